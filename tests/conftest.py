@@ -42,7 +42,7 @@ def ref_lib():
     """The reference's own CPU path (oracle/_ref). Built here when the reference
     checkout is present; it also travels prebuilt to GPU hosts."""
     import oracle
-    if not os.path.exists(oracle.REF_LIB) and os.path.isdir(REFERENCE):
+    if not os.path.exists(oracle.REF_LIB) and os.path.isdir(os.path.join(REFERENCE, "src")):
         _make(os.path.join(ROOT, "oracle"), "ref", f"REFERENCE={REFERENCE}")
     if not os.path.exists(oracle.REF_LIB):
         pytest.skip("oracle/_ref not built and the reference sources are not present")
