@@ -8,6 +8,7 @@
 // used. The flux reconstruction has its own switch (EU_EXACT_FLUX).
 #pragma once
 
+#include <cmath>
 #include <cstdint>
 #include <type_traits>
 
@@ -38,26 +39,47 @@ __device__ __forceinline__ void interior_node(const DevGrid &g, long long t, int
     i += g.bc;
 }
 
-// Reciprocal of a nonzero, non-denormal double by the hardware approximation
-// (rcp.approx.ftz.f64) refined with two Newton-Raphson steps
-// y <- y + y (1 - a y); relative error near one unit in the last place.
+// Reciprocal of a nonzero, non-denormal double: the hardware approximation
+// (rcp.approx.ftz.f64, about 20 bits) refined by one third-order step, y + y (e +
+// e^2) with e = 1 - a y (the remainder is e^3 < 2^-59); relative error near one
+// unit in the last place. One operation less than two Newton steps.
 __device__ __forceinline__ double rcp_nr(double a)
 {
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
-    double e = fma(-a, y, 1.0);
-    y = fma(y, e, y);
-    e = fma(-a, y, 1.0);
-    return fma(y, e, y);
+    const double e = fma(-a, y, 1.0);
+    return fma(y, fma(e, e, e), y);
 }
 
-// q = n / d without an IEEE division: exact division only for d == 0 (the
-// hardware approximation is not valid there).
+// x / sqrt(x d) for positive normal x d, the same way: rsqrt.approx.ftz.f64 and
+// one third-order step, y + y e (1/2 + 3/8 e) with e = 1 - x d y^2. Without the
+// special cases of rsqrt(); a negative or NaN argument gives NaN as there.
+__device__ __forceinline__ double sound_speed(double x, double d)
+{
+    const double a = x * d;
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
+    const double e = fma(-(a * y), y, 1.0);
+    return x * fma(y * e, fma(0.375, e, 0.5), y);
+}
+__device__ __forceinline__ float sound_speed(float x, float d) { return x * rsqrt(x * d); }
+
+// min(max(x, 0), 1) on the words of x (one unsigned comparison tells whether x
+// lies in [0, 1)): integer selects instead of FP64 comparisons. A NaN, whose
+// sign the hardware leaves clear, gives 1.
+__device__ __forceinline__ double saturate(double x)
+{
+    const int hi = __double2hiint(x), lo = __double2loint(x);
+    const bool in = unsigned(hi) < 0x3ff00000u;
+    return __hiloint2double(min(max(hi, 0), 0x3ff00000), in ? lo : 0);
+}
+
+// q = n / d without an IEEE division; for d == 0 (where the Newton steps give
+// NaN) the product with the signed infinity is the quotient.
 __device__ __forceinline__ double div_fast(double n, double d)
 {
-    if (d == 0.0)
-        return n / d;
-    return n * rcp_nr(d);
+    const double y = rcp_nr(d);
+    return n * (d == 0.0 ? copysign(INFINITY, d) : y);
 }
 __device__ __forceinline__ float div_fast(float n, float d) { return __fdividef(n, d); }
 
@@ -723,8 +745,10 @@ __device__ __forceinline__ R minmod(R r)
 //   L = A1/(A0+1e-12), R = A1/(A2+1e-12), limiter values minmod(L), minmod(1/L).
 // Fast form: the same limiter written without the reciprocal ratios. For
 // L > 0 the reference's slope term 0.25((1-k) min(L,1) + (1+k) min(1/L,1) L) A0
-// equals 0.5 min(L,1) A0 (k = 1/3); for L <= 0 it is 0. L is formed with a
-// Newton-refined reciprocal. Results agree to a few units in the last place.
+// equals 0.5 min(L,1) A0 (k = 1/3); for L <= 0 it is 0: 0.5 A0 times L
+// saturated to [0, 1], L formed with a refined reciprocal. Results agree to a
+// few units in the last place (A0 = -1e-12 exactly, where L has no value, takes
+// the slope 0.5 A0).
 // The 1e-12 guard is kept in every form: it flattens the slopes of fields
 // whose differences are below it (trace species), so the first-order value
 // the reference takes there is kept.
@@ -745,8 +769,7 @@ __device__ __forceinline__ R muscl_slope(R a, R A1)
         const R L = __saturatef(div_fast(A1, a + R(1e-12)));
         return R(0.5) * a * L;
     } else {
-        const R L = div_fast(A1, a + R(1e-12));
-        return L > R(0) ? R(0.5) * a * fmin(L, R(1)) : R(0);
+        return R(0.5) * a * saturate(A1 * rcp_nr(a + R(1e-12)));
     }
 }
 
@@ -760,72 +783,61 @@ __device__ __forceinline__ void muscl(R fm1, R f0, R f1, R f2, R &left, R &right
     right = f1 - muscl_slope<R, kStrict>(A2, A1);
 }
 
-// Only the upwind side of the face: the left state when up, else the right.
-// The same expression as that side of muscl(), so the same value.
+// Only the upwind side of a face, from the three points it reads: u and w on
+// the upwind side (u next to the face), v across it, e = +1e-12 when the left
+// side is upwind, else -1e-12. The right side's value f1 - t(f2 - f1, f1 - f0)
+// is u + t with every operand of the slope negated, and round-to-nearest is
+// symmetric, so in the strict form the value is bitwise the reference's (a zero
+// denominator takes the sign it has there).
 template <typename R, bool kStrict>
-__device__ __forceinline__ R muscl_upwind(bool up, R fm1, R f0, R f1, R f2)
+__device__ __forceinline__ R muscl_upwind(R u, R w, R v, R e)
 {
-    if constexpr (!kStrict && std::is_same<R, float>::value) {
-        // The side's base u, outer point w and inner point v (up: f0, fm1, f1;
-        // down: f1, f2, f0): the value is u + (u - w)/2 sat((v - u) / ((u - w)
-        // + e)) with e = +1e-12 (up) or -1e-12 (down), one fused multiply-add.
-        // Every term of the down side is the exact negation of the form
-        // f1 - (a/2) sat(A1 / (a + 1e-12)), a = f2 - f1, A1 = f1 - f0
-        // (round-to-nearest is symmetric), so the value is bitwise that form's;
-        // selecting the three points first saves the arithmetic of the side
-        // not taken.
-        const R u = up ? f0 : f1, w = up ? fm1 : f2, v = up ? f1 : f0;
-        const R d = u - w;
-        const R L = __saturatef(div_fast(v - u, d + (up ? R(1e-12) : R(-1e-12))));
-        return fmaf(R(0.5) * d, L, u);
-    }
-    const R A1 = f1 - f0;
-    const R a = up ? f0 - fm1 : f2 - f1;
-    {
-        const R t = muscl_slope<R, kStrict>(a, A1);
-        return up ? f0 + t : f1 - t;
+    const R a = u - w, A1 = v - u;
+    if constexpr (kStrict) {
+        R d = a + e;
+        d = d == R(0) ? copysign(R(0), e) : d;
+        const R kk = R(1.0) / R(3.0);
+        const R L = A1 / d;
+        const R L1 = minmod(L), L2 = minmod(R(1.0) / L);
+        return u + R(0.25) * ((R(1.0) - kk) * L1 + (R(1) + kk) * L2 * L) * a;
+    } else if constexpr (std::is_same<R, float>::value) {
+        return fmaf(R(0.5) * a, __saturatef(div_fast(A1, a + e)), u);
+    } else {
+        return fma(R(0.5) * a, saturate(A1 * rcp_nr(a + e)), u);
     }
 }
 
-// MUSCL reconstruction and AUSM+ flux of one face (src/Flowfield.cpp:1794-1930)
-// for direction DIR (0: x, 1: y, 2: z). get(f, p) returns stencil point p
-// (0..3: cells m-1, m, m+1, m+2 across the face m+1/2) of primitive f.
-//
-// AUSM+ reads both reconstructed sides only of p, rho, gamma and the normal
-// velocity (sound speeds, Mach numbers, pressure split). Every other flux
-// term takes the upwind side (VI >= 0: left, src/Flowfield.cpp:1870): the two
-// tangential velocities, H and the species. Those twelve quantities are
-// reconstructed on the upwind side alone, with the same expression as
-// before, so the flux is the same as with both sides formed.
-template <int NS, int DIR, typename R, bool kStrict, typename FOut, class Get>
-__device__ __forceinline__ void face_ausm(Get get, FOut (&F)[NS + 4])
+// The part of a face's AUSM+ flux that needs both reconstructed sides
+// (src/Flowfield.cpp:1794-1870): sound speeds, split Mach numbers and pressures
+// from p, rho, gamma and the normal velocity.
+template <typename R>
+struct FaceState {
+    R PL, PR, DL, DR, UnL, UnR, G1, G2, VI;
+};
+
+template <typename R, bool kStrict>
+__device__ __forceinline__ void face_split(FaceState<R> &w, R GaL, R GaR)
 {
-    constexpr int kN = kU + DIR;
-    R PL, PR, DL, DR, UnL, UnR, GaL, GaR;
-    muscl<R, kStrict>(get(kP, 0), get(kP, 1), get(kP, 2), get(kP, 3), PL, PR);
-    muscl<R, kStrict>(get(kD, 0), get(kD, 1), get(kD, 2), get(kD, 3), DL, DR);
-    muscl<R, kStrict>(get(kN, 0), get(kN, 1), get(kN, 2), get(kN, 3), UnL, UnR);
-    muscl<R, kStrict>(get(kG, 0), get(kG, 1), get(kG, 2), get(kG, 3), GaL, GaR);
-    R CL, CR, CI, MaL, MaR;
+    R CI, MaL, MaR;
     if (kStrict) {
-        CL = sqrt(GaL * PL / DL);
-        CR = sqrt(GaR * PR / DR);
+        const R CL = sqrt(GaL * w.PL / w.DL);
+        const R CR = sqrt(GaR * w.PR / w.DR);
         CI = R(0.5) * (CL + CR);
-        MaL = UnL / CI;
-        MaR = UnR / CI;
+        MaL = w.UnL / CI;
+        MaR = w.UnR / CI;
     } else {
         // c = sqrt(g p / rho) = (g p) / sqrt(g p rho)
-        const R gpL = GaL * PL, gpR = GaR * PR;
-        CL = gpL * rsqrt(gpL * DL);
-        CR = gpR * rsqrt(gpR * DR);
+        const R gpL = GaL * w.PL, gpR = GaR * w.PR;
+        const R CL = sound_speed(gpL, w.DL);
+        const R CR = sound_speed(gpR, w.DR);
         CI = R(0.5) * (CL + CR);
         const R inv = div_fast(R(1), CI);
-        MaL = UnL * inv;
-        MaR = UnR * inv;
+        MaL = w.UnL * inv;
+        MaR = w.UnR * inv;
     }
     // Split Mach and pressure functions: both regimes formed, then selected
     // (a branch per regime would split a warp whose faces straddle Mach 1)
-    R B1, G1, B2, G2;
+    R B1, B2;
     {
         const R a = MaL + R(1.0), t = MaL * MaL - R(1.0);
         const R Bs = R(0.25) * (a * a) + R(0.125) * (t * t);
@@ -835,7 +847,7 @@ __device__ __forceinline__ void face_ausm(Get get, FOut (&F)[NS + 4])
         const R Gp = kStrict ? Bp / MaL : (MaL > R(0) ? R(1) : R(0));
         const bool sub = fabs(MaL) < R(1.0);
         B1 = sub ? Bs : Bp;
-        G1 = sub ? Gs : Gp;
+        w.G1 = sub ? Gs : Gp;
     }
     {
         const R a = MaR - R(1.0), t = MaR * MaR - R(1.0);
@@ -845,26 +857,98 @@ __device__ __forceinline__ void face_ausm(Get get, FOut (&F)[NS + 4])
         const R Gp = kStrict ? Bp / MaR : (MaR < R(0) ? R(1) : R(0));
         const bool sub = fabs(MaR) < R(1.0);
         B2 = sub ? Bs : Bp;
-        G2 = sub ? Gs : Gp;
+        w.G2 = sub ? Gs : Gp;
     }
-    const R MaI = B1 + B2;
-    const R VI = MaI * CI;
+    w.VI = (B1 + B2) * CI;
+}
+
+// MUSCL reconstruction and AUSM+ flux of one face (src/Flowfield.cpp:1794-1930)
+// for direction DIR (0: x, 1: y, 2: z). get(f, p) returns stencil point p
+// (0..3: cells m-1, m, m+1, m+2 across the face m+1/2) of primitive f; upwind(f,
+// up, u, w, v) the three points of muscl_upwind.
+//
+// AUSM+ reads both reconstructed sides only of p, rho, gamma and the normal
+// velocity (sound speeds, Mach numbers, pressure split). Every other flux
+// term takes the upwind side (VI >= 0: left, src/Flowfield.cpp:1870): the two
+// tangential velocities, H and the species. Those twelve quantities are
+// reconstructed on the upwind side alone, with the same expression, so the
+// flux is the same as with both sides formed.
+template <int NS, int DIR, typename R, class Get, class Upwind>
+__device__ __forceinline__ void face_ausm(Get get, Upwind upwind, R (&F)[NS + 4])
+{
+    constexpr int kN = kU + DIR;
+    FaceState<R> w;
+    R GaL, GaR;
+    muscl<R, false>(get(kP, 0), get(kP, 1), get(kP, 2), get(kP, 3), w.PL, w.PR);
+    muscl<R, false>(get(kD, 0), get(kD, 1), get(kD, 2), get(kD, 3), w.DL, w.DR);
+    muscl<R, false>(get(kN, 0), get(kN, 1), get(kN, 2), get(kN, 3), w.UnL, w.UnR);
+    muscl<R, false>(get(kG, 0), get(kG, 1), get(kG, 2), get(kG, 3), GaL, GaR);
+    face_split<R, false>(w, GaL, GaR);
+    const R VI = w.VI;
     const bool up = VI >= R(0.0);
-    auto side = [&](int f) { return muscl_upwind<R, kStrict>(up, get(f, 0), get(f, 1), get(f, 2), get(f, 3)); };
-    const R Du = up ? DL : DR;
+    const R e = up ? R(1e-12) : R(-1e-12);
+    auto side = [&](int f) {
+        R u, o, v;
+        upwind(f, up, u, o, v);
+        return muscl_upwind<R, false>(u, o, v, e);
+    };
+    const R Du = up ? w.DL : w.DR;
     const R m = VI * Du;
 #pragma unroll
-    for (int s = 0; s < NS; ++s) F[s] = FOut(m * side(kY0 + s));
+    for (int s = 0; s < NS; ++s) F[s] = m * side(kY0 + s);
     R vel[3];
 #pragma unroll
-    for (int d = 0; d < 3; ++d) vel[d] = (d == DIR) ? (up ? UnL : UnR) : side(kU + d);
+    for (int d = 0; d < 3; ++d) vel[d] = (d == DIR) ? (up ? w.UnL : w.UnR) : side(kU + d);
     const R Hu = side(kH);
     R mom[3] = {m * vel[0], m * vel[1], m * vel[2]};
-    mom[DIR] = mom[DIR] + G1 * PL + G2 * PR;
-    F[NS + 0] = FOut(mom[0]);
-    F[NS + 1] = FOut(mom[1]);
-    F[NS + 2] = FOut(mom[2]);
-    F[NS + 3] = FOut(VI * (Du * Hu + R(0.5) * Du * (vel[0] * vel[0] + vel[1] * vel[1] + vel[2] * vel[2])));
+    mom[DIR] = mom[DIR] + w.G1 * w.PL + w.G2 * w.PR;
+    F[NS + 0] = mom[0];
+    F[NS + 1] = mom[1];
+    F[NS + 2] = mom[2];
+    F[NS + 3] = VI * (Du * Hu + R(0.5) * Du * (vel[0] * vel[0] + vel[1] * vel[1] + vel[2] * vel[2]));
+}
+
+// face_ausm with the direction at run time, so that one instance of the code
+// serves the x, y and z faces of a kernel (a third of the instructions in the
+// instruction cache). p: stencil point 0 (cell m-1) of plane 0, points `stride`
+// apart, planes n3 apart. The twelve quantities that only the upwind side
+// enters are read once that side is known: three points instead of four, and
+// no selects between the sides. put(q, v) takes flux component q as soon as
+// it is formed.
+template <int NS, typename R, bool kStrict, class Put>
+__device__ __forceinline__ void face_ausm_dir(int dir, const R *__restrict__ p, unsigned n3, int stride, Put put)
+{
+    const int kN = kU + dir, kA = dir == 0 ? kV : kU, kB = dir == 2 ? kV : kW; // normal, tangential planes
+    FaceState<R> w;
+    R GaL, GaR;
+    auto both = [&](int q, R &l, R &r) {
+        const R *b = p + (unsigned long long)n3 * unsigned(q);
+        muscl<R, kStrict>(__ldg(b), __ldg(b + stride), __ldg(b + 2 * stride), __ldg(b + 3 * stride), l, r);
+    };
+    both(kP, w.PL, w.PR);
+    both(kD, w.DL, w.DR);
+    both(kN, w.UnL, w.UnR);
+    both(kG, GaL, GaR);
+    face_split<R, kStrict>(w, GaL, GaR);
+    const R VI = w.VI;
+    const bool up = VI >= R(0.0);
+    const R e = up ? R(1e-12) : R(-1e-12);
+    const R *pu = p + (up ? stride : 2 * stride), *pw = p + (up ? 0 : 3 * stride), *pv = p + (up ? 2 * stride : stride);
+    auto side = [&](int q) {
+        const unsigned long long o = (unsigned long long)n3 * unsigned(q);
+        return muscl_upwind<R, kStrict>(__ldg(pu + o), __ldg(pw + o), __ldg(pv + o), e);
+    };
+    const R Du = up ? w.DL : w.DR;
+    const R m = VI * Du;
+#pragma unroll
+    for (int s = 0; s < NS; ++s) put(s, m * side(kY0 + s));
+    const R un = up ? w.UnL : w.UnR, va = side(kA), vb = side(kB), Hu = side(kH);
+    const R momn = m * un;
+    put(NS + dir, momn + w.G1 * w.PL + w.G2 * w.PR);
+    put(NS + kA - kU, m * va);
+    put(NS + kB - kU, m * vb);
+    const R v0 = dir == 0 ? un : va, v1 = dir == 0 ? va : (dir == 1 ? un : vb), v2 = dir == 2 ? un : vb;
+    put(NS + 3, VI * (Du * Hu + R(0.5) * Du * (v0 * v0 + v1 * v1 + v2 * v2)));
 }
 
 } // namespace eu3d

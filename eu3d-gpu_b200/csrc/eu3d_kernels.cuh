@@ -176,179 +176,151 @@ __global__ void k_halo_copy(R *planes, R *msg, int nf, int bc, long long n3, lon
 
 // ----------------------------------------------------------------- fluxes
 
-// Face flux between cell c and c + stride along DIR, from the primitive planes
-// (FP64 or FP32 copies): MUSCL_2 on every primitive, then AUSM+.
-template <int NS, int DIR, typename R, bool kStrict>
-__device__ __forceinline__ void face_flux(const R *__restrict__ prim, long long n3, long long c, long long stride,
-                                          R (&F)[NS + 4])
+// Tile of k_flux_update_faces: cells per axis, the divisions of its flat face
+// lists, and the faces they hold. Blocks are kFaceThreadsWide threads on grids
+// that fill the chip once at most (a face a thread, one round), half of that
+// on larger ones.
+constexpr int kFaceThreads = 128, kFaceThreadsWide = 256;
+// Flux slots of a component: the faces of a tile at most. 464 doubles are the
+// most with which four 128-thread blocks share an SM (at 496 three do: 1.30 ms
+// against 0.85 on 256 x 128 x 128).
+template <typename R>
+constexpr int kFacePitch = sizeof(R) == 8 ? 464 : 496;
+struct FaceTile {
+    int ti, tj, tk;
+    FastDiv d_tk, d_tk1, d_area, d_area_y, d_area_z;
+};
+
+template <int NS, typename R>
+constexpr size_t face_smem_bytes()
 {
-    const R *a = prim + c - stride;
-    face_ausm<NS, DIR, R, kStrict, R>([&](int f, int p) { return __ldg(a + f * n3 + p * stride); }, F);
+    return sizeof(R) * (NS + 4) * kFacePitch<R>;
 }
 
 // Flux divergence and the Euler-explicit update (TimeAdv::EE, src/TimeAdv.cpp:42-56,
-// then CS += RHS, src/Flowfield.cpp:1350-1354) with every face flux formed once.
+// then CS += RHS, src/Flowfield.cpp:1350-1354) with one thread per face: every
+// FP64 grid, and FP32 fluxes on thin or small grids.
 //
-// A block owns a kFluxTJ x kFluxTK tile of (j, k) columns and marches along x
-// over ci nodes (a launch parameter the autotuner picks). The x-face flux at
-// i-1/2 stays in registers from the
-// previous node; the y- and z-face fluxes of the current plane go through
-// shared memory (row 0 / column 0 hold the faces below the tile, computed by
-// warp 0 and by eight lanes of warp 1). RHS keeps the reference's order
-// -dt/dx (F+ - F-) - dt/dy (G+ - G-) - dt/dz (Q+ - Q-), accumulated in FP64.
-constexpr int kFluxTK = 32, kFluxTJ = 8;
-
-template <int NS, typename R>
-constexpr size_t flux_smem_bytes()
-{
-    return sizeof(R) * (NS + 4) * ((kFluxTJ + 1) * kFluxTK + kFluxTJ * (kFluxTK + 1));
-}
-
+// A block owns a ti x tj x tk tile of cells (chosen from the grid at run time,
+// FaceTile), marches ci nodes along x in steps of ti, and per step forms the
+// tile's x, y and z faces as one flat list (a face a thread at a time, stencil
+// points through the read-only cache), leaves the fluxes in shared memory and
+// updates the cells from them. The x faces above the last plane are carried to
+// the next step. The RHS keeps the reference's order -dt/dx (F+ - F-) - dt/dy
+// (G+ - G-) - dt/dz (Q+ - Q-): in FP64, or for R = float the differences and
+// their sum in FP32 onto the FP64 conserved value.
+//
+// What bounds it: in FP64 the instruction issue (about 2/5 of the instructions
+// are FP64 ones). A thread that forms one face needs a third of the state of one
+// that forms a cell's three, so 16 warps fit an SM without spills where the
+// cell-a-thread forms ran 8 at 255 registers, and a tile's shape follows the
+// grid, where fixed 32-lane rows left most lanes idle on thin grids and a few
+// blocks marched 16 planes one after the other on small ones. Flux phase of a
+// step on a B200, before and after:
+//   256 x 128 x 128 FP64  1.60 -> 0.85 ms    129 x 65 x 65 FP64   0.367 -> 0.133 ms
+//   281 x 141 x 2 strict  0.92 -> 0.093 ms   33 x 17 x 17 strict  0.396 -> 0.023 ms
+//   4001 x 2 x 2 FP64    0.448 -> 0.014 ms   41 x 24 x 23 FP64    0.144 -> 0.015 ms
+//   1024 x 512 x 2 FP32   0.40 -> 0.18 ms    48 x 32 x 32 FP32    0.073 -> 0.020 ms
 template <int NS, typename R, bool kStrict>
-__global__ void __launch_bounds__(kFluxTK *kFluxTJ, 1)
-    k_flux_update(const DevGrid g, const DevState st, const R *__restrict__ prim, const double *__restrict__ dt_dev,
-                  int ci)
+__global__ void __launch_bounds__(kFaceThreadsWide, 2)
+    k_flux_update_faces(const DevGrid g, const DevState st, const R *__restrict__ prim,
+                        const double *__restrict__ dt_dev, const FaceTile t, int ci)
 {
-    constexpr int NV = NS + 4;
+    constexpr int NV = NS + 4, kPitch = kFacePitch<R>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    R(*sG)[kFluxTJ + 1][kFluxTK] = reinterpret_cast<R(*)[kFluxTJ + 1][kFluxTK]>(smem_raw);
-    R(*sQ)[kFluxTJ][kFluxTK + 1] =
-        reinterpret_cast<R(*)[kFluxTJ][kFluxTK + 1]>(smem_raw + sizeof(R) * NV * (kFluxTJ + 1) * kFluxTK);
-
-    const int tx = threadIdx.x, ty = threadIdx.y;
-    const int k0 = blockIdx.x * kFluxTK, j0 = blockIdx.y * kFluxTJ;
-    const int k = g.bc + k0 + tx, j = g.bc + j0 + ty;
-    const bool valid = (k0 + tx < g.nk) && (j0 + ty < g.nj);
-    const int i_begin = g.bc + blockIdx.z * ci;
-    const int i_end = min(i_begin + ci, g.bc + g.ni);
-    const long long n3 = g.n3, sx = (long long)g.ny * g.nz, sy = g.nz;
+    R *sF = reinterpret_cast<R *>(smem_raw); // [NV][kPitch]
+    const int tid = threadIdx.x, nthreads = blockDim.x;
+    const int area = t.tj * t.tk; // cells of a plane
+    const int nfx = (t.ti + 1) * area, nfy = t.ti * (t.tj + 1) * t.tk, nf = nfx + nfy + t.ti * t.tj * (t.tk + 1);
+    const int k0 = blockIdx.x * t.tk, j0 = blockIdx.y * t.tj;
+    const int rows = min(t.tj, g.nj - j0), cols = min(t.tk, g.nk - k0);
+    const int i_begin = blockIdx.z * ci, i_end = min(i_begin + ci, g.ni);
+    const long long n3 = g.n3;
+    const int sx = g.ny * g.nz, sy = g.nz;
     const double dt = *dt_dev;
-    const double cy = valid ? dt / (g.y[j] - g.y[j - 1]) : 0.0;
-    const double cz = valid ? dt / (g.z[k] - g.z[k - 1]) : 0.0;
-    // lanes of warp 1 that form the z faces below the tile, one per row
-    const int zrow = tx;
-    const bool zlow = (ty == 1) && (tx < kFluxTJ) && (j0 + zrow < g.nj) && (k0 < g.nk);
-
-    R Fm[NV];
-    if (valid)
-        face_flux<NS, 0, R, kStrict>(prim, n3, cell_index(g, i_begin - 1, j, k), sx, Fm);
-    for (int i = i_begin; i < i_end; ++i) {
-        const long long c = cell_index(g, i, j, k);
-        R Fp[NV];
-        if (valid) {
-            face_flux<NS, 0, R, kStrict>(prim, n3, c, sx, Fp);
-            {
-                R G[NV];
-                face_flux<NS, 1, R, kStrict>(prim, n3, c, sy, G);
-#pragma unroll
-                for (int q = 0; q < NV; ++q) sG[q][ty + 1][tx] = G[q];
+    for (int i0 = i_begin; i0 < i_end; i0 += t.ti) {
+        const int planes = min(t.ti, i_end - i0);
+        for (int f = tid + (i0 == i_begin ? 0 : area); f < nf; f += nthreads) {
+            int dir, a, j, k, stride;
+            bool in;
+            if (f < nfx) {
+                dir = 0;
+                stride = sx;
+                a = fdiv(f, t.d_area);
+                const int r = f - a * area;
+                j = fdiv(r, t.d_tk);
+                k = r - j * t.tk;
+                in = a <= planes && j < rows && k < cols;
+                --a;
+            } else if (f < nfx + nfy) {
+                dir = 1;
+                stride = sy;
+                const int e = f - nfx;
+                a = fdiv(e, t.d_area_y);
+                const int r = e - a * (area + t.tk);
+                j = fdiv(r, t.d_tk);
+                k = r - j * t.tk;
+                in = a < planes && j <= rows && k < cols;
+                --j;
+            } else {
+                dir = 2;
+                stride = 1;
+                const int e = f - nfx - nfy;
+                a = fdiv(e, t.d_area_z);
+                const int r = e - a * (area + t.tj);
+                j = fdiv(r, t.d_tk1);
+                k = r - j * (t.tk + 1);
+                in = a < planes && j < rows && k <= cols;
+                --k;
             }
-            {
-                R Q[NV];
-                face_flux<NS, 2, R, kStrict>(prim, n3, c, 1, Q);
-#pragma unroll
-                for (int q = 0; q < NV; ++q) sQ[q][ty][tx + 1] = Q[q];
-            }
-            if (ty == 0) {
-                R G[NV];
-                face_flux<NS, 1, R, kStrict>(prim, n3, c - sy, sy, G);
-#pragma unroll
-                for (int q = 0; q < NV; ++q) sG[q][0][tx] = G[q];
-            }
-        }
-        if (zlow) {
-            R Q[NV];
-            face_flux<NS, 2, R, kStrict>(prim, n3, cell_index(g, i, g.bc + j0 + zrow, g.bc + k0 - 1), 1, Q);
-#pragma unroll
-            for (int q = 0; q < NV; ++q) sQ[q][zrow][0] = Q[q];
-        }
-        __syncthreads();
-        if (valid) {
-            const double cx = -dt / (g.x[i] - g.x[i - 1]);
-#pragma unroll
-            for (int q = 0; q < NV; ++q) {
-                const double rhs = cx * (double(Fp[q]) - double(Fm[q])) -
-                                   cy * (double(sG[q][ty + 1][tx]) - double(sG[q][ty][tx])) -
-                                   cz * (double(sQ[q][ty][tx + 1]) - double(sQ[q][ty][tx]));
-                st.cs[q * n3 + c] = st.cs[q * n3 + c] + rhs;
-                Fm[q] = Fp[q];
+            if (in) {
+                const R *p = prim + cell_index(g, g.bc + i0 + a, g.bc + j0 + j, g.bc + k0 + k) - stride;
+                face_ausm_dir<NS, R, kStrict>(dir, p, unsigned(n3), stride, [&](int q, R v) { sF[q * kPitch + f] = v; });
             }
         }
         __syncthreads();
-    }
-}
-
-// Flux divergence and update for grids thin in z (nk below half a warp),
-// where the (j, k) tiles of the kernels above and below would leave most lanes
-// idle: one thread per (j, k) column (flattened, k fastest) marching ci nodes
-// in x. The x face at i-1/2 is carried in registers from the previous node; the
-// thread forms the y and z faces on both sides of its cell from the stencil in
-// global memory (each interior y or z face twice, once by each of its cells).
-// The RHS is formed in the same order as the other flux kernels (FP32
-// differences and sum onto the FP64 conserved value for R = float, FP64 for
-// R = double).
-template <int NS, typename R, bool kStrict>
-__global__ void __launch_bounds__(128) k_flux_update_cols(const DevGrid g, const DevState st,
-                                                          const R *__restrict__ prim,
-                                                          const double *__restrict__ dt_dev, int ci)
-{
-    constexpr int NV = NS + 4;
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= g.nj * g.nk)
-        return;
-    const int jj = t / g.nk;
-    const int j = g.bc + jj, k = g.bc + (t - jj * g.nk);
-    const int i_begin = g.bc + blockIdx.y * ci;
-    const int i_end = min(i_begin + ci, g.bc + g.ni);
-    const long long n3 = g.n3, sx = (long long)g.ny * g.nz, sy = g.nz;
-    const double dt = *dt_dev;
-    const double cy = dt / (g.y[j] - g.y[j - 1]);
-    const double cz = dt / (g.z[k] - g.z[k - 1]);
-    R Fm[NV];
-    face_flux<NS, 0, R, kStrict>(prim, n3, cell_index(g, i_begin - 1, j, k), sx, Fm);
-    for (int i = i_begin; i < i_end; ++i) {
-        const long long c = cell_index(g, i, j, k);
-        const double cx = -dt / (g.x[i] - g.x[i - 1]);
-        R Fp[NV], A[NV], B[NV];
-        face_flux<NS, 0, R, kStrict>(prim, n3, c, sx, Fp);
-        face_flux<NS, 1, R, kStrict>(prim, n3, c, sy, A);      // y face above
-        face_flux<NS, 1, R, kStrict>(prim, n3, c - sy, sy, B); // y face below
-        if (sizeof(R) == 4) {
-            const float cx32 = float(cx), cy32 = float(cy), cz32 = float(cz);
-            float rhs[NV];
+        for (int e = tid; e < t.ti * area; e += nthreads) {
+            const int a = fdiv(e, t.d_area), r = e - a * area, j = fdiv(r, t.d_tk), k = r - j * t.tk;
+            if (a >= planes || j >= rows || k >= cols)
+                continue;
+            const int i = g.bc + i0 + a, jj = g.bc + j0 + j, kk = g.bc + k0 + k;
+            const long long c = cell_index(g, i, jj, kk);
+            const double cx = -dt / (g.x[i] - g.x[i - 1]), cy = dt / (g.y[jj] - g.y[jj - 1]),
+                         cz = dt / (g.z[kk] - g.z[kk - 1]);
+            const int fx = e, fy = nfx + e + a * t.tk, fz = nfx + nfy + e + a * t.tj + j;
+            double old[NV];
 #pragma unroll
-            for (int q = 0; q < NV; ++q) rhs[q] = cx32 * float(Fp[q] - Fm[q]) - cy32 * float(A[q] - B[q]);
-            face_flux<NS, 2, R, kStrict>(prim, n3, c, 1, A);     // z face right
-            face_flux<NS, 2, R, kStrict>(prim, n3, c - 1, 1, B); // z face left
+            for (int q = 0; q < NV; ++q) old[q] = st.cs[q * n3 + c];
 #pragma unroll
             for (int q = 0; q < NV; ++q) {
-                const float r = rhs[q] - cz32 * float(A[q] - B[q]);
-                st.cs[q * n3 + c] = st.cs[q * n3 + c] + double(r);
-                Fm[q] = Fp[q];
+                const R *F = sF + q * kPitch;
+                const R xp = F[fx + area], xm = F[fx], yp = F[fy + t.tk], ym = F[fy], zp = F[fz + 1], zm = F[fz];
+                if constexpr (sizeof(R) == 4) {
+                    const float rhs = float(cx) * float(xp - xm) - float(cy) * float(yp - ym) - float(cz) * float(zp - zm);
+                    st.cs[q * n3 + c] = old[q] + double(rhs);
+                } else {
+                    const double rhs = cx * (xp - xm) - cy * (yp - ym) - cz * (zp - zm);
+                    st.cs[q * n3 + c] = old[q] + rhs;
+                }
             }
-        } else {
-            double rhs[NV];
-#pragma unroll
-            for (int q = 0; q < NV; ++q)
-                rhs[q] = cx * (double(Fp[q]) - double(Fm[q])) - cy * (double(A[q]) - double(B[q]));
-            face_flux<NS, 2, R, kStrict>(prim, n3, c, 1, A);
-            face_flux<NS, 2, R, kStrict>(prim, n3, c - 1, 1, B);
-#pragma unroll
-            for (int q = 0; q < NV; ++q) {
-                const double r = rhs[q] - cz * (double(A[q]) - double(B[q]));
-                st.cs[q * n3 + c] = st.cs[q * n3 + c] + r;
-                Fm[q] = Fp[q];
+        }
+        if (i0 + t.ti < i_end) {
+            __syncthreads();
+            for (int e = tid; e < NV * area; e += nthreads) {
+                const int q = fdiv(e, t.d_area), r = e - q * area;
+                sF[q * kPitch + r] = sF[q * kPitch + t.ti * area + r];
             }
+            __syncthreads();
         }
     }
 }
 
-// Plane-tiled flux divergence and update: the same faces, arithmetic and RHS
-// order as k_flux_update (bitwise the same result), with every primitive read
-// from HBM once per plane instead of once per stencil point, and the loads of
-// the next plane overlapped with the current plane's arithmetic.
+// Plane-tiled flux divergence and update (FP32 fluxes): the same faces and RHS
+// order as k_flux_update_faces, with every primitive read from HBM once per
+// plane instead of once per stencil point, and the loads of the next plane
+// overlapped with the current plane's arithmetic.
 //
-// A block owns a kTileJ x kTileK tile of (j, k) columns (TileShape) and
+// A block owns a kTileJ x kTileK tile of (j, k) columns  and
 // marches along x with kTileJ + 1 warps. Warps 0 .. kTileJ-1 own a row of cells each: every
 // thread keeps its column's x-stencil (planes i-1 .. i+2 of every primitive) in
 // registers and loads plane i+3 one node ahead. Plane i of the tile plus a
@@ -367,53 +339,64 @@ __global__ void __launch_bounds__(128) k_flux_update_cols(const DevGrid g, const
 // extra face. Partial tiles: the faces of the valid rows/columns are formed,
 // including the one past the last valid row/column.
 //
-// Tile height: 7 cell rows (8 warps) in FP32; 3 cell rows (4 warps) in FP64,
-// whose x-stencil window takes twice the registers, so that two blocks still
-// fit per SM (98 KB of shared memory each).
+// Tile height: 7 cell rows (8 warps), so that two blocks fit per SM (98 KB of
+// shared memory each).
 constexpr int kTileK = 32, kTileCols = kTileK + 4;
-template <typename R>
-struct TileShape {
-    static constexpr int J = sizeof(R) == 4 ? 7 : 3; // cell rows
-    static constexpr int Warps = J + 1, Rows = J + 4;
-    // staged by cp.async: rows 0, 1 and J + 3 over the full width, and the
-    // two columns each side of rows 2 .. J + 2 (the cell rows and the edge
-    // warp's row)
-    static constexpr int Halo = 3 * kTileCols + 4 * (J + 1);
-};
+constexpr int kTileJ = 7, kTileWarps = kTileJ + 1, kTileRows = kTileJ + 4;
+// staged by cp.async: rows 0, 1 and kTileJ + 3 over the full width, and the two
+// columns each side of rows 2 .. kTileJ + 2 (the cell rows and the edge warp's row)
+constexpr int kTileHalo = 3 * kTileCols + 4 * (kTileJ + 1);
 
-template <int NS, typename R>
+template <int NS>
 constexpr size_t tiled_flux_smem_bytes()
 {
-    constexpr int J = TileShape<R>::J, Rows = TileShape<R>::Rows;
-    return sizeof(double) * (NS + 4) * J * kTileK + sizeof(R) * 2 * (7 + NS) * Rows * kTileCols +
-           sizeof(R) * (NS + 4) * ((J + 1) * kTileK + J * (kTileK + 1));
+    return sizeof(double) * (NS + 4) * kTileJ * kTileK + sizeof(float) * 2 * (7 + NS) * kTileRows * kTileCols +
+           sizeof(float) * (NS + 4) * ((kTileJ + 1) * kTileK + kTileJ * (kTileK + 1));
 }
 
 // Face flux from four consecutive stencil points of the staged plane tile,
 // starting at (r, c) and stepping (DR, DC). own: the values of stencil point 2
 // when that point is the thread's own node (kept in registers), else null.
-template <int NS, int DIR, int DR, int DC, typename R, bool kStrict, bool kOwn>
-__device__ __forceinline__ void tile_face_flux(const R (*sP)[TileShape<R>::Rows][kTileCols], int r, int c,
-                                               const R *own, R (&F)[NS + 4])
+template <int NS, int DIR, int DR, int DC, bool kOwn>
+__device__ __forceinline__ void tile_face_flux(const float (*sP)[kTileRows][kTileCols], int r, int c, const float *own,
+                                               float (&F)[NS + 4])
 {
-    face_ausm<NS, DIR, R, kStrict, R>(
-        [&](int f, int p) { return (kOwn && p == 2) ? own[f] : sP[f][r + p * DR][c + p * DC]; }, F);
+    constexpr int S = DR * kTileCols + DC, N = kTileRows * kTileCols;
+    const float *p = &sP[0][r][c];
+    face_ausm<NS, DIR, float>([&](int f, int q) { return (kOwn && q == 2) ? own[f] : p[f * N + q * S]; },
+                              [&](int f, bool up, float &u, float &w, float &v) {
+                                  w = p[f * N + (up ? 0 : 3 * S)];
+                                  if (kOwn) {
+                                      const float a = p[f * N + S];
+                                      u = up ? a : own[f];
+                                      v = up ? own[f] : a;
+                                  } else {
+                                      u = p[f * N + (up ? S : 2 * S)];
+                                      v = p[f * N + (up ? 2 * S : S)];
+                                  }
+                              },
+                              F);
 }
 
-template <int NS, typename R, bool kStrict>
-__device__ __forceinline__ void window_face_flux(const R (&w)[4][7 + NS], R (&F)[NS + 4])
+template <int NS>
+__device__ __forceinline__ void window_face_flux(const float (&w)[4][7 + NS], float (&F)[NS + 4])
 {
-    face_ausm<NS, 0, R, kStrict, R>([&](int f, int p) { return w[p][f]; }, F);
+    face_ausm<NS, 0, float>([&](int f, int p) { return w[p][f]; },
+                            [&](int f, bool up, float &u, float &o, float &v) {
+                                u = up ? w[1][f] : w[2][f];
+                                o = up ? w[0][f] : w[3][f];
+                                v = up ? w[2][f] : w[1][f];
+                            },
+                            F);
 }
 
-template <int NS, typename R, bool kStrict>
-__global__ void __launch_bounds__(kTileK *TileShape<R>::Warps, 2)
-    k_flux_update_tiled(const DevGrid g, const DevState st, const R *__restrict__ prim, const double *__restrict__ dt_dev,
-                        int ci)
+template <int NS>
+__global__ void __launch_bounds__(kTileK *kTileWarps, 2)
+    k_flux_update_tiled(const DevGrid g, const DevState st, const float *__restrict__ prim,
+                        const double *__restrict__ dt_dev, int ci)
 {
+    using R = float;
     constexpr int NP = 7 + NS, NV = NS + 4;
-    constexpr int kTileJ = TileShape<R>::J, kTileWarps = TileShape<R>::Warps, kTileRows = TileShape<R>::Rows;
-    constexpr int kTileHalo = TileShape<R>::Halo;
     using Plane = R[NP][kTileRows][kTileCols];
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double(*sC)[kTileJ][kTileK] = reinterpret_cast<double(*)[kTileJ][kTileK]>(smem_raw);
@@ -472,12 +455,7 @@ __global__ void __launch_bounds__(kTileK *TileShape<R>::Warps, 2)
         }
         if (halo) {
 #pragma unroll
-            for (int f = 0; f < NP; ++f) {
-                if constexpr (sizeof(R) == 4)
-                    tc::cp_async4(&stage[s][f][hr][hc], prim + f * n3 + hcol + p * sx);
-                else
-                    tc::cp_async8(&stage[s][f][hr][hc], prim + f * n3 + hcol + p * sx);
-            }
+            for (int f = 0; f < NP; ++f) tc::cp_async4(&stage[s][f][hr][hc], prim + f * n3 + hcol + p * sx);
         }
         tc::cp_async_commit();
     };
@@ -489,7 +467,7 @@ __global__ void __launch_bounds__(kTileK *TileShape<R>::Warps, 2)
         for (int f = 0; f < NP; ++f) w[p][f] = resident ? __ldg(prim + f * n3 + col + (i_begin - 2 + p) * sx) : R(0);
     R Fm[NV];
     if (valid)
-        window_face_flux<NS, R, kStrict>(w, Fm);
+        window_face_flux<NS>(w, Fm);
 #pragma unroll
     for (int f = 0; f < NP; ++f) {
         w[0][f] = w[1][f];
@@ -522,22 +500,22 @@ __global__ void __launch_bounds__(kTileK *TileShape<R>::Warps, 2)
         __syncthreads();
         R Fp[NV];
         if (valid)
-            window_face_flux<NS, R, kStrict>(w, Fp);
+            window_face_flux<NS>(w, Fp);
         if (yface) {
             R G[NV];
-            tile_face_flux<NS, 1, 1, 0, R, kStrict, true>(stage[s], ty, tx + 2, w[1], G);
+            tile_face_flux<NS, 1, 1, 0, true>(stage[s], ty, tx + 2, w[1], G);
 #pragma unroll
             for (int q = 0; q < NV; ++q) sG[q][ty][tx] = G[q];
         }
         if (zface) {
             R Q[NV];
-            tile_face_flux<NS, 2, 0, 1, R, kStrict, true>(stage[s], ty + 2, tx, w[1], Q);
+            tile_face_flux<NS, 2, 0, 1, true>(stage[s], ty + 2, tx, w[1], Q);
 #pragma unroll
             for (int q = 0; q < NV; ++q) sQ[q][ty][tx] = Q[q];
         }
         if (zright) {
             R Q[NV];
-            tile_face_flux<NS, 2, 0, 1, R, kStrict, false>(stage[s], zrow + 2, kTileK, nullptr, Q);
+            tile_face_flux<NS, 2, 0, 1, false>(stage[s], zrow + 2, kTileK, nullptr, Q);
 #pragma unroll
             for (int q = 0; q < NV; ++q) sQ[q][zrow][kTileK] = Q[q];
         }
@@ -546,27 +524,16 @@ __global__ void __launch_bounds__(kTileK *TileShape<R>::Warps, 2)
         if (valid) {
             const long long c = col + i * sx;
             const double cx = -dt / (g.x[i] - g.x[i - 1]);
-            if (sizeof(R) == 4) {
-                // FP32 fluxes: the flux differences and their sum in FP32 (a
-                // difference of two FP32 values within a factor of two is exact),
-                // accumulated onto the FP64 conserved value
-                const float cx32 = float(cx), cy32 = float(cy), cz32 = float(cz);
+            // the flux differences and their sum in FP32 (a difference of two
+            // FP32 values within a factor of two is exact), accumulated onto
+            // the FP64 conserved value
+            const float cx32 = float(cx), cy32 = float(cy), cz32 = float(cz);
 #pragma unroll
-                for (int q = 0; q < NV; ++q) {
-                    const float rhs = cx32 * float(Fp[q] - Fm[q]) - cy32 * float(sG[q][ty + 1][tx] - sG[q][ty][tx]) -
-                                      cz32 * float(sQ[q][ty][tx + 1] - sQ[q][ty][tx]);
-                    st.cs[q * n3 + c] = sC[q][ty][tx] + double(rhs);
-                    Fm[q] = Fp[q];
-                }
-            } else {
-#pragma unroll
-                for (int q = 0; q < NV; ++q) {
-                    const double rhs = cx * (double(Fp[q]) - double(Fm[q])) -
-                                       cy * (double(sG[q][ty + 1][tx]) - double(sG[q][ty][tx])) -
-                                       cz * (double(sQ[q][ty][tx + 1]) - double(sQ[q][ty][tx]));
-                    st.cs[q * n3 + c] = sC[q][ty][tx] + rhs;
-                    Fm[q] = Fp[q];
-                }
+            for (int q = 0; q < NV; ++q) {
+                const float rhs = cx32 * float(Fp[q] - Fm[q]) - cy32 * float(sG[q][ty + 1][tx] - sG[q][ty][tx]) -
+                                  cz32 * float(sQ[q][ty][tx + 1] - sQ[q][ty][tx]);
+                st.cs[q * n3 + c] = sC[q][ty][tx] + double(rhs);
+                Fm[q] = Fp[q];
             }
         }
 #pragma unroll

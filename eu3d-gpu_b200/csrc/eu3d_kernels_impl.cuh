@@ -29,66 +29,94 @@ cudaError_t boundary_t(const LaunchArgs &a)
 // division-light limiter form.
 constexpr bool kStrictFlux = EU_EXACT_FLUX != 0;
 
-template <int NS, typename R, bool kStrict>
-cudaError_t flux_launch(const LaunchArgs &a, const R *prim)
+template <int NS>
+cudaError_t tiled_flux_launch(const LaunchArgs &a)
 {
     const DevGrid &g = a.g;
-    const size_t smem = flux_smem_bytes<NS, R>();
+    const size_t smem = tiled_flux_smem_bytes<NS>();
     static SmemLimit limit; // per instantiation, per device
-    const cudaError_t e = limit.ensure(k_flux_update<NS, R, kStrict>, smem);
+    const cudaError_t e = limit.ensure(k_flux_update_tiled<NS>, smem);
     if (e != cudaSuccess)
         return e;
-    const dim3 block(kFluxTK, kFluxTJ);
+    const dim3 block(kTileK, kTileWarps);
     const int ci = a.flux_ci > 0 ? a.flux_ci : 16;
-    const dim3 grid((g.nk + kFluxTK - 1) / kFluxTK, (g.nj + kFluxTJ - 1) / kFluxTJ, (g.ni + ci - 1) / ci);
-    k_flux_update<NS, R, kStrict><<<grid, block, smem, a.stream>>>(g, a.st, prim, a.dt_dev, ci);
+    const dim3 grid((g.nk + kTileK - 1) / kTileK, (g.nj + kTileJ - 1) / kTileJ, (g.ni + ci - 1) / ci);
+    k_flux_update_tiled<NS><<<grid, block, smem, a.stream>>>(g, a.st, a.st.prim32, a.dt_dev, ci);
     return cudaGetLastError();
 }
 
+// n cut into pieces of about `want`, all but the last equally long (129 at 8:
+// 17 pieces of 8, the last of 1; 65 at 16: five of 13).
+inline int even_piece(int n, int want)
+{
+    const int pieces = (n + want - 1) / want;
+    return (n + pieces - 1) / pieces;
+}
+
+// Grids below this many cells leave SMs without blocks when the tiles hold 128
+// cells (fewer than 8 blocks of 128 cells per SM of 148): there a tile holds
+// half the cells and the block twice the threads, so that a step is one round
+// of faces a block (33 x 17 x 17 strict: 0.023 ms against 0.033-0.054 with the
+// large grids' tiles; 129 x 65 x 65 FP64 the other way: 0.133 against 0.145).
+constexpr long long kFaceSmallCells = 148LL * 8 * 128;
+
+// The tile of k_flux_update_faces for a grid: 128 (small grids: 64) cells, rows
+// along z cut evenly into about 8 FP64 or 16 FP32 values (the whole of a thin
+// grid), 4 of them (16 on thin grids of many cells) along y, the rest along x.
+template <typename R>
+FaceTile face_tile(const DevGrid &g)
+{
+    const bool small = (long long)g.ni * g.nj * g.nk < kFaceSmallCells;
+    const int cells = small ? 64 : 128;
+    FaceTile t;
+    t.tk = even_piece(g.nk, sizeof(R) == 8 ? 8 : 16);
+    t.tj = even_piece(g.nj, t.tk <= 3 && !small ? 16 : 4);
+    t.ti = std::min(g.ni, std::max(1, cells / (t.tj * t.tk)));
+    while (t.ti > 1 && (t.ti + 1) * t.tj * t.tk + t.ti * (t.tj + 1) * t.tk + t.ti * t.tj * (t.tk + 1) > kFacePitch<R>)
+        --t.ti;
+    t.d_tk = make_fastdiv(unsigned(t.tk));
+    t.d_tk1 = make_fastdiv(unsigned(t.tk + 1));
+    t.d_area = make_fastdiv(unsigned(t.tj * t.tk));
+    t.d_area_y = make_fastdiv(unsigned((t.tj + 1) * t.tk));
+    t.d_area_z = make_fastdiv(unsigned(t.tj * (t.tk + 1)));
+    return t;
+}
+
 template <int NS, typename R, bool kStrict>
-cudaError_t tiled_flux_launch(const LaunchArgs &a, const R *prim)
+cudaError_t faces_flux_launch(const LaunchArgs &a, const R *prim)
 {
     const DevGrid &g = a.g;
-    const size_t smem = tiled_flux_smem_bytes<NS, R>();
+    constexpr size_t smem = face_smem_bytes<NS, R>();
     static SmemLimit limit; // per instantiation, per device
-    const cudaError_t e = limit.ensure(k_flux_update_tiled<NS, R, kStrict>, smem);
+    const cudaError_t e = limit.ensure(k_flux_update_faces<NS, R, kStrict>, smem);
     if (e != cudaSuccess)
         return e;
-    const dim3 block(kTileK, TileShape<R>::Warps);
-    const int ci = a.flux_ci > 0 ? a.flux_ci : 16;
-    const dim3 grid((g.nk + kTileK - 1) / kTileK, (g.nj + TileShape<R>::J - 1) / TileShape<R>::J,
-                    (g.ni + ci - 1) / ci);
-    k_flux_update_tiled<NS, R, kStrict><<<grid, block, smem, a.stream>>>(g, a.st, prim, a.dt_dev, ci);
+    const FaceTile t = face_tile<R>(g);
+    const int ci = std::max(std::max(a.flux_ci, t.ti), (g.ni + 65534) / 65535); // gridDim.z < 2^16
+    const int threads = (long long)g.ni * g.nj * g.nk < kFaceSmallCells ? kFaceThreadsWide : kFaceThreads;
+    const dim3 grid(unsigned((g.nk + t.tk - 1) / t.tk), unsigned((g.nj + t.tj - 1) / t.tj), unsigned((g.ni + ci - 1) / ci));
+    k_flux_update_faces<NS, R, kStrict><<<grid, threads, smem, a.stream>>>(g, a.st, prim, a.dt_dev, t, ci);
     return cudaGetLastError();
 }
 
-// Grids thin in z: one thread per (j, k) column.
+// FP32 fluxes (mixed precision, always the division-light forms) on grids thick
+// enough in z for the tiled kernel's 32-lane rows and large enough for its
+// blocks to fill the chip take that kernel (192 x 96 x 96: 0.215 ms against
+// 0.239, 256 x 128 x 128: 0.46 against 0.54), smaller and thinner ones a face a
+// thread (128 x 64 x 64: 0.079 ms against 0.105, 48 x 32 x 32: 0.020 against
+// 0.073). The two give the same bits. FP64 fluxes (the reference's forms when strict, the division-light
+// limiter when fast) are always formed a face a thread.
 constexpr int kThinNk = 16;
-
-template <int NS, typename R, bool kStrict>
-cudaError_t cols_flux_launch(const LaunchArgs &a, const R *prim)
-{
-    const DevGrid &g = a.g;
-    const int ci = a.flux_ci > 0 ? a.flux_ci : 16;
-    const dim3 grid(unsigned((g.nj * g.nk + 127) / 128), unsigned((g.ni + ci - 1) / ci));
-    k_flux_update_cols<NS, R, kStrict><<<grid, 128, 0, a.stream>>>(g, a.st, prim, a.dt_dev, ci);
-    return cudaGetLastError();
-}
+constexpr long long kTiledCells = 1000000;
 
 template <int NS, int NR>
 cudaError_t flux_t(const LaunchArgs &a)
 {
-    if (a.g.nk < kThinNk) {
-        if (a.precision == 1)
-            return cols_flux_launch<NS, float, false>(a, a.st.prim32);
-        return cols_flux_launch<NS, double, kStrictFlux>(a, a.st.prim);
-    }
-    // mixed precision: FP32 reconstruction and AUSM (always the division-light
-    // forms); FP64: the reference's forms (strict) or the division-light
-    // limiter (fast). Both plane-tiled.
-    if (a.precision == 1)
-        return tiled_flux_launch<NS, float, false>(a, a.st.prim32);
-    return tiled_flux_launch<NS, double, kStrictFlux>(a, a.st.prim);
+    if (a.precision != 1)
+        return faces_flux_launch<NS, double, kStrictFlux>(a, a.st.prim);
+    if (a.g.nk >= kThinNk && (long long)a.g.ni * a.g.nj * a.g.nk >= kTiledCells)
+        return tiled_flux_launch<NS>(a);
+    return faces_flux_launch<NS, float, false>(a, a.st.prim32);
 }
 
 template <int NS, int NR>

@@ -2209,7 +2209,7 @@ eu_status eu_autotune(eu_handle *h, int reps, eu_tune_report *report)
             e = cudaMemcpyAsync(snap + off, q.p, q.bytes, cudaMemcpyDeviceToDevice, h->stream);
         off += q.bytes;
     }
-    const int ci_cand[] = {8, 12, 16, 20, 24, 29, 32, 43, 64};
+    const int ci_cand[] = {1, 8, 12, 16, 20, 24, 29, 32, 43, 64}; // 1: one tile of the face kernel
     const int rb_cand[] = {64, 96, 128};
     eu_tune_report rep;
     std::memset(&rep, 0, sizeof rep);

@@ -131,7 +131,7 @@ def test_mixed_precision_error_is_bounded(gpu):
     assert rel_linf(interior(b.get("CS")), interior(a.get("CS"))).max() <= 1e-3
 
 
-@pytest.mark.parametrize("dims", [(40, 20, 45), (17, 7, 32), (17, 8, 32), (33, 9, 5)])
+@pytest.mark.parametrize("dims", [(40, 20, 45), (17, 7, 32), (17, 8, 32), (33, 9, 5), (264, 62, 65)])
 def test_mixed_precision_tiles_match_fp64_closely(gpu, dims):
     """The plane-tiled FP32 flux kernel on grids whose (j, k) extent is not a
     multiple of its 7 x 32 tile, on one that is exactly one tile, and on one
@@ -167,6 +167,37 @@ def test_mixed_precision_tiles_match_fp64_closely(gpu, dims):
     d = np.abs(a - b).max(axis=1)
     err = np.concatenate([d[:9] / b[:9].sum(axis=0).max(), d[9:12] / np.abs(b[9:12]).max(), d[12:] / np.abs(b[12]).max()])
     assert err.max() <= 2e-6, err
+
+
+@pytest.mark.parametrize("dims", [(2, 2, 2), (5, 3, 9), (67, 2, 2), (9, 33, 3), (3, 5, 17), (18, 9, 13)])
+def test_face_kernel_tiles_match_restatement(gpu, port_lib, dims):
+    """k_flux_update_faces (strict FP64) on grids smaller than a tile, thin in
+    one or two directions and ragged against its tiles, against the pinned C
+    restatement: the fluxes round as the reference's, so after three steps the
+    conserved state differs by what the kinetics' exp, log and pow leave (the
+    bound of the golden three-step test, momentum planes against the largest
+    momentum)."""
+    from helpers import cs_rel_linf
+    ni, nj, nk = dims
+    h = 5e-4
+    ext = (0.0, h * (ni - 1), 0.0, h * (nj - 1), 0.0, h * (nk - 1))
+    mech = golden_mechanism()
+    x, y, z = (cases.node_coordinates(n, 0.0, h * (n - 1)) for n in dims)
+    rng = np.random.default_rng(sum(dims))
+    shape = (ni + 4, nj + 4, nk + 4)
+    P, T = 1e5 * rng.uniform(0.7, 1.4, shape), rng.uniform(400.0, 1300.0, shape)
+    U, V, W = (rng.uniform(-900.0, 900.0, shape) for _ in range(3))
+    f = rng.uniform(0.0, 1.0, shape)
+    Y = np.zeros((9,) + shape)
+    Y[5], Y[4], Y[8] = 0.1 * f, 0.8 * f, 1 - 0.9 * f
+    port = port_lib(ni, nj, nk, x, y, z, mech)
+    port.set_primitive(P, T, U, V, W, Y)
+    s = gpu.Solver(ni, nj, nk, ext)
+    s.set_mechanism(mech)
+    s.set_primitive(P, T, U, V, W, Y)
+    port.step(3, 2e-8)
+    s.step(3, 2e-8)
+    assert cs_rel_linf(interior(s.get("CS")), interior(port.get("CS"))).max() <= 1e-12
 
 
 def test_deterministic(gpu):
