@@ -1,11 +1,11 @@
 // eu3d_device.cuh — device-side types and per-cell / per-face arithmetic of the
 // EU3D reacting-Euler timestep for sm_100a.
 //
-// Included by the kernel translation units. EU_EXACT_CHEM selects thermo,
-// temperature-inversion and rate expressions with the reference's operand
-// order and divisions (compiled with --fmad=false they round exactly as the
-// reference's CPU build); without it, algebraically equivalent fast forms are
-// used. The flux reconstruction has its own switch (EU_EXACT_FLUX).
+// Included by the kernel translation units. EU_EXACT_THERMO selects the state
+// recovery and EU_EXACT_RATES the rate and trapezoid expressions with the
+// reference's operand order and divisions (compiled with --fmad=false they
+// round exactly as the reference's CPU build); without them, algebraically
+// equivalent fast forms are used. The flux reconstruction has its own switch (EU_EXACT_FLUX).
 #pragma once
 
 #include <cmath>
@@ -83,6 +83,34 @@ __device__ __forceinline__ double div_fast(double n, double d)
 }
 __device__ __forceinline__ float div_fast(float n, float d) { return __fdividef(n, d); }
 
+// exp(x): x = k ln 2 + r, |r| <= ln(2)/2, e^r = 1 + r + r^2 q(r) with q the
+// degree-9 polynomial through (e^r - 1 - r) / r^2 at the ten Chebyshev nodes of
+// that interval (relative error of e^r below 2e-17), scaled by 2^k. Within one
+// unit in the last place for results in the normal range; 0 below it, at most
+// the largest power-of-two range's end above it; a NaN stays a NaN. Straight
+// code (no special-case branches), so that a cell's twenty-odd exponentials
+// interleave.
+__device__ __forceinline__ double exp_fast(double x)
+{
+    constexpr double kShift = 6755399441055744.0; // 1.5 * 2^52: rounds to an integer in the low word
+    const double t = fma(x, 1.4426950408889634, kShift), kd = t - kShift;
+    const int k = min(max(__double2loint(t), -1023), 1023);
+    double r = fma(kd, -0x1.62e42fefa39efp-1, x);
+    r = fma(kd, -0x1.abc9e3b39803fp-56, r);
+    double q = 0x1.af38b4925be09p-26;
+    q = fma(q, r, 0x1.28918e390a71ep-22);
+    q = fma(q, r, 0x1.71de0da9d06acp-19);
+    q = fma(q, r, 0x1.a019b905bafb1p-16);
+    q = fma(q, r, 0x1.a01a01a7c54aep-13);
+    q = fma(q, r, 0x1.6c16c1788dc33p-10);
+    q = fma(q, r, 0x1.11111111109b2p-7);
+    q = fma(q, r, 0x1.5555555553d5ep-5);
+    q = fma(q, r, 0x1.5555555555556p-3);
+    q = fma(q, r, 0.5);
+    const double scale = __hiloint2double((k + 1023) << 20, 0);
+    return fma(scale, fma(r * r, q, r), scale);
+}
+
 // ------------------------------------------------------------------ thermo
 // NASA 9-coefficient polynomials (src/Reaction.cpp:1165-1220). T powers are
 // formed once per temperature.
@@ -103,23 +131,6 @@ __device__ __forceinline__ TPow make_tpow(double T, bool need_log)
     p.t4 = p.t3 * T;
     p.t5 = p.t4 * T;
     p.lnT = need_log ? log(T) : 0.0;
-    return p;
-}
-
-// The powers of T with 1/T and log T already known (a caller that carries
-// them from the temperature Newton).
-__device__ __forceinline__ TPow make_tpow_known(double T, double inv, double lnT)
-{
-    TPow p;
-    p.T = T;
-    p.low = T < kThermoSwitch;
-    p.inv = inv;
-    p.inv2 = inv * inv;
-    p.t2 = T * T;
-    p.t3 = p.t2 * T;
-    p.t4 = p.t3 * T;
-    p.t5 = p.t4 * T;
-    p.lnT = lnT;
     return p;
 }
 
@@ -170,7 +181,7 @@ __device__ __forceinline__ double h_species(const DevMech &m, const TPow &p, dou
     const double a0 = coeff<NS, kRange>(m, p, 0, s), a1 = coeff<NS, kRange>(m, p, 1, s), a2 = coeff<NS, kRange>(m, p, 2, s),
                  a3 = coeff<NS, kRange>(m, p, 3, s), a4 = coeff<NS, kRange>(m, p, 4, s), a5 = coeff<NS, kRange>(m, p, 5, s),
                  a6 = coeff<NS, kRange>(m, p, 6, s), a7 = coeff<NS, kRange>(m, p, 7, s);
-#ifdef EU_EXACT_CHEM
+#ifdef EU_EXACT_RATES
     return R * (-a0 * p.inv + a1 * p.lnT + a2 * p.T + a3 * p.t2 / 2 + a4 * p.t3 / 3 + a5 * p.t4 / 4 +
                 a6 * p.t5 / 5 + a7);
 #else
@@ -186,7 +197,7 @@ __device__ __forceinline__ double s_species(const DevMech &m, const TPow &p, dou
     const double a0 = coeff<NS, kRange>(m, p, 0, s), a1 = coeff<NS, kRange>(m, p, 1, s), a2 = coeff<NS, kRange>(m, p, 2, s),
                  a3 = coeff<NS, kRange>(m, p, 3, s), a4 = coeff<NS, kRange>(m, p, 4, s), a5 = coeff<NS, kRange>(m, p, 5, s),
                  a6 = coeff<NS, kRange>(m, p, 6, s), a8 = coeff<NS, kRange>(m, p, 8, s);
-#ifdef EU_EXACT_CHEM
+#ifdef EU_EXACT_RATES
     return R * (-a0 * p.inv2 / 2 - a1 * p.inv + a2 * p.lnT + a3 * p.T + a4 * p.t2 / 2 + a5 * p.t3 / 3 +
                 a6 * p.t4 / 4 + a8);
 #else
@@ -195,6 +206,7 @@ __device__ __forceinline__ double s_species(const DevMech &m, const TPow &p, dou
 #endif
 }
 
+#ifdef EU_EXACT_RATES
 // G_s = H_s - S_s T of every species (src/Reaction.cpp:597-600), the
 // reference's per-species expression.
 template <int NS>
@@ -206,13 +218,51 @@ __device__ __forceinline__ void gibbs_all(const DevMech &m, const TPow &p, doubl
         for (int s = 0; s < NS; ++s) G[s] = h_species<NS, kR>(m, p, kRUniv, s) - s_species<NS, kR>(m, p, kRUniv, s) * T;
     });
 }
+#else
+// The nine functions of T whose sums with a species' coefficients give G_s/(R T):
+// the enthalpy's term over R T minus the entropy's over R, coefficient by
+// coefficient (src/Reaction.cpp:597-600, 1180-1220).
+__device__ __forceinline__ void gibbs_terms(double T, double inv, double lnT, double (&f)[9])
+{
+    const double t2 = T * T;
+    f[0] = -0.5 * (inv * inv);
+    f[1] = (lnT + 1.0) * inv;
+    f[2] = 1.0 - lnT;
+    f[3] = -0.5 * T;
+    f[4] = t2 * (-1.0 / 6.0);
+    f[5] = (t2 * T) * (-1.0 / 12.0);
+    f[6] = (t2 * t2) * (-1.0 / 20.0);
+    f[7] = inv;
+    f[8] = -1.0;
+}
+
+// g_s = G_s/(R T) of every species: nine multiply-adds each.
+template <int NS>
+__device__ __forceinline__ void gibbs_rt(const DevMech &m, double T, double inv, double lnT, double (&g)[NS])
+{
+    double f[9];
+    gibbs_terms(T, inv, lnT, f);
+    by_range(T < kThermoSwitch, [&](auto range) {
+        constexpr int kR = decltype(range)::value;
+        TPow p;
+        p.low = T < kThermoSwitch;
+#pragma unroll
+        for (int s = 0; s < NS; ++s) {
+            double v = f[0] * coeff<NS, kR>(m, p, 0, s);
+#pragma unroll
+            for (int k = 1; k < 9; ++k) v = fma(f[k], coeff<NS, kR>(m, p, k, s), v);
+            g[s] = v;
+        }
+    });
+}
+#endif
 
 // --------------------------------------------------------- state recovery
 
 // Flowfield::Get_temp (src/Flowfield.cpp:2072-2131): Newton on
 // sum_s Y_s h_s(T) - E*1e-3 - (sum_s Y_s R_s) T = 0, at most 10 iterations,
 // stop when |dT| < 1e-6 K. E is the cell's previous internal energy.
-#ifdef EU_EXACT_CHEM
+#ifdef EU_EXACT_THERMO
 template <int NS>
 __device__ __forceinline__ double newton_temperature(const DevMech &m, double T, double E, const double (&Y)[NS])
 {
@@ -304,7 +354,7 @@ __device__ __forceinline__ void mix_poly(const DevMech &m, const double (&Y)[NS]
 template <int NS>
 struct ThermoCache {
     MixPoly<NS> c;
-    bool low;
+    int low = -1; // 1: low range, 0: high, -1: no sums
 };
 
 template <int NS>
@@ -315,9 +365,8 @@ __device__ __forceinline__ double newton_temperature(const DevMech &m, double T,
 #pragma unroll
     for (int s = 0; s < NS; ++s) rsum += Y[s] * m.ri[s];
     const double e_scaled = E * 1e-3;
-    bool &low = tc.low;
+    bool low = T < kThermoSwitch;
     MixPoly<NS> &c = tc.c;
-    low = T < kThermoSwitch;
     mix_poly<NS>(m, Y, low, c);
     double T_temp = T;
     for (int count = 0; count < 10; ++count) {
@@ -338,6 +387,7 @@ __device__ __forceinline__ double newton_temperature(const DevMech &m, double T,
         if (fabs(T_temp - T0) < 1e-6)
             break;
     }
+    tc.low = low;
     return T_temp;
 }
 
@@ -370,12 +420,11 @@ __device__ __forceinline__ double advance_log(double ln0, double x, double T1)
     return fabs(x) <= 0x1p-6 ? ln0 + log1p_small(x) : log(T1);
 }
 
-// The Newton above for a caller that carries 1/T and log T from one solve to
-// the next (the warp-per-cell kinetics: every substep's rates and rebuild
-// start from the last rebuild's temperature). On entry inv and lnT are those
-// of T; each iterate's log comes from the previous one's (advance_log), not
-// from a logarithm; on return they are those of the result. Same iterates as
-// the Newton above to within rounding.
+// The Newton above for the kinetics, whose substeps' rates and rebuilds each
+// start from the last rebuild's temperature: inv and lnT are 1/T and log T of
+// the starting temperature on entry and of the result on return, and each
+// iterate's log comes from the previous one's (advance_log), so that a cell's
+// substeps take one logarithm.
 template <int NS>
 __device__ __forceinline__ double newton_temperature_carry(const DevMech &m, double T, double E, const double (&Y)[NS],
                                                            ThermoCache<NS> &tc, double &inv, double &lnT)
@@ -384,9 +433,8 @@ __device__ __forceinline__ double newton_temperature_carry(const DevMech &m, dou
 #pragma unroll
     for (int s = 0; s < NS; ++s) rsum += Y[s] * m.ri[s];
     const double e_scaled = E * 1e-3;
-    bool &low = tc.low;
+    bool low = T < kThermoSwitch;
     MixPoly<NS> &c = tc.c;
-    low = T < kThermoSwitch;
     mix_poly<NS>(m, Y, low, c);
     double T0 = T, inv0 = inv, ln0 = lnT, T_temp = T;
     for (int count = 0; count < 10; ++count) {
@@ -411,6 +459,7 @@ __device__ __forceinline__ double newton_temperature_carry(const DevMech &m, dou
         if (fabs(T_temp - T0) < 1e-6)
             break;
     }
+    tc.low = low;
     lnT = advance_log(ln0, (T_temp - T0) * inv0, T_temp);
     inv = rcp_nr(T_temp);
     return T_temp;
@@ -423,22 +472,37 @@ struct CellState {
     double cs[NS + 4];
     double Y[NS];
     double D, T, E, U, V, W;
+    double inv, lnT; // 1/T and log T (fast forms; carried by the temperature Newton)
 };
+
+// 1/T and log T of a temperature just loaded.
+template <int NS>
+__device__ __forceinline__ void load_temperature(CellState<NS> &c, double T)
+{
+    c.T = T;
+#ifndef EU_EXACT_RATES
+    c.inv = rcp_nr(T);
+    c.lnT = log(T);
+#endif
+}
 
 // Flowfield::Update_after_CS (src/Flowfield.cpp:1579-1617 / :1639-1673) for one
 // cell, up to the point where P, H, Gamma are needed (those are formed by
-// finish_primitives when the cell's primitives are written).
-template <int NS>
+// finish_primitives when the cell's primitives are written). kCarry: within the
+// kinetics, whose rates read c.inv and c.lnT (newton_temperature_carry).
+template <int NS, bool kCarry = false>
 __device__ __forceinline__ void recover_state(const DevMech &m, CellState<NS> &c, ThermoCache<NS> &tcache)
 {
     double D = 0;
 #pragma unroll
     for (int s = 0; s < NS; ++s) D += c.cs[s];
-#ifdef EU_EXACT_CHEM
+#ifdef EU_EXACT_THERMO
 #pragma unroll
     for (int s = 0; s < NS; ++s) c.Y[s] = c.cs[s] / D;
     c.D = D;
     c.T = newton_temperature<NS>(m, c.T, c.E, c.Y);
+    if (kCarry)
+        load_temperature<NS>(c, c.T);
     c.U = c.cs[NS + 0] / D;
     c.V = c.cs[NS + 1] / D;
     c.W = c.cs[NS + 2] / D;
@@ -449,41 +513,16 @@ __device__ __forceinline__ void recover_state(const DevMech &m, CellState<NS> &c
 #pragma unroll
     for (int s = 0; s < NS; ++s) c.Y[s] = c.cs[s] * invD;
     c.D = D;
-    c.T = newton_temperature<NS>(m, c.T, c.E, c.Y, tcache);
+    if (kCarry)
+        c.T = newton_temperature_carry<NS>(m, c.T, c.E, c.Y, tcache, c.inv, c.lnT);
+    else
+        c.T = newton_temperature<NS>(m, c.T, c.E, c.Y, tcache);
     c.U = c.cs[NS + 0] * invD;
     c.V = c.cs[NS + 1] * invD;
     c.W = c.cs[NS + 2] * invD;
     c.E = (c.cs[NS + 3] - 0.5 * D * (c.U * c.U + c.V * c.V + c.W * c.W)) * invD;
 #endif
 }
-
-template <int NS>
-__device__ __forceinline__ void recover_state(const DevMech &m, CellState<NS> &c)
-{
-    ThermoCache<NS> tcache;
-    recover_state<NS>(m, c, tcache);
-}
-
-#ifndef EU_EXACT_CHEM
-// recover_state with 1/T and log T carried (newton_temperature_carry).
-template <int NS>
-__device__ __forceinline__ void recover_state_carry(const DevMech &m, CellState<NS> &c, double &inv, double &lnT)
-{
-    double D = 0;
-#pragma unroll
-    for (int s = 0; s < NS; ++s) D += c.cs[s];
-    const double invD = rcp_nr(D);
-#pragma unroll
-    for (int s = 0; s < NS; ++s) c.Y[s] = c.cs[s] * invD;
-    c.D = D;
-    ThermoCache<NS> tcache;
-    c.T = newton_temperature_carry<NS>(m, c.T, c.E, c.Y, tcache, inv, lnT);
-    c.U = c.cs[NS + 0] * invD;
-    c.V = c.cs[NS + 1] * invD;
-    c.W = c.cs[NS + 2] * invD;
-    c.E = (c.cs[NS + 3] - 0.5 * D * (c.U * c.U + c.V * c.V + c.W * c.W)) * invD;
-}
-#endif
 
 // P, H, Gamma of Update_after_CS (src/Flowfield.cpp:1606-1614). tcache: the
 // recovery's thermo sums for this state, or null.
@@ -491,7 +530,7 @@ template <int NS>
 __device__ __forceinline__ void finish_primitives(const DevMech &m, const CellState<NS> &c,
                                                   const ThermoCache<NS> *tcache, double &P, double &H, double &G)
 {
-#ifdef EU_EXACT_CHEM
+#ifdef EU_EXACT_THERMO
     double inv_w = 0;
 #pragma unroll
     for (int s = 0; s < NS; ++s) inv_w += c.Y[s] / m.mw[s];
@@ -518,7 +557,7 @@ __device__ __forceinline__ void finish_primitives(const DevMech &m, const CellSt
     H = c.T * Rgas + c.E;
     MixPoly<NS> mp;
     const bool low = c.T < kThermoSwitch;
-    if (tcache && tcache->low == low)
+    if (tcache && tcache->low == int(low))
         mp = tcache->c;
     else
         mix_poly<NS>(m, c.Y, low, mp);
@@ -564,15 +603,24 @@ __device__ __forceinline__ double pow_int_or_real(double x, double e)
 // every species; terms whose stoichiometric coefficients vanish are exact zeros
 // in the reference and are skipped here. P and Q do not depend on the substep
 // length, so the prediction's evaluation serves the first substep too.
+// Per reaction W's term is Q's minus P's, and the fast forms take W from the
+// sums: W_s = mw_s (Q_s - P_s), a third of the sums less to keep.
 template <int NS>
 struct SpeciesRates {
-    double P[NS], Q[NS], W[NS]; // W = Wi (mass rate, g/cm^3/s)
+    double P[NS], Q[NS];
+#ifdef EU_EXACT_RATES
+    double W[NS]; // Wi (mass rate, g/cm^3/s)
+    __device__ __forceinline__ double w(const DevMech &, int s) const { return W[s]; }
+#else
+    __device__ __forceinline__ double w(const DevMech &m, int s) const { return m.mw[s] * (Q[s] - P[s]); }
+#endif
 };
 
-#ifdef EU_EXACT_CHEM
+#ifdef EU_EXACT_RATES
 // Strict form: the reference's expressions (pow, exp of each Kp, divisions).
 template <int NS, int NR>
-__device__ __forceinline__ void eval_rates(const DevMech &m, double T, const double (&mc)[NS], SpeciesRates<NS> &k)
+__device__ __forceinline__ void eval_rates(const DevMech &m, double T, double, double, const double (&mc)[NS],
+                                           SpeciesRates<NS> &k)
 {
     double Gi[NS];
     {
@@ -629,26 +677,24 @@ __device__ __forceinline__ void eval_rates(const DevMech &m, double T, const dou
 //   kb_r = kf_r * prod_s exp(g_s)^nu_rs * (RT/p0)^Xr  (one exp per species);
 //   kf_r = A_r exp(b_r ln T - E_r/(Ru T))            (one exp per reaction).
 template <int NS, int NR>
-__device__ __forceinline__ void eval_rates(const DevMech &m, double T, const double (&mc)[NS], SpeciesRates<NS> &k)
+__device__ __forceinline__ void eval_rates(const DevMech &m, double T, double inv, double lnT, const double (&mc)[NS],
+                                           SpeciesRates<NS> &k)
 {
-    double eg[NS], ieg[NS], Gs[NS];
-    const TPow p = make_tpow(T, true);
-    const double invRT = 1.0 / (kRUniv * T);
-    gibbs_all<NS>(m, p, T, Gs);
+    double eg[NS], ieg[NS];
+    gibbs_rt<NS>(m, T, inv, lnT, eg);
 #pragma unroll
     for (int s = 0; s < NS; ++s) {
-        const double g = Gs[s] * invRT;
-        eg[s] = exp(g);
+        eg[s] = exp_fast(eg[s]);
         ieg[s] = rcp_nr(eg[s]);
     }
-    const double invRuT = 1.0 / (kRuCal * T);
-    const double rt_p0 = (kRUniv * T) / (kP0 * 1e-6);
-    const double p0_rt = rcp_nr(rt_p0);
+    const double inv2 = inv * inv;
+    const double invRuT = inv * (1.0 / kRuCal);
+    const double rt_p0 = T * (kRUniv / (kP0 * 1e-6));
+    const double p0_rt = inv * (kP0 * 1e-6 / kRUniv);
 #pragma unroll
     for (int s = 0; s < NS; ++s) {
         k.P[s] = 0.0;
         k.Q[s] = 0.0;
-        k.W[s] = 0.0;
     }
 #pragma unroll
     for (int r = 0; r < NR; ++r) {
@@ -656,9 +702,9 @@ __device__ __forceinline__ void eval_rates(const DevMech &m, double T, const dou
         const double b = m.bf[r];
         double kf;
         if (m.eaf[r] == 0.0 && (b == 0.0 || b == 1.0 || b == -1.0 || b == -2.0))
-            kf = m.af[r] * (b == 0.0 ? 1.0 : b == 1.0 ? T : b == -1.0 ? p.inv : p.inv2);
+            kf = m.af[r] * (b == 0.0 ? 1.0 : b == 1.0 ? T : b == -1.0 ? inv : inv2);
         else
-            kf = m.af[r] * exp(b * p.lnT - m.eaf[r] * invRuT);
+            kf = m.af[r] * exp_fast(b * lnT - m.eaf[r] * invRuT);
 #pragma unroll
         for (int s = 0; s < NS; ++s) {
             const double f = m.sf[r][s], bb = m.sb[r][s];
@@ -675,19 +721,25 @@ __device__ __forceinline__ void eval_rates(const DevMech &m, double T, const dou
         if (rtb == 0.0)
             rtb = 1.0;
         const double fwd = kf * rrf, bwd = kb * rrb;
-        const double rr = fwd - bwd;
 #pragma unroll
         for (int s = 0; s < NS; ++s) {
             const double bb = m.sb[r][s], f = m.sf[r][s];
             if (bb != 0.0 || f != 0.0) {
-                k.W[s] += (bb - f) * rtb * rr;
                 k.Q[s] += (bb * fwd + f * bwd) * rtb;
                 k.P[s] += (bb * bwd + f * fwd) * rtb;
             }
         }
     }
-#pragma unroll
-    for (int s = 0; s < NS; ++s) k.W[s] = m.mw[s] * k.W[s];
+}
+
+// P_s / mc_s, the trapezoid's loss frequency (0 where the species is absent,
+// src/Reaction.cpp:786-797), with a refined reciprocal. Traces below 1e-200,
+// whose reciprocal would leave the normal range, are scaled first.
+__device__ __forceinline__ double loss_frequency(double P, double mc)
+{
+    const double s = fabs(mc) < 1e-200 ? 0x1p+300 : 1.0;
+    const double q = (P * s) * rcp_nr(mc * s);
+    return mc == 0.0 ? 0.0 : q;
 }
 #endif
 
@@ -697,19 +749,28 @@ __device__ __forceinline__ void eval_rates(const DevMech &m, double T, const dou
 // densities are cs * 1e-3.
 template <int NS>
 __device__ __forceinline__ void trapezoid_substep(const DevMech &m, const SpeciesRates<NS> &k, double dts,
-                                                  const double (&mc)[NS], CellState<NS> &c)
+                                                  const double (&mc)[NS], CellState<NS> &c, ThermoCache<NS> &tcache)
 {
+#ifdef EU_EXACT_RATES
     const double half = dts / 2.0;
+#else
+    const double half = dts * 0.5;
+#endif
     double D = 0.0;
 #pragma unroll
     for (int s = 0; s < NS; ++s) {
         const double di = c.cs[s] * 1e-3;
         const double q = m.mw[s] * k.Q[s];
+#ifdef EU_EXACT_RATES
         // the quotient formed before the choice: a select, not a branch on
         // which the threads (cells with and without the species) diverge
         const double pq = k.P[s] / mc[s];
         const double p = (mc[s] == 0) ? 0.0 : pq;
         const double nd = ((1.0 - half * p) * di + dts * q) / (1.0 + half * p) * 1e3;
+#else
+        const double hp = half * loss_frequency(k.P[s], mc[s]);
+        const double nd = fma(dts, q, fma(-hp, di, di)) * rcp_nr(1.0 + hp) * 1e3;
+#endif
         c.cs[s] = nd;
         D += nd;
     }
@@ -717,7 +778,7 @@ __device__ __forceinline__ void trapezoid_substep(const DevMech &m, const Specie
     c.cs[NS + 1] = c.V * D;
     c.cs[NS + 2] = c.W * D;
     c.cs[NS + 3] = D * c.E + 0.5 * (c.U * c.U + c.V * c.V + c.W * c.W) * D;
-    recover_state<NS>(m, c);
+    recover_state<NS, true>(m, c, tcache);
 }
 
 // Concentrations scaled to mol/cm^3 as the kinetics reads them: Mc = Di/Mw*1000

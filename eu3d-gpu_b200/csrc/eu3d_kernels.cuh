@@ -1,6 +1,6 @@
 // eu3d_kernels.cuh — the timestep kernels, templated on the species and
 // reaction counts. Instantiated twice: eu3d_kernels_strict.cu (--fmad=false,
-// EU_EXACT_CHEM/EU_EXACT_FLUX) and eu3d_kernels_fast.cu.
+// EU_EXACT_RATES/EU_EXACT_FLUX) and eu3d_kernels_fast.cu.
 #pragma once
 
 #include "eu3d_device.cuh"
@@ -626,9 +626,10 @@ __device__ __forceinline__ void mark_z_fresh(const DevState &st)
 template <int NS_, int NR_>
 struct TableRates {
     static constexpr int NS = NS_, NR = NR_;
-    __device__ __forceinline__ static void rates(const DevMech &m, double T, const double (&mc)[NS], SpeciesRates<NS> &k)
+    __device__ __forceinline__ static void rates(const DevMech &m, double T, double inv, double lnT,
+                                                 const double (&mc)[NS], SpeciesRates<NS> &k)
     {
-        eval_rates<NS, NR>(m, T, mc, k);
+        eval_rates<NS, NR>(m, T, inv, lnT, mc, k);
     }
 };
 
@@ -639,110 +640,146 @@ struct TableRates {
 // the first substep: both evaluate the same expression on the same state.
 // Returns Nchem; a prediction <= 0 or above max_substeps is counted as an error.
 // Nchem = ceil(dtm / min_s |Di_s / Wi_s|) over species with Y_s >= 1e-6
-// (src/Reaction.cpp:919-940); a prediction <= 0 or above max_substeps is
-// counted as an error and gives 0 or max_substeps.
-__device__ __forceinline__ int nchem_from_dt(double dtm, double dt, int max_substeps, unsigned long long *counters)
+// (src/Reaction.cpp:919-940); a prediction <= 0 or above max_substeps is bad
+// (counted as an error) and gives 0 or max_substeps.
+__device__ __forceinline__ int nchem_from_dt(double dtm, double dt, int max_substeps, bool &bad)
 {
     const double ratio = ceil(dtm / dt);
-    if (!(ratio >= 1.0) || ratio > double(max_substeps)) {
-        atomicAdd(&counters[kCntBadNchem], 1ULL);
+    bad = !(ratio >= 1.0) || ratio > double(max_substeps);
+    if (bad)
         return (ratio > double(max_substeps)) ? max_substeps : 0;
-    }
     return int(ratio);
 }
 
-__device__ __forceinline__ void count_nchem(unsigned long long *counters, int nchem)
+// The threads that arrive here together with the same pointer (in a batch's
+// shared stage a warp's cells may belong to several instances).
+__device__ __forceinline__ unsigned peers(const void *p)
 {
-    if (nchem > 0) {
-        atomicMax(&counters[kCntMaxNchem], (unsigned long long)nchem);
-        atomicAdd(&counters[kCntSumNchem], (unsigned long long)nchem);
+    const unsigned here = __activemask();
+    int same;
+    __match_all_sync(here, reinterpret_cast<unsigned long long>(p), &same);
+    return same ? here : __match_any_sync(here, reinterpret_cast<unsigned long long>(p));
+}
+
+// The statistics of the cells' predictions, by the kernel that advances them:
+// one set of atomics for the threads that arrive together. (One a cell on the
+// two counters, all on one L2 slice, were what the kinetics waited for: 545,025
+// cells of one substep each took 0.75 ms with the rates in either form, 0.26
+// with a set a warp.)
+__device__ __forceinline__ void count_nchem(unsigned long long *counters, int nchem, bool bad)
+{
+    const unsigned here = peers(counters);
+    const unsigned errors = __ballot_sync(here, bad);
+    const int most = __reduce_max_sync(here, nchem);
+    const unsigned sum = __reduce_add_sync(here, unsigned(nchem)); // 32 x 2^20 at most by default
+    const bool big = most >= (1 << 26);
+    if (big) { // max_substeps beyond the sum's range: a cell at a time
+        if (nchem > 0)
+            atomicAdd(&counters[kCntSumNchem], (unsigned long long)nchem);
     }
+    if ((threadIdx.x & 31) == __ffs(here) - 1) {
+        if (errors)
+            atomicAdd(&counters[kCntBadNchem], (unsigned long long)__popc(errors));
+        if (most > 0) {
+            if (!big)
+                atomicAdd(&counters[kCntSumNchem], (unsigned long long)sum);
+            if (*(volatile unsigned long long *)&counters[kCntMaxNchem] < (unsigned long long)most)
+                atomicMax(&counters[kCntMaxNchem], (unsigned long long)most);
+        }
+    }
+}
+
+// One more on a counter for every thread that arrives.
+__device__ __forceinline__ void count_threads(unsigned long long *counter)
+{
+    const unsigned here = peers(counter);
+    if ((threadIdx.x & 31) == __ffs(here) - 1)
+        atomicAdd(counter, (unsigned long long)__popc(here));
 }
 
 // The prediction: start-of-step rates (kept in `rates` for the first substep)
 // and Nchem.
 template <int NS, class Rt>
 __device__ __forceinline__ int predict_nchem(const DevMech &m, const CellState<NS> &cell, double dtm,
-                                             int max_substeps, unsigned long long *counters, double (&mc)[NS],
+                                             int max_substeps, bool &bad, double (&mc)[NS],
                                              SpeciesRates<NS> &rates)
 {
     scaled_concentrations<NS>(m, cell, mc);
-    Rt::rates(m, cell.T, mc, rates);
+    Rt::rates(m, cell.T, cell.inv, cell.lnT, mc, rates);
     double dt = dtm;
 #pragma unroll
     for (int s = 0; s < NS; ++s) {
         // formed for every species, then chosen: a select instead of a branch
         // that the cells diverge on
-        const double dt_temp = fabs(-(cell.cs[s] * 1e-3) / rates.W[s]);
-        dt = (cell.Y[s] >= 1e-6 && rates.W[s] != 0 && dt_temp < dt) ? dt_temp : dt;
+        const double w = rates.w(m, s);
+#ifdef EU_EXACT_RATES
+        const double dt_temp = fabs(-(cell.cs[s] * 1e-3) / w);
+#else
+        const double dt_temp = fabs(cell.cs[s] * 1e-3 * rcp_nr(w));
+#endif
+        dt = (cell.Y[s] >= 1e-6 && w != 0 && dt_temp < dt) ? dt_temp : dt;
     }
-    return nchem_from_dt(dtm, dt, max_substeps, counters);
+    return nchem_from_dt(dtm, dt, max_substeps, bad);
 }
 
 // The Nchem substeps, the first one on the prediction's rates.
 template <int NS, class Rt>
 __device__ __forceinline__ void run_substeps(const DevMech &m, CellState<NS> &cell, double dtm, int nchem,
                                              double (&mc)[NS], SpeciesRates<NS> &rates, double *cms,
-                                             long long cms_stride)
+                                             long long cms_stride, ThermoCache<NS> &tcache)
 {
     const double dts = dtm / nchem;
     for (int step = 0; step < nchem; ++step) {
         if (step > 0) {
             scaled_concentrations<NS>(m, cell, mc);
-            Rt::rates(m, cell.T, mc, rates);
+            Rt::rates(m, cell.T, cell.inv, cell.lnT, mc, rates);
         }
         if (cms) {
 #pragma unroll
-            for (int s = 0; s < NS; ++s) cms[s * cms_stride] = rates.W[s] * 1e3;
+            for (int s = 0; s < NS; ++s) cms[s * cms_stride] = rates.w(m, s) * 1e3;
         }
-        trapezoid_substep<NS>(m, rates, dts, mc, cell);
+        trapezoid_substep<NS>(m, rates, dts, mc, cell, tcache);
     }
 }
 
-template <int NS, class Rt>
-__device__ __forceinline__ int react_cell(const DevMech &m, CellState<NS> &cell, double dtm, int max_substeps,
-                                          unsigned long long *counters, double *cms, long long cms_stride)
-{
-    double mc[NS];
-    SpeciesRates<NS> rates;
-    const int nchem = predict_nchem<NS, Rt>(m, cell, dtm, max_substeps, counters, mc, rates);
-    count_nchem(counters, nchem);
-    run_substeps<NS, Rt>(m, cell, dtm, nchem, mc, rates, cms, cms_stride);
-    return nchem;
-}
-
-// Cells whose predicted Nchem exceeds kHeavyNchem are, in the mixed-precision
-// flavour (EU_HEAVY_QUEUE), deferred to k_react_heavy: one warp per cell
-// instead of one thread, so the long serial substep chains of igniting cells
-// do not set the step's time. st.heavy = {count, next, cells...}. On the
-// 48x32x32 igniting block the step takes 0.865 / 0.81 / 0.764 / 0.78 / 1.11 ms
-// with the threshold at 16 / 8 / 4 / 2 / 0: below 4 a warp per cell costs more
-// than the few substeps it shortens.
+// Cells whose predicted Nchem exceeds kHeavyNchem are deferred to k_react_heavy:
+// one warp per cell instead of one thread, so the long serial substep chains of
+// igniting cells do not set the step's time. st.heavy = {count, next, cells...}
+// (null: every cell on its own thread). On the 48x32x32 igniting block in mixed
+// precision the step took 0.865 / 0.81 / 0.764 / 0.78 / 1.11 ms with the
+// threshold at 16 / 8 / 4 / 2 / 0: below 4 a warp per cell costs more than the
+// few substeps it shortens.
 constexpr int kHeavyNchem = 4;
 
 __device__ __forceinline__ void push_heavy(int *heavy, long long c)
 {
-    const int q = atomicAdd(&heavy[0], 1);
+    const unsigned here = peers(heavy), lane = threadIdx.x & 31;
+    const int first = __ffs(here) - 1;
+    int q = 0;
+    if (int(lane) == first)
+        q = atomicAdd(&heavy[0], __popc(here));
+    q = __shfl_sync(here, q, first) + __popc(here & ((1u << lane) - 1));
     heavy[2 + q] = int(c);
 }
 
-// React one recovered cell, or (mixed flavour, heavy queue present) defer it
-// when its Nchem is large. Returns false when deferred.
+// React one recovered cell, or (heavy queue present) defer it when its Nchem is
+// large. Returns false when deferred. tcache: the last substep's thermo sums out.
 template <int NS, class Rt>
 __device__ __forceinline__ bool react_or_defer(const DevMech &m, const DevState &st, long long n3, long long c,
-                                               CellState<NS> &cell, double dtm, int max_substeps)
+                                               CellState<NS> &cell, double dtm, int max_substeps,
+                                              ThermoCache<NS> &tcache)
 {
     double mc[NS];
     SpeciesRates<NS> rates;
-    const int nchem = predict_nchem<NS, Rt>(m, cell, dtm, max_substeps, st.counters, mc, rates);
-#ifdef EU_HEAVY_QUEUE
+    bool bad;
+    load_temperature<NS>(cell, cell.T); // as a cell loaded from a queue
+    const int nchem = predict_nchem<NS, Rt>(m, cell, dtm, max_substeps, bad, mc, rates);
     if (st.heavy && nchem > kHeavyNchem) {
         push_heavy(st.heavy, c);
         return false;
     }
-#endif
-    count_nchem(st.counters, nchem);
-    run_substeps<NS, Rt>(m, cell, dtm, nchem, mc, rates, st.cms ? st.cms + c : nullptr, n3);
+    count_nchem(st.counters, nchem, bad);
+    run_substeps<NS, Rt>(m, cell, dtm, nchem, mc, rates, st.cms ? st.cms + c : nullptr, n3, tcache);
     st.nchem[c] = nchem;
     return true;
 }
@@ -752,7 +789,7 @@ __device__ __forceinline__ void load_cell(const DevState &st, long long n3, long
 {
 #pragma unroll
     for (int q = 0; q < NS + 4; ++q) cell.cs[q] = st.cs[q * n3 + c];
-    cell.T = st.T[c];
+    load_temperature<NS>(cell, st.T[c]);
     cell.E = st.E[c];
 }
 
@@ -767,7 +804,7 @@ __device__ __forceinline__ void load_recovered(const DevState &st, long long n3,
 #pragma unroll
     for (int s = 0; s < NS; ++s) D += cell.cs[s];
     cell.D = D;
-#ifdef EU_EXACT_CHEM
+#ifdef EU_EXACT_THERMO
 #pragma unroll
     for (int s = 0; s < NS; ++s) cell.Y[s] = cell.cs[s] / D;
     cell.U = cell.cs[NS + 0] / D;
@@ -843,20 +880,17 @@ __global__ void __launch_bounds__(128, MINB) k_recover_react(const __grid_consta
     const long long c = cell_index(g, i, j, k);
     CellState<NS> cell;
     load_cell<NS>(st, n3, c, cell);
+    ThermoCache<NS> recovered;
+    recover_state<NS>(m, cell, recovered);
     if (!kReact) {
-        ThermoCache<NS> tcache;
-        recover_state<NS>(m, cell, tcache);
-        store_cell<NS, false>(m, st, n3, c, cell, &tcache);
+        store_cell<NS, false>(m, st, n3, c, cell, &recovered);
         return;
     }
-    recover_state<NS>(m, cell);
-    if (kReact) {
-        if (!react_or_defer<NS, Rt>(m, st, n3, c, cell, *dt_dev, max_substeps)) {
-            store_cell<NS, false>(m, st, n3, c, cell); // recovered state for k_react_heavy
-            return;
-        }
-    }
-    store_cell<NS, kReact>(m, st, n3, c, cell);
+    ThermoCache<NS> tcache;
+    if (react_or_defer<NS, Rt>(m, st, n3, c, cell, *dt_dev, max_substeps, tcache))
+        store_cell<NS>(m, st, n3, c, cell, &tcache);
+    else
+        store_cell<NS, false>(m, st, n3, c, cell); // recovered state for k_react_heavy
 }
 
 // ------------------------------------------------- learned chemistry
@@ -997,9 +1031,9 @@ __global__ void __launch_bounds__(128) k_learned_apply(const __grid_constant__ D
                     cell.Y[s] = Y[s] / sum;
                     cell.cs[s] = cell.D * cell.Y[s];
                 }
-                cell.T = newton_temperature<NS>(m, cell.T + mean[NS], cell.E, cell.Y);
+                load_temperature<NS>(cell, newton_temperature<NS>(m, cell.T + mean[NS], cell.E, cell.Y));
                 store_cell<NS>(m, st, n3, c, cell);
-                atomicAdd(&st.counters[kCntLearned], 1ULL);
+                count_threads(&st.counters[kCntLearned]);
             } else {
                 fallback = true;
             }
@@ -1024,9 +1058,10 @@ __device__ __forceinline__ void react_queued(const DevMech &m, const DevState &s
 {
     CellState<NS> cell;
     load_recovered<NS>(st, n3, c, cell);
-    atomicAdd(&st.counters[counter], 1ULL);
-    if (react_or_defer<NS, Rt>(m, st, n3, c, cell, dtm, max_substeps))
-        store_cell<NS>(m, st, n3, c, cell);
+    count_threads(&st.counters[counter]);
+    ThermoCache<NS> tcache;
+    if (react_or_defer<NS, Rt>(m, st, n3, c, cell, dtm, max_substeps, tcache))
+        store_cell<NS>(m, st, n3, c, cell, &tcache);
 }
 
 // Position `pos` of the batch's queues taken end to end: the instance holding
@@ -1142,19 +1177,18 @@ __global__ void __launch_bounds__(128) k_learned_route(const __grid_constant__ D
                 double mc[NS];
                 SpeciesRates<NS> rates;
                 const double dtm = *dt_dev;
-                const int nchem = predict_nchem<NS, Rt>(m, cell, dtm, max_substeps, st.counters, mc, rates);
+                bool bad;
+                const int nchem = predict_nchem<NS, Rt>(m, cell, dtm, max_substeps, bad, mc, rates);
                 if (nchem <= lp.min_nchem) {
                     to_model = false;
-#ifdef EU_HEAVY_QUEUE
                     if (st.heavy && nchem > kHeavyNchem) {
                         push_heavy(st.heavy, c);
-                    } else
-#endif
-                    {
-                        count_nchem(st.counters, nchem);
-                        run_substeps<NS, Rt>(m, cell, dtm, nchem, mc, rates, st.cms ? st.cms + c : nullptr, n3);
+                    } else {
+                        count_nchem(st.counters, nchem, bad);
+                        ThermoCache<NS> tcache;
+                        run_substeps<NS, Rt>(m, cell, dtm, nchem, mc, rates, st.cms ? st.cms + c : nullptr, n3, tcache);
                         st.nchem[c] = nchem;
-                        store_cell<NS>(m, st, n3, c, cell);
+                        store_cell<NS>(m, st, n3, c, cell, &tcache);
                     }
                 }
             }
@@ -1170,392 +1204,6 @@ __global__ void __launch_bounds__(128) k_learned_route(const __grid_constant__ D
             at = __shfl_sync(0xffffffffu, at, __ffs(mask) - 1);
             if (to_model)
                 lp.queue[at + __popc(mask & ((1u << lane) - 1))] = int(c);
-        }
-    }
-}
-
-// ------------------------------------------------- warp-per-cell kinetics
-// The same kinetics as react_cell (prediction, Nchem trapezoid substeps,
-// state rebuild after each) with one warp per cell: lane r evaluates reaction
-// r, lane s owns species s's sums and trapezoid update, and every lane keeps
-// the whole cell state (the rebuild runs redundantly on all lanes). The sums
-// run in the same order as the one-thread form. Tables that lanes index by
-// reaction or species are read from a shared-memory copy of the mechanism;
-// the uniform reads of the state rebuild stay on the kernel parameter.
-
-template <int NS>
-__device__ __forceinline__ double lane_pick(const double (&v)[NS], int lane)
-{
-    double r = 0.0;
-#pragma unroll
-    for (int s = 0; s < NS; ++s) r = (lane == s) ? v[s] : r;
-    return r;
-}
-
-// Per-lane constants of the warp-per-cell kinetics, read once per warp from
-// the mechanism tables: lane r's reaction (r < NR; others repeat reaction 0)
-// and lane s's species (s < NS; others repeat species 0).
-template <int NS, int NR>
-struct HeavyLane {
-    double af, bf, eaf, xr, mw;
-};
-
-template <int NS, int NR>
-__device__ __forceinline__ HeavyLane<NS, NR> heavy_lane(const DevMech &m, int lane)
-{
-    static_assert(NR <= 32 && NS <= 32, "one lane per reaction and per species");
-    HeavyLane<NS, NR> h;
-    const int r = lane < NR ? lane : 0, sl = lane < NS ? lane : 0;
-    h.af = m.af[r];
-    h.bf = m.bf[r];
-    h.eaf = m.eaf[r];
-    h.xr = m.xr[r];
-    h.mw = m.mw[sl];
-    return h;
-}
-
-// The mechanism's sparse structure for the warp-per-cell kinetics, built once
-// per block, every array [entry][lane] so that a warp reads 32 consecutive
-// elements. Lane r's reaction (lanes past NR repeat reaction 0) lists the
-// species it involves, ascending: rent = s | nu' << 4 | nu'' << 6, then
-// entries with nu' = nu'' = 0 (factors of exactly 1). Lane s's species (lanes
-// past NS repeat species 0) lists the reactions it takes part in, ascending:
-// sent = q with its coefficients as doubles in sbv, sfv, then entries of
-// reaction slot 31, whose rates are zero (addends of exactly 0). So the
-// loops run a fixed count without branches and the products and sums are
-// the per-thread form's, whose other terms are factors of 1 and addends of
-// 0. tb: third-body efficiencies [s][r]; imw: 1e-3 / W_s.
-template <int NS, int NR>
-struct HeavyTablesT {
-    static_assert(NR < 32, "slot 31 holds zero rates");
-    double tb[NS][32];
-    double sbv[NR][32], sfv[NR][32];
-    double imw[NS];
-    unsigned char rent[NS][32], sent[NR][32];
-};
-
-// A warp's exchange buffers in shared memory: the species' exp(g) and
-// exp(-g), the reactions' forward and backward rates and third-body sums.
-struct HeavyScratch {
-    double eg[32], ieg[32], fwd[32], bwd[32], rtb[32], mc[32];
-};
-
-// Fast-form rates (the mixed flavour's eval_rates) across a warp. On return
-// lane s < NS holds P_s, Q_s and W_s (W with the molecular weight applied).
-// The species' Gibbs exponentials and the reactions' rates change hands
-// through the warp's shared buffers (one store each, broadcast loads); a
-// reaction lane reads its coefficients from the transposed tables (tt), a
-// species lane from the mechanism's (ms): the arithmetic and its order are
-// the per-thread form's. inv, lnT: 1/T and log T (carried from the last
-// rebuild's Newton).
-template <int NS, int NR>
-__device__ __forceinline__ void warp_rates(const DevMech &ms, const HeavyLane<NS, NR> &hl,
-                                           const HeavyTablesT<NS, NR> &tt, HeavyScratch &x, double T, double inv,
-                                           double lnT, const double (&mc)[NS], int lane, double &Pl, double &Ql,
-                                           double &Wl)
-{
-    const TPow p = make_tpow_known(T, inv, lnT);
-    const double invRT = inv * (1.0 / kRUniv);
-    const int sl = lane < NS ? lane : 0;
-    const double egl = exp((h_species<NS>(ms, p, kRUniv, sl) - s_species<NS>(ms, p, kRUniv, sl) * T) * invRT);
-    x.eg[lane] = egl;
-    x.ieg[lane] = rcp_nr(egl);
-    x.mc[lane] = lane_pick<NS>(mc, sl);
-    const double invRuT = inv * (1.0 / kRuCal);
-    const double rt_p0 = (kRUniv * T) / (kP0 * 1e-6);
-    const double p0_rt = rcp_nr(rt_p0);
-    double rrf = 1.0, rrb = 1.0, kc_inv = 1.0, rtb = 0.0;
-    const double b = hl.bf;
-    // Every candidate is formed before it is chosen, so the choices are
-    // selects: a conditional whose arms compute is a branch, and the lanes,
-    // holding different reactions and species, diverge on it.
-    const double kf_exp = hl.af * exp(b * p.lnT - hl.eaf * invRuT);
-    double tpow = 1.0;
-    tpow = b == 1.0 ? T : tpow;
-    tpow = b == -1.0 ? p.inv : tpow;
-    tpow = b == -2.0 ? p.inv2 : tpow;
-    const double kf_pow = hl.af * tpow;
-    const double kf = (hl.eaf == 0.0 && (b == 0.0 || b == 1.0 || b == -1.0 || b == -2.0)) ? kf_pow : kf_exp;
-#pragma unroll
-    for (int s = 0; s < NS; ++s) rtb += mc[s] * tt.tb[s][lane];
-    __syncwarp();
-    // a fixed count without branches: every entry's loads issue together
-#pragma unroll
-    for (int i = 0; i < NS; ++i) {
-        const unsigned e = tt.rent[i][lane];
-        const int s = int(e & 15u), fi = int((e >> 4) & 3u), bi = int(e >> 6);
-        const double m = x.mc[s], eg = x.eg[s], ieg = x.ieg[s];
-        const double m2 = m * m, eg2 = eg * eg, ieg2 = ieg * ieg;
-        double ff = fi == 1 ? m : 1.0, fb = bi == 1 ? m : 1.0;
-        ff = fi == 2 ? m2 : ff;
-        fb = bi == 2 ? m2 : fb;
-        rrf *= ff;
-        rrb *= fb;
-        const int d = bi - fi;
-        double fk = d == 1 ? eg : 1.0;
-        fk = d == -1 ? ieg : fk;
-        fk = d == 2 ? eg2 : fk;
-        fk = d == -2 ? ieg2 : fk;
-        kc_inv *= fk;
-    }
-    const double Xr = hl.xr;
-    kc_inv *= (Xr == 0.0 ? 1.0 : Xr == 1.0 ? rt_p0 : p0_rt);
-    if (rtb == 0.0)
-        rtb = 1.0;
-    const bool real = lane < NR; // slot 31 (and every slot past NR) holds zero rates
-    x.fwd[lane] = real ? kf * rrf : 0.0;
-    x.bwd[lane] = real ? kf * kc_inv * rrb : 0.0;
-    x.rtb[lane] = real ? rtb : 0.0;
-    __syncwarp();
-    double P = 0.0, Q = 0.0, W = 0.0;
-#pragma unroll
-    for (int i = 0; i < NR; ++i) {
-        const int q = tt.sent[i][lane];
-        const double bb = tt.sbv[i][lane], f = tt.sfv[i][lane];
-        const double fr = x.fwd[q], br = x.bwd[q], tr = x.rtb[q];
-        W += (bb - f) * tr * (fr - br);
-        Q += (bb * fr + f * br) * tr;
-        P += (bb * br + f * fr) * tr;
-    }
-    __syncwarp(); // the buffers are free for the next evaluation
-    Pl = P;
-    Ql = Q;
-    Wl = hl.mw * W;
-}
-
-// The scaled concentrations of a deferred cell: one multiplication by
-// 1e-3 / W_s per species instead of a division (within rounding of
-// scaled_concentrations).
-template <int NS, int NR>
-__device__ __forceinline__ void heavy_concentrations(const DevMech &m, const HeavyTablesT<NS, NR> &tt,
-                                                     const CellState<NS> &c, double (&mc)[NS])
-{
-#ifdef EU_EXACT_CHEM
-    scaled_concentrations<NS>(m, c, mc);
-#else
-#pragma unroll
-    for (int s = 0; s < NS; ++s) mc[s] = c.cs[s] * tt.imw[s];
-#endif
-}
-
-// One deferred cell advanced by a whole warp: lane r evaluates reaction r,
-// lane s owns species s's sums and trapezoid update, every lane rebuilds the
-// state (ms: the mechanism tables in shared memory; hl, tt, x: see
-// warp_rates).
-template <int NS, int NR>
-__device__ __forceinline__ void react_heavy_cell(const DevMech &m, const DevMech &ms, const HeavyLane<NS, NR> &hl,
-                                                 const HeavyTablesT<NS, NR> &tt, HeavyScratch &x, const DevState &st,
-                                                 long long n3, long long c, double dtm, int max_substeps, int lane)
-{
-    CellState<NS> cell;
-    load_recovered<NS>(st, n3, c, cell);
-    // 1/T and log T of the current temperature, carried through the substeps
-    // by the rebuild's Newton
-    double inv = rcp_nr(cell.T), lnT = log(cell.T);
-    double mc[NS], P, Q, W;
-    heavy_concentrations<NS, NR>(m, tt, cell, mc);
-    warp_rates<NS, NR>(ms, hl, tt, x, cell.T, inv, lnT, mc, lane, P, Q, W);
-    // prediction: min over the species lanes, then every lane has Nchem
-    double dt = dtm;
-    if (lane < NS && lane_pick<NS>(cell.Y, lane) >= 1e-6 && W != 0)
-        dt = fmin(dt, fabs(-(lane_pick<NS + 4>(cell.cs, lane) * 1e-3) / W));
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) dt = fmin(dt, __shfl_xor_sync(0xffffffffu, dt, o));
-    int nchem = 0;
-    if (lane == 0) {
-        nchem = nchem_from_dt(dtm, dt, max_substeps, st.counters);
-        count_nchem(st.counters, nchem);
-    }
-    nchem = __shfl_sync(0xffffffffu, nchem, 0);
-    const double dts = dtm / nchem, half = dts / 2.0;
-    for (int step = 0; step < nchem; ++step) {
-        if (step > 0) {
-            heavy_concentrations<NS, NR>(m, tt, cell, mc);
-            warp_rates<NS, NR>(ms, hl, tt, x, cell.T, inv, lnT, mc, lane, P, Q, W);
-        }
-        if (st.cms && lane < NS)
-            st.cms[lane * n3 + c] = W * 1e3;
-        double nd = 0.0;
-        if (lane < NS) {
-            const double di = lane_pick<NS + 4>(cell.cs, lane) * 1e-3;
-            const double mcl = lane_pick<NS>(mc, lane);
-            const double qv = hl.mw * Q;
-#ifdef EU_EXACT_CHEM
-            const double pv = (mcl == 0) ? 0.0 : P / mcl;
-            nd = ((1.0 - half * pv) * di + dts * qv) / (1.0 + half * pv) * 1e3;
-#else
-            // refined reciprocals instead of IEEE divisions (1 + half pv >= 1);
-            // the reciprocal formed before the choice (a select, not a branch)
-            const double pq = P * rcp_nr(mcl);
-            const double pv = (mcl == 0) ? 0.0 : pq;
-            nd = ((1.0 - half * pv) * di + dts * qv) * rcp_nr(1.0 + half * pv) * 1e3;
-#endif
-        }
-        double D = 0.0;
-#pragma unroll
-        for (int s = 0; s < NS; ++s) {
-            cell.cs[s] = __shfl_sync(0xffffffffu, nd, s);
-            D += cell.cs[s];
-        }
-        cell.cs[NS + 0] = cell.U * D;
-        cell.cs[NS + 1] = cell.V * D;
-        cell.cs[NS + 2] = cell.W * D;
-        cell.cs[NS + 3] = D * cell.E + 0.5 * (cell.U * cell.U + cell.V * cell.V + cell.W * cell.W) * D;
-#ifdef EU_EXACT_CHEM
-        recover_state<NS>(m, cell);
-        inv = 1.0 / cell.T;
-        lnT = log(cell.T);
-#else
-        recover_state_carry<NS>(m, cell, inv, lnT);
-#endif
-    }
-    if (lane == 0) {
-        st.nchem[c] = nchem;
-        store_cell<NS>(m, st, n3, c, cell);
-    }
-    __syncwarp();
-}
-
-__device__ __forceinline__ void copy_mech_to_shared(const DevMech &m, DevMech &ms)
-{
-    const int *src = reinterpret_cast<const int *>(&m);
-    int *dst = reinterpret_cast<int *>(&ms);
-    for (int w = threadIdx.x; w < int(sizeof(DevMech) / sizeof(int)); w += blockDim.x) dst[w] = src[w];
-}
-
-// The block's tables of the warp-per-cell kinetics: the mechanism and its
-// per-reaction tables transposed. Blocks are 128 threads: four warps, four
-// exchange buffers.
-template <int NS, int NR>
-struct HeavyShared {
-    DevMech ms;
-    HeavyTablesT<NS, NR> tt;
-    HeavyScratch x[4];
-};
-
-__device__ __forceinline__ unsigned coef2(double v) { return v <= 0.0 ? 0u : v <= 1.0 ? 1u : 2u; }
-
-template <int NS, int NR>
-__device__ __forceinline__ void heavy_shared_setup(const DevMech &m, HeavyShared<NS, NR> &sh)
-{
-    static_assert(NS <= 16 && NR <= 32, "4-bit species and 5-bit reaction indices");
-    copy_mech_to_shared(m, sh.ms);
-    HeavyTablesT<NS, NR> &t = sh.tt;
-    for (int i = threadIdx.x; i < NS * 32; i += blockDim.x) {
-        const int sp = i / 32, r = i % 32, rr = r < NR ? r : 0;
-        t.tb[sp][r] = m.tb[rr][sp];
-    }
-    if (threadIdx.x < NS)
-        t.imw[threadIdx.x] = 1e-3 / m.mw[threadIdx.x];
-    if (threadIdx.x < 32) { // lane l's lists
-        const int l = threadIdx.x, r = l < NR ? l : 0, sp = l < NS ? l : 0;
-        int n = 0;
-        for (int s = 0; s < NS; ++s) {
-            const unsigned fi = coef2(m.sf[r][s]), bi = coef2(m.sb[r][s]);
-            if (fi | bi)
-                t.rent[n++][l] = (unsigned char)(s | fi << 4 | bi << 6);
-        }
-        for (; n < NS; ++n) t.rent[n][l] = 0;
-        n = 0;
-        for (int q = 0; q < NR; ++q) {
-            const double bb = m.sb[q][sp], f = m.sf[q][sp];
-            if (bb != 0.0 || f != 0.0) {
-                t.sent[n][l] = (unsigned char)q;
-                t.sbv[n][l] = bb;
-                t.sfv[n][l] = f;
-                ++n;
-            }
-        }
-        for (; n < NR; ++n) {
-            t.sent[n][l] = 31;
-            t.sbv[n][l] = 0.0;
-            t.sfv[n][l] = 0.0;
-        }
-    }
-}
-
-// The order in which the warps of a persistent grid take deferred cells:
-// position p of n is entry p * s mod n, s near 0.618 n and coprime with n (a
-// bijection of [0, n)). The queue holds the cells in about the order the
-// recovery met them, so neighbouring cells, whose stiffness is alike, sit
-// next to each other; the warps that start together belong to few blocks,
-// and without the scatter the stiffest cells would share a few SMs.
-__device__ __forceinline__ long long scatter_stride(long long n)
-{
-    long long s = static_cast<long long>(0.6180339887498949 * double(n)) | 1;
-    for (;;) {
-        long long a = s, b = n;
-        while (b != 0) {
-            const long long t = a % b;
-            a = b;
-            b = t;
-        }
-        if (a == 1)
-            return s;
-        s += 2;
-    }
-}
-
-template <int NS, int NR>
-__global__ void __launch_bounds__(128, 3) k_react_heavy(const __grid_constant__ DevMech m, const DevGrid g,
-                                                     const DevState st, const double *__restrict__ dt_dev,
-                                                     int max_substeps)
-{
-    __shared__ HeavyShared<NS, NR> sh;
-    const int count = st.heavy[0];
-    if (count == 0) // no deferred cell this step: skip the table copy
-        return;
-    heavy_shared_setup<NS, NR>(m, sh);
-    __syncthreads();
-    const int lane = threadIdx.x & 31;
-    const HeavyLane<NS, NR> hl = heavy_lane<NS, NR>(sh.ms, lane);
-    HeavyScratch &x = sh.x[threadIdx.x / 32];
-    const double dtm = *dt_dev;
-    const long long stride = scatter_stride(count);
-    for (;;) {
-        int q = 0;
-        if (lane == 0)
-            q = atomicAdd(&st.heavy[1], 1);
-        q = __shfl_sync(0xffffffffu, q, 0);
-        if (q >= count)
-            break;
-        const int e = int((q * stride) % count);
-        react_heavy_cell<NS, NR>(m, sh.ms, hl, sh.tt, x, st, g.n3, st.heavy[2 + e], dtm, max_substeps, lane);
-    }
-}
-
-// The deferred cells of every instance of a batch, their heavy queues taken
-// end to end, drained by one persistent grid (one warp per cell, one counter).
-template <int NS, int NR>
-__global__ void __launch_bounds__(128, 3) k_react_heavy_batch(const __grid_constant__ DevMech m,
-                                                           const BatchCell *__restrict__ tab, int n, int *next,
-                                                           int max_substeps)
-{
-    __shared__ HeavyShared<NS, NR> sh;
-    auto len = [&](int q) { return tab[q].st.heavy ? *(volatile const int *)tab[q].st.heavy : 0; };
-    int total = 0;
-    for (int q = 0; q < n; ++q) total += len(q);
-    if (total == 0)
-        return;
-    heavy_shared_setup<NS, NR>(m, sh);
-    __syncthreads();
-    const int lane = threadIdx.x & 31;
-    const HeavyLane<NS, NR> hl = heavy_lane<NS, NR>(sh.ms, lane);
-    HeavyScratch &x = sh.x[threadIdx.x / 32];
-    const long long stride = scatter_stride(total);
-    for (;;) {
-        int pos = 0;
-        if (lane == 0)
-            pos = atomicAdd(next, 1);
-        pos = __shfl_sync(0xffffffffu, pos, 0);
-        if (pos >= total)
-            break;
-        int local = 0;
-        const int q = batch_locate(n, int((pos * stride) % total), len, local);
-        if (q < n) {
-            const BatchCell &b = tab[q];
-            react_heavy_cell<NS, NR>(m, sh.ms, hl, sh.tt, x, b.st, b.n3, b.st.heavy[2 + local], *b.dt, max_substeps,
-                                     lane);
         }
     }
 }
@@ -1592,19 +1240,14 @@ __global__ void k_state_from_tpy(const __grid_constant__ DevMech m, long long n,
     E[i] = e * 1000;
 }
 
-// One chemistry step (react_cell) of each sample with its own dt, in place.
-template <int NS, class Rt>
-__global__ void __launch_bounds__(128) k_chem_samples(const __grid_constant__ DevMech m, long long n, double *cs,
-                                                      double *T, double *E, const double *__restrict__ dt,
-                                                      int *nchem, int max_substeps, unsigned long long *counters)
+// A sample's state (planes of n values) and back.
+template <int NS>
+__device__ __forceinline__ void load_sample(long long n, long long i, const double *cs, const double *T, const double *E,
+                                            CellState<NS> &cell)
 {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n)
-        return;
-    CellState<NS> cell;
 #pragma unroll
     for (int q = 0; q < NS + 4; ++q) cell.cs[q] = cs[q * n + i];
-    cell.T = T[i];
+    load_temperature<NS>(cell, T[i]);
     cell.E = E[i];
     double D = 0;
 #pragma unroll
@@ -1615,14 +1258,51 @@ __global__ void __launch_bounds__(128) k_chem_samples(const __grid_constant__ De
     cell.U = cell.cs[NS] / D;
     cell.V = cell.cs[NS + 1] / D;
     cell.W = cell.cs[NS + 2] / D;
-    const int nc = react_cell<NS, Rt>(m, cell, dt[i], max_substeps, counters, nullptr, 0);
-    if (nchem)
-        nchem[i] = nc;
+}
+
+template <int NS>
+__device__ __forceinline__ void store_sample(long long n, long long i, double *cs, double *T, double *E,
+                                             const CellState<NS> &cell)
+{
 #pragma unroll
     for (int q = 0; q < NS + 4; ++q) cs[q * n + i] = cell.cs[q];
     T[i] = cell.T;
     E[i] = cell.E;
 }
+
+// One chemistry step of each sample with its own dt, in place; samples of a
+// large Nchem are left to k_chem_heavy (heavy = {count, next, samples...}, null:
+// every sample on its own thread).
+template <int NS, class Rt>
+__global__ void __launch_bounds__(128) k_chem_samples(const __grid_constant__ DevMech m, long long n, double *cs,
+                                                      double *T, double *E, const double *__restrict__ dt,
+                                                      int *nchem, int max_substeps, unsigned long long *counters,
+                                                      int *heavy)
+{
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n)
+        return;
+    CellState<NS> cell;
+    load_sample<NS>(n, i, cs, T, E, cell);
+    double mc[NS];
+    SpeciesRates<NS> rates;
+    bool bad;
+    const int nc = predict_nchem<NS, Rt>(m, cell, dt[i], max_substeps, bad, mc, rates);
+    if (heavy && nc > kHeavyNchem) {
+        push_heavy(heavy, i);
+        return;
+    }
+    count_nchem(counters, nc, bad);
+    ThermoCache<NS> tcache;
+    run_substeps<NS, Rt>(m, cell, dt[i], nc, mc, rates, nullptr, 0, tcache);
+    if (nchem)
+        nchem[i] = nc;
+    store_sample<NS>(n, i, cs, T, E, cell);
+}
+
+// ------------------------------------------------- warp-per-cell kinetics
+
+#include "eu3d_heavy.cuh"
 
 // Derived output fields of Update_after_CS that the timestep does not keep
 // (Wav, Rgas, Cp, C, Ma; src/Flowfield.cpp:1606-1616), from the stored state.

@@ -236,17 +236,20 @@ cudaError_t state_from_tpy_t(const LaunchArgs &a, long long n, const double *T, 
 
 template <int NS, int NR>
 cudaError_t chem_samples_t(const LaunchArgs &a, long long n, double *cs, double *T, double *E, const double *dt,
-                           int *nchem)
+                           int *nchem, int *heavy)
 {
     if (n <= 0)
         return cudaSuccess;
     const dim3 grid(unsigned((n + 127) / 128));
     if (a.spec == 1 && NS == Mech_JA919::NS && NR == Mech_JA919::NR)
         k_chem_samples<NS, Mech_JA919><<<grid, 128, 0, a.stream>>>(*a.mech, n, cs, T, E, dt, nchem, a.max_substeps,
-                                                                   a.st.counters);
+                                                                   a.st.counters, heavy);
     else
         k_chem_samples<NS, TableRates<NS, NR>><<<grid, 128, 0, a.stream>>>(*a.mech, n, cs, T, E, dt, nchem,
-                                                                           a.max_substeps, a.st.counters);
+                                                                           a.max_substeps, a.st.counters, heavy);
+    if (heavy) // one warp a deferred sample, at most a warp for each
+        k_chem_heavy<NS, NR><<<dim3(unsigned(std::min<long long>((n + 3) / 4, queue_grid(a, kHeavyBlocksPerSm)))), 128,
+                               0, a.stream>>>(*a.mech, n, cs, T, E, dt, nchem, a.max_substeps, a.st.counters, heavy);
     return cudaGetLastError();
 }
 
@@ -322,9 +325,9 @@ cudaError_t launch_state_from_tpy(const LaunchArgs &a, long long n, const double
     EU3D_DISPATCH(state_from_tpy_t, a, n, T, p, Y, cs, E)
 }
 cudaError_t launch_chem_samples(const LaunchArgs &a, long long n, double *cs, double *T, double *E, const double *dt,
-                                int *nchem)
+                                int *nchem, int *heavy)
 {
-    EU3D_DISPATCH(chem_samples_t, a, n, cs, T, E, dt, nchem)
+    EU3D_DISPATCH(chem_samples_t, a, n, cs, T, E, dt, nchem, heavy)
 }
 
 cudaError_t launch_react_heavy(const LaunchArgs &a, int blocks) { EU3D_DISPATCH(heavy_t, a, blocks) }

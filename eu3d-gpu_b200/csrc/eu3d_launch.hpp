@@ -62,7 +62,7 @@ struct Launchers {
     cudaError_t launch_state_from_tpy(const LaunchArgs &a, long long n, const double *T,           \
                                       const double *p, const double *Y, double *cs, double *E);    \
     cudaError_t launch_chem_samples(const LaunchArgs &a, long long n, double *cs, double *T,       \
-                                    double *E, const double *dt, int *nchem);                      \
+                                    double *E, const double *dt, int *nchem, int *heavy);                      \
     cudaError_t launch_react_heavy(const LaunchArgs &a, int blocks);                               \
     cudaError_t launch_react_queue_batch(const LaunchArgs &a, const BatchCell *tab, int n, int *next, \
                                          int counter);                                             \

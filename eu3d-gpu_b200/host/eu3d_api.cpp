@@ -54,6 +54,10 @@ struct eu_handle {
     long long lp_capacity = 0;
     int *h_counts = nullptr; // pinned [2]
     int heavy_blocks = 0;    // persistent grid of the warp-per-cell kinetics
+    bool heavy_fits = false; // whether the mechanism has that form
+    int *heavy_queue = nullptr;
+    int *sample_queue = nullptr; // eu_chem_advance's deferred samples (grown with the calls, kept)
+    long long sample_capacity = 0;
     // mixed precision: the timestep keeps only the FP32 primitive planes
     // current; the FP64 ones are formed on demand (k_materialize) for output
     bool prim_stale = false;
@@ -189,9 +193,22 @@ eu_status install_mechanism(eu_handle *h, const MechanismTables &m)
     if (!nu_int)
         return fail(h, EU_ERR_UNSUPPORTED, "stoichiometric coefficients other than 0, 1, 2 are not supported");
     d.nu_int = nu_int;
+    // the warp-per-cell kinetics' tables hold reactions of at most three molecules
+    // a side whose sides differ by at most one; other mechanisms' cells all run
+    // on a thread each
+    h->heavy_fits = true;
+    for (int r = 0; r < m.nr; ++r) {
+        double f = 0, b = 0;
+        for (int s = 0; s < m.ns; ++s) {
+            f += d.sf[r][s];
+            b += d.sb[r][s];
+        }
+        h->heavy_fits &= f <= 3 && b <= 3 && std::fabs(f - b) <= 1;
+    }
+    h->st.heavy = h->heavy_fits ? h->heavy_queue : nullptr;
     const bool first = !h->has_mech;
-    h->spec = matches_JA919(m.ns, m.nr, m.mw.data(), m.coeff_lo.data(), m.coeff_hi.data(), m.af.data(), m.bf.data(),
-                            m.eaf.data(), m.stoi_f.data(), m.stoi_b.data(), m.tb.data())
+    h->spec = matches_JA919(m.ns, m.nr, m.af.data(), m.bf.data(), m.eaf.data(), m.stoi_f.data(), m.stoi_b.data(),
+                            m.tb.data())
                   ? 1
                   : 0;
     h->mech = m;
@@ -216,9 +233,10 @@ eu_status install_mechanism(eu_handle *h, const MechanismTables &m)
         if ((s = dalloc(h, &h->st.cms, size_t(ns) * n3)) != EU_OK) return s;
     if ((s = dalloc(h, &h->st.counters, size_t(kCntCount))) != EU_OK) return s;
     if ((s = dalloc(h, &h->d_scratch, size_t(n3))) != EU_OK) return s;
-    if (h->cfg.precision == EU_PREC_MIXED) {
-        if ((s = dalloc(h, &h->st.heavy, size_t(2) + size_t(h->ni) * h->nj * h->nk)) != EU_OK) return s;
-        CK(h, cudaMemsetAsync(h->st.heavy, 0, 2 * sizeof(int), h->stream));
+    if (h->cfg.chemistry != EU_CHEM_FROZEN) {
+        if ((s = dalloc(h, &h->heavy_queue, size_t(2) + size_t(h->ni) * h->nj * h->nk)) != EU_OK) return s;
+        CK(h, cudaMemsetAsync(h->heavy_queue, 0, 2 * sizeof(int), h->stream));
+        h->st.heavy = h->heavy_fits ? h->heavy_queue : nullptr;
     }
     CK(h, cudaMemsetAsync(h->st.prim, 0, size_t(7 + ns) * n3 * sizeof(double), h->stream));
     if (h->st.prim32)
@@ -529,6 +547,7 @@ eu_status eu_destroy(eu_handle *h)
         cudaStreamSynchronize(h->stream);
     drop_graph(h);
     free_all(h);
+    if (h->sample_queue) cudaFree(h->sample_queue);
     if (h->d_snap) cudaFree(h->d_snap);
     if (h->h_snap) cudaFreeHost(h->h_snap);
     if (h->ev_snap) cudaEventDestroy(h->ev_snap);
@@ -864,6 +883,12 @@ void element_projector(const MechanismTables &m, double (&P)[kMaxS][kMaxS])
         }
 }
 
+// Whether the stiff fallback of the learned mode hands its long substep chains
+// to the warp-per-cell kinetics. In FP64 only the cells of the recovery and the
+// routing are handed over (inside the instance's own branch of a batch), so a
+// batch's shared stage holds one launch for an FP64 flavour.
+bool defers_fallback(const eu_handle *h) { return h->cfg.precision == EU_PREC_MIXED; }
+
 // One learned-chemistry phase of a step: recover + classify every cell,
 // features of the queued cells, the ensemble, gate + apply, stiff fallback.
 // The queue kernels read the queue lengths on the device; with the model's
@@ -910,7 +935,10 @@ eu_status learned_chemistry(eu_handle *h, const LaunchArgs &a, const Launchers &
     CK(h, L.learned_apply(a, lp));
     ++*launches;
     if (fallback) {
-        CK(h, L.react_queue(a, lp.fallback, lp.counts + 1, kCntFallback));
+        LaunchArgs f = a;
+        if (!defers_fallback(h))
+            f.st.heavy = nullptr;
+        CK(h, L.react_queue(f, lp.fallback, lp.counts + 1, kCntFallback));
         ++*launches;
     }
     return EU_OK;
@@ -974,7 +1002,7 @@ eu_status step_launches(eu_handle *h, const LaunchArgs &a, const Launchers &L, b
         CK(h, L.recover_react(a, react));
         ++*launches;
     }
-    if (heavy && !shared_tail) { // warp-per-cell kinetics of the cells deferred above
+    if (heavy && !(shared_tail && defers_fallback(h))) { // warp-per-cell kinetics of the cells deferred above
         CK(h, L.react_heavy(a, h->heavy_blocks));
         ++*launches;
     }
@@ -1039,7 +1067,19 @@ eu_status eu_chem_advance(eu_handle *h, long long n, double *cs, double *T, doub
     cudaSetDevice(h->cfg.device);
     LaunchArgs a = launch_args(h);
     CK(h, cudaMemsetAsync(h->st.counters, 0, kCntCount * sizeof(unsigned long long), h->stream));
-    CK(h, strict::launch_chem_samples(a, n, cs, T, E, dt, nchem));
+    if (h->heavy_fits && n < (1LL << 31)) {
+        if (h->sample_capacity < n) {
+            if (h->sample_queue)
+                CK(h, cudaFree(h->sample_queue));
+            h->sample_queue = nullptr;
+            h->sample_capacity = 0;
+            CK(h, cudaMalloc(&h->sample_queue, (size_t(2) + size_t(n)) * sizeof(int)));
+            h->sample_capacity = n;
+        }
+        CK(h, cudaMemsetAsync(h->sample_queue, 0, 2 * sizeof(int), h->stream));
+    }
+    CK(h, strict::launch_chem_samples(a, n, cs, T, E, dt, nchem,
+                                      h->heavy_fits && n < (1LL << 31) ? h->sample_queue : nullptr));
     unsigned long long cnt[kCntCount];
     CK(h, cudaMemcpyAsync(cnt, h->st.counters, sizeof cnt, cudaMemcpyDeviceToHost, h->stream));
     CK(h, cudaStreamSynchronize(h->stream));
@@ -1880,7 +1920,7 @@ void drop_batch_graph(eu_batch *b)
 bool needs_shared_stage(const eu_handle *h)
 {
     const bool learned = h->cfg.chemistry == EU_CHEM_LEARNED;
-    return learned || (h->st.heavy && h->cfg.chemistry == EU_CHEM_STIFF);
+    return learned || (h->st.heavy && h->cfg.chemistry == EU_CHEM_STIFF && defers_fallback(h));
 }
 
 // The shared kinetics stage: the groups' table on the device, then the
@@ -1915,7 +1955,7 @@ eu_status build_shared_stage(eu_batch *b, cudaGraph_t *out)
                 c.count = o->lp.counts + 1;
                 grp.fallback = true;
             }
-            if (o->st.heavy)
+            if (o->st.heavy && defers_fallback(o))
                 grp.heavy = true;
             else
                 c.st.heavy = nullptr;

@@ -119,20 +119,31 @@ void emit_strict(std::ostream &o, const MechanismTables &m)
 void emit_fast(std::ostream &o, const MechanismTables &m)
 {
     const int ns = m.ns, nr = m.nr;
-    o << "    double eg[" << ns << "], ieg[" << ns << "], Gs[" << ns << "];\n"
-      << "    const TPow p = make_tpow(T, true);\n"
-      << "    const double invRT = 1.0 / (kRUniv * T);\n"
-      << "    gibbs_all<" << ns << ">(m, p, T, Gs);\n"
-      << "#pragma unroll\n"
-      << "    for (int s = 0; s < " << ns << "; ++s) {\n"
-      << "        const double g = Gs[s] * invRT;\n"
-      << "        eg[s] = exp(g);\n"
-      << "        ieg[s] = exp(-g);\n"
-      << "    }\n"
-      << "    const double invRuT = 1.0 / (kRuCal * T);\n"
-      << "    const double rt_p0 = (kRUniv * T) * " << hex(1.0 / (101325.0 * 1e-6)) << ";\n"
-      << "#pragma unroll\n"
-      << "    for (int s = 0; s < " << ns << "; ++s) { k.P[s] = 0.0; k.Q[s] = 0.0; k.W[s] = 0.0; }\n";
+    o << "    double g[" << ns << "], eg[" << ns << "], ieg[" << ns << "];\n"
+      << "    gibbs_rt<" << ns << ">(m, T, inv, lnT, g);\n";
+    for (int sp = 0; sp < ns; ++sp) {
+        bool used = false;
+        for (int r = 0; r < nr; ++r) used |= m.stoi_f[sp * nr + r] != m.stoi_b[sp * nr + r];
+        if (used)
+            o << "    eg[" << sp << "] = exp_fast(g[" << sp << "]);\n    ieg[" << sp << "] = rcp_nr(eg[" << sp << "]);\n";
+    }
+    o << "    const double invRuT = inv * (1.0 / kRuCal), inv2 = inv * inv;\n"
+      << "    const double rt_p0 = T * (kRUniv / (kP0 * 1e-6)), p0_rt = inv * (kP0 * 1e-6 / kRUniv);\n"
+      << "    (void)inv2;\n    (void)rt_p0;\n    (void)p0_rt;\n";
+    // third-body sums: every species once, then the efficiencies' differences
+    // from 1 (where that is the shorter form)
+    bool total = false;
+    for (int r = 0; r < nr; ++r) {
+        int ones = 0;
+        for (int sp = 0; sp < ns; ++sp) ones += m.tb[sp * nr + r] == 1.0;
+        total |= 2 * ones > ns;
+    }
+    if (total) {
+        o << "    double mtot = mc[0];\n";
+        for (int sp = 1; sp < ns; ++sp) o << "    mtot += mc[" << sp << "];\n";
+    }
+    o << "#pragma unroll\n"
+      << "    for (int s = 0; s < " << ns << "; ++s) { k.P[s] = 0.0; k.Q[s] = 0.0; }\n";
     for (int r = 0; r < nr; ++r) {
         o << "    { // reaction " << r + 1 << "\n";
         std::string rrf = "1.0", rrb = "1.0", kc = "1.0";
@@ -154,16 +165,19 @@ void emit_fast(std::ostream &o, const MechanismTables &m)
             if (!fac.empty()) kc = (kc == "1.0") ? fac : kc + " * " + fac;
         }
         if (xr == 1.0) kc += " * rt_p0";
-        else if (xr == -1.0) kc += " / rt_p0";
+        else if (xr == -1.0) kc += " * p0_rt";
         else if (xr != 0.0) kc += " * pow(rt_p0, " + hex(xr) + ")";
         o << "        const double rrf = " << rrf << ";\n";
         o << "        const double rrb = " << rrb << ";\n";
         bool has_tb = false;
         for (int s = 0; s < ns; ++s) has_tb |= m.tb[s * nr + r] != 0.0;
         if (has_tb) {
-            o << "        double rtb = 0.0;\n";
+            int ones = 0;
+            for (int s = 0; s < ns; ++s) ones += m.tb[s * nr + r] == 1.0;
+            const double base = 2 * ones > ns ? 1.0 : 0.0;
+            o << "        double rtb = " << (base == 1.0 ? "mtot" : "0.0") << ";\n";
             for (int s = 0; s < ns; ++s) {
-                const double e = m.tb[s * nr + r];
+                const double e = m.tb[s * nr + r] - base;
                 if (e != 0.0) o << "        rtb = fma(mc[" << s << "], " << hex(e) << ", rtb);\n";
             }
             o << "        if (rtb == 0.0) rtb = 1.0;\n";
@@ -173,15 +187,16 @@ void emit_fast(std::ostream &o, const MechanismTables &m)
         const double A = m.af[r], b = m.bf[r], E = m.eaf[r];
         std::string kf;
         if (E == 0.0 && (b == 0.0 || b == 1.0 || b == -1.0 || b == -2.0)) {
-            const char *tp = b == 0.0 ? "1.0" : b == 1.0 ? "T" : b == -1.0 ? "p.inv" : "p.inv2";
+            const char *tp = b == 0.0 ? "1.0" : b == 1.0 ? "T" : b == -1.0 ? "inv" : "inv2";
             kf = hex(A) + " * " + tp;
+        } else if (b == 0.0) {
+            kf = hex(A) + " * exp_fast(" + hex(-E) + " * invRuT)";
         } else {
-            kf = hex(A) + " * exp(" + hex(b) + " * p.lnT - " + hex(E) + " * invRuT)";
+            kf = hex(A) + " * exp_fast(" + hex(b) + " * lnT - " + hex(E) + " * invRuT)";
         }
         o << "        const double kf = " << kf << ";\n";
         o << "        const double kb = kf * (" << kc << ");\n";
         o << "        const double fwd = kf * rrf, bwd = kb * rrb;\n";
-        o << "        const double rrt = (fwd - bwd) * rtb;\n";
         o << "        const double fr = fwd * rtb, br = bwd * rtb;\n";
         for (int s = 0; s < ns; ++s) {
             const double f = m.stoi_f[s * nr + r], bb = m.stoi_b[s * nr + r];
@@ -190,8 +205,6 @@ void emit_fast(std::ostream &o, const MechanismTables &m)
                 if (c == 1.0) return v;
                 return hex(c) + " * " + v;
             };
-            const double d = bb - f;
-            if (d != 0.0) o << "        k.W[" << s << "] = fma(" << hex(d) << ", rrt, k.W[" << s << "]);\n";
             std::string q, pl;
             if (bb != 0.0) q = scaled(bb, "fr");
             if (f != 0.0) q = q.empty() ? scaled(f, "br") : q + " + " + scaled(f, "br");
@@ -202,7 +215,6 @@ void emit_fast(std::ostream &o, const MechanismTables &m)
         }
         o << "    }\n";
     }
-    o << "#pragma unroll\n    for (int s = 0; s < " << ns << "; ++s) k.W[s] = m.mw[s] * k.W[s];\n";
 }
 
 void emit_tables(std::ostream &o, const MechanismTables &m, const std::string &name)
@@ -212,28 +224,23 @@ void emit_tables(std::ostream &o, const MechanismTables &m, const std::string &n
         for (size_t i = 0; i < v.size(); ++i) o << (i ? ", " : "") << hex(v[i]);
         o << "};\n";
     };
-    arr("mw", m.mw);
-    arr("coeff_lo", m.coeff_lo);
-    arr("coeff_hi", m.coeff_hi);
     arr("af", m.af);
     arr("bf", m.bf);
     arr("eaf", m.eaf);
     arr("stoi_f", m.stoi_f);
     arr("stoi_b", m.stoi_b);
     arr("tb", m.tb);
-    o << "\n// True when tables m are bitwise the ones this code was generated from.\n"
-      << "inline bool matches_" << name << "(int ns, int nr, const double *mw, const double *clo, const double *chi,\n"
-      << "                            const double *af, const double *bf, const double *eaf, const double *sf,\n"
-      << "                            const double *sb, const double *tb)\n{\n"
+    o << "\n// True when the reactions are bitwise the ones this code was generated from (it\n"
+      << "// reads the molecular weights and NASA coefficients from the handle's tables, so\n"
+      << "// a mechanism that differs in those alone, such as the Ar variant, uses it too).\n"
+      << "inline bool matches_" << name << "(int ns, int nr, const double *af, const double *bf, const double *eaf,\n"
+      << "                            const double *sf, const double *sb, const double *tb)\n{\n"
       << "    if (ns != " << m.ns << " || nr != " << m.nr << ") return false;\n"
       << "    auto same = [](const double *a, const double *b, int n) {\n"
       << "        for (int i = 0; i < n; ++i)\n"
       << "            if (std::memcmp(&a[i], &b[i], sizeof(double)) != 0) return false;\n"
       << "        return true;\n    };\n"
-      << "    return same(mw, k" << name << "_mw, " << m.ns << ") && same(clo, k" << name << "_coeff_lo, "
-      << 9 * m.ns << ") &&\n"
-      << "           same(chi, k" << name << "_coeff_hi, " << 9 * m.ns << ") && same(af, k" << name << "_af, " << m.nr
-      << ") &&\n"
+      << "    return same(af, k" << name << "_af, " << m.nr << ") &&\n"
       << "           same(bf, k" << name << "_bf, " << m.nr << ") && same(eaf, k" << name << "_eaf, " << m.nr
       << ") &&\n"
       << "           same(sf, k" << name << "_stoi_f, " << m.ns * m.nr << ") && same(sb, k" << name << "_stoi_b, "
@@ -267,8 +274,8 @@ int main(int argc, char **argv)
           << ". Do not edit.\n#pragma once\n#include \"eu3d_device.cuh\"\n\nnamespace eu3d {\n\n"
           << "// Rates of mechanism " << name << " (" << m.ns << " species, " << m.nr << " reactions).\n"
           << "struct Mech_" << name << " {\n    static constexpr int NS = " << m.ns << ", NR = " << m.nr << ";\n"
-          << "    __device__ __forceinline__ static void rates(const DevMech &m, double T, const double (&mc)[" << m.ns
-          << "], SpeciesRates<" << m.ns << "> &k)\n    {\n#ifdef EU_EXACT_CHEM\n";
+          << "    __device__ __forceinline__ static void rates(const DevMech &m, double T, double inv, double lnT, const double (&mc)[" << m.ns
+          << "], SpeciesRates<" << m.ns << "> &k)\n    {\n#ifdef EU_EXACT_RATES\n    (void)inv;\n    (void)lnT;\n";
         emit_strict(o, m);
         o << "#else\n";
         emit_fast(o, m);
