@@ -3,8 +3,7 @@
 //   C[M x N] = act(A[M x K] * B[N x K]^T + bias[N])
 //
 // A and B are row-major with K contiguous (both operands "K-major"); C is
-// written as fp32 and/or bf16, optionally with the pre-activation values kept
-// for a backward pass. One CTA of 128 threads computes a 128 x BN tile:
+// written as fp32 and/or bf16, optionally with the pre-activation values. One CTA of 128 threads computes a 128 x BN tile:
 // all threads stage K-slabs of 64 into shared memory with cp.async (two stages),
 // one elected thread issues the tcgen05.mma instructions (M=128, N=BN, K=16)
 // into a TMEM accumulator and commits them to the stage's mbarrier, and each
@@ -21,11 +20,9 @@ namespace eu3d {
 
 constexpr int kGemmBM = 128, kGemmBK = 64, kGemmThreads = 128;
 
-// Epilogue modes: 0 none, 1 SiLU, 2 multiply by SiLU'(Z) (backward through an
-// activation whose pre-activation Z is given), 3 accumulate into Cf with
-// atomics (split-K partial sums; no bias), 4 SiLU in its inference form
-// (silu_fast, the fused inference kernel's activation).
-enum GemmAct { kActNone = 0, kActSilu = 1, kActSiluGrad = 2, kActAccumulate = 3, kActSiluFast = 4 };
+// Epilogue modes: 0 none, 1 SiLU, 4 SiLU in its inference form (silu_fast, the
+// fused inference kernel's activation).
+enum GemmAct { kActNone = 0, kActSilu = 1, kActSiluFast = 4 };
 
 // SiLU with the hardware's approximate division (reciprocal and multiply, about
 // two units in the last place): the activations are rounded to bf16 next, eight
@@ -54,7 +51,7 @@ __device__ __forceinline__ float silu_fast_half(float h) { return fmaf(h, tanh_a
 __device__ __forceinline__ float silu_fast(float x) { return silu_fast_half(0.5f * x); }
 __device__ __forceinline__ float silu_grad(float z)
 {
-    const float s = 1.0f / (1.0f + __expf(-z));
+    const float s = __fdividef(1.0f, 1.0f + __expf(-z));
     return s * (1.0f + z * (1.0f - s));
 }
 
@@ -85,7 +82,7 @@ template <int BN>
 __global__ void __launch_bounds__(kGemmThreads, 1)
     k_gemm_bf16(const __nv_bfloat16 *__restrict__ A, int lda, const __nv_bfloat16 *__restrict__ B, int ldb, int M,
                 int N, int K, const float *__restrict__ bias, int act, float *Cf, __nv_bfloat16 *Cb, float *Cpre,
-                int ldc, const float *__restrict__ Z, int k_split, int *err)
+                int ldc, int *err)
 {
     static_assert(BN % 32 == 0 && BN >= 32 && BN <= 256, "BN");
     constexpr int BM = kGemmBM, BK = kGemmBK;
@@ -98,12 +95,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
-    // split-K: CTA z handles K slabs [kt0, kt1)
-    const int KT_all = (K + BK - 1) / BK;
-    const int per = (KT_all + k_split - 1) / k_split;
-    const int kt0 = blockIdx.z * per;
-    const int KT = max(0, min(KT_all, kt0 + per) - kt0);
-    const int kbase = kt0 * BK;
+    const int KT = (K + BK - 1) / BK;
 
     if (warp == 0) {
         tc::tmem_alloc(tslot, BN);
@@ -121,8 +113,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     bool ok = true;
 
     if (KT > 0) {
-        stage_slab<BM>(sa[0], A, lda, m0, M, kbase, K);
-        stage_slab<BN>(sb[0], B, ldb, n0, N, kbase, K);
+        stage_slab<BM>(sa[0], A, lda, m0, M, 0, K);
+        stage_slab<BN>(sb[0], B, ldb, n0, N, 0, K);
     }
     tc::cp_async_commit();
 
@@ -142,8 +134,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
                     break;
                 }
             }
-            stage_slab<BM>(sa[s1], A, lda, m0, M, kbase + (kt + 1) * BK, K);
-            stage_slab<BN>(sb[s1], B, ldb, n0, N, kbase + (kt + 1) * BK, K);
+            stage_slab<BM>(sa[s1], A, lda, m0, M, (kt + 1) * BK, K);
+            stage_slab<BN>(sb[s1], B, ldb, n0, N, (kt + 1) * BK, K);
             tc::cp_async_commit();
             tc::cp_async_wait<1>();
         } else {
@@ -184,10 +176,6 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
                     const int n = n0 + c0 + q;
                     if (n < N) {
                         const size_t o = (size_t)row * ldc + n;
-                        if (act == kActAccumulate) {
-                            atomicAdd(&Cf[o], v[q]);
-                            continue;
-                        }
                         float x = v[q] + (bias ? bias[n] : 0.0f);
                         if (Cpre)
                             Cpre[o] = x;
@@ -195,8 +183,6 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
                             x = silu(x);
                         else if (act == kActSiluFast)
                             x = silu_fast(x);
-                        else if (act == kActSiluGrad)
-                            x *= silu_grad(Z[o]);
                         if (Cf)
                             Cf[o] = x;
                         if (Cb)

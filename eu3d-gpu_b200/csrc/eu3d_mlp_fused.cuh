@@ -365,17 +365,4 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
         tc::tmem_dealloc(tmem, kFusedTmemCols);
 }
 
-// Weights of one layer, bf16 [N x K] row-major, into its K-slabs of
-// kFusedSlabK columns, each in the core-matrix layout: element (n, k) of slab s
-// at ((k' / 8) * N + n) * 8 + k' % 8, k' = k - kFusedSlabK s, slabs back to back.
-__global__ void k_pack_slabs(const __nv_bfloat16 *__restrict__ W, int N, int K, __nv_bfloat16 *__restrict__ out)
-{
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long long)N * K)
-        return;
-    const int n = int(t / K), k = int(t % K);
-    const int s = k / kFusedSlabK, kl = k % kFusedSlabK;
-    out[(long long)s * N * kFusedSlabK + ((kl / 8) * N + n) * 8 + kl % 8] = W[t];
-}
-
 } // namespace eu3d

@@ -1,8 +1,8 @@
 // eu3d_mlp_kernels.hpp — host launch interface of the learned-chemistry kernels
-// (eu3d_mlp.cu). bf16 buffers are passed as void pointers so host code needs
-// no CUDA half-precision headers.
+// (eu3d_mlp.cu).
 #pragma once
 
+#include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
 namespace eu3d {
@@ -71,25 +71,51 @@ inline int fused_grid(long long tiles, int sms)
 // member * s_mem + o]. `grid` CTAs (one per SM is the intent).
 cudaError_t mlp_fused(const FusedMlpParams &p, const float *feat, int ld_feat, int count_host, const int *count_dev,
                       int max_rows, float *out, long long s_row, long long s_mem, int *err, int grid, cudaStream_t s);
-// One layer's bf16 [N x K] weights into K-slabs (see k_pack_slabs).
-cudaError_t pack_slabs(const void *W, int N, int K, void *out, cudaStream_t s);
+
+// A training step (eu3d_mlp_train.cuh): one member's parameters (fp32 P, gradient
+// G, Adam's M and V: per layer W [out_pad x in_pad], then b), their bf16 copies
+// (row-major Wb, K-slabs of it and of its transpose) and its scratch for a batch
+// of n rows.
+constexpr int kTrainRows = 128; // rows of a tile
+// Leading dimension of the transposed arrays of an n-row batch: whole 128-byte
+// lines, one more than the batch's, so that the rows of a power-of-two batch
+// do not all start on the same memory channels.
+inline int train_ld(int n) { return (n + 63) / 64 * 64 + 64; }
+struct TrainMember {
+    float *P, *G, *M, *V;
+    const float *bias[kFusedMaxLayers];
+    float *gW[kFusedMaxLayers], *gb[kFusedMaxLayers];
+    __nv_bfloat16 *Wb[kFusedMaxLayers], *slabs[kFusedMaxLayers], *slabs_t[kFusedMaxLayers];
+    float *Z;                      // pre-activations [hidden][n x width]
+    // transposed (rows along the leading dimension ld): [in_pad], [hidden][width]
+    // twice, [out_pad]
+    __nv_bfloat16 *XT, *HT, *dZT, *dYT;
+    unsigned long long key;        // of the batch's draw
+};
+struct TrainParams {
+    int n, n_in, in_pad, width, hidden, n_out, out_pad;
+    int ld;                        // of the transposed arrays (train_ld)
+    int params;                    // padded parameters of a member
+    int first, members;            // members [first, first + members)
+    const float *X, *T;            // fp32 rows [rows x n_in], [rows x n_out]
+    long long rows;
+    bool drawn;                    // batch rows drawn at random (else the first n)
+    const float *in_shift, *in_scale, *out_shift, *out_scale;
+    float *loss;                   // [members of the model] squared errors summed
+    int *err;
+    TrainMember member[kFusedMaxMembers];
+};
+cudaError_t train_rows(const TrainParams &p, cudaStream_t s);
+cudaError_t train_weights(const TrainParams &p, int sms, cudaStream_t s);
+// lr 0: only pack the bf16 weights
+cudaError_t train_adam(const TrainParams &p, float lr, float b1, float b2, float eps, float c1, float c2, cudaStream_t s);
 
 // C = epilogue(A B^T): A (M x K), B (N x K) row-major bf16; act 0 none, 1 SiLU,
-// 2 times SiLU'(Z), 3 atomically accumulate into Cf (split-K partial sums).
+// 4 SiLU in its inference form.
 cudaError_t gemm_bf16(const void *A, int lda, const void *B, int ldb, int M, int N, int K, const float *bias, int act,
-                      float *Cf, void *Cb, float *Cpre, int ldc, const float *Z, int k_split, int *err, cudaStream_t s);
-cudaError_t transpose_bf16(const void *in, int R, int C, int ldi, void *out, int ldo, cudaStream_t s);
-cudaError_t pack_features(const float *X, long long n, int n_in, const int *rows, const float *shift,
-                          const float *scale, void *out, int ld, cudaStream_t s);
-cudaError_t mse_grad(const float *Y, int ldy, const float *T, long long n, int n_out, const int *rows,
-                     const float *shift, const float *scale, void *dY, float *loss, cudaStream_t s);
-cudaError_t colsum_f32(const float *A, long long R, int C, int lda, float *out, cudaStream_t s);
-cudaError_t colsum_bf16(const void *A, long long R, int C, int lda, float *out, cudaStream_t s);
-cudaError_t adam(float *p, const float *g, float *m, float *v, long long n, float lr, float b1, float b2, float eps,
-                 float c1, float c2, cudaStream_t s);
-cudaError_t refresh_weights(const float *W, int out, int in, int out_pad, int in_pad, void *Wb, void *Wt,
-                            cudaStream_t s);
-cudaError_t random_rows(int *rows, int count, long long n, unsigned long long key, cudaStream_t s);
+                      float *Cf, void *Cb, float *Cpre, int ldc, int *err, cudaStream_t s);
+cudaError_t pack_features(const float *X, long long n, int n_in, const float *shift, const float *scale, void *out,
+                          int ld, cudaStream_t s);
 cudaError_t unscale_outputs(const float *Y, long long n, int ld, int n_out, const float *shift, const float *scale,
                             float *out, cudaStream_t s);
 

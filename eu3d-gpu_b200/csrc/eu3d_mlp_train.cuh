@@ -1,0 +1,501 @@
+// eu3d_mlp_train.cuh — a training step of the learned-chemistry ensemble in
+// three kernels over all members: rows (forward, loss and the gradients'
+// way back to the first layer), weight gradients, Adam.
+//
+// A batch's rows are independent up to the weight gradients, so k_train_rows
+// gives each 128-row tile of each member to one CTA, which runs every layer
+// forward and back on the tensor cores with the tile's activations, and on the
+// way back its layer gradients, in shared memory as the next MMA's A operand
+// (two CTAs per SM: one's epilogue under the other's MMAs). What the weight
+// gradients need, the bf16 inputs and gradients of every layer, goes to global
+// memory transposed (rows along K), which costs no extra pass: a lane holds a
+// row, so a column's 32 values are one contiguous store. The pre-activations
+// (fp32, for SiLU') are written and read back by the same thread. k_train_dw
+// then forms every layer's dW = dZ^T H of every member in one launch, split
+// along the rows to fill the chip. k_train_adam updates the parameters, packs
+// the bf16 weights for the next step and clears the gradients.
+//
+// Rounding points are the layer-wise path's: bf16 inputs, weights, activations
+// and layer gradients, fp32 accumulation, bias gradients from the fp32 layer
+// gradients. Launched layer by layer, with transposes, column sums and
+// one-value-a-lane epilogues of their own, a step of three members at batch
+// 16384 took 3.2 ms (about 165 launches).
+#pragma once
+
+#include <cuda_bf16.h>
+
+#include "eu3d_gemm.cuh"
+#include "eu3d_mlp_kernels.hpp"
+#include "eu3d_tc.cuh"
+
+namespace eu3d {
+
+// three slabs in flight: two CTAs' shared memory then just fits an SM
+constexpr int kTrainThreads = 256, kTrainSlots = 3, kTrainSlabBytes = 256 * kFusedSlabK * 2;
+constexpr size_t kTrainSmem = size_t(kTrainRows) * 256 * 2 + kTrainSlots * kTrainSlabBytes + 64;
+
+__device__ __forceinline__ unsigned long long train_row(unsigned long long key, int i, long long n)
+{
+    // uniform index in [0, n) from a counter-based hash (splitmix64) of the key
+    // and the batch position: batches drawn on the device, no host copies
+    unsigned long long z = key + 0x9E3779B97F4A7C15ull * (unsigned long long)(i + 1);
+    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
+    z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
+    z ^= z >> 31;
+    return z % (unsigned long long)n;
+}
+
+// Sum over the warp's lanes of each of 32 values: lane q returns value q's sum.
+__device__ __forceinline__ float column_sum(float (&v)[32], int lane)
+{
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int q = 0; q < o; ++q) {
+            const bool hi = (lane & o) != 0;
+            const float send = hi ? v[q] : v[q + o], keep = hi ? v[q + o] : v[q];
+            v[q] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    return v[0];
+}
+
+// 8 bf16 of one row into an A operand (core-matrix layout).
+__device__ __forceinline__ void put_operand(unsigned char *act, int col, int row, const __nv_bfloat16 *v)
+{
+    *reinterpret_cast<uint4 *>(act + ((col / 8) * kTrainRows + row) * 16) = *reinterpret_cast<const uint4 *>(v);
+}
+
+__global__ void __launch_bounds__(kTrainThreads, 2) k_train_rows(const __grid_constant__ TrainParams p)
+{
+    extern __shared__ __align__(128) unsigned char smem[];
+    unsigned char *act = smem;                                    // [256 / 8][128][16 B]
+    unsigned char *ring = smem + kTrainRows * 256 * 2;            // weight slabs
+    uint64_t *full = reinterpret_cast<uint64_t *>(ring + kTrainSlots * kTrainSlabBytes), *empty = full + kTrainSlots;
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(empty + kTrainSlots);
+    volatile int *abort_flag = reinterpret_cast<volatile int *>(tslot + 1);
+
+    const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32, quad = warp % 4, half = warp / 4;
+    const int e = p.first + blockIdx.y;
+    const TrainMember &mem = p.member[e];
+    const int lrow = quad * 32 + lane, row = blockIdx.x * kTrainRows + lrow;
+    const bool valid = row < p.n;
+    const long long src = !valid ? 0 : p.drawn ? (long long)train_row(mem.key, row, p.rows) : row;
+    const unsigned ld = unsigned(p.ld);
+    const size_t wide = size_t(p.width) * ld, zwide = size_t(p.width) * p.n; // one layer's planes
+
+    if (warp == 0) {
+        tc::tmem_alloc(tslot, 256);
+        tc::tmem_relinquish();
+    }
+    if (tid == 0) {
+        for (int q = 0; q < kTrainSlots; ++q) {
+            tc::mbar_init(&full[q], 1);
+            tc::mbar_init(&empty[q], 1);
+        }
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    // features -> first A operand and, transposed, the first layer's input
+    for (int kc = half; kc < p.in_pad / 8; kc += 2) {
+        __align__(16) __nv_bfloat16 v[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const int c = kc * 8 + q;
+            float f = 0.0f;
+            if (valid && c < p.n_in)
+                f = (p.X[src * p.n_in + c] - p.in_shift[c]) * p.in_scale[c];
+            v[q] = __float2bfloat16_rn(f);
+            if (valid)
+                mem.XT[unsigned(c) * ld + unsigned(row)] = v[q];
+        }
+        put_operand(act, kc * 8, lrow, v);
+    }
+    tc::fence_proxy_async();
+    tc::tc_fence_before();
+    __syncthreads();
+    tc::tc_fence_after();
+    const uint32_t tmem = *tslot;
+    const uint32_t trow = tmem + (uint32_t(quad * 32) << 16);
+    const int L = p.hidden;       // hidden layers; GEMMs 0 .. L forward, then L .. 1 back
+    const int ngemm = 2 * L + 1;
+    int issued = 0, done = 0;     // weight slabs requested and consumed (thread 0)
+    bool ok = true;
+
+    // GEMM q: its weights, K and N
+    auto shape = [&](int q, const __nv_bfloat16 *&w, int &K, int &N) {
+        if (q <= L) {
+            K = q == 0 ? p.in_pad : p.width;
+            N = q == L ? p.out_pad : p.width;
+            w = mem.slabs[q];
+        } else {
+            const int l = L - (q - L - 1); // back through layer l
+            K = l == L ? p.out_pad : p.width;
+            N = p.width;
+            w = mem.slabs_t[l];
+        }
+    };
+    auto request = [&](int q, int s) { // slab s of GEMM q into the next slot
+        const __nv_bfloat16 *w;
+        int K, N;
+        shape(q, w, K, N);
+        const int slot = issued % kTrainSlots;
+        if (issued >= kTrainSlots && !tc::mbar_wait(&empty[slot], uint32_t((issued / kTrainSlots - 1) & 1)))
+            return false;
+        const uint32_t bytes = uint32_t(N) * min(kFusedSlabK, K - s * kFusedSlabK) * 2;
+        tc::mbar_arrive_expect_tx(&full[slot], bytes);
+        tc::bulk_g2s(ring + slot * kTrainSlabBytes, w + (size_t)s * N * kFusedSlabK, bytes, &full[slot]);
+        ++issued;
+        return true;
+    };
+    auto slabs_of = [&](int q) {
+        const __nv_bfloat16 *w;
+        int K, N;
+        shape(q, w, K, N);
+        return (K + kFusedSlabK - 1) / kFusedSlabK;
+    };
+
+    // 32 pre-activations of this thread's row, columns c0 ..
+    float zz[32];
+    auto load_z = [&](const float *z, int c0) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (valid && c0 + j * 4 < p.width)
+                a = *reinterpret_cast<const float4 *>(z + c0 + j * 4);
+            zz[j * 4] = a.x, zz[j * 4 + 1] = a.y, zz[j * 4 + 2] = a.z, zz[j * 4 + 3] = a.w;
+        }
+    };
+
+    for (int q = 0; q < ngemm; ++q) {
+        // the way back: the first pre-activations come while the MMAs run
+        if (q > L)
+            load_z(mem.Z + (2 * L - q) * zwide + (size_t)row * p.width, half * 32);
+        // ------------------------------------------------------------ MMAs
+        if (tid == 0) {
+            const __nv_bfloat16 *w;
+            int K, N;
+            shape(q, w, K, N);
+            const int ns = slabs_of(q), first = done;
+            const uint32_t idesc = tc::idesc_bf16_f32(kTrainRows, N);
+            bool good = true;
+            while (good && issued < first + min(ns, kTrainSlots)) good = request(q, issued - first);
+            for (int s = 0; good && s < ns; ++s) {
+                const int slot = done % kTrainSlots;
+                good = good && tc::mbar_wait(&full[slot], uint32_t((done / kTrainSlots) & 1));
+                if (!good)
+                    break;
+                tc::tc_fence_after();
+                const int kw = min(kFusedSlabK, K - s * kFusedSlabK);
+                const uint32_t a0 = tc::smem_u32(act), b0 = tc::smem_u32(ring + slot * kTrainSlabBytes);
+                for (int kk = 0; kk < kw / 16; ++kk) {
+                    const int kg = s * (kFusedSlabK / 16) + kk;
+                    tc::mma_bf16(tmem, tc::smem_desc(a0 + kg * 2 * kTrainRows * 16, kTrainRows * 16, 128),
+                                 tc::smem_desc(b0 + kk * 2 * N * 16, N * 16, 128), idesc, (s > 0 || kk > 0) ? 1u : 0u);
+                }
+                tc::mma_commit(&empty[slot]);
+                ++done;
+                // refill the slot of the MMAs before these, which run meanwhile
+                if (s >= 1 && issued < first + ns)
+                    good = request(q, issued - first);
+            }
+            // the last slab's commit follows every MMA of the GEMM
+            if (good)
+                good = tc::mbar_wait(&empty[(done - 1) % kTrainSlots], uint32_t(((done - 1) / kTrainSlots) & 1));
+            // the next GEMM's first slabs arrive under this one's epilogue
+            if (q + 1 < ngemm)
+                for (int s = 0; good && s < min(slabs_of(q + 1), kTrainSlots); ++s) good = request(q + 1, s);
+            if (!good) {
+                *abort_flag = 1;
+                atomicExch(p.err, 1);
+            }
+        }
+        __syncthreads();
+        tc::tc_fence_after();
+        if (*abort_flag) {
+            ok = false;
+            break;
+        }
+        // -------------------------------------------------------- epilogue
+        if (q < L) { // hidden layer: z, silu(z) as bf16
+            float *z = mem.Z + q * zwide + (size_t)row * p.width;
+            __nv_bfloat16 *ht = mem.HT + q * wide + row;
+            const float *bias = mem.bias[q];
+            for (int c0 = half * 32; c0 < p.width; c0 += 64) {
+                float v[32];
+                tc::tmem_ld32(trow + c0, v);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int c = c0 + j * 8;
+                    if (c < p.width) {
+                        __align__(16) __nv_bfloat16 h[8];
+                        const float4 b0 = __ldg(reinterpret_cast<const float4 *>(bias + c)),
+                                     b1 = __ldg(reinterpret_cast<const float4 *>(bias + c + 4));
+                        const float bb[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+#pragma unroll
+                        for (int u = 0; u < 8; ++u) {
+                            v[j * 8 + u] += bb[u];
+                            h[u] = __float2bfloat16_rn(silu(v[j * 8 + u]));
+                        }
+                        put_operand(act, c, lrow, h);
+                        if (valid) {
+#pragma unroll
+                            for (int u = 0; u < 8; ++u) ht[unsigned(c + u) * ld] = h[u];
+                            *reinterpret_cast<float4 *>(z + c) = make_float4(v[j * 8], v[j * 8 + 1], v[j * 8 + 2], v[j * 8 + 3]);
+                            *reinterpret_cast<float4 *>(z + c + 4) =
+                                make_float4(v[j * 8 + 4], v[j * 8 + 5], v[j * 8 + 6], v[j * 8 + 7]);
+                        }
+                    }
+                }
+            }
+        } else if (q == L) { // output: loss and its gradient
+            float sq = 0.0f;
+            for (int c0 = half * 32; c0 < p.out_pad; c0 += 64) {
+                float v[32];
+                tc::tmem_ld32(trow + c0, v);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int c = c0 + j * 8;
+                    __align__(16) __nv_bfloat16 g[8];
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) {
+                        float d = 0.0f;
+                        if (valid && c + u < p.n_out) {
+                            const float target = (p.T[src * p.n_out + c + u] - p.out_shift[c + u]) * p.out_scale[c + u];
+                            d = v[j * 8 + u] + __ldg(mem.bias[L] + c + u) - target;
+                            sq += d * d;
+                            d = 2.0f * d / float(p.n * p.n_out);
+                        }
+                        g[u] = __float2bfloat16_rn(d);
+                        v[j * 8 + u] = __bfloat162float(g[u]);
+                        if (valid && c + u < p.out_pad)
+                            mem.dYT[unsigned(c + u) * ld + unsigned(row)] = g[u];
+                    }
+                    if (c < p.out_pad)
+                        put_operand(act, c, lrow, g);
+                }
+                const float s = column_sum(v, lane);
+                if (c0 + lane < p.out_pad)
+                    atomicAdd(&mem.gb[L][c0 + lane], s);
+            }
+            for (int o = 16; o > 0; o >>= 1) sq += __shfl_down_sync(0xffffffffu, sq, o);
+            if (lane == 0 && sq != 0.0f)
+                atomicAdd(&p.loss[e], sq);
+        } else { // back through layer l into hidden layer l - 1
+            const int l = L - (q - L - 1);
+            const float *z = mem.Z + (l - 1) * zwide + (size_t)row * p.width;
+            __nv_bfloat16 *zt = mem.dZT + (l - 1) * wide + row;
+            for (int c0 = half * 32; c0 < p.width; c0 += 64) {
+                if (c0 > half * 32)
+                    load_z(z, c0);
+                float v[32];
+                tc::tmem_ld32(trow + c0, v);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int c = c0 + j * 8;
+                    __align__(16) __nv_bfloat16 g[8];
+                    // (rows past the batch have zero gradients: no loss)
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) {
+                        const float d = c < p.width ? v[j * 8 + u] * silu_grad(zz[j * 8 + u]) : 0.0f;
+                        v[j * 8 + u] = d;
+                        g[u] = __float2bfloat16_rn(d);
+                    }
+                    if (c < p.width) {
+                        if (valid) {
+#pragma unroll
+                            for (int u = 0; u < 8; ++u) zt[unsigned(c + u) * ld] = g[u];
+                        }
+                        put_operand(act, c, lrow, g);
+                    }
+                }
+                const float s = column_sum(v, lane);
+                if (c0 + lane < p.width)
+                    atomicAdd(&mem.gb[l - 1][c0 + lane], s);
+            }
+        }
+        tc::fence_proxy_async();
+        tc::tc_fence_before();
+        __syncthreads();
+        tc::tc_fence_after();
+    }
+    if (!ok && tid == 0) {
+        // copies in flight land and MMAs issued finish (bounded) before the
+        // CTA's memory goes away
+        for (int s = issued > kTrainSlots ? issued - kTrainSlots : 0; s < issued; ++s)
+            tc::mbar_wait(&full[s % kTrainSlots], uint32_t((s / kTrainSlots) & 1));
+        if (done > 0)
+            tc::mbar_wait(&empty[(done - 1) % kTrainSlots], uint32_t(((done - 1) / kTrainSlots) & 1));
+    }
+    tc::tc_fence_before();
+    __syncthreads();
+    if (warp == 0)
+        tc::tmem_dealloc(tmem, 256);
+}
+
+// dW = dZ^T H of every layer of every member: one CTA per (K split, 128-row
+// piece of a layer's outputs, member), partial sums added to the fp32 gradient
+// four values at a time. Two cp.async stages of 64 rows feed the MMAs.
+constexpr int kDwThreads = 128, kDwK = 64;
+constexpr size_t kDwSmem = 2 * size_t(128 + 256) * kDwK * 2 + 64;
+
+// rows x kDwK bf16 of a row-major matrix (rows r0.., columns k0..) into the
+// core-matrix layout of a `pitch`-row operand.
+__device__ __forceinline__ void dw_stage(unsigned char *dst, int pitch, const __nv_bfloat16 *src, int ld, int r0, int nrows,
+                                         int k0, int k1)
+{
+    for (int c = threadIdx.x; c < pitch * (kDwK / 8); c += kDwThreads) {
+        const int r = c / (kDwK / 8), kc = c % (kDwK / 8), gk = k0 + kc * 8;
+        const bool in = r0 + r < nrows && gk < k1;
+        tc::cp_async16(dst + (kc * pitch + r) * 16, in ? src + (size_t)(r0 + r) * ld + gk : src, in);
+    }
+}
+
+__global__ void __launch_bounds__(kDwThreads, 2) k_train_dw(const __grid_constant__ TrainParams p, int splits)
+{
+    extern __shared__ __align__(128) unsigned char smem[];
+    constexpr uint32_t kA = 128 * kDwK * 2, kB = 256 * kDwK * 2;
+    unsigned char *sa[2] = {smem, smem + kA + kB}, *sb[2] = {smem + kA, smem + 2 * kA + kB};
+    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + 2 * (kA + kB));
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(bars + 2);
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    const int e = p.first + blockIdx.z;
+    const TrainMember &mem = p.member[e];
+    const size_t wide = size_t(p.width) * p.ld;
+    // the job: layer l, output rows m0 ..
+    int job = blockIdx.y, l = 0;
+    const int pieces = (p.width + 127) / 128;
+    l = min(job / pieces, p.hidden);
+    const int m0 = (job - l * pieces) * 128;
+    const int M = l == p.hidden ? p.out_pad : p.width, N = l == 0 ? p.in_pad : p.width;
+    const __nv_bfloat16 *A = l == p.hidden ? mem.dYT : mem.dZT + l * wide;
+    const __nv_bfloat16 *B = l == 0 ? mem.XT : mem.HT + (l - 1) * wide;
+    const int slabs = (p.n + kDwK - 1) / kDwK, per = (slabs + splits - 1) / splits;
+    const int k0 = blockIdx.x * per, KT = max(0, min(slabs, k0 + per) - k0);
+    if (KT == 0)
+        return;
+    if (warp == 0) {
+        tc::tmem_alloc(tslot, 256);
+        tc::tmem_relinquish();
+    }
+    if (threadIdx.x == 0) {
+        tc::mbar_init(&bars[0], 1);
+        tc::mbar_init(&bars[1], 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    tc::tc_fence_before();
+    __syncthreads();
+    tc::tc_fence_after();
+    const uint32_t tmem = *tslot;
+    bool ok = true;
+    dw_stage(sa[0], 128, A, p.ld, m0, M, k0 * kDwK, p.n);
+    dw_stage(sb[0], N, B, p.ld, 0, N, k0 * kDwK, p.n);
+    tc::cp_async_commit();
+    const uint32_t idesc = tc::idesc_bf16_f32(128, N);
+    for (int kt = 0; kt < KT; ++kt) {
+        const int s = kt & 1;
+        if (kt + 1 < KT) {
+            if (kt >= 1) { // the MMAs of slab kt - 1 have read the other stage
+                bool w = true;
+                if (threadIdx.x == 0)
+                    w = tc::mbar_wait(&bars[s ^ 1], ((kt - 1) >> 1) & 1);
+                if (!__syncthreads_and(w)) {
+                    ok = false;
+                    break;
+                }
+            }
+            dw_stage(sa[s ^ 1], 128, A, p.ld, m0, M, (k0 + kt + 1) * kDwK, p.n);
+            dw_stage(sb[s ^ 1], N, B, p.ld, 0, N, (k0 + kt + 1) * kDwK, p.n);
+            tc::cp_async_commit();
+            tc::cp_async_wait<1>();
+        } else {
+            tc::cp_async_wait<0>();
+        }
+        tc::fence_proxy_async();
+        __syncthreads();
+        tc::tc_fence_after();
+        if (threadIdx.x == 0) {
+            const uint32_t a0 = tc::smem_u32(sa[s]), b0 = tc::smem_u32(sb[s]);
+#pragma unroll
+            for (int kk = 0; kk < kDwK / 16; ++kk)
+                tc::mma_bf16(tmem, tc::smem_desc(a0 + kk * 2 * 128 * 16, 128 * 16, 128),
+                             tc::smem_desc(b0 + kk * 2 * N * 16, N * 16, 128), idesc, (kt > 0 || kk > 0) ? 1u : 0u);
+            tc::mma_commit(&bars[s]);
+        }
+    }
+    {
+        bool w = true;
+        if (threadIdx.x == 0 && ok)
+            w = tc::mbar_wait(&bars[(KT - 1) & 1], ((KT - 1) >> 1) & 1);
+        ok = __syncthreads_and(ok && w);
+    }
+    tc::cp_async_wait<0>();
+    tc::tc_fence_after();
+    if (ok) {
+        const int m = m0 + warp * 32 + lane;
+        float *g = mem.gW[l] + (size_t)m * N;
+        for (int c0 = 0; c0 < N; c0 += 32) {
+            float v[32];
+            tc::tmem_ld32(tmem + (uint32_t(warp * 32) << 16) + c0, v);
+            if (m < M)
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    if (c0 + j * 4 < N)
+                        asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(g + c0 + j * 4), "f"(v[j * 4]),
+                                     "f"(v[j * 4 + 1]), "f"(v[j * 4 + 2]), "f"(v[j * 4 + 3])
+                                     : "memory");
+        }
+    } else if (threadIdx.x == 0) {
+        atomicExch(p.err, 1);
+    }
+    tc::tc_fence_before();
+    __syncthreads();
+    if (warp == 0)
+        tc::tmem_dealloc(tmem, 256);
+}
+
+// Position of element (n, k) of an [N x K] operand in its K-slabs of kFusedSlabK
+// columns, each in the core-matrix layout, slabs back to back.
+__device__ __forceinline__ size_t slab_at(int n, int k, int N)
+{
+    const int s = k / kFusedSlabK, kl = k % kFusedSlabK;
+    return (size_t)s * N * kFusedSlabK + ((size_t)(kl / 8) * N + n) * 8 + kl % 8;
+}
+
+// Adam on every parameter of the members (pads have zero gradients and stay
+// zero), or with lr == 0 the packing of the weights alone; the gradients are
+// cleared for the next step.
+__global__ void k_train_adam(const __grid_constant__ TrainParams p, float lr, float b1, float b2, float eps, float c1, float c2)
+{
+    const TrainMember &mem = p.member[p.first + blockIdx.y];
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < p.params; t += gridDim.x * blockDim.x) {
+        int l = 0, base = 0, in = 0, out = 0;
+        for (l = 0; l <= p.hidden; ++l) {
+            in = l == 0 ? p.in_pad : p.width;
+            out = l == p.hidden ? p.out_pad : p.width;
+            if (t < base + out * in + out)
+                break;
+            base += out * in + out;
+        }
+        const int at = t - base;
+        float w = mem.P[t];
+        if (lr > 0.0f) {
+            const float g = mem.G[t];
+            const float mi = b1 * mem.M[t] + (1.0f - b1) * g;
+            const float vi = b2 * mem.V[t] + (1.0f - b2) * g * g;
+            mem.M[t] = mi;
+            mem.V[t] = vi;
+            w -= lr * (mi * c1) / (sqrtf(vi * c2) + eps);
+            mem.P[t] = w;
+            mem.G[t] = 0.0f;
+        }
+        if (at < out * in) {
+            const int o = at / in, i = at % in;
+            const __nv_bfloat16 b = __float2bfloat16_rn(w);
+            mem.Wb[l][at] = b;
+            mem.slabs[l][slab_at(o, i, out)] = b;
+            mem.slabs_t[l][slab_at(i, o, in)] = b;
+        }
+    }
+}
+
+} // namespace eu3d

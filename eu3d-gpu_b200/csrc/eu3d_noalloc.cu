@@ -139,7 +139,7 @@ extern "C" eu_status eu_mlp_predict_noalloc(eu_mlp *m, const float *X, long long
             return fail_cuda(m, e_, #call);                                                        \
     } while (0)
     NCK(cudaMemsetAsync(err, 0, sizeof(int), s));
-    NCK(eu3d::pack_features(X, n, v.n_in, nullptr, v.in_shift, v.in_scale, xs, v.in_pad, s));
+    NCK(eu3d::pack_features(X, n, v.n_in, v.in_shift, v.in_scale, xs, v.in_pad, s));
     const int rows = int(n);
     for (int member = 0; member < v.members; ++member) {
         eu3d::MlpLayerView L;
@@ -148,11 +148,11 @@ extern "C" eu_status eu_mlp_predict_noalloc(eu_mlp *m, const float *X, long long
             const void *A = l == 0 ? xs : h[(l - 1) & 1];
             const int lda = l == 0 ? v.in_pad : v.width;
             NCK(eu3d::gemm_bf16(A, lda, L.Wb, L.in_pad, rows, L.out_pad, L.in_pad, L.b, 4, nullptr, h[l & 1],
-                                nullptr, v.width, nullptr, 1, err, s));
+                                nullptr, v.width, err, s));
         }
         eu3d::mlp_layer_view(m, member, v.hidden, &L);
         NCK(eu3d::gemm_bf16(h[(v.hidden - 1) & 1], v.width, L.Wb, L.in_pad, rows, L.out_pad, L.in_pad, L.b, 0, ys,
-                            nullptr, nullptr, v.out_pad, nullptr, 1, err, s));
+                            nullptr, nullptr, v.out_pad, err, s));
         NCK(eu3d::unscale_outputs(ys, n, v.out_pad, v.n_out, v.out_shift, v.out_scale,
                                   out + (long long)member * n * v.n_out, s));
     }

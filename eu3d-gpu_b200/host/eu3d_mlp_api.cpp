@@ -22,10 +22,11 @@ namespace {
 
 struct Layer {
     int in = 0, out = 0, in_pad = 0, out_pad = 0;
+    long long at = 0;                   // of W in the member's parameters; b follows
     float *W = nullptr, *b = nullptr;   // fp32 master, padded [out_pad x in_pad], [out_pad]
     float *gW = nullptr, *gb = nullptr; // gradients
-    float *mW = nullptr, *vW = nullptr, *mb = nullptr, *vb = nullptr;
-    void *Wb = nullptr, *Wt = nullptr; // bf16 [out_pad x in_pad] and [in_pad x out_pad]
+    __nv_bfloat16 *Wb = nullptr;        // [out_pad x in_pad]
+    __nv_bfloat16 *slabs = nullptr, *slabs_t = nullptr; // its K-slabs and its transpose's
 };
 
 int pad16(int n) { return (n + 15) / 16 * 16; }
@@ -42,22 +43,22 @@ struct eu_mlp {
     int in_pad = 0, out_pad = 0;
     std::vector<std::vector<Layer>> net;
     float *in_shift = nullptr, *in_scale = nullptr, *out_shift = nullptr, *out_scale = nullptr;
-    void *X = nullptr;                  // bf16 [B x in_pad]
-    std::vector<float *> Z;             // fp32 [B x width] per hidden layer
-    std::vector<void *> H;              // bf16 [B x width]
-    float *Y = nullptr;                 // fp32 [B x out_pad]
-    void *dY = nullptr;                 // bf16 [B x out_pad]
-    float *dZf[2] = {nullptr, nullptr}; // fp32 [B x width]
-    void *dZb[2] = {nullptr, nullptr};  // bf16 [B x width]
-    void *T1 = nullptr, *T2 = nullptr;  // bf16 transposes [width x B]
-    float *loss = nullptr;
-    int *rows = nullptr;
+    // fp32 parameters, gradients and Adam's moments: `params` padded values a member
+    float *P = nullptr, *G = nullptr, *M = nullptr, *V = nullptr;
+    long long params = 0;
+    void *X = nullptr;    // bf16 [B x in_pad]
+    std::vector<void *> H; // bf16 [B x width]
+    float *Y = nullptr;   // fp32 [B x out_pad]
+    float *loss = nullptr; // [members]
     long long adam_t = 0;
     std::vector<void *> allocs;
-    // inference in one persistent kernel (eu3d_mlp_fused.cuh): the bf16 weights
-    // repacked into K-slabs whenever they change
+    // training scratch of every member for batches of up to train_rows rows
+    // (allocated by the first training call, grown with the batch, kept)
+    void *train = nullptr;
+    long long train_rows = 0;
+    // inference in one persistent kernel (eu3d_mlp_fused.cuh), on the K-slabs
     bool fused = false;
-    void *slabs = nullptr;
+    __nv_bfloat16 *slabs = nullptr;
     long long slab_off[eu3d::kFusedMaxMembers][eu3d::kFusedMaxLayers] = {};
     int sms = 0;
 };
@@ -101,8 +102,11 @@ void free_all(eu_mlp *m)
 {
     for (void *p : m->allocs) cudaFree(p);
     m->allocs.clear();
+    if (m->train)
+        cudaFree(m->train);
+    m->train = nullptr;
+    m->train_rows = 0;
     m->net.clear();
-    m->Z.clear();
     m->H.clear();
     m->ready = false;
 }
@@ -114,11 +118,9 @@ long long params_per_member(const eu_mlp *m)
     return n;
 }
 
-// forward of member e over n packed rows in m->X (on stream s). Training keeps
-// the pre-activations and uses the exact-form SiLU (epilogue mode 1);
-// inference uses the fused kernel's form (mode 4), so the layer-wise and fused
-// predictions agree bitwise.
-eu_status forward(eu_mlp *m, int e, int n, cudaStream_t s = nullptr, bool keep_pre = true)
+// layer-wise inference of member e over n packed rows in m->X (on stream s), with
+// the fused kernel's activation, so that the two predictions agree bitwise
+eu_status forward(eu_mlp *m, int e, int n, cudaStream_t s = nullptr)
 {
     if (!s)
         s = m->stream;
@@ -127,66 +129,93 @@ eu_status forward(eu_mlp *m, int e, int n, cudaStream_t s = nullptr, bool keep_p
         const void *A = l == 0 ? m->X : m->H[l - 1];
         const int lda = l == 0 ? m->in_pad : m->width;
         const Layer &L = net[l];
-        MCK(m, eu3d::gemm_bf16(A, lda, L.Wb, L.in_pad, n, L.out_pad, L.in_pad, L.b, keep_pre ? 1 : 4, nullptr,
-                               m->H[l], keep_pre ? m->Z[l] : nullptr, m->width, nullptr, 1, m->d_err, s));
+        MCK(m, eu3d::gemm_bf16(A, lda, L.Wb, L.in_pad, n, L.out_pad, L.in_pad, L.b, 4, nullptr, m->H[l], nullptr,
+                               m->width, m->d_err, s));
     }
     const Layer &L = net[m->hidden];
     MCK(m, eu3d::gemm_bf16(m->H[m->hidden - 1], m->width, L.Wb, L.in_pad, n, L.out_pad, L.in_pad, L.b, 0, m->Y, nullptr,
-                           nullptr, m->out_pad, nullptr, 1, m->d_err, s));
+                           nullptr, m->out_pad, m->d_err, s));
     return EU_OK;
 }
 
-// gradients of member e for the n rows whose forward is in the scratch buffers
-// and whose output gradient is in m->dY (n % 16 == 0)
-eu_status backward(eu_mlp *m, int e, int n)
+// The training kernels' parameters for members [first, first + count), without a
+// batch.
+eu3d::TrainParams train_params(const eu_mlp *m, int first, int count)
 {
-    auto &net = m->net[e];
-    const int ksplit = n >= 2048 ? 16 : (n >= 512 ? 4 : 1);
-    for (Layer &L : net) {
-        MCK(m, cudaMemsetAsync(L.gW, 0, sizeof(float) * L.out_pad * L.in_pad, m->stream));
-        MCK(m, cudaMemsetAsync(L.gb, 0, sizeof(float) * L.out_pad, m->stream));
-    }
-    // output layer
-    {
-        Layer &L = net[m->hidden];
-        void *Hl = m->H[m->hidden - 1];
-        MCK(m, eu3d::transpose_bf16(m->dY, n, L.out_pad, L.out_pad, m->T1, n, m->stream));
-        MCK(m, eu3d::transpose_bf16(Hl, n, m->width, m->width, m->T2, n, m->stream));
-        MCK(m, eu3d::gemm_bf16(m->T1, n, m->T2, n, L.out_pad, L.in_pad, n, nullptr, 3, L.gW, nullptr, nullptr, L.in_pad,
-                               nullptr, ksplit, m->d_err, m->stream));
-        MCK(m, eu3d::colsum_bf16(m->dY, n, L.out_pad, L.out_pad, L.gb, m->stream));
-        MCK(m, eu3d::gemm_bf16(m->dY, L.out_pad, L.Wt, L.out_pad, n, m->width, L.out_pad, nullptr, 2, m->dZf[0],
-                               m->dZb[0], nullptr, m->width, m->Z[m->hidden - 1], 1, m->d_err, m->stream));
-    }
-    int cur = 0;
-    for (int l = m->hidden - 1; l >= 0; --l) {
-        Layer &L = net[l];
-        const void *A = l == 0 ? m->X : m->H[l - 1];
-        const int in_pad = L.in_pad;
-        MCK(m, eu3d::transpose_bf16(m->dZb[cur], n, m->width, m->width, m->T1, n, m->stream));
-        MCK(m, eu3d::transpose_bf16(A, n, in_pad, in_pad, m->T2, n, m->stream));
-        MCK(m, eu3d::gemm_bf16(m->T1, n, m->T2, n, m->width, in_pad, n, nullptr, 3, L.gW, nullptr, nullptr, in_pad,
-                               nullptr, ksplit, m->d_err, m->stream));
-        MCK(m, eu3d::colsum_f32(m->dZf[cur], n, m->width, m->width, L.gb, m->stream));
-        if (l > 0) {
-            MCK(m, eu3d::gemm_bf16(m->dZb[cur], m->width, L.Wt, L.out_pad, n, m->width, m->width, nullptr, 2,
-                                   m->dZf[cur ^ 1], m->dZb[cur ^ 1], nullptr, m->width, m->Z[l - 1], 1, m->d_err,
-                                   m->stream));
-            cur ^= 1;
+    eu3d::TrainParams p{};
+    p.n_in = m->n_in;
+    p.in_pad = m->in_pad;
+    p.width = m->width;
+    p.hidden = m->hidden;
+    p.n_out = m->n_out;
+    p.out_pad = m->out_pad;
+    p.params = int(m->params);
+    p.first = first;
+    p.members = count;
+    p.in_shift = m->in_shift;
+    p.in_scale = m->in_scale;
+    p.out_shift = m->out_shift;
+    p.out_scale = m->out_scale;
+    p.loss = m->loss;
+    p.err = m->d_err;
+    for (int e = 0; e < m->members; ++e) {
+        eu3d::TrainMember &t = p.member[e];
+        t.P = m->P + e * m->params;
+        t.G = m->G + e * m->params;
+        t.M = m->M + e * m->params;
+        t.V = m->V + e * m->params;
+        for (int l = 0; l <= m->hidden; ++l) {
+            const Layer &L = m->net[e][l];
+            t.bias[l] = L.b;
+            t.gW[l] = L.gW;
+            t.gb[l] = L.gb;
+            t.Wb[l] = L.Wb;
+            t.slabs[l] = L.slabs;
+            t.slabs_t[l] = L.slabs_t;
         }
     }
+    return p;
+}
+
+// A batch of n rows of the caller's arrays, with the members' scratch for it.
+eu_status train_batch(eu_mlp *m, eu3d::TrainParams &p, const float *X, const float *T, long long rows, int n, bool drawn)
+{
+    const int ld = eu3d::train_ld(n);
+    const size_t wide = size_t(m->hidden) * m->width * ld;
+    // every piece a multiple of 64 values, so 128-byte aligned
+    const size_t bytes = wide * (4 + 2 + 2) + size_t(ld) * (m->in_pad + m->out_pad) * 2;
+    if (m->train_rows < n) {
+        if (m->train) {
+            MCK(m, cudaStreamSynchronize(m->stream));
+            MCK(m, cudaFree(m->train));
+        }
+        m->train = nullptr;
+        m->train_rows = 0;
+        MCK(m, cudaMalloc(&m->train, bytes * m->members));
+        m->train_rows = n;
+    }
+    p.X = X;
+    p.T = T;
+    p.rows = rows;
+    p.n = n;
+    p.ld = ld;
+    p.drawn = drawn;
+    for (int e = 0; e < m->members; ++e) {
+        eu3d::TrainMember &t = p.member[e];
+        unsigned char *at = static_cast<unsigned char *>(m->train) + e * bytes;
+        t.Z = reinterpret_cast<float *>(at);
+        t.HT = reinterpret_cast<__nv_bfloat16 *>(at + wide * 4);
+        t.dZT = t.HT + wide;
+        t.XT = t.dZT + wide;
+        t.dYT = t.XT + size_t(ld) * m->in_pad;
+    }
     return EU_OK;
 }
 
-eu_status refresh(eu_mlp *m, int e)
+// The bf16 weights of members [first, first + count) from the fp32 masters.
+eu_status refresh(eu_mlp *m, int first, int count)
 {
-    for (size_t l = 0; l < m->net[e].size(); ++l) {
-        Layer &L = m->net[e][l];
-        MCK(m, eu3d::refresh_weights(L.W, L.out_pad, L.in_pad, L.out_pad, L.in_pad, L.Wb, L.Wt, m->stream));
-        if (m->fused)
-            MCK(m, eu3d::pack_slabs(L.Wb, L.out_pad, L.in_pad,
-                                    static_cast<uint16_t *>(m->slabs) + m->slab_off[e][l], m->stream));
-    }
+    MCK(m, eu3d::train_adam(train_params(m, first, count), 0.0f, 0, 0, 0, 0, 0, m->stream));
     return EU_OK;
 }
 
@@ -289,10 +318,10 @@ eu_status mlp_predict_stream(eu_mlp *m, const float *X, long long n, float *out,
 {
     for (long long r0 = 0; r0 < n; r0 += m->max_batch) {
         const int nb = int(n - r0 < m->max_batch ? n - r0 : m->max_batch);
-        MCK(m, eu3d::pack_features(X + r0 * m->n_in, nb, m->n_in, nullptr, m->in_shift, m->in_scale, m->X, m->in_pad,
+        MCK(m, eu3d::pack_features(X + r0 * m->n_in, nb, m->n_in, m->in_shift, m->in_scale, m->X, m->in_pad,
                                    s));
         for (int e = 0; e < m->members; ++e) {
-            eu_status st = forward(m, e, nb, s, false);
+            eu_status st = forward(m, e, nb, s);
             if (st != EU_OK)
                 return st;
             MCK(m, eu3d::unscale_outputs(m->Y, nb, m->out_pad, m->n_out, m->out_shift, m->out_scale,
@@ -360,7 +389,7 @@ eu_status eu_mlp_gemm(eu_mlp *m, const void *A, int lda, const void *B, int ldb,
         return EU_OK;
     cudaSetDevice(m->device);
     cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : m->stream;
-    cudaError_t e = eu3d::gemm_bf16(A, lda, B, ldb, M, N, K, bias, act, Cf, Cb, Cpre, ldc, nullptr, 1, m->d_err, s);
+    cudaError_t e = eu3d::gemm_bf16(A, lda, B, ldb, M, N, K, bias, act, Cf, Cb, Cpre, ldc, m->d_err, s);
     if (e != cudaSuccess)
         return mfail(m, EU_ERR_CUDA, "gemm launch: %s", cudaGetErrorString(e));
     int herr = 0;
@@ -397,33 +426,53 @@ eu_status eu_mlp_init(eu_mlp *m, int n_in, int width, int hidden_layers, int n_o
     m->adam_t = 0;
     std::mt19937_64 rng(seed);
     m->net.assign(members, std::vector<Layer>(hidden_layers + 1));
-    for (int e = 0; e < members; ++e)
+    m->params = 0;
+    long long slab_values = 0;
+    for (int l = 0; l <= hidden_layers; ++l) {
+        const long long in = pad16(l == 0 ? n_in : width), out = pad16(l == hidden_layers ? n_out : width);
+        m->params += out * in + out;
+        slab_values += out * in;
+    }
+    const size_t all = size_t(m->params) * members * 4;
+    __nv_bfloat16 *Wb = nullptr, *slabs_t = nullptr;
+    MCK(m, malloc_zero(m, &m->P, all));
+    MCK(m, malloc_zero(m, &m->G, all));
+    MCK(m, malloc_zero(m, &m->M, all));
+    MCK(m, malloc_zero(m, &m->V, all));
+    MCK(m, malloc_zero(m, &Wb, size_t(slab_values) * members * 2));
+    MCK(m, malloc_zero(m, &m->slabs, size_t(slab_values) * members * 2));
+    MCK(m, malloc_zero(m, &slabs_t, size_t(slab_values) * members * 2));
+    std::vector<float> init(size_t(m->params) * members, 0.0f);
+    long long slab = 0;
+    for (int e = 0; e < members; ++e) {
+        long long at = 0;
         for (int l = 0; l <= hidden_layers; ++l) {
             Layer &L = m->net[e][l];
             L.in = l == 0 ? n_in : width;
             L.out = l == hidden_layers ? n_out : width;
             L.in_pad = pad16(L.in);
             L.out_pad = pad16(L.out);
-            const size_t nw = size_t(L.out_pad) * L.in_pad, nb = L.out_pad;
-            MCK(m, malloc_zero(m, &L.W, nw * 4));
-            MCK(m, malloc_zero(m, &L.b, nb * 4));
-            MCK(m, malloc_zero(m, &L.gW, nw * 4));
-            MCK(m, malloc_zero(m, &L.gb, nb * 4));
-            MCK(m, malloc_zero(m, &L.mW, nw * 4));
-            MCK(m, malloc_zero(m, &L.vW, nw * 4));
-            MCK(m, malloc_zero(m, &L.mb, nb * 4));
-            MCK(m, malloc_zero(m, &L.vb, nb * 4));
-            MCK(m, malloc_zero(m, &L.Wb, nw * 2));
-            MCK(m, malloc_zero(m, &L.Wt, nw * 2));
+            const long long nw = (long long)L.out_pad * L.in_pad, base = e * m->params + at;
+            L.at = at;
+            L.W = m->P + base;
+            L.b = L.W + nw;
+            L.gW = m->G + base;
+            L.gb = L.gW + nw;
+            L.Wb = Wb + slab;
+            L.slabs = m->slabs + slab;
+            L.slabs_t = slabs_t + slab;
+            m->slab_off[e][l] = slab;
+            slab += nw;
+            at += nw + L.out_pad;
             // He-uniform initialisation (SiLU layers), zero biases
-            std::vector<float> w(nw, 0.0f);
             const double bound = std::sqrt(6.0 / L.in) * (l == hidden_layers ? 0.5 : 1.0);
             std::uniform_real_distribution<double> u(-bound, bound);
             for (int o = 0; o < L.out; ++o)
-                for (int i = 0; i < L.in; ++i) w[size_t(o) * L.in_pad + i] = float(u(rng));
-            MCK(m, cudaMemcpyAsync(L.W, w.data(), nw * 4, cudaMemcpyHostToDevice, m->stream));
-            MCK(m, cudaStreamSynchronize(m->stream));
+                for (int i = 0; i < L.in; ++i) init[size_t(base) + size_t(o) * L.in_pad + i] = float(u(rng));
         }
+    }
+    MCK(m, cudaMemcpyAsync(m->P, init.data(), all, cudaMemcpyHostToDevice, m->stream));
+    MCK(m, cudaStreamSynchronize(m->stream));
     const int B = max_batch;
     MCK(m, malloc_zero(m, &m->in_shift, size_t(m->in_pad) * 4));
     MCK(m, malloc_zero(m, &m->in_scale, size_t(m->in_pad) * 4));
@@ -433,38 +482,16 @@ eu_status eu_mlp_init(eu_mlp *m, int n_in, int width, int hidden_layers, int n_o
         std::vector<float> one(256, 1.0f);
         MCK(m, cudaMemcpyAsync(m->in_scale, one.data(), size_t(m->in_pad) * 4, cudaMemcpyHostToDevice, m->stream));
         MCK(m, cudaMemcpyAsync(m->out_scale, one.data(), size_t(m->out_pad) * 4, cudaMemcpyHostToDevice, m->stream));
+        MCK(m, cudaStreamSynchronize(m->stream));
     }
     MCK(m, malloc_zero(m, &m->X, size_t(B) * m->in_pad * 2));
-    m->Z.assign(hidden_layers, nullptr);
     m->H.assign(hidden_layers, nullptr);
-    for (int l = 0; l < hidden_layers; ++l) {
-        MCK(m, malloc_zero(m, &m->Z[l], size_t(B) * width * 4));
-        MCK(m, malloc_zero(m, &m->H[l], size_t(B) * width * 2));
-    }
+    for (int l = 0; l < hidden_layers; ++l) MCK(m, malloc_zero(m, &m->H[l], size_t(B) * width * 2));
     MCK(m, malloc_zero(m, &m->Y, size_t(B) * m->out_pad * 4));
-    MCK(m, malloc_zero(m, &m->dY, size_t(B) * m->out_pad * 2));
-    for (int q = 0; q < 2; ++q) {
-        MCK(m, malloc_zero(m, &m->dZf[q], size_t(B) * width * 4));
-        MCK(m, malloc_zero(m, &m->dZb[q], size_t(B) * width * 2));
-    }
-    int tw = width > m->in_pad ? width : m->in_pad;
-    tw = tw > m->out_pad ? tw : m->out_pad;
-    MCK(m, malloc_zero(m, &m->T1, size_t(B) * tw * 2));
-    MCK(m, malloc_zero(m, &m->T2, size_t(B) * tw * 2));
-    MCK(m, malloc_zero(m, &m->loss, 4 * sizeof(float)));
-    MCK(m, malloc_zero(m, &m->rows, size_t(B) * sizeof(int)));
+    MCK(m, malloc_zero(m, &m->loss, eu3d::kFusedMaxMembers * sizeof(float)));
     m->fused = eu3d::fused_supported(m->in_pad, width, m->out_pad, members, hidden_layers + 1);
-    if (m->fused) {
-        long long n = 0;
-        for (int e = 0; e < members; ++e)
-            for (int l = 0; l <= hidden_layers; ++l) {
-                m->slab_off[e][l] = n;
-                n += (long long)m->net[e][l].out_pad * m->net[e][l].in_pad;
-            }
-        MCK(m, malloc_zero(m, &m->slabs, size_t(n) * 2));
-    }
-    for (int e = 0; e < members; ++e) {
-        eu_status s = refresh(m, e);
+    {
+        eu_status s = refresh(m, 0, members);
         if (s != EU_OK)
             return s;
     }
@@ -499,6 +526,34 @@ long long eu_mlp_num_params(const eu_mlp *m)
     return params_per_member(m) * m->members;
 }
 
+namespace {
+// The member's values without the layers' padding, in the order of the flat
+// parameters, and back.
+long long unpad(const eu_mlp *m, const float *padded, float *out)
+{
+    long long n = 0;
+    for (const Layer &L : m->net[0]) {
+        const float *w = padded + L.at, *b = w + (long long)L.out_pad * L.in_pad;
+        for (int o = 0; o < L.out; ++o, n += L.in) std::memcpy(out + n, w + (long long)o * L.in_pad, size_t(L.in) * 4);
+        std::memcpy(out + n, b, size_t(L.out) * 4);
+        n += L.out;
+    }
+    return n;
+}
+
+long long pad(const eu_mlp *m, const float *in, float *padded)
+{
+    long long n = 0;
+    for (const Layer &L : m->net[0]) {
+        float *w = padded + L.at, *b = w + (long long)L.out_pad * L.in_pad;
+        for (int o = 0; o < L.out; ++o, n += L.in) std::memcpy(w + (long long)o * L.in_pad, in + n, size_t(L.in) * 4);
+        std::memcpy(b, in + n, size_t(L.out) * 4);
+        n += L.out;
+    }
+    return n;
+}
+} // namespace
+
 eu_status eu_mlp_get_params(eu_mlp *m, float *out)
 {
     if (!m || !out)
@@ -506,17 +561,10 @@ eu_status eu_mlp_get_params(eu_mlp *m, float *out)
     if (!m->ready)
         return mfail(m, EU_ERR_NOT_READY, "eu_mlp_init first");
     cudaSetDevice(m->device);
-    long long off = 0;
-    for (auto &net : m->net)
-        for (Layer &L : net) {
-            std::vector<float> w(size_t(L.out_pad) * L.in_pad), b(L.out_pad);
-            MCK(m, cudaMemcpyAsync(w.data(), L.W, w.size() * 4, cudaMemcpyDeviceToHost, m->stream));
-            MCK(m, cudaMemcpyAsync(b.data(), L.b, b.size() * 4, cudaMemcpyDeviceToHost, m->stream));
-            MCK(m, cudaStreamSynchronize(m->stream));
-            for (int o = 0; o < L.out; ++o)
-                for (int i = 0; i < L.in; ++i) out[off++] = w[size_t(o) * L.in_pad + i];
-            for (int o = 0; o < L.out; ++o) out[off++] = b[o];
-        }
+    std::vector<float> all(size_t(m->params) * m->members);
+    MCK(m, cudaMemcpyAsync(all.data(), m->P, all.size() * 4, cudaMemcpyDeviceToHost, m->stream));
+    MCK(m, cudaStreamSynchronize(m->stream));
+    for (int e = 0; e < m->members; ++e) out += unpad(m, all.data() + e * m->params, out);
     return EU_OK;
 }
 
@@ -527,21 +575,13 @@ eu_status eu_mlp_set_params(eu_mlp *m, const float *in)
     if (!m->ready)
         return mfail(m, EU_ERR_NOT_READY, "eu_mlp_init first");
     cudaSetDevice(m->device);
-    long long off = 0;
-    for (int e = 0; e < m->members; ++e) {
-        for (Layer &L : m->net[e]) {
-            std::vector<float> w(size_t(L.out_pad) * L.in_pad, 0.0f), b(L.out_pad, 0.0f);
-            for (int o = 0; o < L.out; ++o)
-                for (int i = 0; i < L.in; ++i) w[size_t(o) * L.in_pad + i] = in[off++];
-            for (int o = 0; o < L.out; ++o) b[o] = in[off++];
-            MCK(m, cudaMemcpyAsync(L.W, w.data(), w.size() * 4, cudaMemcpyHostToDevice, m->stream));
-            MCK(m, cudaMemcpyAsync(L.b, b.data(), b.size() * 4, cudaMemcpyHostToDevice, m->stream));
-            MCK(m, cudaStreamSynchronize(m->stream));
-        }
-        eu_status s = refresh(m, e);
-        if (s != EU_OK)
-            return s;
-    }
+    std::vector<float> all(size_t(m->params) * m->members, 0.0f);
+    for (int e = 0; e < m->members; ++e) in += pad(m, in, all.data() + e * m->params);
+    MCK(m, cudaMemcpyAsync(m->P, all.data(), all.size() * 4, cudaMemcpyHostToDevice, m->stream));
+    MCK(m, cudaStreamSynchronize(m->stream));
+    const eu_status s = refresh(m, 0, m->members);
+    if (s != EU_OK)
+        return s;
     MCK(m, cudaStreamSynchronize(m->stream));
     return EU_OK;
 }
@@ -556,31 +596,25 @@ eu_status eu_mlp_loss_grad(eu_mlp *m, int member, const float *X, const float *T
     if (member < 0 || member >= m->members || n < 16 || n > m->max_batch || (n % 16))
         return mfail(m, EU_ERR_INVALID_ARGUMENT, "member or batch size (multiple of 16 up to max_batch)");
     cudaSetDevice(m->device);
-    MCK(m, eu3d::pack_features(X, n, m->n_in, nullptr, m->in_shift, m->in_scale, m->X, m->in_pad, m->stream));
-    eu_status s = forward(m, member, n);
+    eu3d::TrainParams p = train_params(m, member, 1);
+    eu_status s = train_batch(m, p, X, T, n, n, false);
     if (s != EU_OK)
         return s;
-    MCK(m, cudaMemsetAsync(m->loss, 0, sizeof(float), m->stream));
-    MCK(m, eu3d::mse_grad(m->Y, m->out_pad, T, n, m->n_out, nullptr, m->out_shift, m->out_scale, m->dY, m->loss,
-                          m->stream));
-    if ((s = backward(m, member, n)) != EU_OK)
-        return s;
+    float *g = m->G + member * m->params;
+    MCK(m, cudaMemsetAsync(g, 0, size_t(m->params) * 4, m->stream));
+    MCK(m, cudaMemsetAsync(m->loss + member, 0, sizeof(float), m->stream));
+    MCK(m, eu3d::train_rows(p, m->stream));
+    MCK(m, eu3d::train_weights(p, m->sms, m->stream));
+    float sq = 0;
+    std::vector<float> all(grads_out ? size_t(m->params) : 0);
+    MCK(m, cudaMemcpyAsync(&sq, m->loss + member, sizeof(float), cudaMemcpyDeviceToHost, m->stream));
+    if (grads_out)
+        MCK(m, cudaMemcpyAsync(all.data(), g, all.size() * 4, cudaMemcpyDeviceToHost, m->stream));
     if ((s = check_err(m)) != EU_OK)
         return s;
-    float sq = 0;
-    MCK(m, cudaMemcpy(&sq, m->loss, sizeof(float), cudaMemcpyDeviceToHost));
     *loss_out = sq / float(n * m->n_out);
-    if (grads_out) {
-        long long off = 0;
-        for (Layer &L : m->net[member]) {
-            std::vector<float> w(size_t(L.out_pad) * L.in_pad), b(L.out_pad);
-            MCK(m, cudaMemcpy(w.data(), L.gW, w.size() * 4, cudaMemcpyDeviceToHost));
-            MCK(m, cudaMemcpy(b.data(), L.gb, b.size() * 4, cudaMemcpyDeviceToHost));
-            for (int o = 0; o < L.out; ++o)
-                for (int i = 0; i < L.in; ++i) grads_out[off++] = w[size_t(o) * L.in_pad + i];
-            for (int o = 0; o < L.out; ++o) grads_out[off++] = b[o];
-        }
-    }
+    if (grads_out)
+        unpad(m, all.data(), grads_out);
     return EU_OK;
 }
 
@@ -594,46 +628,31 @@ eu_status eu_mlp_train(eu_mlp *m, const float *X, const float *T, long long n, i
     if (batch < 16 || batch > m->max_batch || (batch % 16) || n < batch || steps < 0 || !(lr > 0))
         return mfail(m, EU_ERR_INVALID_ARGUMENT, "batch must be a multiple of 16, <= max_batch and <= n");
     cudaSetDevice(m->device);
-    std::vector<double> total(m->members, 0.0);
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
+    eu3d::TrainParams p = train_params(m, 0, m->members);
+    eu_status s = train_batch(m, p, X, T, n, batch, true);
+    if (s != EU_OK)
+        return s;
+    MCK(m, cudaMemsetAsync(m->G, 0, size_t(m->params) * m->members * 4, m->stream));
     for (int it = 0; it < steps; ++it) {
         ++m->adam_t;
         const float c1 = 1.0f / (1.0f - std::pow(b1, float(m->adam_t)));
         const float c2 = 1.0f / (1.0f - std::pow(b2, float(m->adam_t)));
-        for (int e = 0; e < m->members; ++e) {
-            const unsigned long long key =
-                (unsigned long long)seed * 0x100000001B3ull + (unsigned long long)m->adam_t * 131ull + e;
-            MCK(m, eu3d::random_rows(m->rows, batch, n, key, m->stream));
-            MCK(m, eu3d::pack_features(X, batch, m->n_in, m->rows, m->in_shift, m->in_scale, m->X, m->in_pad,
-                                       m->stream));
-            eu_status s = forward(m, e, batch);
-            if (s != EU_OK)
-                return s;
-            MCK(m, cudaMemsetAsync(m->loss, 0, sizeof(float), m->stream));
-            MCK(m, eu3d::mse_grad(m->Y, m->out_pad, T, batch, m->n_out, m->rows, m->out_shift, m->out_scale, m->dY,
-                                  m->loss, m->stream));
-            if ((s = backward(m, e, batch)) != EU_OK)
-                return s;
-            for (Layer &L : m->net[e]) {
-                MCK(m, eu3d::adam(L.W, L.gW, L.mW, L.vW, (long long)L.out_pad * L.in_pad, lr, b1, b2, eps, c1, c2,
-                                  m->stream));
-                MCK(m, eu3d::adam(L.b, L.gb, L.mb, L.vb, L.out_pad, lr, b1, b2, eps, c1, c2, m->stream));
-            }
-            if ((s = refresh(m, e)) != EU_OK)
-                return s;
-            if (it + 1 == steps) {
-                float sq = 0;
-                MCK(m, cudaMemcpyAsync(&sq, m->loss, sizeof(float), cudaMemcpyDeviceToHost, m->stream));
-                MCK(m, cudaStreamSynchronize(m->stream));
-                total[e] = sq / double(batch * m->n_out);
-            }
-        }
+        for (int e = 0; e < m->members; ++e)
+            p.member[e].key = (unsigned long long)seed * 0x100000001B3ull + (unsigned long long)m->adam_t * 131ull + e;
+        if (it + 1 == steps) // the last batch's loss is the one returned
+            MCK(m, cudaMemsetAsync(m->loss, 0, size_t(m->members) * sizeof(float), m->stream));
+        MCK(m, eu3d::train_rows(p, m->stream));
+        MCK(m, eu3d::train_weights(p, m->sms, m->stream));
+        MCK(m, eu3d::train_adam(p, lr, b1, b2, eps, c1, c2, m->stream));
     }
-    eu_status s = check_err(m);
-    if (s != EU_OK)
+    std::vector<float> sq(m->members, 0.0f);
+    if (steps > 0)
+        MCK(m, cudaMemcpyAsync(sq.data(), m->loss, sq.size() * sizeof(float), cudaMemcpyDeviceToHost, m->stream));
+    if ((s = check_err(m)) != EU_OK)
         return s;
     if (mean_loss)
-        for (int e = 0; e < m->members; ++e) mean_loss[e] = float(total[e]);
+        for (int e = 0; e < m->members; ++e) mean_loss[e] = float(sq[e] / double(batch * m->n_out));
     return EU_OK;
 }
 
@@ -700,10 +719,10 @@ eu_status eu_mlp_predict(eu_mlp *m, const float *X, long long n, float *out)
     cudaSetDevice(m->device);
     for (long long r0 = 0; r0 < n; r0 += m->max_batch) {
         const int nb = int(n - r0 < m->max_batch ? n - r0 : m->max_batch);
-        MCK(m, eu3d::pack_features(X + r0 * m->n_in, nb, m->n_in, nullptr, m->in_shift, m->in_scale, m->X, m->in_pad,
+        MCK(m, eu3d::pack_features(X + r0 * m->n_in, nb, m->n_in, m->in_shift, m->in_scale, m->X, m->in_pad,
                                    m->stream));
         for (int e = 0; e < m->members; ++e) {
-            eu_status s = forward(m, e, nb, nullptr, false);
+            eu_status s = forward(m, e, nb);
             if (s != EU_OK)
                 return s;
             MCK(m, eu3d::unscale_outputs(m->Y, nb, m->out_pad, m->n_out, m->out_shift, m->out_scale,

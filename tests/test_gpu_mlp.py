@@ -95,6 +95,36 @@ def test_training_fits_a_smooth_map(gpu):
     assert (l1 < l0 / 20).all(), (l0, l1)
 
 
+@pytest.mark.parametrize("shape,n", [((5, 64, 2, 3, 2), 16), ((20, 96, 1, 40, 1), 144), ((N_IN, WIDTH, HIDDEN, N_OUT, 1), 1008),
+                                     ((3, 16, 1, 1, 2), 128), ((200, 128, 2, 130, 1), 272)])
+def test_gradients_of_other_shapes(gpu, shape, n):
+    """The training kernels at widths and batches off their tiles (16 to 256
+    wide, one to several 128-row tiles with a partial last one, inputs and
+    outputs wider than a slab), against the CPU checker with the bounds of
+    test_gradients_match_cpu_oracle."""
+    import torch
+    n_in, width, hidden, n_out, members = shape
+    m = gpu.Mlp()
+    m.init(n_in, width, hidden, n_out, members, max_batch=1024, seed=6)
+    rng = np.random.default_rng(n)
+    scal = [np.asarray(v, np.float32) for v in (rng.normal(size=n_in), rng.uniform(0.5, 2, n_in), rng.normal(size=n_out),
+                                                rng.uniform(0.5, 2, n_out))]
+    m.set_scaling(*scal)
+    X, T = rng.normal(size=(n, n_in)).astype(np.float32), rng.normal(size=(n, n_out)).astype(np.float32)
+    params = m.get_params()
+    per = params.size // members
+    for e in range(members):
+        loss, g = m.loss_grad(e, torch.from_numpy(X).cuda(), torch.from_numpy(T).cuda())
+        ref_loss, ref = mo.loss_and_grads(params[e * per:(e + 1) * per], X, T, n_in, width, hidden, n_out, *scal)
+        assert abs(loss - ref_loss) <= 1e-4 * ref_loss, (loss, ref_loss)
+        off = 0
+        for a, b in mo.layer_sizes(n_in, width, hidden, n_out):
+            for size in (a * b, b):
+                d = np.abs(g[off:off + size] - ref[off:off + size]).max()
+                assert d <= 2e-3 * np.abs(ref[off:off + size]).max() + 1e-12, (off, d)
+                off += size
+
+
 @pytest.mark.parametrize("shape", [(N_IN, WIDTH, HIDDEN, N_OUT, MEMBERS), (5, 64, 2, 3, 2), (20, 96, 1, 40, 1)])
 def test_fused_inference_matches_layerwise(gpu, shape):
     """The one-kernel inference (every member's network per 128-row tile, the
