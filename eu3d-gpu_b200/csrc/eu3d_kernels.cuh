@@ -34,7 +34,12 @@ __global__ void __launch_bounds__(256) k_boundary(const __grid_constant__ DevMec
                                                   const DevState st)
 {
     const int bc = g.bc, ni = g.ni, nj = g.nj, nk = g.nk;
-    const long long nxf = 2LL * bc * nj * nk, nyf = 2LL * bc * ni * nk, nzf = 2LL * bc * ni * nj;
+    // z ghosts of a row: on a grid two nodes thick every interior node is the
+    // mirror source of one ghost below and one above, and a thread fills both
+    // from one read and one rebuild (1024 x 512 x 2 ODW: 0.122 -> 0.093 ms)
+    const bool both = nk == bc;
+    const int zper = both ? bc : 2 * bc;
+    const long long nxf = 2LL * bc * nj * nk, nyf = 2LL * bc * ni * nk, nzf = (long long)zper * ni * nj;
     long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= nxf + nyf + nzf)
         return;
@@ -43,6 +48,7 @@ __global__ void __launch_bounds__(256) k_boundary(const __grid_constant__ DevMec
     double su = 1, sv = 1, sw = 1;
     bool rebuild = false;
     long long inflow = -1; // ODW x-low: index into the inflow tables
+    long long again = 0;   // distance to a second ghost of the same value
     if (t < nxf) {
         const int jk = fdiv(t, g.d_nk), q = fdiv(t, g.d_njnk); // q: 0 .. 2bc-1
         const int k = bc + int(t - (long long)jk * nk);
@@ -85,7 +91,8 @@ __global__ void __launch_bounds__(256) k_boundary(const __grid_constant__ DevMec
         if (st.zm_fresh && *st.zm_fresh) // EU_GHOSTS_STORED: stored with the interior
             return;
         const int jq = fdiv(t, g.d_ghost), ii = fdiv(t, g.d_ghost_nj);
-        const int q = int(t - (long long)jq * (2 * bc));
+        const int q = int(t - (long long)jq * zper);
+        again = both ? nk + bc : 0;
         const int j = bc + (jq - ii * nj);
         const int i = bc + ii;
         const int k = q < bc ? q : nk + q;
@@ -118,6 +125,23 @@ __global__ void __launch_bounds__(256) k_boundary(const __grid_constant__ DevMec
     v[kW] = sw * v[kW];
     const double T = st.T[src];
     if (rebuild) {
+#ifndef EU_EXACT_THERMO
+        double rg = 0, Y[NS];
+#pragma unroll
+        for (int s = 0; s < NS; ++s) {
+            Y[s] = v[kY0 + s];
+            rg = fma(Y[s], m.ri[s], rg);
+        }
+        MixPoly<NS> mp;
+        mix_poly<NS>(m, Y, T < kThermoSwitch, mp);
+        const double Rgas = rg * 1000, inv = rcp_nr(T);
+        const double h = fma(T, fma(T, fma(T, fma(T, fma(T, mp.h6, mp.h5), mp.h4), mp.h3), mp.a2), mp.a7) - mp.a0 * inv +
+                         mp.a1 * log(T);
+        const double cp = fma(T, fma(T, fma(T, fma(T, mp.a6, mp.a5), mp.a4), mp.a3), mp.a2) + inv * fma(mp.a0, inv, mp.a1);
+        v[kD] = div_fast(v[kP], T * Rgas);
+        v[kH] = h * 1000;
+        v[kG] = div_fast(cp * 1000, cp * 1000 - Rgas);
+#else
         const TPow p = make_tpow(T, true);
         double rg = 0, cp = 0, h = 0, e = 0;
         double Cpi[NS], Hi[NS];
@@ -141,14 +165,21 @@ __global__ void __launch_bounds__(256) k_boundary(const __grid_constant__ DevMec
         const double Cp = cp * 1000;
         v[kH] = h * 1000;
         v[kG] = Cp / (Cp - Rgas);
+#endif
     }
-    st.T[dst] = T;
+    for (;;) {
+        st.T[dst] = T;
 #pragma unroll
-    for (int f = 0; f < 7 + NS; ++f) {
-        if (st.prim32)
-            st.prim32[f * n3 + dst] = float(v[f]);
-        else
-            st.prim[f * n3 + dst] = v[f];
+        for (int f = 0; f < 7 + NS; ++f) {
+            if (st.prim32)
+                st.prim32[f * n3 + dst] = float(v[f]);
+            else
+                st.prim[f * n3 + dst] = v[f];
+        }
+        if (!again)
+            break;
+        dst += again;
+        again = 0;
     }
 }
 

@@ -18,7 +18,9 @@ template <int NS, int NR>
 cudaError_t boundary_t(const LaunchArgs &a)
 {
     const DevGrid &g = a.g;
-    const long long n = 2LL * g.bc * ((long long)g.nj * g.nk + (long long)g.ni * g.nk + (long long)g.ni * g.nj);
+    // a thread per ghost node; on a grid bc nodes thick one per pair of z ghosts
+    const long long n = 2LL * g.bc * ((long long)g.nj * g.nk + (long long)g.ni * g.nk) +
+                        (g.nk == g.bc ? 1LL : 2LL) * g.bc * g.ni * g.nj;
     const int threads = 256;
     const long long blocks = (n + threads - 1) / threads;
     k_boundary<NS><<<dim3((unsigned)blocks), threads, 0, a.stream>>>(*a.mech, g, a.st);

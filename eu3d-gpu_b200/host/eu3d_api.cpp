@@ -516,8 +516,9 @@ eu_status eu_create(const eu_config *cfg, eu_handle **out)
     h->g.d_nk = make_fastdiv(unsigned(h->nk));
     h->g.d_njnk = make_fastdiv(unsigned(h->nj) * unsigned(h->nk));
     h->g.d_nink = make_fastdiv(unsigned(h->ni) * unsigned(h->nk));
-    h->g.d_ghost = make_fastdiv(unsigned(2 * h->bc));
-    h->g.d_ghost_nj = make_fastdiv(unsigned(2 * h->bc) * unsigned(h->nj));
+    const unsigned zper = unsigned(h->nk == h->bc ? h->bc : 2 * h->bc); // threads a row of z ghosts
+    h->g.d_ghost = make_fastdiv(zper);
+    h->g.d_ghost_nj = make_fastdiv(zper * unsigned(h->nj));
     h->g.d_nz = make_fastdiv(unsigned(h->nz));
     h->g.d_nynz = make_fastdiv(unsigned(h->ny) * unsigned(h->nz));
     h->g.bc_kind = cfg->boundary;
