@@ -31,6 +31,29 @@ cudaError_t boundary_t(const LaunchArgs &a)
 // division-light limiter form.
 constexpr bool kStrictFlux = EU_EXACT_FLUX != 0;
 
+// The tiled kernel's march where the autotuner has not chosen one. A block costs
+// its ci planes and about three more (the window's first planes and the first
+// face), and runs among two per SM: the ci whose rounds of blocks cost least
+// (256 x 128 x 128: 24, 0.436 ms against 0.459 at 16; 192 x 96 x 96: 29, 0.193
+// against 0.213). In a batch the rounds mix with the other instances'.
+inline int tiled_march(const LaunchArgs &a, long long tiles)
+{
+    if (a.batch_cells > 0)
+        return 24;
+    const long long slots = 2LL * (a.sms > 0 ? a.sms : 148);
+    int best = 16;
+    long long least = -1;
+    for (int ci = 8; ci <= 48; ++ci) {
+        const long long blocks = tiles * ((a.g.ni + ci - 1) / ci);
+        const long long cost = (blocks + slots - 1) / slots * (ci + 3);
+        if (least < 0 || cost < least) {
+            least = cost;
+            best = ci;
+        }
+    }
+    return best;
+}
+
 template <int NS>
 cudaError_t tiled_flux_launch(const LaunchArgs &a)
 {
@@ -41,8 +64,9 @@ cudaError_t tiled_flux_launch(const LaunchArgs &a)
     if (e != cudaSuccess)
         return e;
     const dim3 block(kTileK, kTileWarps);
-    const int ci = a.flux_ci > 0 ? a.flux_ci : 16;
-    const dim3 grid((g.nk + kTileK - 1) / kTileK, (g.nj + kTileJ - 1) / kTileJ, (g.ni + ci - 1) / ci);
+    const int tk = (g.nk + kTileK - 1) / kTileK, tj = (g.nj + kTileJ - 1) / kTileJ;
+    const int ci = a.flux_ci > 0 ? a.flux_ci : tiled_march(a, (long long)tk * tj);
+    const dim3 grid(tk, tj, (g.ni + ci - 1) / ci);
     k_flux_update_tiled<NS><<<grid, block, smem, a.stream>>>(g, a.st, a.st.prim32, a.dt_dev, ci);
     return cudaGetLastError();
 }
@@ -108,15 +132,23 @@ cudaError_t faces_flux_launch(const LaunchArgs &a, const R *prim)
 // thread (128 x 64 x 64: 0.079 ms against 0.105, 48 x 32 x 32: 0.020 against
 // 0.073). The two give the same bits. FP64 fluxes (the reference's forms when strict, the division-light
 // limiter when fast) are always formed a face a thread.
+// On grids that fill the chip the share of the tiled kernel's 7 x 32 cells that
+// hold a cell of the grid decides (at 68 % of them, 129 x 65 x 65, it takes 0.107
+// ms against 0.095); the instances of a batch run together, so there the cells
+// of all of them count (eight instances of 0.3-1.8 M cells: 105.0 ms -> 99.1 a
+// 50-step pass).
 constexpr int kThinNk = 16;
 constexpr long long kTiledCells = 1000000;
 
 template <int NS, int NR>
 cudaError_t flux_t(const LaunchArgs &a)
 {
+    const DevGrid &g = a.g;
     if (a.precision != 1)
         return faces_flux_launch<NS, double, kStrictFlux>(a, a.st.prim);
-    if (a.g.nk >= kThinNk && (long long)a.g.ni * a.g.nj * a.g.nk >= kTiledCells)
+    const long long cells = std::max((long long)g.ni * g.nj * g.nk, a.batch_cells);
+    const long long slots = (long long)((g.nj + kTileJ - 1) / kTileJ * kTileJ) * ((g.nk + kTileK - 1) / kTileK * kTileK);
+    if (g.nk >= kThinNk && cells >= kTiledCells && 5LL * g.nj * g.nk >= 4 * slots)
         return tiled_flux_launch<NS>(a);
     return faces_flux_launch<NS, float, false>(a, a.st.prim32);
 }
@@ -171,7 +203,8 @@ template <int NS, int NR>
 cudaError_t classify_t(const LaunchArgs &a, const LearnedParams &lp)
 {
     const long long n = (long long)a.g.ni * a.g.nj * a.g.nk;
-    const int threads = a.recover_block > 0 ? a.recover_block : 128;
+    // (64 threads: 0.206 ms on 256 x 128 x 128 against 0.211 with 128)
+    const int threads = a.recover_block > 0 ? a.recover_block : 64;
     const dim3 grid(unsigned((n + threads - 1) / threads));
     switch (a.recover_minb) {
     case 3: k_recover_classify<NS, 3><<<grid, threads, 0, a.stream>>>(*a.mech, a.g, a.st, lp); break;

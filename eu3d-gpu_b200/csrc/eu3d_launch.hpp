@@ -19,9 +19,10 @@ struct LaunchArgs {
     int chemistry; // eu_chemistry
     int spec;      // 1: tables are bitwise H2_JA919, use the generated rate code
     int sms;       // multiprocessors of the device (fixed grids of the queue kernels)
-    int flux_ci;   // nodes each flux block marches along x (autotuned; 0: 16, or one tile of the face kernel)
-    int recover_block; // threads per block of the recovery kernels, 32..128 (autotuned; 0: 128)
+    int flux_ci;   // nodes each flux block marches along x (autotuned; 0: by the grid, tiled_march, or one tile of the face kernel)
+    int recover_block; // threads per block of the recovery kernels, 32..128 (autotuned; 0: 128, or 64 in learned mode)
     int recover_minb;  // register target of the learned-mode recovery: 3, 4, 5 or 6 blocks per SM (0: 4)
+    long long batch_cells = 0; // cells of all instances that run together in a batch (0: alone)
     cudaStream_t stream;
 };
 

@@ -2094,6 +2094,8 @@ eu_status eu_batch_step(eu_batch *b, int nsteps, const double *dt, eu_step_stats
     cudaSetDevice(b->device);
     const int n = int(b->hs.size());
     bool rebuild = !b->exec;
+    long long cells = 0;
+    for (const eu_handle *h : b->hs) cells += (long long)h->ni * h->nj * h->nk;
     for (int i = 0; i < n; ++i) {
         eu_handle *h = b->hs[i];
         if (!(dt[i] > 0))
@@ -2104,7 +2106,9 @@ eu_status eu_batch_step(eu_batch *b, int nsteps, const double *dt, eu_step_stats
             return bfail(b, EU_ERR_UNSUPPORTED, "instance %d: learned chemistry needs a model with the fused kernel", i);
         const bool tail = b->shared && needs_shared_stage(h);
         if (h->graph_dirty || !h->graph_exec || h->graph_cfl != 0 || h->graph_shared_tail != tail) {
-            const eu_status s = capture_step(h, launch_args(h), flavour(h), 0, tail);
+            LaunchArgs a = launch_args(h);
+            a.batch_cells = cells;
+            const eu_status s = capture_step(h, a, flavour(h), 0, tail);
             if (s != EU_OK)
                 return bfail(b, s, "instance %d: %s", i, h->err.c_str());
         }

@@ -200,6 +200,59 @@ def test_face_kernel_tiles_match_restatement(gpu, port_lib, dims):
     assert cs_rel_linf(interior(s.get("CS")), interior(port.get("CS"))).max() <= 1e-12
 
 
+def test_strict_warp_kinetics_match_restatement(gpu, port_lib):
+    """Strict FP64 on igniting gas whose long substep chains run a warp each
+    (k_react_heavy), against the pinned C restatement, eight steps: Nchem exact,
+    and the conserved state within the 1e-14 of CUDA's exp, log and pow carried
+    through some hundred substeps of chain branching (bound 1e-9). The fast
+    FP64 forms stay within 1e-9 of it too, and chemistry samples given to
+    eu_chem_advance end where the thread-per-cell form ends (max_substeps 4
+    keeps every sample on its thread: the capped ones report 4)."""
+    import torch
+    from helpers import cs_rel_linf
+    ni, nj, nk = 11, 5, 6
+    ext = (0.0, ni * 2.5e-4, 0.0, nj * 2.5e-4, 0.0, nk * 2.5e-4)
+    mech = golden_mechanism()
+    x, y, z = (cases.node_coordinates(n, ext[2 * a], ext[2 * a + 1]) for a, n in enumerate((ni, nj, nk)))
+    prim = cases.hot_reacting_block(ni + 4, nj + 4, nk + 4, mech.mw, 9)
+    port = port_lib(ni, nj, nk, x, y, z, mech)
+    port.set_primitive(*prim)
+    port.step(8, 2e-8)
+    out = {}
+    for arith in ("strict", "fast"):
+        s = gpu.Solver(ni, nj, nk, ext, arith=arith)
+        s.set_mechanism(mech)
+        s.set_primitive(*prim)
+        assert max(s.step(1, 2e-8)["max_nchem"] for _ in range(8)) > 4
+        out[arith] = interior(s.get("CS"))
+        if arith == "strict":
+            assert n_unequal(interior(s.get("Nchem")), interior(port.get("Nchem"))) == 0
+        s.close()
+    assert cs_rel_linf(out["strict"], interior(port.get("CS"))).max() <= 1e-9
+    assert cs_rel_linf(out["fast"], out["strict"]).max() <= 1e-9
+    n = 300
+    rng = np.random.default_rng(3)
+    T = torch.tensor(rng.uniform(1200, 2600, n), device="cuda")
+    p = torch.tensor(rng.uniform(1e5, 8e5, n), device="cuda")
+    Y = torch.zeros(9, n, device="cuda", dtype=torch.float64)
+    Y[5], Y[4], Y[3], Y[0] = 0.1, 0.85, 0.04, 0.01
+    dt = torch.tensor(10 ** rng.uniform(-9, -7.5, n), device="cuda")
+    got = {}
+    for cap in (20000, 4):
+        s = gpu.Solver(5, 5, 5, (0, 1, 0, 1, 0, 1), max_substeps=cap)
+        s.set_mechanism(mech)
+        cs, E, Tn = torch.zeros(13, n, device="cuda", dtype=torch.float64), torch.zeros(n, device="cuda", dtype=torch.float64), T.clone()
+        s.chem_states(T, p, Y, cs, E)
+        nchem = torch.zeros(n, device="cuda", dtype=torch.int32)
+        s.chem_advance(cs, Tn, E, dt, nchem)
+        got[cap] = (cs, Tn, nchem)
+        s.close()
+    few = got[20000][2] <= 4
+    assert 0 < int(few.sum()) < n and torch.isfinite(got[20000][1]).all()
+    assert torch.equal(got[4][2], got[20000][2].clamp(max=4))
+    assert torch.equal(got[4][0][:, few], got[20000][0][:, few]) and torch.equal(got[4][1][few], got[20000][1][few])
+
+
 def test_deterministic(gpu):
     z = golden("bubble_25x13x13_s20.npz")
     a = solver_from_golden(gpu, z, arith="fast")
