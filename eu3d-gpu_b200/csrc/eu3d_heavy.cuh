@@ -1,5 +1,5 @@
 // eu3d_heavy.cuh — the stiff kinetics of one cell advanced by a whole warp: the
-// same prediction, trapezoid substeps and state rebuilds as react_cell, for
+// same prediction, trapezoid substeps and state rebuilds as a thread per cell, for
 // cells whose long serial substep chains would set the step's time on one
 // thread. Included by eu3d_kernels.cuh inside the flavour's namespace.
 //
@@ -192,8 +192,14 @@ __device__ __forceinline__ double heavy_rates(const HeavyTables<NS, NR> &t, Heav
     }
     const double RT = kRUniv * T, RuT = kRuCal * T, p0 = kP0 * 1e-6;
     const double b = t.bf[lane], E = t.eaf[lane], Xr = t.xr[lane];
+    // powers by integer exponents as selects (the thread form's values); the
+    // general power on the lanes that need one
+    double tp = b == 1.0 ? T : b == -1.0 ? p.inv : 1.0;
+    if (b != 0.0 && b != 1.0 && b != -1.0)
+        tp = pow(T, b);
+    const double invRT = 1.0 / RT;
     const double ex = exp(-E / RuT);
-    const double kf = t.af[lane] * pow_int_or_real(T, b) * (E == 0.0 ? 1.0 : ex);
+    const double kf = t.af[lane] * tp * (E == 0.0 ? 1.0 : ex);
     double rtb = 0.0, rrf = 1.0, rrb = 1.0;
 #pragma unroll
     for (int s = 0; s < NS; ++s) rtb += mc[s] * t.tb[s][lane];
@@ -209,8 +215,9 @@ __device__ __forceinline__ double heavy_rates(const HeavyTables<NS, NR> &t, Heav
     double delta_g = 0.0;
 #pragma unroll
     for (int q = 0; q < 6; ++q) delta_g += t.dg[q][lane] * x.g[t.dgi[q][lane]];
-    const double Kp = exp(-delta_g / RT) * pow_int_or_real(p0, Xr);
-    const double Kc = Kp * pow_int_or_real(RT, -Xr);
+    // (|Xr| <= 1 in the mechanisms that come here)
+    const double Kp = exp(-delta_g / RT) * (Xr == 0.0 ? 1.0 : Xr == 1.0 ? p0 : 1.0 / p0);
+    const double Kc = Kp * (Xr == 0.0 ? 1.0 : Xr == 1.0 ? invRT : RT);
     const double kb = kf / Kc;
     const bool real = lane < NR;
     x.fwd[lane] = real ? kf * rrf : 0.0;
@@ -244,13 +251,12 @@ __device__ __forceinline__ int heavy_advance(const DevMech &m, const HeavyTables
     for (int s = 0; s < NS; ++s) csl = sp == s ? cell.cs[s] : csl;
     double mc[NS];
     auto rates = [&](double &W, double &Q, double &P) {
-        scaled_concentrations<NS>(m, cell, mc);
-        double mcl = 0.0;
-#pragma unroll
-        for (int s = 0; s < NS; ++s) mcl = sp == s ? mc[s] : mcl;
+        const double mcl = (csl / mw * 1000) * 1e-6; // scaled_concentrations, a species a lane
         if (lane < NS)
             x.mc[lane] = mcl;
         __syncwarp();
+#pragma unroll
+        for (int s = 0; s < NS; ++s) mc[s] = x.mc[s];
         const double v = heavy_rates<NS, NR>(t, x, cell.T, mc, lane);
         W = mw * v;
         Q = __shfl_sync(0xffffffffu, v, sp + NS);

@@ -33,6 +33,8 @@ template <int NS>
 __global__ void __launch_bounds__(256) k_boundary(const __grid_constant__ DevMech m, const DevGrid g,
                                                   const DevState st)
 {
+    if (blockIdx.x == 0 && threadIdx.x < kStepWords)
+        st.step_words[threadIdx.x] = 0;
     const int bc = g.bc, ni = g.ni, nj = g.nj, nk = g.nk;
     // z ghosts of a row: on a grid two nodes thick every interior node is the
     // mirror source of one ghost below and one above, and a thread fills both
@@ -892,7 +894,7 @@ __global__ void k_to_f32(const double *__restrict__ src, float *__restrict__ dst
 
 // Post-advection state recovery (Flowfield::Update_after_Adv ->
 // Update_after_CS, src/Flowfield.cpp:1579-1617) followed, in the stiff modes,
-// by the kinetics of react_cell. One thread per interior node.
+// by the kinetics (react_or_defer). One thread per interior node.
 // MINB: resident 128-thread blocks per SM the register allocation aims at
 // (2: no spills, 8 warps; 3 and 4 trade spills for warps; the autotuner picks).
 template <int NS, int NR, bool kReact, class Rt, int MINB = 2>
@@ -973,28 +975,22 @@ __global__ void __launch_bounds__(128, MINB) k_recover_classify(const __grid_con
     }
 }
 
-// Model inputs of the queued cells: T, log10 p, Y_0..Y_{NS-1}, log10 dt, with
-// p = rho R T and R = 8314.34 / Wav (Update_after_CS, src/Flowfield.cpp:1606-1608).
+// Model inputs of the cell at position q of the model's queue: T, log10 p, Y_0 ..
+// Y_{NS-1}, log10 dt, with p = rho R T and R = 8314.34 / Wav (Update_after_CS,
+// src/Flowfield.cpp:1606-1608).
 template <int NS>
-__global__ void k_learned_features(const __grid_constant__ DevMech m, const DevGrid g, const DevState st,
-                                   LearnedParams lp, const double *__restrict__ dt_dev)
+__device__ __forceinline__ void learned_features(const DevMech &m, const LearnedParams &lp, long long q,
+                                                 const CellState<NS> &cell, double dt)
 {
-    // a fixed grid walks the queue (its length is read on the device)
-    const int nq = lp.counts[0];
-    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < nq; q += gridDim.x * blockDim.x) {
-        const long long n3 = g.n3, c = lp.queue[q];
-        CellState<NS> cell;
-        load_recovered<NS>(st, n3, c, cell);
-        float *f = lp.feat + (long long)q * (NS + 3);
-        double inv_w = 0;
+    float *f = lp.feat + q * (NS + 3);
+    double inv_w = 0;
 #pragma unroll
-        for (int s = 0; s < NS; ++s) inv_w += cell.Y[s] / m.mw[s];
-        f[0] = float(cell.T);
-        f[1] = float(log10(cell.T * cell.D * (kRUniv * 1000 * inv_w)));
+    for (int s = 0; s < NS; ++s) inv_w += cell.Y[s] / m.mw[s];
+    f[0] = float(cell.T);
+    f[1] = float(log10(cell.T * cell.D * (kRUniv * 1000 * inv_w)));
 #pragma unroll
-        for (int s = 0; s < NS; ++s) f[2 + s] = float(cell.Y[s]);
-        f[NS + 2] = float(log10(*dt_dev));
-    }
+    for (int s = 0; s < NS; ++s) f[2 + s] = float(cell.Y[s]);
+    f[NS + 2] = float(log10(dt));
 }
 
 // Apply the ensemble's prediction to each queued cell, or send it to the stiff
@@ -1176,7 +1172,8 @@ __global__ void __launch_bounds__(128) k_react_queue(const __grid_constant__ Dev
 // (Reaction::TrapezoidPrediction, src/Reaction.cpp:865-942); a cell needing at
 // most lp.min_nchem substeps takes the stiff kinetics here (its substeps cost
 // less than the model's evaluation and carry no model error), the others are
-// appended to the model's queue (lp.queue, length lp.counts[0]). With
+// appended to the model's queue with their inputs (lp.queue, lp.feat, length
+// lp.counts[0]). With
 // lp.min_nchem <= 0 every active cell goes to the model unpredicted. A fixed
 // grid drains the active queue (length lp.counts[3], warp grabs on counts[4]).
 template <int NS, class Rt>
@@ -1199,12 +1196,12 @@ __global__ void __launch_bounds__(128) k_learned_route(const __grid_constant__ D
         const int q = base + lane;
         bool to_model = false;
         long long c = 0;
+        CellState<NS> cell;
         if (q < nq) {
             c = lp.active[q];
             to_model = true;
+            load_recovered<NS>(st, n3, c, cell);
             if (lp.min_nchem > 0) {
-                CellState<NS> cell;
-                load_recovered<NS>(st, n3, c, cell);
                 double mc[NS];
                 SpeciesRates<NS> rates;
                 const double dtm = *dt_dev;
@@ -1233,8 +1230,11 @@ __global__ void __launch_bounds__(128) k_learned_route(const __grid_constant__ D
             if (lane == __ffs(mask) - 1)
                 at = atomicAdd(&lp.counts[0], __popc(mask));
             at = __shfl_sync(0xffffffffu, at, __ffs(mask) - 1);
-            if (to_model)
-                lp.queue[at + __popc(mask & ((1u << lane) - 1))] = int(c);
+            if (to_model) {
+                at += __popc(mask & ((1u << lane) - 1));
+                lp.queue[at] = int(c);
+                learned_features<NS>(m, lp, at, cell, *dt_dev);
+            }
         }
     }
 }

@@ -165,11 +165,22 @@ cudaError_t react_t(const LaunchArgs &a, bool react)
         k_recover_react<NS, NR, false, TableRates<NS, NR>><<<grid, threads, 0, a.stream>>>(*a.mech, g, a.st, a.dt_dev,
                                                                                            a.max_substeps);
     else if (a.spec == 1 && NS == Mech_JA919::NS && NR == Mech_JA919::NR) {
-        // register target (autotuned): 2, 3 or 4 resident blocks per SM
-        if (a.recover_minb == 4)
+        // Register target, 2, 3 or 4 resident blocks per SM (autotuned, or by the
+        // grid): once the cells fill two blocks a SM, more warps pay for the spills
+        // (129 x 65 x 65 fast: 0.253 / 0.199 / 0.189 ms; 281 x 141 x 2 strict: 0.129 /
+        // 0.095 / 0.102); below, a cell's own chain counts (33 x 17 x 17 strict: 0.041 /
+        // 0.043 / 0.043).
+#ifdef EU_EXACT_RATES
+        constexpr int kFull = 3;
+#else
+        constexpr int kFull = 4;
+#endif
+        const bool full = n > 256LL * (a.sms > 0 ? a.sms : 148);
+        const int minb = a.recover_minb > 0 ? a.recover_minb : full ? kFull : 2;
+        if (minb == 4)
             k_recover_react<NS, NR, true, Mech_JA919, 4><<<grid, threads, 0, a.stream>>>(*a.mech, g, a.st, a.dt_dev,
                                                                                        a.max_substeps);
-        else if (a.recover_minb == 3)
+        else if (minb == 3)
             k_recover_react<NS, NR, true, Mech_JA919, 3><<<grid, threads, 0, a.stream>>>(*a.mech, g, a.st, a.dt_dev,
                                                                                        a.max_substeps);
         else
@@ -218,13 +229,6 @@ cudaError_t classify_t(const LaunchArgs &a, const LearnedParams &lp)
 // The learned-chemistry kernels run on fixed grids that read the queue lengths
 // on the device, so a step needs no host-side count and can be captured.
 inline unsigned queue_grid(const LaunchArgs &a, int per_sm) { return unsigned((a.sms > 0 ? a.sms : 148) * per_sm); }
-
-template <int NS, int NR>
-cudaError_t features_t(const LaunchArgs &a, const LearnedParams &lp)
-{
-    k_learned_features<NS><<<dim3(queue_grid(a, 8)), 128, 0, a.stream>>>(*a.mech, a.g, a.st, lp, a.dt_dev);
-    return cudaGetLastError();
-}
 
 template <int NS, int NR>
 cudaError_t apply_t(const LaunchArgs &a, const LearnedParams &lp)
@@ -347,7 +351,6 @@ cudaError_t launch_to_f32(const double *src, float *dst, long long n, cudaStream
 }
 
 cudaError_t launch_recover_classify(const LaunchArgs &a, const LearnedParams &lp) { EU3D_DISPATCH(classify_t, a, lp) }
-cudaError_t launch_learned_features(const LaunchArgs &a, const LearnedParams &lp) { EU3D_DISPATCH(features_t, a, lp) }
 cudaError_t launch_learned_apply(const LaunchArgs &a, const LearnedParams &lp) { EU3D_DISPATCH(apply_t, a, lp) }
 cudaError_t launch_learned_route(const LaunchArgs &a, const LearnedParams &lp) { EU3D_DISPATCH(route_t, a, lp) }
 cudaError_t launch_react_queue(const LaunchArgs &a, const int *queue, int *count, int counter)
@@ -423,10 +426,9 @@ cudaError_t launch_set_value(double *dst, double v, cudaStream_t s)
 }
 
 const Launchers launchers = {&launch_boundary,         &launch_flux_update,      &launch_recover_react,
-                             &launch_derived,          &launch_recover_classify, &launch_learned_features,
-                             &launch_learned_apply,    &launch_react_queue,      &launch_react_heavy,
-                             &launch_materialize,      &launch_learned_route,    &launch_react_queue_batch,
-                             &launch_react_heavy_batch};
+                             &launch_derived,          &launch_recover_classify, &launch_learned_apply,
+                             &launch_react_queue,      &launch_react_heavy,      &launch_materialize,
+                             &launch_learned_route,    &launch_react_queue_batch, &launch_react_heavy_batch};
 
 #undef EU3D_DISPATCH
 

@@ -21,7 +21,8 @@ struct LaunchArgs {
     int sms;       // multiprocessors of the device (fixed grids of the queue kernels)
     int flux_ci;   // nodes each flux block marches along x (autotuned; 0: by the grid, tiled_march, or one tile of the face kernel)
     int recover_block; // threads per block of the recovery kernels, 32..128 (autotuned; 0: 128, or 64 in learned mode)
-    int recover_minb;  // register target of the learned-mode recovery: 3, 4, 5 or 6 blocks per SM (0: 4)
+    int recover_minb;  // register target, blocks per SM: learned-mode recovery 3 .. 6 (0: 4), stiff kinetics
+                       // 2 .. 4 (0: by the grid)
     long long batch_cells = 0; // cells of all instances that run together in a batch (0: alone)
     cudaStream_t stream;
 };
@@ -35,7 +36,6 @@ struct Launchers {
     cudaError_t (*recover_react)(const LaunchArgs &a, bool react);
     cudaError_t (*derived)(const LaunchArgs &a, int which, double *out);
     cudaError_t (*recover_classify)(const LaunchArgs &a, const LearnedParams &lp);
-    cudaError_t (*learned_features)(const LaunchArgs &a, const LearnedParams &lp);
     cudaError_t (*learned_apply)(const LaunchArgs &a, const LearnedParams &lp);
     cudaError_t (*react_queue)(const LaunchArgs &a, const int *queue, int *count, int counter);
     cudaError_t (*react_heavy)(const LaunchArgs &a, int blocks);
@@ -56,7 +56,6 @@ struct Launchers {
     cudaError_t launch_rk_combine(const LaunchArgs &a, const double *cs0, double ca, double cb);   \
     cudaError_t launch_cfl(const LaunchArgs &a, double cfl, unsigned long long *slot, double *time); \
     cudaError_t launch_recover_classify(const LaunchArgs &a, const LearnedParams &lp);             \
-    cudaError_t launch_learned_features(const LaunchArgs &a, const LearnedParams &lp);             \
     cudaError_t launch_learned_apply(const LaunchArgs &a, const LearnedParams &lp);                \
     cudaError_t launch_learned_route(const LaunchArgs &a, const LearnedParams &lp);                \
     cudaError_t launch_react_queue(const LaunchArgs &a, const int *queue, int *count, int counter); \

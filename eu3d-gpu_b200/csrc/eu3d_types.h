@@ -73,6 +73,7 @@ struct DevState {
     int *nchem;       // plane
     double *cms;      // ns planes (or null)
     unsigned long long *counters; // see CounterIdx
+    unsigned *step_words; // kStepWords words cleared by the ghost fill
     int *heavy;       // mixed precision: {count, next, cells...} of cells left to the warp-per-cell kinetics
     const double *inflow; // ODW x-low ghost values per interior (j, k): 7 + ns primitive planes, then T
     // EU_GHOSTS_STORED: store_cell also writes the z-face ghosts a node is the
@@ -84,21 +85,25 @@ struct DevState {
     int zm_nz, zm_nk, zm_bc;
 };
 
-// Device counters. The first kCntPerStep are statistics of the latest step
-// (cleared before each step); the rest accumulate over one eu_step call so an
-// error in any step of the call is reported.
+// Device counters. The first two accumulate over one eu_step call, so an error in
+// any step of the call is reported; the others are statistics of the latest step.
 enum CounterIdx {
-    kCntMaxNchem = 0,
-    kCntSumNchem = 1,
-    kCntReacting = 2,
-    kCntLearned = 3,
-    kCntFallback = 4,
-    kCntRouted = 5, // learned mode: active cells the Nchem routing gave to the stiff kinetics
-    kCntPerStep = 6,
-    kCntNonfinite = 6,
-    kCntBadNchem = 7,
+    kCntNonfinite = 0,
+    kCntBadNchem = 1,
+    kCntMaxNchem = 2,
+    kCntSumNchem = 3,
+    kCntReacting = 4,
+    kCntLearned = 5,
+    kCntFallback = 6,
+    kCntRouted = 7, // learned mode: active cells the Nchem routing gave to the stiff kinetics
     kCntCount = 8
 };
+// The words a step starts from zero, in one piece of memory: the step's
+// counters, the learned mode's queue counts and the deferred queue's {count,
+// next}. The ghost fill, the step's first kernel, clears them (a memset node
+// each cost about as much as a small grid's kernel).
+constexpr int kStepCounterWords = 2 * (kCntCount - 2), kQueueCountWords = 6, kHeavyHeadWords = 2;
+constexpr int kStepWords = kStepCounterWords + kQueueCountWords + kHeavyHeadWords;
 
 // One instance of a batch in the batch's shared kinetics stage: its state, its
 // dt, and its stiff-fallback queue (learned mode; null otherwise). The

@@ -56,6 +56,7 @@ struct eu_handle {
     int heavy_blocks = 0;    // persistent grid of the warp-per-cell kinetics
     bool heavy_fits = false; // whether the mechanism has that form
     int *heavy_queue = nullptr;
+    int *queue_counts = nullptr; // LearnedParams::counts
     int *sample_queue = nullptr; // eu_chem_advance's deferred samples (grown with the calls, kept)
     long long sample_capacity = 0;
     // mixed precision: the timestep keeps only the FP32 primitive planes
@@ -231,13 +232,18 @@ eu_status install_mechanism(eu_handle *h, const MechanismTables &m)
     if ((s = dalloc(h, &h->st.nchem, size_t(n3))) != EU_OK) return s;
     if (h->cfg.record_sources)
         if ((s = dalloc(h, &h->st.cms, size_t(ns) * n3)) != EU_OK) return s;
-    if ((s = dalloc(h, &h->st.counters, size_t(kCntCount))) != EU_OK) return s;
-    if ((s = dalloc(h, &h->d_scratch, size_t(n3))) != EU_OK) return s;
-    if (h->cfg.chemistry != EU_CHEM_FROZEN) {
-        if ((s = dalloc(h, &h->heavy_queue, size_t(2) + size_t(h->ni) * h->nj * h->nk)) != EU_OK) return s;
-        CK(h, cudaMemsetAsync(h->heavy_queue, 0, 2 * sizeof(int), h->stream));
+    // counters, queue counts and the deferred queue in one piece (kStepWords)
+    const size_t deferred = h->cfg.chemistry != EU_CHEM_FROZEN ? size_t(h->ni) * h->nj * h->nk : 0;
+    int *words = nullptr;
+    if ((s = dalloc(h, &words, size_t(4) + kStepWords + deferred)) != EU_OK) return s;
+    h->st.counters = reinterpret_cast<unsigned long long *>(words);
+    h->st.step_words = reinterpret_cast<unsigned *>(words + 4);
+    h->queue_counts = words + 4 + kStepCounterWords;
+    if (deferred) {
+        h->heavy_queue = h->queue_counts + kQueueCountWords;
         h->st.heavy = h->heavy_fits ? h->heavy_queue : nullptr;
     }
+    if ((s = dalloc(h, &h->d_scratch, size_t(n3))) != EU_OK) return s;
     CK(h, cudaMemsetAsync(h->st.prim, 0, size_t(7 + ns) * n3 * sizeof(double), h->stream));
     if (h->st.prim32)
         CK(h, cudaMemsetAsync(h->st.prim32, 0, size_t(7 + ns) * n3 * sizeof(float), h->stream));
@@ -247,7 +253,7 @@ eu_status install_mechanism(eu_handle *h, const MechanismTables &m)
     CK(h, cudaMemsetAsync(h->st.nchem, 0, size_t(n3) * sizeof(int), h->stream));
     if (h->st.cms)
         CK(h, cudaMemsetAsync(h->st.cms, 0, size_t(ns) * n3 * sizeof(double), h->stream));
-    CK(h, cudaMemsetAsync(h->st.counters, 0, kCntCount * sizeof(unsigned long long), h->stream));
+    CK(h, cudaMemsetAsync(h->st.counters, 0, (4 + kStepWords) * sizeof(int), h->stream));
     return EU_OK;
 }
 
@@ -891,7 +897,7 @@ void element_projector(const MechanismTables &m, double (&P)[kMaxS][kMaxS])
 bool defers_fallback(const eu_handle *h) { return h->cfg.precision == EU_PREC_MIXED; }
 
 // One learned-chemistry phase of a step: recover + classify every cell,
-// features of the queued cells, the ensemble, gate + apply, stiff fallback.
+// routing and features of the active cells, the ensemble, gate + apply, stiff fallback.
 // The queue kernels read the queue lengths on the device; with the model's
 // fused inference kernel nothing here waits on the host, so the phase can be
 // captured in the step's graph. Otherwise (a model shape without the fused
@@ -900,8 +906,7 @@ eu_status learned_chemistry(eu_handle *h, const LaunchArgs &a, const Launchers &
 {
     LearnedParams lp = h->lp;
     const int ns = h->mech.ns;
-    CK(h, cudaMemsetAsync(lp.counts, 0, 5 * sizeof(int), h->stream));
-    // recovery appends the active cells to lp.active (length counts[3]); the
+    // (the counts start from zero, kStepWords) recovery appends the active cells to lp.active (length counts[3]); the
     // routing sends the ones needing few substeps to the stiff kinetics and
     // the rest to the model's queue (lp.queue, length counts[0])
     LearnedParams lpa = lp;
@@ -909,8 +914,7 @@ eu_status learned_chemistry(eu_handle *h, const LaunchArgs &a, const Launchers &
     lpa.counts = lp.counts + 3;
     CK(h, L.recover_classify(a, lpa));
     CK(h, L.learned_route(a, lp));
-    CK(h, L.learned_features(a, lp));
-    *launches += 3;
+    *launches += 2;
     if (mlp_has_fused(h->model)) {
         lp.pred_row = (long long)lp.members * (ns + 1);
         lp.pred_mem = ns + 1;
@@ -918,7 +922,7 @@ eu_status learned_chemistry(eu_handle *h, const LaunchArgs &a, const Launchers &
                                         lp.pred_mem, h->stream);
         if (s != EU_OK)
             return fail(h, s, "learned model: %s", eu_mlp_last_error(h->model));
-        ++*launches;
+        *launches += 2;
     } else {
         CK(h, cudaMemcpyAsync(h->h_counts, lp.counts, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
         CK(h, cudaStreamSynchronize(h->stream));
@@ -956,9 +960,8 @@ eu_status step_launches(eu_handle *h, const LaunchArgs &a, const Launchers &L, b
     const bool learned = h->cfg.chemistry == EU_CHEM_LEARNED;
     if (cfl > 0) { // this step's dt from the current state (Flowfield::CFLcondition)
         CK(h, strict::launch_cfl(a, cfl, h->d_cfl_slot, h->d_time));
-        *launches += 2;
+        ++*launches;
     }
-    CK(h, cudaMemsetAsync(h->st.counters, 0, kCntPerStep * sizeof(unsigned long long), h->stream));
     if (prof) CK(h, cudaEventRecord(h->pev[0], h->stream));
     if (h->time_scheme == EU_TIME_RK3) {
         // three-stage TVD Runge-Kutta advection (Shu-Osher): each stage its ghost
@@ -993,8 +996,6 @@ eu_status step_launches(eu_handle *h, const LaunchArgs &a, const Launchers &L, b
         *launches += 2;
     }
     const bool heavy = h->st.heavy && (learned || react);
-    if (heavy)
-        CK(h, cudaMemsetAsync(h->st.heavy, 0, 2 * sizeof(int), h->stream));
     if (learned) {
         eu_status ls = learned_chemistry(h, a, L, launches, !shared_tail);
         if (ls != EU_OK)
@@ -1115,7 +1116,7 @@ eu_status eu_set_learned(eu_handle *h, eu_mlp *model, const eu_learned_config *l
         if ((s = dalloc(h, &lp.queue, size_t(cap))) != EU_OK) return s;
         if ((s = dalloc(h, &lp.fallback, size_t(cap))) != EU_OK) return s;
         if ((s = dalloc(h, &lp.active, size_t(cap))) != EU_OK) return s;
-        if ((s = dalloc(h, &lp.counts, size_t(5))) != EU_OK) return s;
+        lp.counts = h->queue_counts;
         h->lp_capacity = cap;
     }
     if (!h->h_counts)
