@@ -1402,9 +1402,12 @@ __global__ void k_set_value(double *dst, double v) { *dst = v; }
 // precision). The spacings are the interior ones (the reference takes them
 // from its first two ghost nodes, the same on a uniform grid with three or
 // more nodes per axis). Positive doubles order as their bit patterns, so the
-// block minima combine with an integer atomicMin into *slot (non-finite values
-// map to the largest key and never win).
-__global__ void __launch_bounds__(256) k_cfl_min(const DevGrid g, const DevState st, unsigned long long *slot)
+// block minima combine with an integer atomicMin into slot[0] (non-finite values
+// map to the largest key and never win). The last block to arrive (the ticket in
+// slot[1]) sets dt = cfl times the minimum, which the step's kernels read at
+// *dt_dev, adds it to *time and resets the slot for the next step.
+__global__ void __launch_bounds__(256) k_cfl(const DevGrid g, const DevState st, unsigned long long *slot, double cfl,
+                                             double *dt_dev, double *time)
 {
     const long long ncell = (long long)g.ni * g.nj * g.nk;
     const double dx = g.x[g.bc + 1] - g.x[g.bc], dy = g.y[g.bc + 1] - g.y[g.bc];
@@ -1448,17 +1451,14 @@ __global__ void __launch_bounds__(256) k_cfl_min(const DevGrid g, const DevState
     if (threadIdx.x == 0) {
         for (int w = 1; w < (int)(blockDim.x >> 5); ++w) b = wmin[w] < b ? wmin[w] : b;
         atomicMin(slot, b);
+        __threadfence();
+        unsigned *ticket = reinterpret_cast<unsigned *>(slot + 1);
+        if (atomicInc(ticket, gridDim.x - 1) == gridDim.x - 1) { // wraps to 0
+            const double dt = cfl * __longlong_as_double((long long)atomicExch(slot, 0x7ff0000000000000ULL));
+            *dt_dev = dt;
+            *time += dt;
+        }
     }
-}
-
-// dt = cfl * the minimum; the step's kernels read *dt_dev; *time accumulates
-// the steps' dt; the slot is reset for the next step.
-__global__ void k_cfl_finish(unsigned long long *slot, double cfl, double *dt_dev, double *time)
-{
-    const double dt = cfl * __longlong_as_double((long long)*slot);
-    *dt_dev = dt;
-    *time += dt;
-    *slot = 0x7ff0000000000000ULL;
 }
 
 } // namespace EU3D_NS

@@ -382,8 +382,7 @@ cudaError_t launch_cfl(const LaunchArgs &a, double cfl, unsigned long long *slot
 {
     const long long n = (long long)a.g.ni * a.g.nj * a.g.nk;
     const unsigned blocks = unsigned(std::min<long long>((n + 255) / 256, (long long)(a.sms > 0 ? a.sms : 148) * 8));
-    k_cfl_min<<<blocks, 256, 0, a.stream>>>(a.g, a.st, slot);
-    k_cfl_finish<<<1, 1, 0, a.stream>>>(slot, cfl, const_cast<double *>(a.dt_dev), time);
+    k_cfl<<<blocks, 256, 0, a.stream>>>(a.g, a.st, slot, cfl, const_cast<double *>(a.dt_dev), time);
     return cudaGetLastError();
 }
 

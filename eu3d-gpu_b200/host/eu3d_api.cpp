@@ -39,7 +39,7 @@ struct eu_handle {
     DevState st{};
     double *d_xyz = nullptr;
     double *d_dt = nullptr;
-    unsigned long long *d_cfl_slot = nullptr; // CFL minimum of the step being set up
+    unsigned long long *d_cfl_slot = nullptr; // CFL minimum of the step being set up, and its blocks' ticket
     double *d_time = nullptr;                 // time advanced by the CFL-driven steps of a call
     double *d_scratch = nullptr;
     double *d_inflow = nullptr; // EU_BC_ODW x-low tables ((8 + ns) planes of nj * nk)
@@ -489,13 +489,13 @@ eu_status eu_create(const eu_config *cfg, eu_handle **out)
     eu_status s;
     if ((s = dalloc(h, &h->d_xyz, size_t(h->nx + h->ny + h->nz))) != EU_OK ||
         (s = dalloc(h, &h->d_dt, size_t(1))) != EU_OK || (s = dalloc(h, &h->d_time, size_t(1))) != EU_OK ||
-        (s = dalloc(h, &h->d_cfl_slot, size_t(1))) != EU_OK) {
+        (s = dalloc(h, &h->d_cfl_slot, size_t(2))) != EU_OK) {
         eu_destroy(h);
         return s;
     }
     {
-        const unsigned long long inf_bits = 0x7ff0000000000000ULL; // +inf: no minimum yet
-        if (cudaMemcpy(h->d_cfl_slot, &inf_bits, sizeof inf_bits, cudaMemcpyHostToDevice) != cudaSuccess) {
+        const unsigned long long slot[2] = {0x7ff0000000000000ULL, 0}; // +inf: no minimum yet; the blocks' ticket
+        if (cudaMemcpy(h->d_cfl_slot, slot, sizeof slot, cudaMemcpyHostToDevice) != cudaSuccess) {
             eu_destroy(h);
             return EU_ERR_CUDA;
         }
@@ -922,7 +922,7 @@ eu_status learned_chemistry(eu_handle *h, const LaunchArgs &a, const Launchers &
                                         lp.pred_mem, h->stream);
         if (s != EU_OK)
             return fail(h, s, "learned model: %s", eu_mlp_last_error(h->model));
-        *launches += 2;
+        ++*launches;
     } else {
         CK(h, cudaMemcpyAsync(h->h_counts, lp.counts, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
         CK(h, cudaStreamSynchronize(h->stream));
