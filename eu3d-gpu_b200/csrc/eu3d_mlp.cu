@@ -99,11 +99,10 @@ cudaError_t train_weights(const TrainParams &p, int sms, cudaStream_t s)
     const cudaError_t e = limit.ensure(k_train_dw, kDwSmem);
     if (e != cudaSuccess)
         return e;
-    // the rows split so that about two CTAs per SM run, 64 rows at the least
-    const int jobs = p.hidden * ((p.width + 127) / 128) + (p.out_pad + 127) / 128;
-    const int slabs = (p.n + kDwK - 1) / kDwK;
-    const int want = 2 * sms / (jobs * p.members), splits = want < 1 ? 1 : want > slabs ? slabs : want;
-    k_train_dw<<<dim3(unsigned(splits), unsigned(jobs), unsigned(p.members)), kDwThreads, kDwSmem, s>>>(p, splits);
+    // one CTA per SM: `unit` for the narrow first layer and outputs, twice that for
+    // the layers between
+    const int parts = 2 * p.hidden * p.members, unit = sms / parts > 1 ? sms / parts : 1;
+    k_train_dw<<<dim3(unsigned(2 * p.hidden * unit), unsigned(p.members)), kDwThreads, kDwSmem, s>>>(p, unit);
     return cudaGetLastError();
 }
 

@@ -77,24 +77,20 @@ cudaError_t mlp_fused(const FusedMlpParams &p, const float *feat, int ld_feat, i
 // (row-major Wb, K-slabs of it and of its transpose) and its scratch for a batch
 // of n rows.
 constexpr int kTrainRows = 128; // rows of a tile
-// Leading dimension of the transposed arrays of an n-row batch: whole 128-byte
-// lines, one more than the batch's, so that the rows of a power-of-two batch
-// do not all start on the same memory channels.
-inline int train_ld(int n) { return (n + 63) / 64 * 64 + 64; }
 struct TrainMember {
     float *P, *G, *M, *V;
     const float *bias[kFusedMaxLayers];
     float *gW[kFusedMaxLayers], *gb[kFusedMaxLayers];
     __nv_bfloat16 *Wb[kFusedMaxLayers], *slabs[kFusedMaxLayers], *slabs_t[kFusedMaxLayers];
-    float *Z;                      // pre-activations [hidden][n x width]
-    // transposed (rows along the leading dimension ld): [in_pad], [hidden][width]
-    // twice, [out_pad]
+    // planes of a batch, 128-row tile by tile: pre-activations [hidden][tile][width][128];
+    // inputs, activations, layer gradients and output gradients with the rows along K
+    // in the core-matrix layout, [layer][tile][128 / 8][columns][8]
+    float *ZT;
     __nv_bfloat16 *XT, *HT, *dZT, *dYT;
     unsigned long long key;        // of the batch's draw
 };
 struct TrainParams {
     int n, n_in, in_pad, width, hidden, n_out, out_pad;
-    int ld;                        // of the transposed arrays (train_ld)
     int params;                    // padded parameters of a member
     int first, members;            // members [first, first + members)
     const float *X, *T;            // fp32 rows [rows x n_in], [rows x n_out]

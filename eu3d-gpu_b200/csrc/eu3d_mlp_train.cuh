@@ -8,18 +8,21 @@
 // way back its layer gradients, in shared memory as the next MMA's A operand
 // (two CTAs per SM: one's epilogue under the other's MMAs). What the weight
 // gradients need, the bf16 inputs and gradients of every layer, goes to global
-// memory transposed (rows along K), which costs no extra pass: a lane holds a
-// row, so a column's 32 values are one contiguous store. The pre-activations
-// (fp32, for SiLU') are written and read back by the same thread. k_train_dw
-// then forms every layer's dW = dZ^T H of every member in one launch, split
-// along the rows to fill the chip. k_train_adam updates the parameters, packs
-// the bf16 weights for the next step and clears the gradients.
+// memory as K slabs with the rows along K, in the layout the MMAs read, tile by
+// tile. The pre-activations (fp32, for SiLU') are kept a column at a time and
+// read back by the same thread. k_train_dw then forms every layer's dW = dZ^T H
+// of every member in one launch, split along the rows to fill the chip.
+// k_train_adam updates the parameters, packs the bf16 weights for the next step
+// and clears the gradients.
 //
 // Rounding points are the layer-wise path's: bf16 inputs, weights, activations
 // and layer gradients, fp32 accumulation, bias gradients from the fp32 layer
 // gradients. Launched layer by layer, with transposes, column sums and
 // one-value-a-lane epilogues of their own, a step of three members at batch
-// 16384 took 3.2 ms (about 165 launches).
+// 16384 took 3.2 ms (about 165 launches); in three kernels, with the planes
+// transposed row by row and staged into the MMAs' layout by k_train_dw, 0.35 ms
+// (rows 0.25, weight gradients 0.10); with the planes written in that layout
+// 0.26 ms.
 #pragma once
 
 #include <cuda_bf16.h>
@@ -80,8 +83,13 @@ __global__ void __launch_bounds__(kTrainThreads, 2) k_train_rows(const __grid_co
     const int lrow = quad * 32 + lane, row = blockIdx.x * kTrainRows + lrow;
     const bool valid = row < p.n;
     const long long src = !valid ? 0 : p.drawn ? (long long)train_row(mem.key, row, p.rows) : row;
-    const unsigned ld = unsigned(p.ld);
-    const size_t wide = size_t(p.width) * ld, zwide = size_t(p.width) * p.n; // one layer's planes
+    // this tile's part of a plane of `cols` columns: as K slabs (K = rows) in the
+    // core-matrix layout, and of the fp32 pre-activations, columns outermost
+    const size_t tiles = gridDim.x, tile = blockIdx.x;
+    auto slab_rows = [&](__nv_bfloat16 *plane, int layer, int cols) {
+        return plane + (layer * tiles + tile) * size_t(cols) * kTrainRows + (size_t(lrow / 8) * cols) * 8 + lrow % 8;
+    };
+    auto z_rows = [&](int layer) { return mem.ZT + (layer * tiles + tile) * size_t(p.width) * kTrainRows + lrow; };
 
     if (warp == 0) {
         tc::tmem_alloc(tslot, 256);
@@ -96,6 +104,7 @@ __global__ void __launch_bounds__(kTrainThreads, 2) k_train_rows(const __grid_co
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     // features -> first A operand and, transposed, the first layer's input
+    __nv_bfloat16 *xt = slab_rows(mem.XT, 0, p.in_pad);
     for (int kc = half; kc < p.in_pad / 8; kc += 2) {
         __align__(16) __nv_bfloat16 v[8];
 #pragma unroll
@@ -105,8 +114,7 @@ __global__ void __launch_bounds__(kTrainThreads, 2) k_train_rows(const __grid_co
             if (valid && c < p.n_in)
                 f = (p.X[src * p.n_in + c] - p.in_shift[c]) * p.in_scale[c];
             v[q] = __float2bfloat16_rn(f);
-            if (valid)
-                mem.XT[unsigned(c) * ld + unsigned(row)] = v[q];
+            xt[c * 8] = v[q];
         }
         put_operand(act, kc * 8, lrow, v);
     }
@@ -157,19 +165,20 @@ __global__ void __launch_bounds__(kTrainThreads, 2) k_train_rows(const __grid_co
     // 32 pre-activations of this thread's row, columns c0 ..
     float zz[32];
     auto load_z = [&](const float *z, int c0) {
+        z += c0 * kTrainRows;
+        if (c0 + 32 <= p.width) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if (valid && c0 + j * 4 < p.width)
-                a = *reinterpret_cast<const float4 *>(z + c0 + j * 4);
-            zz[j * 4] = a.x, zz[j * 4 + 1] = a.y, zz[j * 4 + 2] = a.z, zz[j * 4 + 3] = a.w;
+            for (int u = 0; u < 32; ++u) zz[u] = z[u * kTrainRows];
+        } else {
+#pragma unroll
+            for (int u = 0; u < 32; ++u) zz[u] = c0 + u < p.width ? z[u * kTrainRows] : 0.0f;
         }
     };
 
     for (int q = 0; q < ngemm; ++q) {
         // the way back: the first pre-activations come while the MMAs run
         if (q > L)
-            load_z(mem.Z + (2 * L - q) * zwide + (size_t)row * p.width, half * 32);
+            load_z(z_rows(2 * L - q), half * 32);
         // ------------------------------------------------------------ MMAs
         if (tid == 0) {
             const __nv_bfloat16 *w;
@@ -217,8 +226,8 @@ __global__ void __launch_bounds__(kTrainThreads, 2) k_train_rows(const __grid_co
         }
         // -------------------------------------------------------- epilogue
         if (q < L) { // hidden layer: z, silu(z) as bf16
-            float *z = mem.Z + q * zwide + (size_t)row * p.width;
-            __nv_bfloat16 *ht = mem.HT + q * wide + row;
+            float *z0 = z_rows(q);
+            __nv_bfloat16 *ht0 = slab_rows(mem.HT, q, p.width);
             const float *bias = mem.bias[q];
             for (int c0 = half * 32; c0 < p.width; c0 += 64) {
                 float v[32];
@@ -237,18 +246,19 @@ __global__ void __launch_bounds__(kTrainThreads, 2) k_train_rows(const __grid_co
                             h[u] = __float2bfloat16_rn(silu(v[j * 8 + u]));
                         }
                         put_operand(act, c, lrow, h);
-                        if (valid) {
+                        __nv_bfloat16 *ht = ht0 + c * 8;
+                        float *z = z0 + c * kTrainRows;
 #pragma unroll
-                            for (int u = 0; u < 8; ++u) ht[unsigned(c + u) * ld] = h[u];
-                            *reinterpret_cast<float4 *>(z + c) = make_float4(v[j * 8], v[j * 8 + 1], v[j * 8 + 2], v[j * 8 + 3]);
-                            *reinterpret_cast<float4 *>(z + c + 4) =
-                                make_float4(v[j * 8 + 4], v[j * 8 + 5], v[j * 8 + 6], v[j * 8 + 7]);
+                        for (int u = 0; u < 8; ++u) {
+                            ht[u * 8] = h[u];
+                            z[u * kTrainRows] = v[j * 8 + u];
                         }
                     }
                 }
             }
         } else if (q == L) { // output: loss and its gradient
             float sq = 0.0f;
+            __nv_bfloat16 *yt = slab_rows(mem.dYT, 0, p.out_pad);
             for (int c0 = half * 32; c0 < p.out_pad; c0 += 64) {
                 float v[32];
                 tc::tmem_ld32(trow + c0, v);
@@ -267,8 +277,8 @@ __global__ void __launch_bounds__(kTrainThreads, 2) k_train_rows(const __grid_co
                         }
                         g[u] = __float2bfloat16_rn(d);
                         v[j * 8 + u] = __bfloat162float(g[u]);
-                        if (valid && c + u < p.out_pad)
-                            mem.dYT[unsigned(c + u) * ld + unsigned(row)] = g[u];
+                        if (c + u < p.out_pad)
+                            yt[(c + u) * 8] = g[u];
                     }
                     if (c < p.out_pad)
                         put_operand(act, c, lrow, g);
@@ -282,8 +292,8 @@ __global__ void __launch_bounds__(kTrainThreads, 2) k_train_rows(const __grid_co
                 atomicAdd(&p.loss[e], sq);
         } else { // back through layer l into hidden layer l - 1
             const int l = L - (q - L - 1);
-            const float *z = mem.Z + (l - 1) * zwide + (size_t)row * p.width;
-            __nv_bfloat16 *zt = mem.dZT + (l - 1) * wide + row;
+            const float *z = z_rows(l - 1);
+            __nv_bfloat16 *zt0 = slab_rows(mem.dZT, l - 1, p.width);
             for (int c0 = half * 32; c0 < p.width; c0 += 64) {
                 if (c0 > half * 32)
                     load_z(z, c0);
@@ -301,10 +311,9 @@ __global__ void __launch_bounds__(kTrainThreads, 2) k_train_rows(const __grid_co
                         g[u] = __float2bfloat16_rn(d);
                     }
                     if (c < p.width) {
-                        if (valid) {
+                        __nv_bfloat16 *zt = zt0 + c * 8;
 #pragma unroll
-                            for (int u = 0; u < 8; ++u) zt[unsigned(c + u) * ld] = g[u];
-                        }
+                        for (int u = 0; u < 8; ++u) zt[u * 8] = g[u];
                         put_operand(act, c, lrow, g);
                     }
                 }
@@ -332,54 +341,44 @@ __global__ void __launch_bounds__(kTrainThreads, 2) k_train_rows(const __grid_co
         tc::tmem_dealloc(tmem, 256);
 }
 
-// dW = dZ^T H of every layer of every member: one CTA per (K split, 128-row
-// piece of a layer's outputs, member), partial sums added to the fp32 gradient
-// four values at a time. Two cp.async stages of 64 rows feed the MMAs.
-constexpr int kDwThreads = 128, kDwK = 64;
-constexpr size_t kDwSmem = 2 * size_t(128 + 256) * kDwK * 2 + 64;
+// dW = dZ^T H of every layer of every member: a CTA takes a share of the batch's
+// 64-row slabs for one layer (all its outputs and inputs, two 128 x 256
+// accumulators at most) and adds its sums to the fp32 gradient four values at a
+// time. The operands lie in global memory as the MMAs read them, so a slab is one
+// bulk copy each, three of them in flight.
+constexpr int kDwThreads = 256, kDwK = 64, kDwSlots = 3, kDwOperand = 256 * kDwK * 2;
+constexpr size_t kDwSmem = size_t(kDwSlots) * 2 * kDwOperand + 8 * (2 * kDwSlots + 1) + 16;
 
-// rows x kDwK bf16 of a row-major matrix (rows r0.., columns k0..) into the
-// core-matrix layout of a `pitch`-row operand.
-__device__ __forceinline__ void dw_stage(unsigned char *dst, int pitch, const __nv_bfloat16 *src, int ld, int r0, int nrows,
-                                         int k0, int k1)
-{
-    for (int c = threadIdx.x; c < pitch * (kDwK / 8); c += kDwThreads) {
-        const int r = c / (kDwK / 8), kc = c % (kDwK / 8), gk = k0 + kc * 8;
-        const bool in = r0 + r < nrows && gk < k1;
-        tc::cp_async16(dst + (kc * pitch + r) * 16, in ? src + (size_t)(r0 + r) * ld + gk : src, in);
-    }
-}
-
-__global__ void __launch_bounds__(kDwThreads, 2) k_train_dw(const __grid_constant__ TrainParams p, int splits)
+__global__ void __launch_bounds__(kDwThreads, 1) k_train_dw(const __grid_constant__ TrainParams p, int unit)
 {
     extern __shared__ __align__(128) unsigned char smem[];
-    constexpr uint32_t kA = 128 * kDwK * 2, kB = 256 * kDwK * 2;
-    unsigned char *sa[2] = {smem, smem + kA + kB}, *sb[2] = {smem + kA, smem + 2 * kA + kB};
-    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + 2 * (kA + kB));
-    uint32_t *tslot = reinterpret_cast<uint32_t *>(bars + 2);
+    uint64_t *full = reinterpret_cast<uint64_t *>(smem + size_t(kDwSlots) * 2 * kDwOperand), *empty = full + kDwSlots;
+    uint64_t *acc = empty + kDwSlots;
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(acc + 1);
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-    const int e = p.first + blockIdx.z;
-    const TrainMember &mem = p.member[e];
-    const size_t wide = size_t(p.width) * p.ld;
-    // the job: layer l, output rows m0 ..
-    int job = blockIdx.y, l = 0;
-    const int pieces = (p.width + 127) / 128;
-    l = min(job / pieces, p.hidden);
-    const int m0 = (job - l * pieces) * 128;
-    const int M = l == p.hidden ? p.out_pad : p.width, N = l == 0 ? p.in_pad : p.width;
-    const __nv_bfloat16 *A = l == p.hidden ? mem.dYT : mem.dZT + l * wide;
-    const __nv_bfloat16 *B = l == 0 ? mem.XT : mem.HT + (l - 1) * wide;
-    const int slabs = (p.n + kDwK - 1) / kDwK, per = (slabs + splits - 1) / splits;
-    const int k0 = blockIdx.x * per, KT = max(0, min(slabs, k0 + per) - k0);
+    const TrainMember &mem = p.member[p.first + blockIdx.y];
+    // the job: `unit` CTAs for the first layer and for the outputs (one narrow
+    // operand), twice as many for each layer between
+    const int L = p.hidden;
+    const int l = int(blockIdx.x) < unit ? 0 : min(L, (int(blockIdx.x) - unit) / (2 * unit) + 1);
+    const int splits = l == 0 || l == L ? unit : 2 * unit, split = int(blockIdx.x) - (l == 0 ? 0 : unit + (l - 1) * 2 * unit);
+    const int M = l == L ? p.out_pad : p.width, N = l == 0 ? p.in_pad : p.width;
+    const int tiles = (p.n + kTrainRows - 1) / kTrainRows, slabs = tiles * (kTrainRows / kDwK);
+    const __nv_bfloat16 *A = l == L ? mem.dYT : mem.dZT + size_t(l) * tiles * p.width * kTrainRows;
+    const __nv_bfloat16 *B = l == 0 ? mem.XT : mem.HT + size_t(l - 1) * tiles * p.width * kTrainRows;
+    const int per = (slabs + splits - 1) / splits, k0 = split * per, KT = max(0, min(slabs, k0 + per) - k0);
     if (KT == 0)
         return;
     if (warp == 0) {
-        tc::tmem_alloc(tslot, 256);
+        tc::tmem_alloc(tslot, 512);
         tc::tmem_relinquish();
     }
     if (threadIdx.x == 0) {
-        tc::mbar_init(&bars[0], 1);
-        tc::mbar_init(&bars[1], 1);
+        for (int q = 0; q < kDwSlots; ++q) {
+            tc::mbar_init(&full[q], 1);
+            tc::mbar_init(&empty[q], 1);
+        }
+        tc::mbar_init(acc, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     tc::tc_fence_before();
@@ -387,70 +386,64 @@ __global__ void __launch_bounds__(kDwThreads, 2) k_train_dw(const __grid_constan
     tc::tc_fence_after();
     const uint32_t tmem = *tslot;
     bool ok = true;
-    dw_stage(sa[0], 128, A, p.ld, m0, M, k0 * kDwK, p.n);
-    dw_stage(sb[0], N, B, p.ld, 0, N, k0 * kDwK, p.n);
-    tc::cp_async_commit();
-    const uint32_t idesc = tc::idesc_bf16_f32(128, N);
-    for (int kt = 0; kt < KT; ++kt) {
-        const int s = kt & 1;
-        if (kt + 1 < KT) {
-            if (kt >= 1) { // the MMAs of slab kt - 1 have read the other stage
-                bool w = true;
-                if (threadIdx.x == 0)
-                    w = tc::mbar_wait(&bars[s ^ 1], ((kt - 1) >> 1) & 1);
-                if (!__syncthreads_and(w)) {
-                    ok = false;
-                    break;
-                }
+    if (threadIdx.x == 0) { // copies
+        int k = 0;
+        for (; ok && k < KT; ++k) {
+            const int slot = k % kDwSlots;
+            if (k >= kDwSlots && !tc::mbar_wait(&empty[slot], uint32_t((k / kDwSlots - 1) & 1))) {
+                ok = false;
+                break;
             }
-            dw_stage(sa[s ^ 1], 128, A, p.ld, m0, M, (k0 + kt + 1) * kDwK, p.n);
-            dw_stage(sb[s ^ 1], N, B, p.ld, 0, N, (k0 + kt + 1) * kDwK, p.n);
-            tc::cp_async_commit();
-            tc::cp_async_wait<1>();
-        } else {
-            tc::cp_async_wait<0>();
+            unsigned char *a = smem + size_t(slot) * 2 * kDwOperand;
+            tc::mbar_arrive_expect_tx(&full[slot], uint32_t(M + N) * kDwK * 2);
+            tc::bulk_g2s(a, A + size_t(k0 + k) * M * kDwK, uint32_t(M) * kDwK * 2, &full[slot]);
+            tc::bulk_g2s(a + kDwOperand, B + size_t(k0 + k) * N * kDwK, uint32_t(N) * kDwK * 2, &full[slot]);
         }
-        tc::fence_proxy_async();
-        __syncthreads();
-        tc::tc_fence_after();
-        if (threadIdx.x == 0) {
-            const uint32_t a0 = tc::smem_u32(sa[s]), b0 = tc::smem_u32(sb[s]);
+        // copies in flight land before the CTA's memory goes away
+        for (int q = max(0, k - kDwSlots); q < k; ++q) ok = tc::mbar_wait(&full[q % kDwSlots], uint32_t((q / kDwSlots) & 1)) && ok;
+    } else if (threadIdx.x == 32) { // MMAs
+        const uint32_t idesc = tc::idesc_bf16_f32(128, N);
+        for (int k = 0; ok && k < KT; ++k) {
+            const int slot = k % kDwSlots;
+            ok = tc::mbar_wait(&full[slot], uint32_t((k / kDwSlots) & 1));
+            if (!ok)
+                break;
+            tc::tc_fence_after();
+            const uint32_t a0 = tc::smem_u32(smem + size_t(slot) * 2 * kDwOperand), b0 = a0 + kDwOperand;
 #pragma unroll
             for (int kk = 0; kk < kDwK / 16; ++kk)
-                tc::mma_bf16(tmem, tc::smem_desc(a0 + kk * 2 * 128 * 16, 128 * 16, 128),
-                             tc::smem_desc(b0 + kk * 2 * N * 16, N * 16, 128), idesc, (kt > 0 || kk > 0) ? 1u : 0u);
-            tc::mma_commit(&bars[s]);
+                for (int h = 0; h * 128 < M; ++h) // (rows past M are accumulated from what lies there and not read)
+                    tc::mma_bf16(tmem + 256 * h, tc::smem_desc(a0 + kk * 2 * M * 16 + h * 128 * 16, M * 16, 128),
+                                 tc::smem_desc(b0 + kk * 2 * N * 16, N * 16, 128), idesc, (k > 0 || kk > 0) ? 1u : 0u);
+            tc::mma_commit(&empty[slot]);
         }
+        tc::mma_commit(acc); // every MMA issued so far
+        ok = tc::mbar_wait(acc, 0) && ok;
     }
-    {
-        bool w = true;
-        if (threadIdx.x == 0 && ok)
-            w = tc::mbar_wait(&bars[(KT - 1) & 1], ((KT - 1) >> 1) & 1);
-        ok = __syncthreads_and(ok && w);
-    }
-    tc::cp_async_wait<0>();
+    ok = __syncthreads_and(ok);
     tc::tc_fence_after();
     if (ok) {
-        const int m = m0 + warp * 32 + lane;
-        float *g = mem.gW[l] + (size_t)m * N;
-        for (int c0 = 0; c0 < N; c0 += 32) {
-            float v[32];
-            tc::tmem_ld32(tmem + (uint32_t(warp * 32) << 16) + c0, v);
-            if (m < M)
+        const int h = warp / 4, m = warp * 32 + lane;
+        float *g = mem.gW[l] + size_t(m) * N;
+        if (h * 128 < M)
+            for (int c0 = 0; c0 < N; c0 += 32) {
+                float v[32];
+                tc::tmem_ld32(tmem + 256 * h + (uint32_t((warp % 4) * 32) << 16) + c0, v);
+                if (m < M)
 #pragma unroll
-                for (int j = 0; j < 8; ++j)
-                    if (c0 + j * 4 < N)
-                        asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(g + c0 + j * 4), "f"(v[j * 4]),
-                                     "f"(v[j * 4 + 1]), "f"(v[j * 4 + 2]), "f"(v[j * 4 + 3])
-                                     : "memory");
-        }
+                    for (int j = 0; j < 8; ++j)
+                        if (c0 + j * 4 < N)
+                            asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(g + c0 + j * 4),
+                                         "f"(v[j * 4]), "f"(v[j * 4 + 1]), "f"(v[j * 4 + 2]), "f"(v[j * 4 + 3])
+                                         : "memory");
+            }
     } else if (threadIdx.x == 0) {
         atomicExch(p.err, 1);
     }
     tc::tc_fence_before();
     __syncthreads();
     if (warp == 0)
-        tc::tmem_dealloc(tmem, 256);
+        tc::tmem_dealloc(tmem, 512);
 }
 
 // Position of element (n, k) of an [N x K] operand in its K-slabs of kFusedSlabK

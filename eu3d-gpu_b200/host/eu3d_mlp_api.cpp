@@ -180,10 +180,10 @@ eu3d::TrainParams train_params(const eu_mlp *m, int first, int count)
 // A batch of n rows of the caller's arrays, with the members' scratch for it.
 eu_status train_batch(eu_mlp *m, eu3d::TrainParams &p, const float *X, const float *T, long long rows, int n, bool drawn)
 {
-    const int ld = eu3d::train_ld(n);
-    const size_t wide = size_t(m->hidden) * m->width * ld;
-    // every piece a multiple of 64 values, so 128-byte aligned
-    const size_t bytes = wide * (4 + 2 + 2) + size_t(ld) * (m->in_pad + m->out_pad) * 2;
+    // whole tiles: every piece a multiple of 128 values
+    const size_t rows_pad = size_t(n + eu3d::kTrainRows - 1) / eu3d::kTrainRows * eu3d::kTrainRows;
+    const size_t wide = size_t(m->hidden) * m->width * rows_pad;
+    const size_t bytes = wide * (4 + 2 + 2) + rows_pad * (m->in_pad + m->out_pad) * 2;
     if (m->train_rows < n) {
         if (m->train) {
             MCK(m, cudaStreamSynchronize(m->stream));
@@ -198,16 +198,15 @@ eu_status train_batch(eu_mlp *m, eu3d::TrainParams &p, const float *X, const flo
     p.T = T;
     p.rows = rows;
     p.n = n;
-    p.ld = ld;
     p.drawn = drawn;
     for (int e = 0; e < m->members; ++e) {
         eu3d::TrainMember &t = p.member[e];
         unsigned char *at = static_cast<unsigned char *>(m->train) + e * bytes;
-        t.Z = reinterpret_cast<float *>(at);
+        t.ZT = reinterpret_cast<float *>(at);
         t.HT = reinterpret_cast<__nv_bfloat16 *>(at + wide * 4);
         t.dZT = t.HT + wide;
         t.XT = t.dZT + wide;
-        t.dYT = t.XT + size_t(ld) * m->in_pad;
+        t.dYT = t.XT + rows_pad * m->in_pad;
     }
     return EU_OK;
 }
