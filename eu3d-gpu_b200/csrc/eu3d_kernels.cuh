@@ -353,16 +353,23 @@ __global__ void __launch_bounds__(kFaceThreadsWide, 2)
 // plane instead of once per stencil point, and the loads of the next plane
 // overlapped with the current plane's arithmetic.
 //
-// A block owns a kTileJ x kTileK tile of (j, k) columns  and
-// marches along x with kTileJ + 1 warps. Warps 0 .. kTileJ-1 own a row of cells each: every
-// thread keeps its column's x-stencil (planes i-1 .. i+2 of every primitive) in
+// A block owns a kTileJ x kTileK tile of (j, k) columns and marches along x with
+// kTileJ + 1 warps. Warps 0 .. kTileJ-1 own a row of cells each: every thread
+// keeps its column's x-stencil (planes i-1 .. i+2 of every primitive) in
 // registers and loads plane i+3 one node ahead. Plane i of the tile plus a
 // two-node halo in j and k is staged in shared memory, from which the y- and
 // z-face fluxes are formed; two stages alternate, and while plane i is computed
-// the halo of plane i+1 (cp.async) and the conserved values of plane i
-// (cp.async, read by the update) are in flight. Face indices: sG[q][r] is the y
-// face below tile row r (r = kTileJ: above the last row), sQ[q][r][c] the z
-// face left of column c.
+// the halo of plane i+1 (cp.async) is in flight. The update of a plane waits for
+// the next plane's barrier, so a plane has one (the face fluxes lie twice), and
+// is an FP64 addition that the L2 carries out. sG: [r] the y face below
+// tile row r (r = kTileJ: above the last row); sQ: [r][c] the z face left
+// of column c.
+//
+// What bounds it is instruction issue (57 % active at 16 warps per SM). With two
+// barriers a plane, the conserved values staged by cp.async and 64-bit node
+// numbers it took 0.459 ms at 256 x 128 x 128 (278 M warp instructions); now
+// 0.403 ms, the same bits. The addresses count most of that: a node number of 32 bits
+// and a plane's offset as one wide multiply-add (0.460 -> 0.403 ms).
 //
 // Each cell warp forms three faces per plane (x, y, z). The edge warp (warp
 // kTileJ) owns the first halo row above the tile, which it stages from its
@@ -372,7 +379,7 @@ __global__ void __launch_bounds__(kFaceThreadsWide, 2)
 // extra face. Partial tiles: the faces of the valid rows/columns are formed,
 // including the one past the last valid row/column.
 //
-// Tile height: 7 cell rows (8 warps), so that two blocks fit per SM (98 KB of
+// Tile height: 7 cell rows (8 warps), so that two blocks fit per SM (99 KB of
 // shared memory each).
 constexpr int kTileK = 32, kTileCols = kTileK + 4;
 constexpr int kTileJ = 7, kTileWarps = kTileJ + 1, kTileRows = kTileJ + 4;
@@ -383,8 +390,8 @@ constexpr int kTileHalo = 3 * kTileCols + 4 * (kTileJ + 1);
 template <int NS>
 constexpr size_t tiled_flux_smem_bytes()
 {
-    return sizeof(double) * (NS + 4) * kTileJ * kTileK + sizeof(float) * 2 * (7 + NS) * kTileRows * kTileCols +
-           sizeof(float) * (NS + 4) * ((kTileJ + 1) * kTileK + kTileJ * (kTileK + 1));
+    return sizeof(float) * 2 * ((7 + NS) * kTileRows * kTileCols +
+                                (NS + 4) * ((kTileJ + 1) * kTileK + kTileJ * (kTileK + 1)));
 }
 
 // Face flux from four consecutive stencil points of the staged plane tile,
@@ -432,12 +439,12 @@ __global__ void __launch_bounds__(kTileK *kTileWarps, 2)
     constexpr int NP = 7 + NS, NV = NS + 4;
     using Plane = R[NP][kTileRows][kTileCols];
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    double(*sC)[kTileJ][kTileK] = reinterpret_cast<double(*)[kTileJ][kTileK]>(smem_raw);
-    Plane *stage = reinterpret_cast<Plane *>(smem_raw + sizeof(double) * NV * kTileJ * kTileK);
-    unsigned char *flux_raw = reinterpret_cast<unsigned char *>(stage + 2);
-    R(*sG)[kTileJ + 1][kTileK] = reinterpret_cast<R(*)[kTileJ + 1][kTileK]>(flux_raw);
-    R(*sQ)[kTileJ][kTileK + 1] =
-        reinterpret_cast<R(*)[kTileJ][kTileK + 1]>(flux_raw + sizeof(R) * NV * (kTileJ + 1) * kTileK);
+    using FacesY = R[NV][kTileJ + 1][kTileK];
+    using FacesZ = R[NV][kTileJ][kTileK + 1];
+    Plane *stage = reinterpret_cast<Plane *>(smem_raw);
+    FacesY *sG2 = reinterpret_cast<FacesY *>(stage + 2);
+    FacesZ *sQ2 = reinterpret_cast<FacesZ *>(sG2 + 2);
+    __shared__ float sX[2]; // -dt / dx of a plane
 
     const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * kTileK + tx;
     const int k0 = blockIdx.x * kTileK, j0 = blockIdx.y * kTileJ;
@@ -470,14 +477,19 @@ __global__ void __launch_bounds__(kTileK *kTileWarps, 2)
     const int hj = g.bc + j0 - 2 + hr, hk = g.bc + k0 - 2 + hc;
     const bool halo = hr >= 0 && hj < g.ny && hk < g.nz;
 
-    const long long n3 = g.n3, sx = (long long)g.ny * g.nz;
+    // node numbers fit 32 bits; a plane times n3 is formed in 64
+    const unsigned n3 = unsigned(g.n3), sx = unsigned(g.ny) * unsigned(g.nz);
+    auto node = [&](const R *base, int f, unsigned c) {
+        return reinterpret_cast<const R *>(reinterpret_cast<const char *>(base + c) +
+                                           (unsigned long long)n3 * unsigned(f * int(sizeof(R))));
+    };
     const double dt = *dt_dev;
-    const double cy = valid ? dt / (g.y[j] - g.y[j - 1]) : 0.0;
-    const double cz = valid ? dt / (g.z[k] - g.z[k - 1]) : 0.0;
+    const float cy32 = valid ? float(dt / (g.y[j] - g.y[j - 1])) : 0.0f;
+    const float cz32 = valid ? float(dt / (g.z[k] - g.z[k - 1])) : 0.0f;
     const int i_begin = g.bc + blockIdx.z * ci;
     const int i_end = min(i_begin + ci, g.bc + g.ni);
-    const long long col = resident ? cell_index(g, 0, j, k) : 0;
-    const long long hcol = halo ? cell_index(g, 0, hj, hk) : 0;
+    const unsigned col = resident ? unsigned(cell_index(g, 0, j, k)) : 0;
+    const unsigned hcol = halo ? unsigned(cell_index(g, 0, hj, hk)) : 0;
 
     // plane p of the tile into stage s: the own node from registers, the halo
     // node by cp.async; one commit group per call (empty when nothing to copy)
@@ -488,7 +500,7 @@ __global__ void __launch_bounds__(kTileK *kTileWarps, 2)
         }
         if (halo) {
 #pragma unroll
-            for (int f = 0; f < NP; ++f) tc::cp_async4(&stage[s][f][hr][hc], prim + f * n3 + hcol + p * sx);
+            for (int f = 0; f < NP; ++f) tc::cp_async4(&stage[s][f][hr][hc], node(prim, f, hcol + unsigned(p) * sx));
         }
         tc::cp_async_commit();
     };
@@ -497,7 +509,7 @@ __global__ void __launch_bounds__(kTileK *kTileWarps, 2)
 #pragma unroll
     for (int p = 0; p < 4; ++p)
 #pragma unroll
-        for (int f = 0; f < NP; ++f) w[p][f] = resident ? __ldg(prim + f * n3 + col + (i_begin - 2 + p) * sx) : R(0);
+        for (int f = 0; f < NP; ++f) w[p][f] = resident ? __ldg(node(prim, f, col + unsigned(i_begin - 2 + p) * sx)) : R(0);
     R Fm[NV];
     if (valid)
         window_face_flux<NS>(w, Fm);
@@ -506,34 +518,42 @@ __global__ void __launch_bounds__(kTileK *kTileWarps, 2)
         w[0][f] = w[1][f];
         w[1][f] = w[2][f];
         w[2][f] = w[3][f];
-        w[3][f] = resident ? __ldg(prim + f * n3 + col + (i_begin + 2) * sx) : R(0);
+        w[3][f] = resident ? __ldg(node(prim, f, col + unsigned(i_begin + 2) * sx)) : R(0);
     }
     stage_plane(i_begin, w[1], 0);
+    R dF[NV]; // F_{i+1/2} - F_{i-1/2} of the plane whose update is due
 
-    for (int i = i_begin; i < i_end; ++i) {
-        // window: planes i-1, i, i+1, i+2. Stage s holds plane i (its halo may
-        // still be in flight); the other stage was last read before the
-        // previous iteration's second barrier.
+    for (int i = i_begin;; ++i) {
+        // window: planes i-1, i, i+1, i+2. One barrier a plane: it shows plane i's
+        // halo (stage s) and the y and z faces of plane i-1 (the other pair of
+        // face arrays), and closes the reads of plane i-1's stage and of plane
+        // i-2's faces, which this iteration overwrites.
         const int s = (i - i_begin) & 1;
-        if (valid) {
+        tc::cp_async_wait<0>();
+        __syncthreads();
+        if (i > i_begin && valid) { // update plane i-1
+            const auto &sG = sG2[s ^ 1];
+            const auto &sQ = sQ2[s ^ 1];
+            const unsigned c = col + unsigned(i - 1) * sx;
+            const float cx32 = sX[s ^ 1];
+            // the flux differences and their sum in FP32 (a difference of two
+            // FP32 values within a factor of two is exact), accumulated onto
+            // the FP64 conserved value by the L2: nothing waits for its read
 #pragma unroll
-            for (int q = 0; q < NV; ++q) tc::cp_async8(&sC[q][ty][tx], st.cs + q * n3 + col + i * sx);
+            for (int q = 0; q < NV; ++q) {
+                const float rhs = cx32 * dF[q] - cy32 * float(sG[q][ty + 1][tx] - sG[q][ty][tx]) -
+                                  cz32 * float(sQ[q][ty][tx + 1] - sQ[q][ty][tx]);
+                atomicAdd(reinterpret_cast<double *>(reinterpret_cast<char *>(st.cs + c) +
+                                                     (unsigned long long)n3 * unsigned(q * int(sizeof(double)))),
+                          double(rhs));
+            }
         }
-        tc::cp_async_commit();
+        if (i == i_end)
+            break;
+        auto &sG = sG2[s];
+        auto &sQ = sQ2[s];
         if (i + 1 < i_end)
             stage_plane(i + 1, w[2], s ^ 1);
-        else
-            tc::cp_async_commit();
-        R next[NP];
-        const bool more = resident && i + 1 < i_end;
-#pragma unroll
-        for (int f = 0; f < NP; ++f) next[f] = more ? __ldg(prim + f * n3 + col + (i + 3) * sx) : R(0);
-        // groups in flight, oldest first: halo(i), conserved(i), halo(i+1)
-        tc::cp_async_wait<2>();
-        __syncthreads();
-        R Fp[NV];
-        if (valid)
-            window_face_flux<NS>(w, Fp);
         if (yface) {
             R G[NV];
             tile_face_flux<NS, 1, 1, 0, true>(stage[s], ty, tx + 2, w[1], G);
@@ -552,23 +572,21 @@ __global__ void __launch_bounds__(kTileK *kTileWarps, 2)
 #pragma unroll
             for (int q = 0; q < NV; ++q) sQ[q][zrow][kTileK] = Q[q];
         }
-        __syncthreads();
-        tc::cp_async_wait<1>(); // this thread's conserved values of plane i
+        R next[NP];
+        const bool more = resident && i + 1 < i_end;
+#pragma unroll
+        for (int f = 0; f < NP; ++f) next[f] = more ? __ldg(node(prim, f, col + unsigned(i + 3) * sx)) : R(0);
         if (valid) {
-            const long long c = col + i * sx;
-            const double cx = -dt / (g.x[i] - g.x[i - 1]);
-            // the flux differences and their sum in FP32 (a difference of two
-            // FP32 values within a factor of two is exact), accumulated onto
-            // the FP64 conserved value
-            const float cx32 = float(cx), cy32 = float(cy), cz32 = float(cz);
+            R Fp[NV];
+            window_face_flux<NS>(w, Fp);
 #pragma unroll
             for (int q = 0; q < NV; ++q) {
-                const float rhs = cx32 * float(Fp[q] - Fm[q]) - cy32 * float(sG[q][ty + 1][tx] - sG[q][ty][tx]) -
-                                  cz32 * float(sQ[q][ty][tx + 1] - sQ[q][ty][tx]);
-                st.cs[q * n3 + c] = sC[q][ty][tx] + double(rhs);
+                dF[q] = Fp[q] - Fm[q];
                 Fm[q] = Fp[q];
             }
         }
+        if (tid == kTileWarps * kTileK - 1)
+            sX[s] = float(-dt / (g.x[i] - g.x[i - 1]));
 #pragma unroll
         for (int f = 0; f < NP; ++f) {
             w[0][f] = w[1][f];
@@ -577,7 +595,6 @@ __global__ void __launch_bounds__(kTileK *kTileWarps, 2)
             w[3][f] = next[f];
         }
     }
-    tc::cp_async_wait<0>();
 }
 
 // ------------------------------------------------- recovery + kinetics

@@ -77,14 +77,10 @@ __device__ __forceinline__ void cp_async16(void *smem_dst, const void *gmem_src,
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(smem_dst)), "l"(gmem_src), "r"(n)
                  : "memory");
 }
-// 4- and 8-byte copies (cached in L1: stencil halos are re-read by neighbours)
+// 4-byte copies (cached in L1: stencil halos are re-read by neighbours)
 __device__ __forceinline__ void cp_async4(void *smem_dst, const void *gmem_src)
 {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(smem_dst)), "l"(gmem_src) : "memory");
-}
-__device__ __forceinline__ void cp_async8(void *smem_dst, const void *gmem_src)
-{
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(smem_dst)), "l"(gmem_src) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
