@@ -49,9 +49,22 @@ __device__ __forceinline__ float tanh_approx(float x)
 // rounding, so h is bitwise 0.5f * (a + b) (outside the subnormal range).
 __device__ __forceinline__ float silu_fast_half(float h) { return fmaf(h, tanh_approx(h), h); }
 __device__ __forceinline__ float silu_fast(float x) { return silu_fast_half(0.5f * x); }
+// SiLU' with the reciprocal of 1 + e^-z to half a unit in the last place (the bias
+// gradients take it in full fp32): the hardware's approximation and a Newton step,
+// on a denominator scaled by 2^-64 so that no e^-z below infinity leaves the normal
+// range (an infinite one gives 0). The bits matter: they move the bf16 rounding of
+// the layer gradients, Adam divides by the gradients' size, and passes over one
+// model carry the difference on. Against the form with an IEEE division, 30 sets of
+// inputs, a first batch's gradients differed by up to 3.5e-6 of their norm with the
+// approximate division (single values 1.4e-4), with this form by 6e-7 (2e-6), which
+// the order of the fp32 sums leaves. Time of a training pass: the same (6.27 ms;
+// 6.88 with the compiler's division and its range branch).
 __device__ __forceinline__ float silu_grad(float z)
 {
-    const float s = __fdividef(1.0f, 1.0f + __expf(-z));
+    const float d = fminf(fmaf(__expf(-z), 0x1p-64f, 0x1p-64f), 0x1p+100f);
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(d));
+    const float s = fmaf(y, fmaf(-d, y, 1.0f), y) * 0x1p-64f;
     return s * (1.0f + z * (1.0f - s));
 }
 

@@ -125,6 +125,41 @@ def test_gradients_of_other_shapes(gpu, shape, n):
                 off += size
 
 
+def test_silu_gradient_divides_exactly(gpu):
+    """SiLU' = s (1 + z (1 - s)), s = 1 / (1 + e^-z), in the training step: read
+    off the bias gradients of a one-layer net that does nothing else (zero first
+    weights, so z is the bias; unit output weights; sixteen equal rows, whose sum
+    is exact; one output, whose own bias gradient is the common factor). For z in
+    [8, 16] the error of e^-z stays below 4e-10, so 1 + e^-z rounds as the exact
+    sum except within 4e-10 of a midpoint (spacing 1.2e-7: 0.7 %), and from there
+    on every value is the fp32 expression's with a quotient rounded to nearest: at
+    most 2 % of the 1,024 may differ in a bit."""
+    import torch
+    f32 = np.float32
+    m = gpu.Mlp()
+    m.init(1, 256, 1, 1, 1, max_batch=16, seed=1)
+    rng = np.random.default_rng(4)
+    X, T = torch.zeros(16, 1, device="cuda"), torch.zeros(16, 1, device="cuda")
+
+    def gradients(z):
+        m.set_params(np.concatenate([np.zeros(256), z, np.ones(256), [0.0]]).astype(f32))
+        g = m.loss_grad(0, X, T)[1]
+        return g[256:512] / f32(16), g[768] / f32(16)
+
+    off = 0
+    for _ in range(4):
+        z = rng.uniform(8.0, 16.0, 256).astype(f32)
+        got, dh = gradients(z)
+        s = f32(1) / (1 + np.exp(-z.astype(np.float64))).astype(f32)
+        u = (z.astype(np.float64) * (f32(1) - s) + 1).astype(f32)  # fused
+        off += int((got != dh * (s * u)).sum())
+    assert off <= 20, off
+    # far out e^-z leaves the fp32 range: the limits 0 and 1, no NaN
+    z = np.array([-1e4, -89.0, -88.0, -87.0, 87.0, 89.0, 1e4] + [1.0] * 249, f32)
+    got, dh = gradients(z)
+    assert np.abs(got[:7] / dh - [0, 0, 0, 0, 1, 1, 1]).max() <= 1e-7
+
+
 @pytest.mark.parametrize("shape", [(N_IN, WIDTH, HIDDEN, N_OUT, MEMBERS), (5, 64, 2, 3, 2), (20, 96, 1, 40, 1)])
 def test_fused_inference_matches_layerwise(gpu, shape):
     """The one-kernel inference (every member's network per 128-row tile, the
