@@ -36,8 +36,12 @@ constexpr bool kStrictFlux = EU_EXACT_FLUX != 0;
 // face), and runs among two per SM: the ci whose rounds of blocks cost least
 // (256 x 128 x 128: 24, 0.436 ms against 0.459 at 16; 192 x 96 x 96: 29, 0.193
 // against 0.213). In a batch the rounds mix with the other instances'.
-inline int tiled_march(const LaunchArgs &a, long long tiles)
+inline int tiles_j(const DevGrid &g) { return (g.nj + kTileJ - 1) / kTileJ; }
+inline int tiles_k(const DevGrid &g) { return (g.nk + kTileK - 1) / kTileK; }
+
+inline int tiled_march(const LaunchArgs &a)
 {
+    const long long tiles = (long long)tiles_j(a.g) * tiles_k(a.g);
     if (a.batch_cells > 0)
         return 24;
     const long long slots = 2LL * (a.sms > 0 ? a.sms : 148);
@@ -54,6 +58,8 @@ inline int tiled_march(const LaunchArgs &a, long long tiles)
     return best;
 }
 
+inline int tiled_ci(const LaunchArgs &a) { return a.flux_ci > 0 ? a.flux_ci : tiled_march(a); }
+
 template <int NS>
 cudaError_t tiled_flux_launch(const LaunchArgs &a)
 {
@@ -64,9 +70,8 @@ cudaError_t tiled_flux_launch(const LaunchArgs &a)
     if (e != cudaSuccess)
         return e;
     const dim3 block(kTileK, kTileWarps);
-    const int tk = (g.nk + kTileK - 1) / kTileK, tj = (g.nj + kTileJ - 1) / kTileJ;
-    const int ci = a.flux_ci > 0 ? a.flux_ci : tiled_march(a, (long long)tk * tj);
-    const dim3 grid(tk, tj, (g.ni + ci - 1) / ci);
+    const int ci = tiled_ci(a);
+    const dim3 grid(tiles_k(g), tiles_j(g), (g.ni + ci - 1) / ci);
     k_flux_update_tiled<NS><<<grid, block, smem, a.stream>>>(g, a.st, a.st.prim32, a.dt_dev, ci);
     return cudaGetLastError();
 }
@@ -140,15 +145,20 @@ cudaError_t faces_flux_launch(const LaunchArgs &a, const R *prim)
 constexpr int kThinNk = 16;
 constexpr long long kTiledCells = 1000000;
 
+inline bool takes_tiled(const LaunchArgs &a)
+{
+    const DevGrid &g = a.g;
+    const long long cells = std::max((long long)g.ni * g.nj * g.nk, a.batch_cells);
+    const long long slots = (long long)tiles_j(g) * kTileJ * (tiles_k(g) * kTileK);
+    return a.precision == 1 && g.nk >= kThinNk && cells >= kTiledCells && 5LL * g.nj * g.nk >= 4 * slots;
+}
+
 template <int NS, int NR>
 cudaError_t flux_t(const LaunchArgs &a)
 {
-    const DevGrid &g = a.g;
     if (a.precision != 1)
         return faces_flux_launch<NS, double, kStrictFlux>(a, a.st.prim);
-    const long long cells = std::max((long long)g.ni * g.nj * g.nk, a.batch_cells);
-    const long long slots = (long long)((g.nj + kTileJ - 1) / kTileJ * kTileJ) * ((g.nk + kTileK - 1) / kTileK * kTileK);
-    if (g.nk >= kThinNk && cells >= kTiledCells && 5LL * g.nj * g.nk >= 4 * slots)
+    if (takes_tiled(a))
         return tiled_flux_launch<NS>(a);
     return faces_flux_launch<NS, float, false>(a, a.st.prim32);
 }
@@ -339,6 +349,7 @@ cudaError_t heavy_batch_t(const LaunchArgs &a, const BatchCell *tab, int n, int 
 
 cudaError_t launch_boundary(const LaunchArgs &a) { EU3D_DISPATCH(boundary_t, a) }
 cudaError_t launch_flux_update(const LaunchArgs &a) { EU3D_DISPATCH(flux_t, a) }
+int flux_plan(const LaunchArgs &a) { return takes_tiled(a) ? tiled_ci(a) : 0; }
 cudaError_t launch_recover_react(const LaunchArgs &a, bool react) { EU3D_DISPATCH(react_t, a, react) }
 cudaError_t launch_derived(const LaunchArgs &a, int which, double *out) { EU3D_DISPATCH(derived_t, a, which, out) }
 cudaError_t launch_materialize(const LaunchArgs &a) { EU3D_DISPATCH(materialize_t, a) }
@@ -427,7 +438,8 @@ cudaError_t launch_set_value(double *dst, double v, cudaStream_t s)
 const Launchers launchers = {&launch_boundary,         &launch_flux_update,      &launch_recover_react,
                              &launch_derived,          &launch_recover_classify, &launch_learned_apply,
                              &launch_react_queue,      &launch_react_heavy,      &launch_materialize,
-                             &launch_learned_route,    &launch_react_queue_batch, &launch_react_heavy_batch};
+                             &launch_learned_route,    &launch_react_queue_batch, &launch_react_heavy_batch,
+                             &flux_plan};
 
 #undef EU3D_DISPATCH
 

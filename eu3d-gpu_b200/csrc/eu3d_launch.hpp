@@ -44,6 +44,8 @@ struct Launchers {
     // a batch's shared kinetics stage over the instances of tab[0..n)
     cudaError_t (*react_queue_batch)(const LaunchArgs &a, const BatchCell *tab, int n, int *next, int counter);
     cudaError_t (*react_heavy_batch)(const LaunchArgs &a, const BatchCell *tab, int n, int *next, int blocks);
+    // what flux_update launches: 0 the face kernel, else the tiled kernel with this march
+    int (*flux_plan)(const LaunchArgs &a);
 };
 
 #define EU3D_DECLARE_LAUNCHERS(NSP)                                                                \

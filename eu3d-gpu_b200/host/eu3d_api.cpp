@@ -73,6 +73,7 @@ struct eu_handle {
     double graph_cfl = 0;   // the CFL number the captured step sets its dt from (0: a fixed dt)
     bool graph_shared_tail = false; // captured for a batch: the stiff-fallback and deferred-cell
                                     // kinetics left to the batch's shared stage
+    int graph_flux_plan = 0; // Launchers::flux_plan of the captured step (a batch's differs from the handle's alone)
     unsigned graph_gen = 0; // captures so far (batches rebuild when it changes)
     // launch shapes picked by eu_autotune (0: defaults)
     int flux_ci = 0, recover_block = 0, recover_minb = 0;
@@ -1036,6 +1037,7 @@ eu_status capture_step(eu_handle *h, const LaunchArgs &a, const Launchers &L, do
     h->graph_dirty = false;
     h->graph_cfl = cfl;
     h->graph_shared_tail = shared_tail;
+    h->graph_flux_plan = L.flux_plan(a);
     ++h->graph_gen;
     return EU_OK;
 }
@@ -1276,7 +1278,8 @@ eu_status step_impl(eu_handle *h, int nsteps, double dt, double cfl, eu_step_sta
     if (h->st.prim32 && nsteps > 0)
         h->prim_stale = true;
     int n = 0;
-    if (graphs && nsteps > 0 && (h->graph_dirty || !h->graph_exec || h->graph_cfl != cfl || h->graph_shared_tail)) {
+    if (graphs && nsteps > 0 && (h->graph_dirty || !h->graph_exec || h->graph_cfl != cfl || h->graph_shared_tail ||
+                                 h->graph_flux_plan != L.flux_plan(a))) {
         // the first step runs eagerly (one-time kernel attribute set-up), then
         // the step is captured
         eu_status s = step_launches(h, a, L, false, &launches, cfl);
@@ -2106,10 +2109,12 @@ eu_status eu_batch_step(eu_batch *b, int nsteps, const double *dt, eu_step_stats
         if (h->cfg.chemistry == EU_CHEM_LEARNED && (!h->model || !mlp_has_fused(h->model)))
             return bfail(b, EU_ERR_UNSUPPORTED, "instance %d: learned chemistry needs a model with the fused kernel", i);
         const bool tail = b->shared && needs_shared_stage(h);
-        if (h->graph_dirty || !h->graph_exec || h->graph_cfl != 0 || h->graph_shared_tail != tail) {
-            LaunchArgs a = launch_args(h);
-            a.batch_cells = cells;
-            const eu_status s = capture_step(h, a, flavour(h), 0, tail);
+        LaunchArgs a = launch_args(h);
+        a.batch_cells = cells;
+        const Launchers &L = flavour(h);
+        if (h->graph_dirty || !h->graph_exec || h->graph_cfl != 0 || h->graph_shared_tail != tail ||
+            h->graph_flux_plan != L.flux_plan(a)) {
+            const eu_status s = capture_step(h, a, L, 0, tail);
             if (s != EU_OK)
                 return bfail(b, s, "instance %d: %s", i, h->err.c_str());
         }

@@ -253,6 +253,49 @@ def test_strict_warp_kinetics_match_restatement(gpu, port_lib):
     assert torch.equal(got[4][0][:, few], got[20000][0][:, few]) and torch.equal(got[4][1][few], got[20000][1][few])
 
 
+def mixed_block(gpu, dims, **kw):
+    """A mixed-precision solver on random reacting gas with O(1) changes between nodes."""
+    h = 5e-4
+    s = gpu.Solver(*dims, tuple(v for n in dims for v in (0.0, h * (n - 1))), precision="mixed", arith="fast", **kw)
+    s.set_mechanism(golden_mechanism())
+    rng = np.random.default_rng(sum(dims))
+    shape = tuple(n + 4 for n in dims)
+    f = rng.uniform(0.0, 1.0, shape)
+    Y = np.zeros((9,) + shape)
+    Y[5], Y[4], Y[8] = 0.1 * f, 0.8 * f, 1 - 0.9 * f
+    s.set_primitive(1e5 * rng.uniform(0.7, 1.4, shape), rng.uniform(400.0, 1300.0, shape),
+                    *(rng.uniform(-900.0, 900.0, shape) for _ in range(3)), Y)
+    return s
+
+
+def flux_kernels(fn):
+    """Names of the flux kernels that fn launches."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+    with profile(activities=[ProfilerActivity.CUDA], acc_events=True) as p:
+        fn()
+        torch.cuda.synchronize()
+    return {k for k in ("k_flux_update_faces", "k_flux_update_tiled") if any(k in e.key for e in p.key_averages())}
+
+
+def test_flux_kernel_follows_the_call(gpu):
+    """Which FP32 flux kernel a handle runs depends on the cells that run together:
+    its own alone (too few here for the tiled kernel), all instances' in a batch.
+    The captured step follows each call, whatever the calls before it were, also
+    where the kinetics leave nothing to a batch's shared stage (frozen)."""
+    a, b = (mixed_block(gpu, (50, 7, 32), chemistry="frozen") for _ in range(2))
+    big = mixed_block(gpu, (128, 98, 96), chemistry="frozen")  # 1.2 M cells
+    small = mixed_block(gpu, (10, 7, 32), chemistry="frozen")
+    large, little = gpu.Batch([b, big]), gpu.Batch([b, small])
+    calls = [(lambda: a.step(2, 2e-8), "k_flux_update_faces"), (lambda: large.step(2, 2e-8), "k_flux_update_tiled"),
+             (lambda: b.step(2, 2e-8), "k_flux_update_faces"), (lambda: large.step(2, 2e-8), "k_flux_update_tiled"),
+             (lambda: little.step(2, 2e-8), "k_flux_update_faces"), (lambda: large.step(2, 2e-8), "k_flux_update_tiled")]
+    for k, (call, kernel) in enumerate(calls):
+        assert flux_kernels(call) == {kernel}, k
+    a.step(8, 2e-8)  # b's steps one by one
+    assert np.array_equal(a.get("CS"), b.get("CS"))
+
+
 def test_deterministic(gpu):
     z = golden("bubble_25x13x13_s20.npz")
     a = solver_from_golden(gpu, z, arith="fast")
