@@ -58,7 +58,10 @@ inline int tiled_march(const LaunchArgs &a)
     return best;
 }
 
-inline int tiled_ci(const LaunchArgs &a) { return a.flux_ci > 0 ? a.flux_ci : tiled_march(a); }
+inline int tiled_ci(const LaunchArgs &a)
+{
+    return std::max(a.tiled_ci > 0 ? a.tiled_ci : tiled_march(a), (a.g.ni + 65534) / 65535); // gridDim.z < 2^16
+}
 
 template <int NS>
 cudaError_t tiled_flux_launch(const LaunchArgs &a)
@@ -123,7 +126,7 @@ cudaError_t faces_flux_launch(const LaunchArgs &a, const R *prim)
     if (e != cudaSuccess)
         return e;
     const FaceTile t = face_tile<R>(g);
-    const int ci = std::max(std::max(a.flux_ci, t.ti), (g.ni + 65534) / 65535); // gridDim.z < 2^16
+    const int ci = std::max(std::max(a.face_ci, t.ti), (g.ni + 65534) / 65535); // gridDim.z < 2^16
     const int threads = (long long)g.ni * g.nj * g.nk < kFaceSmallCells ? kFaceThreadsWide : kFaceThreads;
     const dim3 grid(unsigned((g.nk + t.tk - 1) / t.tk), unsigned((g.nj + t.tj - 1) / t.tj), unsigned((g.ni + ci - 1) / ci));
     k_flux_update_faces<NS, R, kStrict><<<grid, threads, smem, a.stream>>>(g, a.st, prim, a.dt_dev, t, ci);

@@ -19,7 +19,8 @@ struct LaunchArgs {
     int chemistry; // eu_chemistry
     int spec;      // 1: tables are bitwise H2_JA919, use the generated rate code
     int sms;       // multiprocessors of the device (fixed grids of the queue kernels)
-    int flux_ci;   // nodes each flux block marches along x (autotuned; 0: by the grid, tiled_march, or one tile of the face kernel)
+    int face_ci;   // nodes a block of the face kernel marches along x (autotuned; 0: one tile)
+    int tiled_ci;  // the same of the tiled kernel (0: by the grid, tiled_march)
     int recover_block; // threads per block of the recovery kernels, 32..128 (autotuned; 0: 128, or 64 in learned mode)
     int recover_minb;  // register target, blocks per SM: learned-mode recovery 3 .. 6 (0: 4), stiff kinetics
                        // 2 .. 4 (0: by the grid)

@@ -76,7 +76,8 @@ struct eu_handle {
     int graph_flux_plan = 0; // Launchers::flux_plan of the captured step (a batch's differs from the handle's alone)
     unsigned graph_gen = 0; // captures so far (batches rebuild when it changes)
     // launch shapes picked by eu_autotune (0: defaults)
-    int flux_ci = 0, recover_block = 0, recover_minb = 0;
+    // (a march belongs to the flux kernel that it was timed on: alone and in a batch a handle may take either)
+    int face_ci = 0, tiled_ci = 0, recover_block = 0, recover_minb = 0;
     // advection time scheme (eu_set_time_scheme) and the RK start-of-step state
     int time_scheme = EU_TIME_EE;
     double *d_cs0 = nullptr;
@@ -270,7 +271,8 @@ LaunchArgs launch_args(eu_handle *h)
     a.chemistry = h->cfg.chemistry;
     a.spec = h->spec;
     a.sms = h->sms;
-    a.flux_ci = h->flux_ci;
+    a.face_ci = h->face_ci;
+    a.tiled_ci = h->tiled_ci;
     a.recover_block = h->recover_block;
     a.recover_minb = h->recover_minb;
     a.stream = h->stream;
@@ -279,7 +281,7 @@ LaunchArgs launch_args(eu_handle *h)
 
 using TuneKey = std::tuple<int, int, int, int, int, int, int>;
 std::mutex g_tune_mutex;                            // guards g_tuned
-std::map<TuneKey, std::array<int, 3>> g_tuned;      // (flux_ci, recover_block, recover_minb) per grid and mode
+std::map<TuneKey, std::array<int, 4>> g_tuned;      // (face_ci, tiled_ci, recover_block, recover_minb) per grid and mode
 
 TuneKey tune_key(const eu_handle *h)
 {
@@ -535,9 +537,10 @@ eu_status eu_create(const eu_config *cfg, eu_handle **out)
         std::lock_guard<std::mutex> lock(g_tune_mutex);
         auto it = g_tuned.find(tune_key(h));
         if (it != g_tuned.end()) {
-            h->flux_ci = it->second[0];
-            h->recover_block = it->second[1];
-            h->recover_minb = it->second[2];
+            h->face_ci = it->second[0];
+            h->tiled_ci = it->second[1];
+            h->recover_block = it->second[2];
+            h->recover_minb = it->second[3];
         }
     }
     *out = h;
@@ -2260,7 +2263,7 @@ eu_status eu_autotune(eu_handle *h, int reps, eu_tune_report *report)
             e = cudaMemcpyAsync(snap + off, q.p, q.bytes, cudaMemcpyDeviceToDevice, h->stream);
         off += q.bytes;
     }
-    const int ci_cand[] = {1, 8, 12, 16, 20, 24, 29, 32, 43, 64}; // 1: one tile of the face kernel
+    const int ci_cand[] = {1, 8, 12, 16, 20, 24, 29, 32, 43, 64}; // 1: one tile of the face kernel alone
     const int rb_cand[] = {64, 96, 128};
     eu_tune_report rep;
     std::memset(&rep, 0, sizeof rep);
@@ -2277,12 +2280,14 @@ eu_status eu_autotune(eu_handle *h, int reps, eu_tune_report *report)
         *ms /= reps;
         return r;
     };
+    const bool tiled = L.flux_plan(a) != 0;
+    int &march = tiled ? a.tiled_ci : a.face_ci;
     int best_ci = 16, best_rb = 128;
     float best = 1e30f;
     for (int ci : ci_cand) {
-        if (e != cudaSuccess || ci > h->ni + 15)
+        if (e != cudaSuccess || ci > h->ni + 15 || (tiled && ci == 1))
             continue;
-        a.flux_ci = ci;
+        march = ci;
         float ms = 0;
         e = time_it([&] { return L.flux_update(a); }, &ms);
         if (rep.flux_candidates < 16) {
@@ -2294,7 +2299,7 @@ eu_status eu_autotune(eu_handle *h, int reps, eu_tune_report *report)
             best_ci = ci;
         }
     }
-    a.flux_ci = best_ci;
+    march = best_ci;
     // the flux launches moved the conserved state: back to the snapshot
     // before timing the recovery on it
     auto restore = [&] {
@@ -2355,13 +2360,14 @@ eu_status eu_autotune(eu_handle *h, int reps, eu_tune_report *report)
     cudaFree(snap);
     if (e != cudaSuccess)
         return cuda_fail(h, e, "autotune");
-    h->flux_ci = best_ci;
+    h->face_ci = a.face_ci;
+    h->tiled_ci = a.tiled_ci;
     h->recover_block = best_rb;
     h->recover_minb = best_minb;
     h->graph_dirty = true;
     {
         std::lock_guard<std::mutex> lock(g_tune_mutex);
-        g_tuned[tune_key(h)] = {best_ci, best_rb, best_minb};
+        g_tuned[tune_key(h)] = {a.face_ci, a.tiled_ci, best_rb, best_minb};
     }
     rep.chosen_flux_ci = best_ci;
     rep.chosen_recover_block = best_rb;

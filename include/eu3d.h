@@ -479,8 +479,9 @@ eu_status eu_set_learned(eu_handle *h, eu_mlp *model, const eu_learned_config *c
 
 /* Autotuner: times the launch shapes that change no arithmetic (every
  * candidate gives bitwise the same state) on the handle's current state, which
- * it restores: the x-march length of the flux kernels, the block size of the
- * recovery kernels and, in learned mode, the recovery's register target. The choice applies to this handle and to handles
+ * it restores: the x-march length of the flux kernel that the handle takes alone,
+ * the block size of the recovery kernels and the register target of the learned
+ * mode's recovery or of the stiff kinetics. The choice applies to this handle and to handles
  * created later in the process with the same grid and mode. reps: timed
  * launches per candidate. report (or NULL) receives the candidates' times.
  * Allocates a temporary copy of the state. No counterpart in the reference. */
@@ -490,7 +491,7 @@ typedef struct {
     float flux_ms[16];
     int recover_candidates;
     int recover_block[16];      /* threads per block */
-    int recover_minblocks[16];  /* register target: resident blocks per SM (learned mode) */
+    int recover_minblocks[16];  /* register target: resident blocks per SM (learned mode, stiff kinetics) */
     float recover_ms[16];
     int chosen_flux_ci;
     int chosen_recover_block;

@@ -268,14 +268,26 @@ def mixed_block(gpu, dims, **kw):
     return s
 
 
-def flux_kernels(fn):
-    """Names of the flux kernels that fn launches."""
+def flux_launches(fn):
+    """The flux kernels that fn launches: {(name, grid)}."""
+    import json
+    import os
+    import tempfile
     import torch
     from torch.profiler import ProfilerActivity, profile
     with profile(activities=[ProfilerActivity.CUDA], acc_events=True) as p:
         fn()
         torch.cuda.synchronize()
-    return {k for k in ("k_flux_update_faces", "k_flux_update_tiled") if any(k in e.key for e in p.key_averages())}
+    with tempfile.TemporaryDirectory() as d:
+        p.export_chrome_trace(os.path.join(d, "trace.json"))
+        with open(os.path.join(d, "trace.json")) as f:
+            events = json.load(f)["traceEvents"]
+    return {(k, tuple(e["args"]["grid"])) for e in events if e.get("cat") == "kernel"
+            for k in ("k_flux_update_faces", "k_flux_update_tiled") if k in e["name"]}
+
+
+def flux_kernels(fn):
+    return {k for k, _ in flux_launches(fn)}
 
 
 def test_flux_kernel_follows_the_call(gpu):
@@ -366,6 +378,45 @@ def test_autotuned_launch_shapes_change_no_bits(gpu, precision, arith, chemistry
         s.close()
     for a, b in zip(*out):
         assert n_unequal(a, b) == 0
+
+
+def test_tuned_march_belongs_to_its_kernel(gpu):
+    """A march tuned on the face kernel, which a small grid takes alone, is not the
+    tiled kernel's in a batch: that one keeps its default there (blocks of 24
+    planes: 3 for the 50 of the small instance, 6 for the large one's 128)."""
+    a = mixed_block(gpu, (50, 7, 32), chemistry="frozen")
+    assert 1 in a.autotune(reps=1)["flux_ms"]
+    big = mixed_block(gpu, (128, 98, 96), chemistry="frozen")
+    b = gpu.Batch([a, big])
+    assert flux_launches(lambda: b.step(1, 2e-8)) == {("k_flux_update_tiled", (1, 1, 3)), ("k_flux_update_tiled", (3, 14, 6))}
+
+
+def test_autotune_beyond_65535_planes(gpu):
+    """A mixed grid that takes the tiled flux kernel with more planes along x than
+    a launch has blocks in z: the tuner offers no march that needs more (nor a
+    single plane, which only the face kernel has), and the tuned steps' bits are
+    XX."""
+    ni, nj, nk = 65560, 7, 26
+    mech = golden_mechanism()
+    rng = np.random.default_rng(1)
+    shape = (24, nj + 4, nk + 4)
+    f = rng.uniform(0.0, 1.0, shape)
+    Y = np.zeros((9,) + shape)
+    Y[5], Y[4], Y[8] = 0.1 * f, 0.8 * f, 1 - 0.9 * f
+    prim = (1e5 * rng.uniform(0.7, 1.4, shape), rng.uniform(400.0, 1300.0, shape), *(rng.uniform(-900.0, 900.0, shape) for _ in range(3)), Y)
+    _, cs, T, E = gpu.initial_state(mech, 20, nj, nk, *prim)
+    planes = 2 + np.arange(ni + 4) % 20  # (the ghost planes of the state are not formed)
+    h = 5e-4
+    s = gpu.Solver(ni, nj, nk, (0.0, h * (ni - 1), 0.0, h * (nj - 1), 0.0, h * (nk - 1)), chemistry="frozen", precision="mixed", arith="fast")
+    s.set_mechanism(mech)
+    got = []
+    for tune in (False, True):
+        s.set_conserved(cs[:, planes], T[:, planes], E[:, planes])
+        if tune:
+            assert min(s.autotune(reps=1)["flux_ms"]) >= 8
+        s.step(1, 2e-8)
+        got.append(s.get("T"))
+    assert np.array_equal(*got) and np.isfinite(got[0]).all()
 
 
 @pytest.mark.parametrize("width,steps,tol", [(2.0, 40, 1e-11), (6.0, 100, 1e-10)])
