@@ -672,6 +672,15 @@ __device__ __forceinline__ void eval_rates(const DevMech &m, double T, double, d
     for (int s = 0; s < NS; ++s) k.W[s] = m.mw[s] * k.W[s];
 }
 #else
+// x^n for a whole n; ix = 1/x.
+__device__ __forceinline__ double pow_whole(double x, double ix, double n)
+{
+    double r = 1.0;
+#pragma unroll 1
+    for (int q = int(fabs(n)); q > 0; --q) r *= n > 0.0 ? x : ix;
+    return r;
+}
+
 // Fast form, algebraically the reference's:
 //   Kc_r = exp(-sum_s nu_rs g_s) (p0/RT)^Xr with g_s = G_s/(R T) per species, so
 //   kb_r = kf_r * prod_s exp(g_s)^nu_rs * (RT/p0)^Xr  (one exp per species);
@@ -716,7 +725,7 @@ __device__ __forceinline__ void eval_rates(const DevMech &m, double T, double in
             rtb += mc[s] * m.tb[r][s];
         }
         const double Xr = m.xr[r];
-        kc_inv *= (Xr == 0.0 ? 1.0 : Xr == 1.0 ? rt_p0 : p0_rt);
+        kc_inv *= (Xr == 0.0 ? 1.0 : Xr == 1.0 ? rt_p0 : Xr == -1.0 ? p0_rt : pow_whole(rt_p0, p0_rt, Xr));
         const double kb = kf * kc_inv;
         if (rtb == 0.0)
             rtb = 1.0;

@@ -253,6 +253,37 @@ def test_strict_warp_kinetics_match_restatement(gpu, port_lib):
     assert torch.equal(got[4][0][:, few], got[20000][0][:, few]) and torch.equal(got[4][1][few], got[20000][1][few])
 
 
+@pytest.mark.parametrize("precision,bound", [("fp64", 1e-9), ("mixed", 1e-5)])
+def test_reactions_that_change_the_mole_number_by_two(gpu, precision, bound):
+    """A mechanism with 2 H + O -> H2O and H2O -> 2 H + O (the sides differ by two
+    moles, so Kc carries (RT/p0)^-2 and ^2): the fast forms of the rates against
+    the strict ones on gas near equilibrium, where the backward rates count. FP64:
+    rounding only; mixed: FP32 fluxes of a gas nearly at rest."""
+    mech = gpu.parse_mechanism(cases.MECH_JA919, cases.THERMO)
+    H, O, H2O = 0, 1, 2
+    for r, (f, b), (A, Bf, E) in ((5, ({H: 2, O: 1}, {H2O: 1}), (1e18, -1.0, 0.0)), (18, ({H2O: 1}, {H: 2, O: 1}), (1e19, 0.0, 2.2e5))):
+        for key, side in (("stoi_f", f), ("stoi_b", b)):
+            mech[key][:, r] = [side.get(s, 0) for s in range(9)]
+        mech["tb"][:, r] = 0
+        mech["af"][r], mech["bf"][r], mech["eaf"][r] = A, Bf, E
+    shape = (10, 9, 8)
+    rng = np.random.default_rng(8)
+    Y = np.zeros((9,) + shape)
+    Y[H], Y[O], Y[H2O], Y[3], Y[4], Y[5] = 0.002, 0.02, 0.2, 0.03, 0.03, 0.004
+    Y[8] = 1 - Y.sum(axis=0)
+    T = rng.uniform(2800.0, 3200.0, shape)
+    got = {}
+    for prec, arith in (("fp64", "strict"), (precision, "fast")):
+        s = gpu.Solver(6, 5, 4, (0.0, 5e-3, 0.0, 4e-3, 0.0, 3e-3), precision=prec, arith=arith)
+        s.set_mechanism(mech)
+        s.set_primitive(np.full(shape, 1e5), T, *(np.zeros(shape) for _ in range(3)), Y)
+        s.step(3, 2e-8)
+        got[arith] = interior(s.get("T")), interior(s.get("CS"))
+    for a, b in zip(got["fast"], got["strict"]):
+        for q in (range(len(b)) if len(b) == 1 else (H, O, H2O, 12)):
+            assert np.abs(a[q] - b[q]).max() <= bound * np.abs(b[q]).max(), q
+
+
 def mixed_block(gpu, dims, **kw):
     """A mixed-precision solver on random reacting gas with O(1) changes between nodes."""
     h = 5e-4
@@ -395,7 +426,7 @@ def test_autotune_beyond_65535_planes(gpu):
     """A mixed grid that takes the tiled flux kernel with more planes along x than
     a launch has blocks in z: the tuner offers no march that needs more (nor a
     single plane, which only the face kernel has), and the tuned steps' bits are
-    XX."""
+    the untuned ones' (a state of 20 different planes repeated along x)."""
     ni, nj, nk = 65560, 7, 26
     mech = golden_mechanism()
     rng = np.random.default_rng(1)
