@@ -83,18 +83,19 @@ __device__ __forceinline__ double div_fast(double n, double d)
 }
 __device__ __forceinline__ float div_fast(float n, float d) { return __fdividef(n, d); }
 
-// exp(x): x = k ln 2 + r, |r| <= ln(2)/2, e^r = 1 + r + r^2 q(r) with q the
-// degree-9 polynomial through (e^r - 1 - r) / r^2 at the ten Chebyshev nodes of
-// that interval (relative error of e^r below 2e-17), scaled by 2^k. Within one
-// unit in the last place for results in the normal range; 0 below it, at most
-// the largest power-of-two range's end above it; a NaN stays a NaN. Straight
-// code (no special-case branches), so that a cell's twenty-odd exponentials
-// interleave.
+// exp(x) for |x| <= kExpMost: x = k ln 2 + r, |r| <= ln(2)/2, e^r = 1 + r + r^2 q(r)
+// with q the degree-9 polynomial through (e^r - 1 - r) / r^2 at the ten Chebyshev
+// nodes of that interval (relative error of e^r below 4e-17), scaled by 2^k. Within
+// one unit in the last place; a NaN stays a NaN. Straight code (no special-case
+// branches), so that a cell's twenty-odd exponentials interleave: whoever calls it
+// keeps to the range (DevMech::t_lo, t_hi).
+constexpr double kExpMost = 708.0;
+
 __device__ __forceinline__ double exp_fast(double x)
 {
     constexpr double kShift = 6755399441055744.0; // 1.5 * 2^52: rounds to an integer in the low word
     const double t = fma(x, 1.4426950408889634, kShift), kd = t - kShift;
-    const int k = min(max(__double2loint(t), -1023), 1023);
+    const int k = __double2loint(t);
     double r = fma(kd, -0x1.62e42fefa39efp-1, x);
     r = fma(kd, -0x1.abc9e3b39803fp-56, r);
     double q = 0x1.af38b4925be09p-26;
@@ -109,6 +110,24 @@ __device__ __forceinline__ double exp_fast(double x)
     q = fma(q, r, 0.5);
     const double scale = __hiloint2double((k + 1023) << 20, 0);
     return fma(scale, fma(r * r, q, r), scale);
+}
+
+// exp_fast with its polynomial's terms paired (a third of the dependent operations).
+__device__ __forceinline__ double exp_paired(double x)
+{
+    constexpr double kShift = 6755399441055744.0;
+    const double t = fma(x, 1.4426950408889634, kShift), kd = t - kShift;
+    const int k = __double2loint(t);
+    double r = fma(kd, -0x1.62e42fefa39efp-1, x);
+    r = fma(kd, -0x1.abc9e3b39803fp-56, r);
+    const double r2 = r * r, r4 = r2 * r2;
+    const double a = fma(0x1.5555555555556p-3, r, 0.5), b = fma(0x1.11111111109b2p-7, r, 0x1.5555555553d5ep-5),
+                 c = fma(0x1.a01a01a7c54aep-13, r, 0x1.6c16c1788dc33p-10),
+                 d = fma(0x1.71de0da9d06acp-19, r, 0x1.a019b905bafb1p-16),
+                 e = fma(0x1.af38b4925be09p-26, r, 0x1.28918e390a71ep-22);
+    const double q = fma(fma(e, r4, fma(d, r2, c)), r4, fma(b, r2, a));
+    const double scale = __hiloint2double((k + 1023) << 20, 0);
+    return fma(scale, fma(r2, q, r), scale);
 }
 
 // ------------------------------------------------------------------ thermo
@@ -681,6 +700,72 @@ __device__ __forceinline__ double pow_whole(double x, double ix, double n)
     return r;
 }
 
+// The rates outside [t_lo, t_hi] (very cold gas: exp(G/RT) of water vapour leaves
+// the normal range below 43 K), where the products of the form below would meet an
+// underflowed factor with an overflowed one: one exponential of each reaction's
+// whole exponent, forward and backward, by exp. Rare, so out of line and rolled.
+template <int NS, int NR>
+__device__ __noinline__ void eval_rates_far(const DevMech &m, double T, double inv, double lnT, const double *mc,
+                                            double *Q, double *P)
+{
+    double g[NS], f[9];
+    gibbs_terms(T, inv, lnT, f);
+    const bool low = T < kThermoSwitch;
+#pragma unroll 1
+    for (int s = 0; s < NS; ++s) {
+        double v = 0.0;
+#pragma unroll
+        for (int k = 0; k < 9; ++k) v = fma(f[k], low ? m.clo[k][s] : m.chi[k][s], v);
+        g[s] = v;
+        P[s] = Q[s] = 0.0;
+    }
+    const double rt_p0 = T * (kRUniv / (kP0 * 1e-6)), p0_rt = inv * (kP0 * 1e-6 / kRUniv);
+#pragma unroll 1
+    for (int r = 0; r < NR; ++r) {
+        double rrf = 1.0, rrb = 1.0, rtb = 0.0, dg = 0.0;
+#pragma unroll 1
+        for (int s = 0; s < NS; ++s) {
+            const double nf = m.sf[r][s], nb = m.sb[r][s], c = mc[s];
+            rrf *= nf == 0.0 ? 1.0 : nf == 1.0 ? c : c * c;
+            rrb *= nb == 0.0 ? 1.0 : nb == 1.0 ? c : c * c;
+            dg = fma(nb - nf, g[s], dg);
+            rtb += c * m.tb[r][s];
+        }
+        if (rtb == 0.0)
+            rtb = 1.0;
+        const double e = m.bf[r] * lnT - m.eaf[r] * (inv * (1.0 / kRuCal));
+        const double fr = m.af[r] * exp(e) * rrf * rtb;
+        const double br = m.af[r] * exp(e + dg) * pow_whole(rt_p0, p0_rt, m.xr[r]) * rrb * rtb;
+#pragma unroll 1
+        for (int s = 0; s < NS; ++s) {
+            const double nf = m.sf[r][s], nb = m.sb[r][s];
+            if (nf != 0.0 || nb != 0.0) {
+                Q[s] += nb * fr + nf * br;
+                P[s] += nb * br + nf * fr;
+            }
+        }
+    }
+}
+
+// Whether the rates at T were formed by eval_rates_far.
+template <int NS, int NR>
+__device__ __forceinline__ bool rates_far(const DevMech &m, double T, double inv, double lnT, const double (&mc)[NS],
+                                          SpeciesRates<NS> &k)
+{
+    if (T >= m.t_lo && T <= m.t_hi)
+        return false;
+    double c[NS], Q[NS], P[NS]; // the call's own copies: the caller's arrays stay in registers
+#pragma unroll
+    for (int s = 0; s < NS; ++s) c[s] = mc[s];
+    eval_rates_far<NS, NR>(m, T, inv, lnT, c, Q, P);
+#pragma unroll
+    for (int s = 0; s < NS; ++s) {
+        k.Q[s] = Q[s];
+        k.P[s] = P[s];
+    }
+    return true;
+}
+
 // Fast form, algebraically the reference's:
 //   Kc_r = exp(-sum_s nu_rs g_s) (p0/RT)^Xr with g_s = G_s/(R T) per species, so
 //   kb_r = kf_r * prod_s exp(g_s)^nu_rs * (RT/p0)^Xr  (one exp per species);
@@ -689,6 +774,8 @@ template <int NS, int NR>
 __device__ __forceinline__ void eval_rates(const DevMech &m, double T, double inv, double lnT, const double (&mc)[NS],
                                            SpeciesRates<NS> &k)
 {
+    if (rates_far<NS, NR>(m, T, inv, lnT, mc, k))
+        return;
     double eg[NS], ieg[NS];
     gibbs_rt<NS>(m, T, inv, lnT, eg);
 #pragma unroll

@@ -373,24 +373,6 @@ __device__ __forceinline__ double log1p_paired(double x)
     return x * fma(fma(1.0 / 9.0, x4, cd), x4, ab);
 }
 
-// exp_fast with its polynomial's terms paired.
-__device__ __forceinline__ double exp_paired(double x)
-{
-    constexpr double kShift = 6755399441055744.0;
-    const double t = fma(x, 1.4426950408889634, kShift), kd = t - kShift;
-    const int k = min(max(__double2loint(t), -1023), 1023);
-    double r = fma(kd, -0x1.62e42fefa39efp-1, x);
-    r = fma(kd, -0x1.abc9e3b39803fp-56, r);
-    const double r2 = r * r, r4 = r2 * r2;
-    const double a = fma(0x1.5555555555556p-3, r, 0.5), b = fma(0x1.11111111109b2p-7, r, 0x1.5555555553d5ep-5),
-                 c = fma(0x1.a01a01a7c54aep-13, r, 0x1.6c16c1788dc33p-10),
-                 d = fma(0x1.71de0da9d06acp-19, r, 0x1.a019b905bafb1p-16),
-                 e = fma(0x1.af38b4925be09p-26, r, 0x1.28918e390a71ep-22);
-    const double q = fma(fma(e, r4, fma(d, r2, c)), r4, fma(b, r2, a));
-    const double scale = __hiloint2double((k + 1023) << 20, 0);
-    return fma(scale, fma(r2, q, r), scale);
-}
-
 // One rate evaluation of the fast form: lane s returns Q and P of species s.
 // mc: every species' concentration is in x.mc, this lane's in mcl.
 template <int NS, int NR>
@@ -409,7 +391,7 @@ __device__ __forceinline__ void heavy_rates(const HeavyTables<NS, NR> &t, HeavyS
     const double b = t.bf[lane], E = t.eaf[lane], Xr = t.xr[lane];
     // Every candidate is formed before it is chosen, so the choices are
     // selects: the lanes hold different reactions.
-    const double ex = exp_paired(fma(b, lnT, -E * (inv * (1.0 / kRuCal))));
+    const double e = fma(b, lnT, -E * (inv * (1.0 / kRuCal))), ex = exp_paired(e);
     double tpow = ex;
     const bool plain = E == 0.0;
     tpow = plain && b == 1.0 ? T : tpow;
@@ -440,8 +422,15 @@ __device__ __forceinline__ void heavy_rates(const HeavyTables<NS, NR> &t, HeavyS
         d1 = fma(t.dg[q + 1][lane], x.g[t.dgi[q + 1][lane]], d1);
     }
     const bool real = lane < NR; // slot 31 (and every slot past NR) holds zero rates
-    x.fwd[lane] = real ? kt * rrf : 0.0;
-    x.bwd[lane] = real ? (kt * back) * exp_paired(d0 + d1) : 0.0;
+    const double dg = d0 + d1;
+    double fr = kt * rrf, br = (kt * back) * exp_paired(dg);
+    if (max(__double2hiint(e) & 0x7fffffff, __double2hiint(dg) & 0x7fffffff) >= __double2hiint(kExpMost)) { // as eval_rates_far
+        const double art = t.af[lane] * rtb;
+        fr = art * exp(e) * rrf;
+        br = art * exp(e + dg) * back;
+    }
+    x.fwd[lane] = real ? fr : 0.0;
+    x.bwd[lane] = real ? br : 0.0;
     __syncwarp();
     // species sums, a third of the reactions a lane
     double q0 = 0.0, p0 = 0.0;

@@ -28,6 +28,9 @@ struct DevMech {
     double xr[kMaxR];       // sum_s (nu_b - nu_f)
     double sf[kMaxR][kMaxS], sb[kMaxR][kMaxS], tb[kMaxR][kMaxS];
     int has_tb[kMaxR];
+    // Temperatures between which the exponentials of the fast rate forms, their
+    // reciprocals and products stay in the range of normal numbers (rate_range)
+    double t_lo, t_hi;
 };
 
 // Division of an index n < 2^31 by a fixed divisor d >= 1 without a divide

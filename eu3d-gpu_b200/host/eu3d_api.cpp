@@ -147,6 +147,47 @@ void free_all(eu_handle *h)
     h->bytes = 0;
 }
 
+// The temperatures between which the fast forms of the rates (eval_rates) meet no
+// exponent beyond 690, in steps of 0.5 % from the thermo switch down to 1 K and up
+// to 100,000 K: every species' g = G/(R T), whose exponential and reciprocal they
+// form, the products of those in the order in which a reaction takes them, and
+// each rate constant's exponent. (An exponent changes by a few units a step, and
+// the exponentials hold to 708.)
+void rate_range(DevMech &d)
+{
+    auto fits = [&](double T) {
+        const double lnT = std::log(T);
+        const auto &c = T < kThermoSwitch ? d.clo : d.chi;
+        double g[kMaxS];
+        for (int s = 0; s < d.ns; ++s) {
+            const double h = (-c[0][s] / T + c[1][s] * lnT + c[7][s]) / T + c[2][s] +
+                             T * (c[3][s] / 2 + T * (c[4][s] / 3 + T * (c[5][s] / 4 + T * c[6][s] / 5)));
+            const double e = -c[0][s] / (2 * T * T) - c[1][s] / T + c[2][s] * lnT + c[8][s] +
+                             T * (c[3][s] + T * (c[4][s] / 2 + T * (c[5][s] / 3 + T * c[6][s] / 4)));
+            g[s] = h - e;
+            if (!(std::fabs(g[s]) <= 690))
+                return false;
+        }
+        for (int r = 0; r < d.nr; ++r) {
+            double sum = 0;
+            for (int s = 0; s < d.ns; ++s) {
+                sum += (d.sb[r][s] - d.sf[r][s]) * g[s];
+                if (!(std::fabs(sum) <= 690))
+                    return false;
+            }
+            if (!(std::fabs(d.bf[r] * lnT - d.eaf[r] / (kRuCal * T)) <= 690))
+                return false;
+        }
+        return true;
+    };
+    d.t_lo = kThermoSwitch;
+    d.t_hi = 0; // no temperature fits
+    if (!fits(kThermoSwitch))
+        return;
+    for (double T = kThermoSwitch; T >= 1 && fits(T); T /= 1.005) d.t_lo = T;
+    for (double T = kThermoSwitch; T <= 1e5 && fits(T); T *= 1.005) d.t_hi = T;
+}
+
 // DevMech from host tables; rejects sizes the kernels are not built for.
 eu_status install_mechanism(eu_handle *h, const MechanismTables &m)
 {
@@ -196,6 +237,7 @@ eu_status install_mechanism(eu_handle *h, const MechanismTables &m)
     if (!nu_int)
         return fail(h, EU_ERR_UNSUPPORTED, "stoichiometric coefficients other than 0, 1, 2 are not supported");
     d.nu_int = nu_int;
+    rate_range(d);
     // the warp-per-cell kinetics' tables hold reactions of at most three molecules
     // a side whose sides differ by at most one; other mechanisms' cells all run
     // on a thread each

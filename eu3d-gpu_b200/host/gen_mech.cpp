@@ -119,7 +119,8 @@ void emit_strict(std::ostream &o, const MechanismTables &m)
 void emit_fast(std::ostream &o, const MechanismTables &m)
 {
     const int ns = m.ns, nr = m.nr;
-    o << "    double g[" << ns << "], eg[" << ns << "], ieg[" << ns << "];\n"
+    o << "    if (rates_far<" << ns << ", " << nr << ">(m, T, inv, lnT, mc, k))\n        return;\n"
+      << "    double g[" << ns << "], eg[" << ns << "], ieg[" << ns << "];\n"
       << "    gibbs_rt<" << ns << ">(m, T, inv, lnT, g);\n";
     for (int sp = 0; sp < ns; ++sp) {
         bool used = false;

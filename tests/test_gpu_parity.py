@@ -284,6 +284,37 @@ def test_reactions_that_change_the_mole_number_by_two(gpu, precision, bound):
             assert np.abs(a[q] - b[q]).max() <= bound * np.abs(b[q]).max(), q
 
 
+@pytest.mark.parametrize("precision,bound,deferred", [("fp64", 1e-9, False), ("fp64", 1e-9, True), ("mixed", 1e-5, False)])
+def test_rates_of_very_cold_gas(gpu, precision, bound, deferred):
+    """The fast forms of the rates at 41 to 42 K, where the exponential of water
+    vapour's G/(R T) has left the range of doubles (43 K), on a thread per cell
+    and, with radicals, a warp per cell, against the strict ones: far below the
+    thermo fit, but a step that the reference's forms take. FP64: rounding, of
+    exponents up to 1,000; mixed: FP32 fluxes of a gas nearly at rest."""
+    shape = (10, 9, 8)
+    rng = np.random.default_rng(8)
+    Y = np.zeros((9,) + shape)
+    Y[4], Y[5] = 0.2, 0.02
+    if deferred:
+        Y[0] = 1e-6
+    else:
+        Y[2], Y[6], Y[7] = 1e-3, 1e-5, 1e-5
+    Y[8] = 1 - Y.sum(axis=0)
+    T, dt = rng.uniform(41.0, 42.0, shape), 1e-9
+    got = {}
+    for prec, arith in (("fp64", "strict"), (precision, "fast")):
+        s = gpu.Solver(6, 5, 4, (0.0, 5e-3, 0.0, 4e-3, 0.0, 3e-3), precision=prec, arith=arith)
+        s.set_mechanism(gpu.parse_mechanism(cases.MECH_JA919, cases.THERMO))
+        s.set_primitive(np.full(shape, 1e4), T, *(np.zeros(shape) for _ in range(3)), Y)
+        stats = s.step(1, dt)
+        assert (stats["max_nchem"] > 4) == deferred, stats
+        got[arith] = interior(s.get("T")), interior(s.get("CS"))
+    for a, b in zip(got["fast"], got["strict"]):
+        assert np.isfinite(a).all()
+        for q in (range(len(b)) if len(b) == 1 else (0, 1, 2, 3, 12)):
+            assert np.abs(a[q] - b[q]).max() <= bound * np.abs(b[q]).max(), q
+
+
 def mixed_block(gpu, dims, **kw):
     """A mixed-precision solver on random reacting gas with O(1) changes between nodes."""
     h = 5e-4
