@@ -273,7 +273,7 @@ __global__ void __launch_bounds__(kTrainThreads, 2) k_train_rows(const __grid_co
                             const float target = (p.T[src * p.n_out + c + u] - p.out_shift[c + u]) * p.out_scale[c + u];
                             d = v[j * 8 + u] + __ldg(mem.bias[L] + c + u) - target;
                             sq += d * d;
-                            d = 2.0f * d / float(p.n * p.n_out);
+                            d = 2.0f * d / float((long long)p.n * p.n_out);
                         }
                         g[u] = __float2bfloat16_rn(d);
                         v[j * 8 + u] = __bfloat162float(g[u]);

@@ -611,7 +611,7 @@ eu_status eu_mlp_loss_grad(eu_mlp *m, int member, const float *X, const float *T
         MCK(m, cudaMemcpyAsync(all.data(), g, all.size() * 4, cudaMemcpyDeviceToHost, m->stream));
     if ((s = check_err(m)) != EU_OK)
         return s;
-    *loss_out = sq / float(n * m->n_out);
+    *loss_out = sq / float((long long)n * m->n_out);
     if (grads_out)
         unpad(m, all.data(), grads_out);
     return EU_OK;
@@ -651,7 +651,7 @@ eu_status eu_mlp_train(eu_mlp *m, const float *X, const float *T, long long n, i
     if ((s = check_err(m)) != EU_OK)
         return s;
     if (mean_loss)
-        for (int e = 0; e < m->members; ++e) mean_loss[e] = float(sq[e] / double(batch * m->n_out));
+        for (int e = 0; e < m->members; ++e) mean_loss[e] = float(sq[e] / double((long long)batch * m->n_out));
     return EU_OK;
 }
 

@@ -160,6 +160,28 @@ def test_silu_gradient_divides_exactly(gpu):
     assert np.abs(got[:7] / dh - [0, 0, 0, 0, 1, 1, 1]).max() <= 1e-7
 
 
+def test_batch_of_two_to_the_31_values(gpu):
+    """A batch whose values (rows x outputs) no longer fit an int: the mean's
+    divisor keeps its sign. Equal rows, so the output biases' gradients are 2 y /
+    outputs, but for one bf16 rounding (2^-9) and an fp32 sum of a value per 32 rows
+    (262,144 additions of half a unit of the sum so far, 2^-25 of the last one on
+    average); the loss adds two values per 32 rows."""
+    import torch
+    n, n_out = 1 << 23, 256
+    m = gpu.Mlp()
+    m.init(1, 16, 1, n_out, 1, max_batch=n, seed=1)
+    y = np.random.default_rng(6).uniform(0.5, 2.0, n_out).astype(np.float32)
+    m.set_params(np.concatenate([np.zeros(16 + 16 + 16 * n_out), y]).astype(np.float32))
+    X, T = torch.zeros(n, 1, device="cuda"), torch.zeros(n, n_out, device="cuda")
+    torch.cuda.synchronize()
+    loss, g = m.loss_grad(0, X, T)
+    m.close()
+    del X, T
+    torch.cuda.empty_cache()
+    assert np.abs(g[-n_out:] / (2 * y / n_out) - 1).max() <= 2.0**-9 + (n // 32) * 2.0**-25
+    assert abs(loss / np.mean(y.astype(np.float64) ** 2) - 1) <= (n // 16) * 2.0**-25
+
+
 @pytest.mark.parametrize("shape", [(N_IN, WIDTH, HIDDEN, N_OUT, MEMBERS), (5, 64, 2, 3, 2), (20, 96, 1, 40, 1)])
 def test_fused_inference_matches_layerwise(gpu, shape):
     """The one-kernel inference (every member's network per 128-row tile, the
