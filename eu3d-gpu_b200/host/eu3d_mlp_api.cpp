@@ -3,6 +3,7 @@
 // evaluated with the BF16 tensor-core GEMM (fp32 accumulation, fp32 master
 // weights, Adam). All tensors stay on the device; training batches are drawn
 // on the device from caller-provided fp32 arrays.
+#include <algorithm>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -52,10 +53,10 @@ struct eu_mlp {
     float *loss = nullptr; // [members]
     long long adam_t = 0;
     std::vector<void *> allocs;
-    // training scratch of every member for batches of up to train_rows rows
-    // (allocated by the first training call, grown with the batch, kept)
+    // training scratch (allocated by the first training call, grown with the
+    // batch and the members that run together, kept)
     void *train = nullptr;
-    long long train_rows = 0;
+    size_t train_bytes = 0;
     // inference in one persistent kernel (eu3d_mlp_fused.cuh), on the K-slabs
     bool fused = false;
     __nv_bfloat16 *slabs = nullptr;
@@ -105,7 +106,7 @@ void free_all(eu_mlp *m)
     if (m->train)
         cudaFree(m->train);
     m->train = nullptr;
-    m->train_rows = 0;
+    m->train_bytes = 0;
     m->net.clear();
     m->H.clear();
     m->ready = false;
@@ -177,22 +178,31 @@ eu3d::TrainParams train_params(const eu_mlp *m, int first, int count)
     return p;
 }
 
-// A batch of n rows of the caller's arrays, with the members' scratch for it.
-eu_status train_batch(eu_mlp *m, eu3d::TrainParams &p, const float *X, const float *T, long long rows, int n, bool drawn)
+// A batch of n rows of the caller's arrays, with scratch for `group` members: all
+// run together with scratch of their own, or, where memory is short, one at a time
+// on one (6.2 KB a row and member at 256 x 3).
+eu_status train_batch(eu_mlp *m, eu3d::TrainParams &p, const float *X, const float *T, long long rows, int n, bool drawn,
+                      int group)
 {
     // whole tiles: every piece a multiple of 128 values
     const size_t rows_pad = size_t(n + eu3d::kTrainRows - 1) / eu3d::kTrainRows * eu3d::kTrainRows;
     const size_t wide = size_t(m->hidden) * m->width * rows_pad;
     const size_t bytes = wide * (4 + 2 + 2) + rows_pad * (m->in_pad + m->out_pad) * 2;
-    if (m->train_rows < n) {
+    if (m->train_bytes < bytes * group) {
         if (m->train) {
             MCK(m, cudaStreamSynchronize(m->stream));
             MCK(m, cudaFree(m->train));
         }
         m->train = nullptr;
-        m->train_rows = 0;
-        MCK(m, cudaMalloc(&m->train, bytes * m->members));
-        m->train_rows = n;
+        m->train_bytes = 0;
+        const cudaError_t e = cudaMalloc(&m->train, bytes * group);
+        if (e != cudaSuccess) {
+            m->train = nullptr;
+            cudaGetLastError(); // the launches' own check starts clean
+            return mfail(m, e == cudaErrorMemoryAllocation ? EU_ERR_OUT_OF_MEMORY : EU_ERR_CUDA, "training scratch: %s",
+                         cudaGetErrorString(e));
+        }
+        m->train_bytes = bytes * group;
     }
     p.X = X;
     p.T = T;
@@ -201,7 +211,7 @@ eu_status train_batch(eu_mlp *m, eu3d::TrainParams &p, const float *X, const flo
     p.drawn = drawn;
     for (int e = 0; e < m->members; ++e) {
         eu3d::TrainMember &t = p.member[e];
-        unsigned char *at = static_cast<unsigned char *>(m->train) + e * bytes;
+        unsigned char *at = static_cast<unsigned char *>(m->train) + e % group * bytes;
         t.ZT = reinterpret_cast<float *>(at);
         t.HT = reinterpret_cast<__nv_bfloat16 *>(at + wide * 4);
         t.dZT = t.HT + wide;
@@ -596,7 +606,7 @@ eu_status eu_mlp_loss_grad(eu_mlp *m, int member, const float *X, const float *T
         return mfail(m, EU_ERR_INVALID_ARGUMENT, "member or batch size (multiple of 16 up to max_batch)");
     cudaSetDevice(m->device);
     eu3d::TrainParams p = train_params(m, member, 1);
-    eu_status s = train_batch(m, p, X, T, n, n, false);
+    eu_status s = train_batch(m, p, X, T, n, n, false, 1);
     if (s != EU_OK)
         return s;
     float *g = m->G + member * m->params;
@@ -629,7 +639,10 @@ eu_status eu_mlp_train(eu_mlp *m, const float *X, const float *T, long long n, i
     cudaSetDevice(m->device);
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     eu3d::TrainParams p = train_params(m, 0, m->members);
-    eu_status s = train_batch(m, p, X, T, n, batch, true);
+    int group = m->members; // members that run together
+    eu_status s = train_batch(m, p, X, T, n, batch, true, group);
+    if (s == EU_ERR_OUT_OF_MEMORY && group > 1)
+        s = train_batch(m, p, X, T, n, batch, true, group = 1);
     if (s != EU_OK)
         return s;
     MCK(m, cudaMemsetAsync(m->G, 0, size_t(m->params) * m->members * 4, m->stream));
@@ -641,8 +654,13 @@ eu_status eu_mlp_train(eu_mlp *m, const float *X, const float *T, long long n, i
             p.member[e].key = (unsigned long long)seed * 0x100000001B3ull + (unsigned long long)m->adam_t * 131ull + e;
         if (it + 1 == steps) // the last batch's loss is the one returned
             MCK(m, cudaMemsetAsync(m->loss, 0, size_t(m->members) * sizeof(float), m->stream));
-        MCK(m, eu3d::train_rows(p, m->stream));
-        MCK(m, eu3d::train_weights(p, m->sms, m->stream));
+        for (p.first = 0; p.first < m->members; p.first += group) {
+            p.members = std::min(group, m->members - p.first);
+            MCK(m, eu3d::train_rows(p, m->stream));
+            MCK(m, eu3d::train_weights(p, m->sms, m->stream));
+        }
+        p.first = 0;
+        p.members = m->members;
         MCK(m, eu3d::train_adam(p, lr, b1, b2, eps, c1, c2, m->stream));
     }
     std::vector<float> sq(m->members, 0.0f);

@@ -182,6 +182,34 @@ def test_batch_of_two_to_the_31_values(gpu):
     assert abs(loss / np.mean(y.astype(np.float64) ** 2) - 1) <= (n // 16) * 2.0**-25
 
 
+def test_training_when_memory_is_short(gpu):
+    """With room for one member's scratch but not for all three's (0.82 GB each at
+    this batch) the members train one after the other, and a gradient takes one
+    member's scratch only. The sums' order differs, so the comparison with a model
+    that trained with room is Adam's: two steps of lr 1e-3 from the same start."""
+    import torch
+    n = 131072
+    rng = np.random.default_rng(3)
+    X, T = (torch.tensor(rng.normal(size=(n, k)), device="cuda", dtype=torch.float32) for k in (N_IN, N_OUT))
+    torch.cuda.synchronize()
+
+    def trained(short):
+        m = gpu.Mlp()
+        m.init(N_IN, WIDTH, HIDDEN, N_OUT, MEMBERS, max_batch=n, seed=3)
+        torch.cuda.empty_cache()
+        room = torch.empty(max(0, torch.cuda.mem_get_info()[0] - (3 << 29)) if short else 0, device="cuda", dtype=torch.uint8)
+        try:
+            loss, g = m.loss_grad(1, X, T)
+            return np.float64(loss), g, m.train(X, T, n, 2, 1e-3, seed=5), m.get_params()
+        finally:
+            m.close()
+            del room
+            torch.cuda.empty_cache()
+
+    for a, b in zip(trained(False), trained(True)):
+        assert np.linalg.norm(a - b) <= 1e-4 * np.linalg.norm(a)
+
+
 @pytest.mark.parametrize("shape", [(N_IN, WIDTH, HIDDEN, N_OUT, MEMBERS), (5, 64, 2, 3, 2), (20, 96, 1, 40, 1)])
 def test_fused_inference_matches_layerwise(gpu, shape):
     """The one-kernel inference (every member's network per 128-row tile, the
