@@ -1116,19 +1116,27 @@ eu_status eu_chem_advance(eu_handle *h, long long n, double *cs, double *T, doub
     cudaSetDevice(h->cfg.device);
     LaunchArgs a = launch_args(h);
     CK(h, cudaMemsetAsync(h->st.counters, 0, kCntCount * sizeof(unsigned long long), h->stream));
-    if (h->heavy_fits && n < (1LL << 31)) {
-        if (h->sample_capacity < n) {
-            if (h->sample_queue)
-                CK(h, cudaFree(h->sample_queue));
-            h->sample_queue = nullptr;
-            h->sample_capacity = 0;
-            CK(h, cudaMalloc(&h->sample_queue, (size_t(2) + size_t(n)) * sizeof(int)));
+    // the queue of the samples left to a warp each; without it (a mechanism that
+    // has no warp form, or no memory) every sample runs on a thread, to the same bits
+    if (h->heavy_fits && n < (1LL << 31) && h->sample_capacity < n) {
+        if (h->sample_queue)
+            CK(h, cudaFree(h->sample_queue));
+        h->sample_queue = nullptr;
+        h->sample_capacity = 0;
+        const cudaError_t e = cudaMalloc(&h->sample_queue, (size_t(2) + size_t(n)) * sizeof(int));
+        if (e == cudaSuccess) {
             h->sample_capacity = n;
+        } else {
+            h->sample_queue = nullptr;
+            cudaGetLastError(); // the launches' own check starts clean
+            if (e != cudaErrorMemoryAllocation)
+                return cuda_fail(h, e, "cudaMalloc(sample queue)");
         }
-        CK(h, cudaMemsetAsync(h->sample_queue, 0, 2 * sizeof(int), h->stream));
     }
-    CK(h, strict::launch_chem_samples(a, n, cs, T, E, dt, nchem,
-                                      h->heavy_fits && n < (1LL << 31) ? h->sample_queue : nullptr));
+    int *queue = h->heavy_fits && h->sample_capacity >= n ? h->sample_queue : nullptr;
+    if (queue)
+        CK(h, cudaMemsetAsync(queue, 0, 2 * sizeof(int), h->stream));
+    CK(h, strict::launch_chem_samples(a, n, cs, T, E, dt, nchem, queue));
     unsigned long long cnt[kCntCount];
     CK(h, cudaMemcpyAsync(cnt, h->st.counters, sizeof cnt, cudaMemcpyDeviceToHost, h->stream));
     CK(h, cudaStreamSynchronize(h->stream));

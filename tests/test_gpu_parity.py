@@ -253,6 +253,50 @@ def test_strict_warp_kinetics_match_restatement(gpu, port_lib):
     assert torch.equal(got[4][0][:, few], got[20000][0][:, few]) and torch.equal(got[4][1][few], got[20000][1][few])
 
 
+def igniting_samples(n, seed=3):
+    """Chemistry samples, more than one in ten beyond four substeps: T, p, Y, dt on the device."""
+    import torch
+    g = torch.Generator(device="cuda")
+    g.manual_seed(seed)
+    u = lambda a, b: a + (b - a) * torch.rand(n, generator=g, device="cuda", dtype=torch.float64)  # noqa: E731
+    Y = torch.zeros(9, n, device="cuda", dtype=torch.float64)
+    Y[5], Y[4], Y[3], Y[0], Y[8] = 0.03, 0.23, 0.005, 0.001, 0.734
+    return u(1200, 2600), u(1e5, 8e5), Y, 10 ** u(-8.5, -6.5)
+
+
+def test_samples_without_memory_for_the_queue(gpu):
+    """eu_chem_advance where the queue of the samples left to a warp each (256 MB)
+    does not fit the device any more: it runs every sample on a thread, to the same
+    bits in every state and Nchem. (The samples compared lie at both ends of a call
+    whose other samples take one substep.)"""
+    import torch
+    n, part = 1 << 26, 1 << 12
+    s = gpu.Solver(5, 5, 5, (0, 1, 0, 1, 0, 1))
+    s.set_mechanism(golden_mechanism())
+    T0, p0, Y0, dt0 = igniting_samples(part)
+    cs0, E0 = torch.zeros(13, part, device="cuda", dtype=torch.float64), torch.zeros(part, device="cuda", dtype=torch.float64)
+    s.chem_states(T0, p0, Y0, cs0, E0)
+    want = [cs0.clone(), T0.clone(), E0.clone(), torch.zeros(part, device="cuda", dtype=torch.int32)]
+    torch.cuda.synchronize()
+    s.chem_advance(*want[:3], dt0, want[3])
+    assert int((want[3] > 4).sum()) > part // 10 and all(torch.isfinite(t).all() for t in want)
+    cs = cs0[:, :1].repeat(1, n)
+    E, nchem = E0[:1].repeat(n), torch.zeros(n, device="cuda", dtype=torch.int32)
+    dt = torch.full((n,), 1e-12, device="cuda", dtype=torch.float64)
+    T = T0[:1].repeat(n)
+    for at in (slice(0, part), slice(n - part, n)):
+        cs[:, at], T[at], E[at], dt[at] = cs0, T0, E0, dt0
+    torch.cuda.empty_cache()
+    torch.cuda.synchronize()
+    room = torch.empty(torch.cuda.mem_get_info()[0] - (64 << 20), device="cuda", dtype=torch.uint8)
+    s.chem_advance(cs, T, E, dt, nchem)
+    del room
+    torch.cuda.empty_cache()
+    for at in (slice(0, part), slice(n - part, n)):
+        for a, b in zip((cs[:, at], T[at], E[at], nchem[at]), want):
+            assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("precision,bound", [("fp64", 1e-9), ("mixed", 1e-5)])
 def test_reactions_that_change_the_mole_number_by_two(gpu, precision, bound):
     """A mechanism with 2 H + O -> H2O and H2O -> 2 H + O (the sides differ by two
