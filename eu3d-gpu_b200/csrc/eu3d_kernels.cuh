@@ -221,6 +221,7 @@ template <typename R>
 constexpr int kFacePitch = sizeof(R) == 8 ? 464 : 496;
 struct FaceTile {
     int ti, tj, tk;
+    bool y_first; // blockIdx.x counts the tiles along y and blockIdx.y those along z (more than 65,535 along y)
     FastDiv d_tk, d_tk1, d_area, d_area_y, d_area_z;
 };
 
@@ -265,7 +266,7 @@ __global__ void __launch_bounds__(kFaceThreadsWide, 2)
     const int tid = threadIdx.x, nthreads = blockDim.x;
     const int area = t.tj * t.tk; // cells of a plane
     const int nfx = (t.ti + 1) * area, nfy = t.ti * (t.tj + 1) * t.tk, nf = nfx + nfy + t.ti * t.tj * (t.tk + 1);
-    const int k0 = blockIdx.x * t.tk, j0 = blockIdx.y * t.tj;
+    const int k0 = (t.y_first ? blockIdx.y : blockIdx.x) * t.tk, j0 = (t.y_first ? blockIdx.x : blockIdx.y) * t.tj;
     const int rows = min(t.tj, g.nj - j0), cols = min(t.tk, g.nk - k0);
     const int i_begin = blockIdx.z * ci, i_end = min(i_begin + ci, g.ni);
     const long long n3 = g.n3;

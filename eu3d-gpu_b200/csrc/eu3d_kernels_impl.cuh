@@ -108,6 +108,7 @@ FaceTile face_tile(const DevGrid &g)
     t.ti = std::min(g.ni, std::max(1, cells / (t.tj * t.tk)));
     while (t.ti > 1 && (t.ti + 1) * t.tj * t.tk + t.ti * (t.tj + 1) * t.tk + t.ti * t.tj * (t.tk + 1) > kFacePitch<R>)
         --t.ti;
+    t.y_first = (g.nj + t.tj - 1) / t.tj > 65535; // gridDim.y < 2^16
     t.d_tk = make_fastdiv(unsigned(t.tk));
     t.d_tk1 = make_fastdiv(unsigned(t.tk + 1));
     t.d_area = make_fastdiv(unsigned(t.tj * t.tk));
@@ -128,7 +129,8 @@ cudaError_t faces_flux_launch(const LaunchArgs &a, const R *prim)
     const FaceTile t = face_tile<R>(g);
     const int ci = std::max(std::max(a.face_ci, t.ti), (g.ni + 65534) / 65535); // gridDim.z < 2^16
     const int threads = (long long)g.ni * g.nj * g.nk < kFaceSmallCells ? kFaceThreadsWide : kFaceThreads;
-    const dim3 grid(unsigned((g.nk + t.tk - 1) / t.tk), unsigned((g.nj + t.tj - 1) / t.tj), unsigned((g.ni + ci - 1) / ci));
+    const unsigned tiles_z = unsigned((g.nk + t.tk - 1) / t.tk), tiles_y = unsigned((g.nj + t.tj - 1) / t.tj);
+    const dim3 grid(t.y_first ? tiles_y : tiles_z, t.y_first ? tiles_z : tiles_y, unsigned((g.ni + ci - 1) / ci));
     k_flux_update_faces<NS, R, kStrict><<<grid, threads, smem, a.stream>>>(g, a.st, prim, a.dt_dev, t, ci);
     return cudaGetLastError();
 }

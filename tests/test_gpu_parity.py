@@ -200,6 +200,35 @@ def test_face_kernel_tiles_match_restatement(gpu, port_lib, dims):
     assert cs_rel_linf(interior(s.get("CS")), interior(port.get("CS"))).max() <= 1e-12
 
 
+@pytest.mark.parametrize("precision,nk", [("fp64", 4), ("mixed", 17)])
+def test_face_kernel_beyond_65535_tiles_along_y(gpu, precision, nk):
+    """Grids with more tiles of four rows along y than a launch has blocks in y: the
+    rows repeat with period 20, so a step gives them, away from the ends, the bits
+    of a grid of 60 rows."""
+    ni, long = 2, 262200
+    mech = golden_mechanism()
+    rng = np.random.default_rng(2)
+    shape = (ni + 4, 24, nk + 4)
+    f = rng.uniform(0.0, 1.0, shape)
+    Y = np.zeros((9,) + shape)
+    Y[5], Y[4], Y[8] = 0.1 * f, 0.8 * f, 1 - 0.9 * f
+    _, cs, T, E = gpu.initial_state(mech, ni, 20, nk, 1e5 * rng.uniform(0.7, 1.4, shape), rng.uniform(400.0, 1300.0, shape),
+                                    *(rng.uniform(-900.0, 900.0, shape) for _ in range(3)), Y)
+    h = 2.0**-11  # every spacing exact
+    got = {}
+    for nj in (60, long):
+        rows = 2 + np.arange(nj + 4) % 20  # (the ghost rows of the state are not formed)
+        s = gpu.Solver(ni, nj, nk, (0.0, h * (ni - 1), 0.0, h * (nj - 1), 0.0, h * (nk - 1)), chemistry="frozen", precision=precision,
+                       arith="fast")
+        s.set_mechanism(mech)
+        s.set_conserved(cs[:, :, rows], T[:, :, rows], E[:, :, rows])
+        s.step(1, 2e-8)
+        got[nj] = interior(s.get("T"))[0]
+        s.close()
+    want = got[60][:, 20:40]
+    assert np.array_equal(got[long][:, 20:long - 20].reshape(ni, -1, 20, nk), np.broadcast_to(want[:, None], (ni, long // 20 - 2, 20, nk)))
+
+
 def test_strict_warp_kinetics_match_restatement(gpu, port_lib):
     """Strict FP64 on igniting gas whose long substep chains run a warp each
     (k_react_heavy), against the pinned C restatement, eight steps: Nchem exact,
