@@ -87,20 +87,24 @@ inline int even_piece(int n, int want)
     return (n + pieces - 1) / pieces;
 }
 
-// Grids below this many cells leave SMs without blocks when the tiles hold 128
-// cells (fewer than 8 blocks of 128 cells per SM of 148): there a tile holds
+// Small grids leave SMs without blocks when the tiles hold 128 cells (fewer than 8
+// blocks of 128 cells per SM): there a tile holds
 // half the cells and the block twice the threads, so that a step is one round
 // of faces a block (33 x 17 x 17 strict: 0.023 ms against 0.033-0.054 with the
 // large grids' tiles; 129 x 65 x 65 FP64 the other way: 0.133 against 0.145).
-constexpr long long kFaceSmallCells = 148LL * 8 * 128;
+inline bool small_grid(const LaunchArgs &a)
+{
+    return (long long)a.g.ni * a.g.nj * a.g.nk < (a.sms > 0 ? a.sms : 148) * 8LL * 128;
+}
 
 // The tile of k_flux_update_faces for a grid: 128 (small grids: 64) cells, rows
 // along z cut evenly into about 8 FP64 or 16 FP32 values (the whole of a thin
 // grid), 4 of them (16 on thin grids of many cells) along y, the rest along x.
 template <typename R>
-FaceTile face_tile(const DevGrid &g)
+FaceTile face_tile(const LaunchArgs &a)
 {
-    const bool small = (long long)g.ni * g.nj * g.nk < kFaceSmallCells;
+    const DevGrid &g = a.g;
+    const bool small = small_grid(a);
     const int cells = small ? 64 : 128;
     FaceTile t;
     t.tk = even_piece(g.nk, sizeof(R) == 8 ? 8 : 16);
@@ -126,9 +130,9 @@ cudaError_t faces_flux_launch(const LaunchArgs &a, const R *prim)
     const cudaError_t e = limit.ensure(k_flux_update_faces<NS, R, kStrict>, smem);
     if (e != cudaSuccess)
         return e;
-    const FaceTile t = face_tile<R>(g);
+    const FaceTile t = face_tile<R>(a);
     const int ci = std::max(std::max(a.face_ci, t.ti), (g.ni + 65534) / 65535); // gridDim.z < 2^16
-    const int threads = (long long)g.ni * g.nj * g.nk < kFaceSmallCells ? kFaceThreadsWide : kFaceThreads;
+    const int threads = small_grid(a) ? kFaceThreadsWide : kFaceThreads;
     const unsigned tiles_z = unsigned((g.nk + t.tk - 1) / t.tk), tiles_y = unsigned((g.nj + t.tj - 1) / t.tj);
     const dim3 grid(t.y_first ? tiles_y : tiles_z, t.y_first ? tiles_z : tiles_y, unsigned((g.ni + ci - 1) / ci));
     k_flux_update_faces<NS, R, kStrict><<<grid, threads, smem, a.stream>>>(g, a.st, prim, a.dt_dev, t, ci);
@@ -155,17 +159,17 @@ inline bool takes_tiled(const LaunchArgs &a)
     const DevGrid &g = a.g;
     const long long cells = std::max((long long)g.ni * g.nj * g.nk, a.batch_cells);
     const long long slots = (long long)tiles_j(g) * kTileJ * (tiles_k(g) * kTileK);
-    return a.precision == 1 && g.nk >= kThinNk && cells >= kTiledCells && 5LL * g.nj * g.nk >= 4 * slots;
+    return g.nk >= kThinNk && cells >= kTiledCells && 5LL * g.nj * g.nk >= 4 * slots;
 }
 
 template <int NS, int NR>
 cudaError_t flux_t(const LaunchArgs &a)
 {
-    if (a.precision != 1)
-        return faces_flux_launch<NS, double, kStrictFlux>(a, a.st.prim);
-    if (takes_tiled(a))
-        return tiled_flux_launch<NS>(a);
-    return faces_flux_launch<NS, float, false>(a, a.st.prim32);
+#ifdef EU_MIXED
+    return takes_tiled(a) ? tiled_flux_launch<NS>(a) : faces_flux_launch<NS, float, false>(a, a.st.prim32);
+#else
+    return faces_flux_launch<NS, double, kStrictFlux>(a, a.st.prim);
+#endif
 }
 
 template <int NS, int NR>
@@ -288,6 +292,7 @@ cudaError_t state_from_tpy_t(const LaunchArgs &a, long long n, const double *T, 
     return cudaGetLastError();
 }
 
+#ifdef EU_EXACT_RATES // the chemistry samples run in the strict flavour alone
 template <int NS, int NR>
 cudaError_t chem_samples_t(const LaunchArgs &a, long long n, double *cs, double *T, double *E, const double *dt,
                            int *nchem, int *heavy)
@@ -306,6 +311,7 @@ cudaError_t chem_samples_t(const LaunchArgs &a, long long n, double *cs, double 
                                0, a.stream>>>(*a.mech, n, cs, T, E, dt, nchem, a.max_substeps, a.st.counters, heavy);
     return cudaGetLastError();
 }
+#endif
 
 template <int NS, int NR>
 cudaError_t heavy_t(const LaunchArgs &a, int blocks)
@@ -332,6 +338,7 @@ cudaError_t react_queue_batch_t(const LaunchArgs &a, const BatchCell *tab, int n
     return cudaGetLastError();
 }
 
+#ifdef EU_MIXED // the FP64 flavours' deferred cells stay in their instance's branch
 template <int NS, int NR>
 cudaError_t heavy_batch_t(const LaunchArgs &a, const BatchCell *tab, int n, int *next, int blocks)
 {
@@ -339,6 +346,7 @@ cudaError_t heavy_batch_t(const LaunchArgs &a, const BatchCell *tab, int n, int 
                                                                                a.max_substeps);
     return cudaGetLastError();
 }
+#endif
 
 } // namespace
 
@@ -354,7 +362,11 @@ cudaError_t heavy_batch_t(const LaunchArgs &a, const BatchCell *tab, int n, int 
 
 cudaError_t launch_boundary(const LaunchArgs &a) { EU3D_DISPATCH(boundary_t, a) }
 cudaError_t launch_flux_update(const LaunchArgs &a) { EU3D_DISPATCH(flux_t, a) }
+#ifdef EU_MIXED
 int flux_plan(const LaunchArgs &a) { return takes_tiled(a) ? tiled_ci(a) : 0; }
+#else
+int flux_plan(const LaunchArgs &) { return 0; }
+#endif
 cudaError_t launch_recover_react(const LaunchArgs &a, bool react) { EU3D_DISPATCH(react_t, a, react) }
 cudaError_t launch_derived(const LaunchArgs &a, int which, double *out) { EU3D_DISPATCH(derived_t, a, which, out) }
 cudaError_t launch_materialize(const LaunchArgs &a) { EU3D_DISPATCH(materialize_t, a) }
@@ -378,21 +390,28 @@ cudaError_t launch_state_from_tpy(const LaunchArgs &a, long long n, const double
 {
     EU3D_DISPATCH(state_from_tpy_t, a, n, T, p, Y, cs, E)
 }
+#ifdef EU_EXACT_RATES
 cudaError_t launch_chem_samples(const LaunchArgs &a, long long n, double *cs, double *T, double *E, const double *dt,
                                 int *nchem, int *heavy)
 {
     EU3D_DISPATCH(chem_samples_t, a, n, cs, T, E, dt, nchem, heavy)
 }
+#endif
 
 cudaError_t launch_react_heavy(const LaunchArgs &a, int blocks) { EU3D_DISPATCH(heavy_t, a, blocks) }
 cudaError_t launch_react_queue_batch(const LaunchArgs &a, const BatchCell *tab, int n, int *next, int counter)
 {
     EU3D_DISPATCH(react_queue_batch_t, a, tab, n, next, counter)
 }
+#ifdef EU_MIXED
 cudaError_t launch_react_heavy_batch(const LaunchArgs &a, const BatchCell *tab, int n, int *next, int blocks)
 {
     EU3D_DISPATCH(heavy_batch_t, a, tab, n, next, blocks)
 }
+constexpr auto react_heavy_batch = &launch_react_heavy_batch;
+#else
+constexpr decltype(Launchers::react_heavy_batch) react_heavy_batch = nullptr;
+#endif
 
 cudaError_t launch_cfl(const LaunchArgs &a, double cfl, unsigned long long *slot, double *time)
 {
@@ -443,7 +462,7 @@ cudaError_t launch_set_value(double *dst, double v, cudaStream_t s)
 const Launchers launchers = {&launch_boundary,         &launch_flux_update,      &launch_recover_react,
                              &launch_derived,          &launch_recover_classify, &launch_learned_apply,
                              &launch_react_queue,      &launch_react_heavy,      &launch_materialize,
-                             &launch_learned_route,    &launch_react_queue_batch, &launch_react_heavy_batch,
+                             &launch_learned_route,    &launch_react_queue_batch, react_heavy_batch,
                              &flux_plan};
 
 #undef EU3D_DISPATCH

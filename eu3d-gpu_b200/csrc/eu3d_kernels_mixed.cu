@@ -5,5 +5,6 @@
 // These round differently from the reference's expressions at the 1e-15
 // level, far below the FP32 flux error the mode already accepts.
 #define EU_EXACT_FLUX 0
+#define EU_MIXED 1
 #define EU3D_NS mixed
 #include "eu3d_kernels_impl.cuh"

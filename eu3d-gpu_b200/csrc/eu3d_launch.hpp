@@ -15,7 +15,6 @@ struct LaunchArgs {
     DevState st;
     const double *dt_dev;
     int max_substeps;
-    int precision; // eu_precision
     int chemistry; // eu_chemistry
     int spec;      // 1: tables are bitwise H2_JA919, use the generated rate code
     int sms;       // multiprocessors of the device (fixed grids of the queue kernels)
@@ -44,6 +43,7 @@ struct Launchers {
     cudaError_t (*learned_route)(const LaunchArgs &a, const LearnedParams &lp);
     // a batch's shared kinetics stage over the instances of tab[0..n)
     cudaError_t (*react_queue_batch)(const LaunchArgs &a, const BatchCell *tab, int n, int *next, int counter);
+    // (null in the FP64 flavours, which leave it no deferred cells)
     cudaError_t (*react_heavy_batch)(const LaunchArgs &a, const BatchCell *tab, int n, int *next, int blocks);
     // what flux_update launches: 0 the face kernel, else the tiled kernel with this march
     int (*flux_plan)(const LaunchArgs &a);

@@ -309,7 +309,6 @@ LaunchArgs launch_args(eu_handle *h)
     a.st = h->st;
     a.dt_dev = h->d_dt;
     a.max_substeps = h->cfg.max_substeps > 0 ? h->cfg.max_substeps : (1 << 20);
-    a.precision = h->cfg.precision;
     a.chemistry = h->cfg.chemistry;
     a.spec = h->spec;
     a.sms = h->sms;
