@@ -133,10 +133,9 @@ def test_mixed_precision_error_is_bounded(gpu):
 
 @pytest.mark.parametrize("dims", [(40, 20, 45), (17, 7, 32), (17, 8, 32), (33, 9, 5), (270, 62, 62)])
 def test_mixed_precision_tiles_match_fp64_closely(gpu, dims):
-    """The plane-tiled FP32 flux kernel on grids whose (j, k) extent is not a
-    multiple of its 7 x 32 tile, on one that is exactly one tile, and on one
-    with a single row in its second tile, and the one-thread-per-column kernel
-    of grids thin in z (nk < 16, both precisions): after
+    """FP32 fluxes against FP64 ones: on grids that the face kernel takes (ragged
+    against its tiles, 7 x 32 cells, one row more, thin in z) and on one that the
+    plane-tiled kernel takes (a million cells, its last tiles partly filled). After
     two steps the conserved state stays within 2e-6 of the all-FP64 run, each
     error measured against the scale of its quantity (species partial
     densities against the largest density, momentum components against the
@@ -234,10 +233,7 @@ def test_strict_warp_kinetics_match_restatement(gpu, port_lib):
     (k_react_heavy), against the pinned C restatement, eight steps: Nchem exact,
     and the conserved state within the 1e-14 of CUDA's exp, log and pow carried
     through some hundred substeps of chain branching (bound 1e-9). The fast
-    FP64 forms stay within 1e-9 of it too, and chemistry samples given to
-    eu_chem_advance end where the thread-per-cell form ends (max_substeps 4
-    keeps every sample on its thread: the capped ones report 4)."""
-    import torch
+    FP64 forms stay within 1e-9 of it too."""
     from helpers import cs_rel_linf
     ni, nj, nk = 11, 5, 6
     ext = (0.0, ni * 2.5e-4, 0.0, nj * 2.5e-4, 0.0, nk * 2.5e-4)
@@ -259,27 +255,6 @@ def test_strict_warp_kinetics_match_restatement(gpu, port_lib):
         s.close()
     assert cs_rel_linf(out["strict"], interior(port.get("CS"))).max() <= 1e-9
     assert cs_rel_linf(out["fast"], out["strict"]).max() <= 1e-9
-    n = 300
-    rng = np.random.default_rng(3)
-    T = torch.tensor(rng.uniform(1200, 2600, n), device="cuda")
-    p = torch.tensor(rng.uniform(1e5, 8e5, n), device="cuda")
-    Y = torch.zeros(9, n, device="cuda", dtype=torch.float64)
-    Y[5], Y[4], Y[3], Y[0] = 0.1, 0.85, 0.04, 0.01
-    dt = torch.tensor(10 ** rng.uniform(-9, -7.5, n), device="cuda")
-    got = {}
-    for cap in (20000, 4):
-        s = gpu.Solver(5, 5, 5, (0, 1, 0, 1, 0, 1), max_substeps=cap)
-        s.set_mechanism(mech)
-        cs, E, Tn = torch.zeros(13, n, device="cuda", dtype=torch.float64), torch.zeros(n, device="cuda", dtype=torch.float64), T.clone()
-        s.chem_states(T, p, Y, cs, E)
-        nchem = torch.zeros(n, device="cuda", dtype=torch.int32)
-        s.chem_advance(cs, Tn, E, dt, nchem)
-        got[cap] = (cs, Tn, nchem)
-        s.close()
-    few = got[20000][2] <= 4
-    assert 0 < int(few.sum()) < n and torch.isfinite(got[20000][1]).all()
-    assert torch.equal(got[4][2], got[20000][2].clamp(max=4))
-    assert torch.equal(got[4][0][:, few], got[20000][0][:, few]) and torch.equal(got[4][1][few], got[20000][1][few])
 
 
 def igniting_samples(n, seed=3):
@@ -291,6 +266,39 @@ def igniting_samples(n, seed=3):
     Y = torch.zeros(9, n, device="cuda", dtype=torch.float64)
     Y[5], Y[4], Y[3], Y[0], Y[8] = 0.03, 0.23, 0.005, 0.001, 0.734
     return u(1200, 2600), u(1e5, 8e5), Y, 10 ** u(-8.5, -6.5)
+
+
+def test_samples_on_a_warp_match_the_thread_form(gpu):
+    """eu_chem_advance's samples beyond four substeps, a warp each, against a thread
+    each, bit for bit in every state, temperature, energy and Nchem: the mechanism's
+    last reaction at rate 0, as it is and with sides of four and three molecules,
+    which the warp form does not take (its terms are exact zeros in either). Calls
+    of one sample, of less and of more than a block, a larger one after a smaller."""
+    import torch
+    OH, H2O, H2 = 3, 2, 5
+    s = gpu.Solver(5, 5, 5, (0, 1, 0, 1, 0, 1))
+    T0, p0, Y0, dt0 = igniting_samples(1000, seed=7)
+    deferred = 0
+    for n in (1, 100, 1000):
+        got = []
+        for warp in (True, False):
+            mech = gpu.parse_mechanism(cases.MECH_JA919, cases.THERMO)
+            mech["af"][18] = 0
+            if not warp:
+                for key, side in (("stoi_f", {OH: 2, H2: 2}), ("stoi_b", {H2O: 2, H2: 1})):
+                    mech[key][:, 18] = [side.get(q, 0) for q in range(9)]
+            s.set_mechanism(mech)
+            T, p, Y, dt = T0[:n].clone(), p0[:n].clone(), Y0[:, :n].contiguous(), dt0[:n].clone()
+            cs, E = torch.zeros(13, n, device="cuda", dtype=torch.float64), torch.zeros(n, device="cuda", dtype=torch.float64)
+            nchem = torch.zeros(n, device="cuda", dtype=torch.int32)
+            torch.cuda.synchronize()
+            s.chem_states(T, p, Y, cs, E)
+            s.chem_advance(cs, T, E, dt, nchem)
+            got.append((cs, T, E, nchem))
+        for a, b in zip(*got):
+            assert torch.isfinite(a).all() and torch.equal(a, b), n
+        deferred = int((got[0][3] > 4).sum())
+    assert deferred > 50
 
 
 def test_samples_without_memory_for_the_queue(gpu):
@@ -425,6 +433,21 @@ def flux_kernels(fn):
     return {k for k, _ in flux_launches(fn)}
 
 
+@pytest.mark.parametrize("dims,chemistry", [((50, 7, 32), "frozen"), ((25, 36, 64), "frozen"), ((24, 14, 161), "frozen"),
+                                            ((2, 7, 26), "frozen"), ((49, 35, 32), "stiff"), ((26, 13, 31), "stiff")])
+def test_tiled_flux_gives_the_face_kernels_bits(gpu, dims, chemistry):
+    """A mixed instance alone takes the face kernel at these sizes, in a batch of a
+    million cells the plane-tiled one: the same bits, on which a batch's equality
+    with its instances alone rests. Exactly one 7 x 32 tile, a last row and a last
+    column of one cell, partly filled tiles, and x extents that the march of 24
+    planes divides, leaves one plane of, or exceeds."""
+    alone, together = (mixed_block(gpu, dims, chemistry=chemistry) for _ in range(2))
+    assert flux_kernels(lambda: alone.step(3, 2e-8)) == {"k_flux_update_faces"}
+    b = gpu.Batch([together, mixed_block(gpu, (128, 98, 96), chemistry="frozen")])
+    assert flux_kernels(lambda: b.step(3, 2e-8)) == {"k_flux_update_tiled"}
+    assert np.array_equal(alone.get("CS"), together.get("CS")) and np.array_equal(alone.get("T"), together.get("T"))
+
+
 def test_flux_kernel_follows_the_call(gpu):
     """Which FP32 flux kernel a handle runs depends on the cells that run together:
     its own alone (too few here for the tiled kernel), all instances' in a batch.
@@ -483,8 +506,8 @@ def test_mixed_stiff_heavy_cells_match_fp64(gpu):
 def test_autotuned_launch_shapes_change_no_bits(gpu, precision, arith, chemistry):
     """Every launch shape the autotuner may pick gives bitwise the same state:
     steps after tuning equal steps with the default shapes, and tuning leaves
-    the state it timed on unchanged (ragged grid: 40 x 21 x 45 nodes). In
-    learned mode the tuner also picks the recovery's register target."""
+    the state it timed on unchanged (ragged grid: 40 x 21 x 45 nodes, which the
+    face kernel takes in either precision). In learned mode the tuner also picks the recovery's register target."""
     ni, nj, nk = 40, 21, 45
     ext = (0.0, 0.02, 0.0, 0.01, 0.0, 0.012)
     x, y, z = (cases.node_coordinates(n, a, b) for n, a, b in ((ni, 0, 0.02), (nj, 0, 0.01), (nk, 0, 0.012)))
@@ -513,6 +536,25 @@ def test_autotuned_launch_shapes_change_no_bits(gpu, precision, arith, chemistry
         s.close()
     for a, b in zip(*out):
         assert n_unequal(a, b) == 0
+
+
+def test_tiled_marches_change_no_bits(gpu):
+    """The marches that the tuner may give the tiled kernel (a grid that takes it
+    alone, 130 planes: last marches of 1, 2, 10, 14 ... planes) against its default
+    one, bitwise: each candidate is timed, one is kept, and steps go on with it."""
+    out = []
+    for tune in (False, True):
+        s = mixed_block(gpu, (130, 84, 96), chemistry="frozen")
+        assert flux_kernels(lambda: s.step(1, 2e-8)) == {"k_flux_update_tiled"}
+        if tune:
+            before = s.get("CS")
+            rep = s.autotune(reps=2)
+            assert len(rep["flux_ms"]) >= 9 and 1 not in rep["flux_ms"] and rep["flux_ci"] in rep["flux_ms"], rep
+            assert np.array_equal(s.get("CS"), before)
+        s.step(3, 2e-8)
+        out.append(s.get("CS"))
+        s.close()
+    assert np.array_equal(*out)
 
 
 def test_tuned_march_belongs_to_its_kernel(gpu):
