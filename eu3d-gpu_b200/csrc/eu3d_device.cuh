@@ -700,9 +700,10 @@ __device__ __forceinline__ double pow_whole(double x, double ix, double n)
     return r;
 }
 
-// The rates outside [t_lo, t_hi] (very cold gas: exp(G/RT) of water vapour leaves
-// the normal range below 43 K), where the products of the form below would meet an
-// underflowed factor with an overflowed one: one exponential of each reaction's
+// The rates outside [t_lo, t_hi] (very cold gas: of H2_JA919's factors the square
+// of atomic hydrogen's exp(G/RT) is the first to leave the range, at 85 K), where
+// the products of the form below would meet an underflowed factor with an
+// overflowed one: one exponential of each reaction's
 // whole exponent, forward and backward, by exp. Rare, so out of line and rolled.
 template <int NS, int NR>
 __device__ __noinline__ void eval_rates_far(const DevMech &m, double T, double inv, double lnT, const double *mc,

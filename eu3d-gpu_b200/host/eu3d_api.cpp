@@ -148,11 +148,12 @@ void free_all(eu_handle *h)
 }
 
 // The temperatures between which the fast forms of the rates (eval_rates) meet no
-// exponent beyond 690, in steps of 0.5 % from the thermo switch down to 1 K and up
-// to 100,000 K: every species' g = G/(R T), whose exponential and reciprocal they
+// exponent beyond 690, searched from the thermo switch down to 1 K and up to
+// 100,000 K: every species' g = G/(R T), whose exponential and reciprocal they
 // form, the products of those in the order in which a reaction takes them, and
-// each rate constant's exponent. (An exponent changes by a few units a step, and
-// the exponentials hold to 708.)
+// each rate constant's exponent. All are smooth and leave the range like 1/T, so
+// steps of 10 % and eight halvings of the last one find the ends (20 us a mechanism;
+// 85 and 44,500 K for H2_JA919; the exponentials hold to 708).
 void rate_range(DevMech &d)
 {
     auto fits = [&](double T) {
@@ -184,8 +185,19 @@ void rate_range(DevMech &d)
     d.t_hi = 0; // no temperature fits
     if (!fits(kThermoSwitch))
         return;
-    for (double T = kThermoSwitch; T >= 1 && fits(T); T /= 1.005) d.t_lo = T;
-    for (double T = kThermoSwitch; T <= 1e5 && fits(T); T *= 1.005) d.t_hi = T;
+    auto end = [&](double step, double last) { // the last temperature that fits on the way to `last`
+        double T = kThermoSwitch;
+        while ((step < 1 ? T * step >= last : T * step <= last) && fits(T * step)) T *= step;
+        for (int q = 0; q < 8; ++q) {
+            step = std::sqrt(step);
+            const double next = T * step;
+            if ((step < 1 ? next >= last : next <= last) && fits(next))
+                T = next;
+        }
+        return T;
+    };
+    d.t_lo = end(1 / 1.1, 1.0);
+    d.t_hi = end(1.1, 1e5);
 }
 
 // DevMech from host tables; rejects sizes the kernels are not built for.
