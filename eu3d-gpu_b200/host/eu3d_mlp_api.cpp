@@ -179,30 +179,44 @@ eu3d::TrainParams train_params(const eu_mlp *m, int first, int count)
 }
 
 // A batch of n rows of the caller's arrays, with scratch for `group` members: all
-// run together with scratch of their own, or, where memory is short, one at a time
-// on one (6.2 KB a row and member at 256 x 3).
+// of them (6.2 KB a row and member at 256 x 3), or, where memory is short, one, on
+// which they run one at a time. (A gradient of one member takes all of them's too:
+// a second allocation for the training that follows costs 0.4 ms.)
 eu_status train_batch(eu_mlp *m, eu3d::TrainParams &p, const float *X, const float *T, long long rows, int n, bool drawn,
-                      int group)
+                      int &group)
 {
+    group = m->members;
     // whole tiles: every piece a multiple of 128 values
     const size_t rows_pad = size_t(n + eu3d::kTrainRows - 1) / eu3d::kTrainRows * eu3d::kTrainRows;
     const size_t wide = size_t(m->hidden) * m->width * rows_pad;
     const size_t bytes = wide * (4 + 2 + 2) + rows_pad * (m->in_pad + m->out_pad) * 2;
     if (m->train_bytes < bytes * group) {
-        if (m->train) {
-            MCK(m, cudaStreamSynchronize(m->stream));
-            MCK(m, cudaFree(m->train));
-        }
-        m->train = nullptr;
-        m->train_bytes = 0;
-        const cudaError_t e = cudaMalloc(&m->train, bytes * group);
-        if (e != cudaSuccess) {
+        auto drop = [&] { // nothing of an earlier call uses it any more
+            cudaStreamSynchronize(m->stream);
+            cudaFree(m->train);
             m->train = nullptr;
+            m->train_bytes = 0;
+        };
+        if (m->train && m->train_bytes < bytes)
+            drop();
+        void *fresh = nullptr;
+        cudaError_t e = cudaMalloc(&fresh, bytes * group);
+        if (e == cudaErrorMemoryAllocation) {
             cudaGetLastError(); // the launches' own check starts clean
+            e = cudaSuccess;
+            group = 1;
+            if (!m->train && (e = cudaMalloc(&fresh, bytes)) != cudaSuccess)
+                cudaGetLastError();
+        }
+        if (e != cudaSuccess)
             return mfail(m, e == cudaErrorMemoryAllocation ? EU_ERR_OUT_OF_MEMORY : EU_ERR_CUDA, "training scratch: %s",
                          cudaGetErrorString(e));
+        if (fresh) {
+            if (m->train)
+                drop();
+            m->train = fresh;
+            m->train_bytes = bytes * group;
         }
-        m->train_bytes = bytes * group;
     }
     p.X = X;
     p.T = T;
@@ -606,7 +620,8 @@ eu_status eu_mlp_loss_grad(eu_mlp *m, int member, const float *X, const float *T
         return mfail(m, EU_ERR_INVALID_ARGUMENT, "member or batch size (multiple of 16 up to max_batch)");
     cudaSetDevice(m->device);
     eu3d::TrainParams p = train_params(m, member, 1);
-    eu_status s = train_batch(m, p, X, T, n, n, false, 1);
+    int group;
+    eu_status s = train_batch(m, p, X, T, n, n, false, group);
     if (s != EU_OK)
         return s;
     float *g = m->G + member * m->params;
@@ -639,10 +654,8 @@ eu_status eu_mlp_train(eu_mlp *m, const float *X, const float *T, long long n, i
     cudaSetDevice(m->device);
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     eu3d::TrainParams p = train_params(m, 0, m->members);
-    int group = m->members; // members that run together
+    int group; // members that run together
     eu_status s = train_batch(m, p, X, T, n, batch, true, group);
-    if (s == EU_ERR_OUT_OF_MEMORY && group > 1)
-        s = train_batch(m, p, X, T, n, batch, true, group = 1);
     if (s != EU_OK)
         return s;
     MCK(m, cudaMemsetAsync(m->G, 0, size_t(m->params) * m->members * 4, m->stream));

@@ -184,8 +184,8 @@ def test_batch_of_two_to_the_31_values(gpu):
 
 def test_training_when_memory_is_short(gpu):
     """With room for one member's scratch but not for all three's (0.82 GB each at
-    this batch) the members train one after the other, and a gradient takes one
-    member's scratch only. The sums' order differs, so the comparison with a model
+    this batch) a gradient takes one's and the members train one after the other,
+    also when it comes to more room or less later. The sums' order differs, so the comparison with a model
     that trained with room is Adam's: two steps of lr 1e-3 from the same start."""
     import torch
     n = 131072
@@ -200,7 +200,10 @@ def test_training_when_memory_is_short(gpu):
         room = torch.empty(max(0, torch.cuda.mem_get_info()[0] - (3 << 29)) if short else 0, device="cuda", dtype=torch.uint8)
         try:
             loss, g = m.loss_grad(1, X, T)
-            return np.float64(loss), g, m.train(X, T, n, 2, 1e-3, seed=5), m.get_params()
+            first = m.train(X, T, n, 2, 1e-3, seed=5)
+            room = None
+            torch.cuda.empty_cache()
+            return np.float64(loss), g, first, m.get_params(), m.loss_grad(2, X, T)[1], m.train(X, T, n, 1, 1e-3, seed=6)
         finally:
             m.close()
             del room
