@@ -1,6 +1,7 @@
 // eu3d_kernels.cuh — the timestep kernels, templated on the species and
-// reaction counts. Instantiated twice: eu3d_kernels_strict.cu (--fmad=false,
-// EU_EXACT_RATES/EU_EXACT_FLUX) and eu3d_kernels_fast.cu.
+// reaction counts. Instantiated three times: eu3d_kernels_strict.cu (--fmad=false,
+// EU_EXACT_THERMO, EU_EXACT_RATES, EU_EXACT_FLUX), eu3d_kernels_fast.cu
+// (EU_EXACT_THERMO) and eu3d_kernels_mixed.cu (EU_MIXED).
 #pragma once
 
 #include "eu3d_device.cuh"
@@ -799,7 +800,10 @@ __device__ __forceinline__ void run_substeps(const DevMech &m, CellState<NS> &ce
 // (null: every cell on its own thread). On the 48x32x32 igniting block in mixed
 // precision the step took 0.865 / 0.81 / 0.764 / 0.78 / 1.11 ms with the
 // threshold at 16 / 8 / 4 / 2 / 0: below 4 a warp per cell costs more than the
-// few substeps it shortens.
+// few substeps it shortens. The other forms, at 16 / 8 / 4: strict igniting blocks of
+// 41x24x23 and 96x48x48, 0.396 / 0.314 / 0.262 and 0.698 / 0.613 / 0.566 ms a step;
+// fast FP64, ten steps of the smaller one with its copies, 4.75 / 4.19 / 3.99 ms;
+// 100,000 chemistry samples, whose longest chain decides, 21.9 / 20.7 / 21.3 ms.
 constexpr int kHeavyNchem = 4;
 
 __device__ __forceinline__ void push_heavy(int *heavy, long long c)

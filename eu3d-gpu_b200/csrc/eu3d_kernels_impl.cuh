@@ -31,14 +31,15 @@ cudaError_t boundary_t(const LaunchArgs &a)
 // division-light limiter form.
 constexpr bool kStrictFlux = EU_EXACT_FLUX != 0;
 
+inline int tiles_j(const DevGrid &g) { return (g.nj + kTileJ - 1) / kTileJ; }
+inline int tiles_k(const DevGrid &g) { return (g.nk + kTileK - 1) / kTileK; }
+
 // The tiled kernel's march where the autotuner has not chosen one. A block costs
 // its ci planes and about three more (the window's first planes and the first
 // face), and runs among two per SM: the ci whose rounds of blocks cost least
 // (256 x 128 x 128: 24, 0.436 ms against 0.459 at 16; 192 x 96 x 96: 29, 0.193
-// against 0.213). In a batch the rounds mix with the other instances'.
-inline int tiles_j(const DevGrid &g) { return (g.nj + kTileJ - 1) / kTileJ; }
-inline int tiles_k(const DevGrid &g) { return (g.nk + kTileK - 1) / kTileK; }
-
+// against 0.213). In a batch the rounds mix with the other instances' and the march
+// counts for little: eight instances, 50 steps, 99.7 / 99.2 / 98.7 ms at 16 / 24 / 32.
 inline int tiled_march(const LaunchArgs &a)
 {
     const long long tiles = (long long)tiles_j(a.g) * tiles_k(a.g);
@@ -141,16 +142,17 @@ cudaError_t faces_flux_launch(const LaunchArgs &a, const R *prim)
 
 // FP32 fluxes (mixed precision, always the division-light forms) on grids thick
 // enough in z for the tiled kernel's 32-lane rows and large enough for its
-// blocks to fill the chip take that kernel (192 x 96 x 96: 0.215 ms against
-// 0.239, 256 x 128 x 128: 0.46 against 0.54), smaller and thinner ones a face a
-// thread (128 x 64 x 64: 0.079 ms against 0.105, 48 x 32 x 32: 0.020 against
-// 0.073). The two give the same bits. FP64 fluxes (the reference's forms when strict, the division-light
-// limiter when fast) are always formed a face a thread.
+// blocks to fill the chip take that kernel (192 x 96 x 96: 0.166 ms against
+// 0.238, 256 x 128 x 128: 0.404 against 0.543), smaller and thinner ones a face a
+// thread (48 x 32 x 32: 0.020 ms against 0.036). The line was drawn for the tiled
+// kernel with two barriers a plane; the present one is ahead at 128 x 64 x 64 too
+// (0.064 against 0.078). The two give the same bits. FP64 fluxes (the reference's forms when
+// strict, the division-light limiter when fast) are always formed a face a thread.
 // On grids that fill the chip the share of the tiled kernel's 7 x 32 cells that
-// hold a cell of the grid decides (at 68 % of them, 129 x 65 x 65, it takes 0.107
-// ms against 0.095); the instances of a batch run together, so there the cells
-// of all of them count (eight instances of 0.3-1.8 M cells: 105.0 ms -> 99.1 a
-// 50-step pass).
+// hold a cell of the grid decides (drawn likewise; at 68 % of them, 129 x 65 x 65,
+// the present kernel takes 0.089 ms against 0.094); the instances of a batch run together, so there the cells
+// of all of them count (eight instances of 0.3-1.8 M cells, a 50-step pass: 99.2 ms,
+// of which 35 are host copies, against 108.9 with each instance's own count).
 constexpr int kThinNk = 16;
 constexpr long long kTiledCells = 1000000;
 

@@ -77,7 +77,7 @@ struct DevState {
     double *cms;      // ns planes (or null)
     unsigned long long *counters; // see CounterIdx
     unsigned *step_words; // kStepWords words cleared by the ghost fill
-    int *heavy;       // mixed precision: {count, next, cells...} of cells left to the warp-per-cell kinetics
+    int *heavy;       // {count, next, cells...} of cells left to the warp-per-cell kinetics (null: none are)
     const double *inflow; // ODW x-low ghost values per interior (j, k): 7 + ns primitive planes, then T
     // EU_GHOSTS_STORED: store_cell also writes the z-face ghosts a node is the
     // mirror source of (W reflected), and the ghost fill skips the z faces while
