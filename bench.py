@@ -73,7 +73,7 @@ FLUX_BYTES = {"fp64": (16 + 26) * 8, "mixed": 16 * 4 + 26 * 8}
 # (dram__bytes_read.sum + dram__bytes_write.sum over the cells of the captured
 # 256 x 128 x 64-node grid; the traffic scales with the cells, so it is scaled
 # to the benchmark grid).
-FLUX_TRAFFIC_PER_CELL = {"mixed": 286.4}  # (the FP64 kernel has no capture at that grid)
+FLUX_TRAFFIC_PER_CELL = {"mixed": 274.4}  # (the FP64 kernel has no capture at that grid)
 # FLOPs per row of the learned ensemble (3 members x 2 (12 256 + 256 256 + 256 256 + 256 10)).
 MLP_FLOP_PER_ROW = 820224
 # FP64 flops per cell-substep of the stiff kinetics (rates, trapezoid update,
