@@ -88,14 +88,16 @@ inline int even_piece(int n, int want)
     return (n + pieces - 1) / pieces;
 }
 
-// Small grids leave SMs without blocks when the tiles hold 128 cells (fewer than 8
-// blocks of 128 cells per SM): there a tile holds
-// half the cells and the block twice the threads, so that a step is one round
-// of faces a block (33 x 17 x 17 strict: 0.023 ms against 0.033-0.054 with the
-// large grids' tiles; 129 x 65 x 65 FP64 the other way: 0.133 against 0.145).
+// Grids of few cells leave SMs without blocks when the tiles hold 128 of them
+// (fewer than 8 blocks of 128 cells per SM): there a tile holds half the cells and
+// the block twice the threads, so that a step is one round of faces a block (33 x 17
+// x 17 strict: 0.023 ms against 0.033-0.054 with the large grids' tiles; 129 x 65 x 65
+// FP64 the other way: 0.133 against 0.145). In a batch the cells of all instances
+// count: 8 mixed ones of 44^3 take 0.154 ms a step, 0.246 with the small grids' tiles;
+// 16 of 32^3 in FP64 0.238 against 0.283 (fast), 0.519 against 0.582 (strict).
 inline bool small_grid(const LaunchArgs &a)
 {
-    return (long long)a.g.ni * a.g.nj * a.g.nk < (a.sms > 0 ? a.sms : 148) * 8LL * 128;
+    return std::max((long long)a.g.ni * a.g.nj * a.g.nk, a.batch_cells) < (a.sms > 0 ? a.sms : 148) * 8LL * 128;
 }
 
 // The tile of k_flux_update_faces for a grid: 128 (small grids: 64) cells, rows
@@ -140,28 +142,33 @@ cudaError_t faces_flux_launch(const LaunchArgs &a, const R *prim)
     return cudaGetLastError();
 }
 
-// FP32 fluxes (mixed precision, always the division-light forms) on grids thick
-// enough in z for the tiled kernel's 32-lane rows and large enough for its
-// blocks to fill the chip take that kernel (192 x 96 x 96: 0.166 ms against
-// 0.238, 256 x 128 x 128: 0.404 against 0.543), smaller and thinner ones a face a
-// thread (48 x 32 x 32: 0.020 ms against 0.036). The line was drawn for the tiled
-// kernel with two barriers a plane; the present one is ahead at 128 x 64 x 64 too
-// (0.064 against 0.078). The two give the same bits. FP64 fluxes (the reference's forms when
-// strict, the division-light limiter when fast) are always formed a face a thread.
-// On grids that fill the chip the share of the tiled kernel's 7 x 32 cells that
-// hold a cell of the grid decides (drawn likewise; at 68 % of them, 129 x 65 x 65,
-// the present kernel takes 0.089 ms against 0.094); the instances of a batch run together, so there the cells
-// of all of them count (eight instances of 0.3-1.8 M cells, a 50-step pass: 99.2 ms,
-// of which 35 are host copies, against 108.9 with each instance's own count).
+// The kernel of FP32 fluxes (mixed precision, always the division-light forms); the
+// two give the same bits. FP64 fluxes (the reference's forms when strict, the
+// division-light limiter when fast) are always formed a face a thread.
+// The tiled kernel reads each primitive once but wants its 32-lane rows in z, its 7 x
+// 32 tiles full and the chip filled by its blocks of eight warps. Flux of a grid
+// alone, ms, tiled against faces (share of the tiles' cells that are the grid's):
+//   96 x 48 x 48    0.050 0.037 (73 %)    200 x 100 x 100  0.242 0.297 (74 %)
+//   100 x 50 x 50   0.051 0.048 (70 %)    129 x 65 x 65    0.089 0.094 (65 %)
+//   112 x 56 x 56   0.052 0.058 (88 %)    200 x 100 x 40   0.123 0.127 (60 %)
+//   128 x 64 x 64   0.064 0.077 (91 %)    256 x 128 x 33   0.189 0.171 (51 %)
+//   256 x 128 x 128 0.404 0.543 (96 %)    200 x 100 x 17   0.062 0.059 (51 %)
+// so it takes grids of 300,000 cells and more at 55 % and more. The instances of a
+// batch share the chip: there the faces' shorter blocks are ahead up to about a
+// million cells in all and the tiles beyond, down to half full (a step, ms):
+//   2 x 64^3 0.129 0.103   6 x 44^3 0.147 0.112   4 x (96 x 48 x 48) 0.180 0.176
+//   4 x 64^3 0.195 0.206  16 x 44^3 0.283 0.321   8 x (96 x 48 x 48) 0.322 0.360
+//   8 x (64 x 33 x 33) 0.158 0.143, 16 of them 0.267 0.298 (49 %)
 constexpr int kThinNk = 16;
-constexpr long long kTiledCells = 1000000;
 
 inline bool takes_tiled(const LaunchArgs &a)
 {
     const DevGrid &g = a.g;
-    const long long cells = std::max((long long)g.ni * g.nj * g.nk, a.batch_cells);
+    const bool batch = a.batch_cells > 0;
+    const long long cells = batch ? a.batch_cells : (long long)g.ni * g.nj * g.nk;
     const long long slots = (long long)tiles_j(g) * kTileJ * (tiles_k(g) * kTileK);
-    return g.nk >= kThinNk && cells >= kTiledCells && 5LL * g.nj * g.nk >= 4 * slots;
+    return g.nk >= kThinNk && cells >= (batch ? 1000000 : 300000) &&
+           100LL * g.nj * g.nk >= (batch ? 45 : 55) * slots;
 }
 
 template <int NS, int NR>
@@ -364,11 +371,14 @@ cudaError_t heavy_batch_t(const LaunchArgs &a, const BatchCell *tab, int n, int 
 
 cudaError_t launch_boundary(const LaunchArgs &a) { EU3D_DISPATCH(boundary_t, a) }
 cudaError_t launch_flux_update(const LaunchArgs &a) { EU3D_DISPATCH(flux_t, a) }
+int flux_plan(const LaunchArgs &a)
+{
 #ifdef EU_MIXED
-int flux_plan(const LaunchArgs &a) { return takes_tiled(a) ? tiled_ci(a) : 0; }
-#else
-int flux_plan(const LaunchArgs &) { return 0; }
+    if (takes_tiled(a))
+        return tiled_ci(a);
 #endif
+    return small_grid(a) ? -1 : 0;
+}
 cudaError_t launch_recover_react(const LaunchArgs &a, bool react) { EU3D_DISPATCH(react_t, a, react) }
 cudaError_t launch_derived(const LaunchArgs &a, int which, double *out) { EU3D_DISPATCH(derived_t, a, which, out) }
 cudaError_t launch_materialize(const LaunchArgs &a) { EU3D_DISPATCH(materialize_t, a) }

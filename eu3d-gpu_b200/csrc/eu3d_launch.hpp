@@ -23,7 +23,7 @@ struct LaunchArgs {
     int recover_block; // threads per block of the recovery kernels, 32..128 (autotuned; 0: 128, or 64 in learned mode)
     int recover_minb;  // register target, blocks per SM: learned-mode recovery 3 .. 6 (0: 4), stiff kinetics
                        // 2 .. 4 (0: by the grid)
-    long long batch_cells = 0; // cells of all instances that run together in a batch (0: alone)
+    long long batch_cells = 0; // cells of all instances that run together in a batch of two or more (0: alone)
     cudaStream_t stream;
 };
 
@@ -45,7 +45,7 @@ struct Launchers {
     cudaError_t (*react_queue_batch)(const LaunchArgs &a, const BatchCell *tab, int n, int *next, int counter);
     // (null in the FP64 flavours, which leave it no deferred cells)
     cudaError_t (*react_heavy_batch)(const LaunchArgs &a, const BatchCell *tab, int n, int *next, int blocks);
-    // what flux_update launches: 0 the face kernel, else the tiled kernel with this march
+    // what flux_update launches: 0 the face kernel, -1 with a small grid's tiles, else the tiled kernel with this march
     int (*flux_plan)(const LaunchArgs &a);
 };
 

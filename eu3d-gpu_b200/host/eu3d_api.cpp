@@ -2174,7 +2174,7 @@ eu_status eu_batch_step(eu_batch *b, int nsteps, const double *dt, eu_step_stats
             return bfail(b, EU_ERR_UNSUPPORTED, "instance %d: learned chemistry needs a model with the fused kernel", i);
         const bool tail = b->shared && needs_shared_stage(h);
         LaunchArgs a = launch_args(h);
-        a.batch_cells = cells;
+        a.batch_cells = n > 1 ? cells : 0;
         const Launchers &L = flavour(h);
         if (h->graph_dirty || !h->graph_exec || h->graph_cfl != 0 || h->graph_shared_tail != tail ||
             h->graph_flux_plan != L.flux_plan(a)) {
@@ -2341,7 +2341,7 @@ eu_status eu_autotune(eu_handle *h, int reps, eu_tune_report *report)
         *ms /= reps;
         return r;
     };
-    const bool tiled = L.flux_plan(a) != 0;
+    const bool tiled = L.flux_plan(a) > 0;
     int &march = tiled ? a.tiled_ci : a.face_ci;
     int best_ci = 16, best_rb = 128;
     float best = 1e30f;

@@ -538,6 +538,31 @@ def test_autotuned_launch_shapes_change_no_bits(gpu, precision, arith, chemistry
         assert n_unequal(a, b) == 0
 
 
+@pytest.mark.parametrize("precision,arith", [("fp64", "strict"), ("fp64", "fast"), ("mixed", "fast")])
+def test_face_tiles_follow_the_batch(gpu, precision, arith):
+    """A small instance's faces come in the small grids' tiles alone and in the large
+    grids' in a batch of many cells (other blocks), with the same bits, whatever the
+    calls before; a batch of one is the instance alone."""
+    mech = golden_mechanism()
+
+    def make(dims):
+        h = 5e-4
+        s = gpu.Solver(*dims, tuple(v for n in dims for v in (0.0, h * (n - 1))), precision=precision, arith=arith, chemistry="frozen")
+        s.set_mechanism(mech)
+        ax = [cases.node_coordinates(n, 0.0, h * (n - 1)) for n in dims]
+        s.set_primitive(*cases.shock_bubble(*ax, mech.mw, 9, radius=2e-3, shock_x=2e-3, standoff=3e-3, seed=4))
+        return s
+
+    a, b, big = make((21, 14, 11)), make((21, 14, 11)), make((64, 60, 41))
+    both, one = gpu.Batch([b, big]), gpu.Batch([b])
+    alone = flux_launches(lambda: a.step(2, 2e-8))
+    together = flux_launches(lambda: both.step(2, 2e-8))
+    assert len(alone) == 1 and {k for k, _ in together} == {"k_flux_update_faces"} and not alone <= together
+    assert flux_launches(lambda: one.step(2, 2e-8)) == alone and flux_launches(lambda: b.step(2, 2e-8)) == alone
+    a.step(4, 2e-8)
+    assert np.array_equal(a.get("CS"), b.get("CS")) and np.array_equal(a.get("T"), b.get("T"))
+
+
 def test_tiled_marches_change_no_bits(gpu):
     """The marches that the tuner may give the tiled kernel (a grid that takes it
     alone, 130 planes: last marches of 1, 2, 10, 14 ... planes) against its default
