@@ -341,11 +341,19 @@ __global__ void __launch_bounds__(kTrainThreads, 2) k_train_rows(const __grid_co
         tc::tmem_dealloc(tmem, 256);
 }
 
-// dW = dZ^T H of every layer of every member: a CTA takes a share of the batch's
-// 64-row slabs for one layer (all its outputs and inputs, two 128 x 256
-// accumulators at most) and adds its sums to the fp32 gradient four values at a
-// time. The operands lie in global memory as the MMAs read them, so a slab is one
-// bulk copy each, three of them in flight.
+// dW = dZ^T H of every layer of every member. The batch's 64-row slabs are cut into
+// pieces; a CTA takes every `splits`-th piece of one layer (all its outputs and
+// inputs, two 128 x 256 accumulators at most) and adds each piece's sums to the fp32
+// gradient four values at a time. The operands lie in global memory as the MMAs
+// read them, so a slab is one bulk copy each, three of them in flight.
+//
+// The pieces are the layer-wise training's splits of K (one below 512 rows, 4 below
+// 2048, else 16), so every piece's sum is bitwise that one's and only the order in
+// which the pieces are added is open: with other pieces a batch of 256 rows, 24
+// steps a pass, was 1e-2 of its gradients' norm off in the second pass (Adam divides
+// a gradient by its size; the layer-wise code is 7e-3 off itself). Where 16 pieces would
+// leave the chip idle (few layers and members, more than 24 CTAs for each) or make a
+// CTA come back often (fewer than 16), there is a piece for each CTA.
 constexpr int kDwThreads = 256, kDwK = 64, kDwSlots = 3, kDwOperand = 256 * kDwK * 2;
 constexpr size_t kDwSmem = size_t(kDwSlots) * 2 * kDwOperand + 8 * (2 * kDwSlots + 1) + 16;
 
@@ -363,11 +371,12 @@ __global__ void __launch_bounds__(kDwThreads, 1) k_train_dw(const __grid_constan
     const int l = int(blockIdx.x) < unit ? 0 : min(L, (int(blockIdx.x) - unit) / (2 * unit) + 1);
     const int splits = l == 0 || l == L ? unit : 2 * unit, split = int(blockIdx.x) - (l == 0 ? 0 : unit + (l - 1) * 2 * unit);
     const int M = l == L ? p.out_pad : p.width, N = l == 0 ? p.in_pad : p.width;
-    const int tiles = (p.n + kTrainRows - 1) / kTrainRows, slabs = tiles * (kTrainRows / kDwK);
+    const int tiles = (p.n + kTrainRows - 1) / kTrainRows, slabs = (p.n + kDwK - 1) / kDwK;
     const __nv_bfloat16 *A = l == L ? mem.dYT : mem.dZT + size_t(l) * tiles * p.width * kTrainRows;
     const __nv_bfloat16 *B = l == 0 ? mem.XT : mem.HT + size_t(l - 1) * tiles * p.width * kTrainRows;
-    const int per = (slabs + splits - 1) / splits, k0 = split * per, KT = max(0, min(slabs, k0 + per) - k0);
-    if (KT == 0)
+    const int pieces = p.n < 512 ? 1 : p.n < 2048 ? 4 : 2 * unit >= 16 && 2 * unit <= 24 ? 16 : splits;
+    const int per = (slabs + pieces - 1) / pieces;
+    if (split >= pieces || split * per >= slabs)
         return;
     if (warp == 0) {
         tc::tmem_alloc(tslot, 512);
@@ -386,62 +395,72 @@ __global__ void __launch_bounds__(kDwThreads, 1) k_train_dw(const __grid_constan
     tc::tc_fence_after();
     const uint32_t tmem = *tslot;
     bool ok = true;
-    if (threadIdx.x == 0) { // copies
-        int k = 0;
-        for (; ok && k < KT; ++k) {
-            const int slot = k % kDwSlots;
-            if (k >= kDwSlots && !tc::mbar_wait(&empty[slot], uint32_t((k / kDwSlots - 1) & 1))) {
-                ok = false;
-                break;
+    int done = 0; // slabs of the pieces before: the ring goes on from piece to piece
+    for (int piece = split, turn = 0; ok && piece < pieces && piece * per < slabs; piece += splits, ++turn) {
+        const int k0 = piece * per, end = done + min(slabs - k0, per);
+        if (threadIdx.x == 0) { // copies
+            int k = done;
+            for (; k < end; ++k) {
+                const int slot = k % kDwSlots;
+                if (k >= kDwSlots && !tc::mbar_wait(&empty[slot], uint32_t((k / kDwSlots - 1) & 1))) {
+                    ok = false;
+                    break;
+                }
+                unsigned char *a = smem + size_t(slot) * 2 * kDwOperand;
+                const size_t at = size_t(k0 + k - done);
+                tc::mbar_arrive_expect_tx(&full[slot], uint32_t(M + N) * kDwK * 2);
+                tc::bulk_g2s(a, A + at * M * kDwK, uint32_t(M) * kDwK * 2, &full[slot]);
+                tc::bulk_g2s(a + kDwOperand, B + at * N * kDwK, uint32_t(N) * kDwK * 2, &full[slot]);
             }
-            unsigned char *a = smem + size_t(slot) * 2 * kDwOperand;
-            tc::mbar_arrive_expect_tx(&full[slot], uint32_t(M + N) * kDwK * 2);
-            tc::bulk_g2s(a, A + size_t(k0 + k) * M * kDwK, uint32_t(M) * kDwK * 2, &full[slot]);
-            tc::bulk_g2s(a + kDwOperand, B + size_t(k0 + k) * N * kDwK, uint32_t(N) * kDwK * 2, &full[slot]);
-        }
-        // copies in flight land before the CTA's memory goes away
-        for (int q = max(0, k - kDwSlots); q < k; ++q) ok = tc::mbar_wait(&full[q % kDwSlots], uint32_t((q / kDwSlots) & 1)) && ok;
-    } else if (threadIdx.x == 32) { // MMAs
-        const uint32_t idesc = tc::idesc_bf16_f32(128, N);
-        for (int k = 0; ok && k < KT; ++k) {
-            const int slot = k % kDwSlots;
-            ok = tc::mbar_wait(&full[slot], uint32_t((k / kDwSlots) & 1));
-            if (!ok)
-                break;
-            tc::tc_fence_after();
-            const uint32_t a0 = tc::smem_u32(smem + size_t(slot) * 2 * kDwOperand), b0 = a0 + kDwOperand;
+            // copies in flight land before the CTA's memory goes away
+            for (int q = max(done, k - kDwSlots); q < k; ++q)
+                ok = tc::mbar_wait(&full[q % kDwSlots], uint32_t((q / kDwSlots) & 1)) && ok;
+        } else if (threadIdx.x == 32) { // MMAs
+            const uint32_t idesc = tc::idesc_bf16_f32(128, N);
+            for (int k = done; k < end; ++k) {
+                const int slot = k % kDwSlots;
+                ok = tc::mbar_wait(&full[slot], uint32_t((k / kDwSlots) & 1));
+                if (!ok)
+                    break;
+                tc::tc_fence_after();
+                const uint32_t a0 = tc::smem_u32(smem + size_t(slot) * 2 * kDwOperand), b0 = a0 + kDwOperand;
 #pragma unroll
-            for (int kk = 0; kk < kDwK / 16; ++kk)
-                for (int h = 0; h * 128 < M; ++h) // (rows past M are accumulated from what lies there and not read)
-                    tc::mma_bf16(tmem + 256 * h, tc::smem_desc(a0 + kk * 2 * M * 16 + h * 128 * 16, M * 16, 128),
-                                 tc::smem_desc(b0 + kk * 2 * N * 16, N * 16, 128), idesc, (k > 0 || kk > 0) ? 1u : 0u);
-            tc::mma_commit(&empty[slot]);
-        }
-        tc::mma_commit(acc); // every MMA issued so far
-        ok = tc::mbar_wait(acc, 0) && ok;
-    }
-    ok = __syncthreads_and(ok);
-    tc::tc_fence_after();
-    if (ok) {
-        const int h = warp / 4, m = warp * 32 + lane;
-        float *g = mem.gW[l] + size_t(m) * N;
-        if (h * 128 < M)
-            for (int c0 = 0; c0 < N; c0 += 32) {
-                float v[32];
-                tc::tmem_ld32(tmem + 256 * h + (uint32_t((warp % 4) * 32) << 16) + c0, v);
-                if (m < M)
-#pragma unroll
-                    for (int j = 0; j < 8; ++j)
-                        if (c0 + j * 4 < N)
-                            asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(g + c0 + j * 4),
-                                         "f"(v[j * 4]), "f"(v[j * 4 + 1]), "f"(v[j * 4 + 2]), "f"(v[j * 4 + 3])
-                                         : "memory");
+                for (int kk = 0; kk < kDwK / 16; ++kk)
+                    for (int h = 0; h * 128 < M; ++h) // (rows past M are accumulated from what lies there and not read)
+                        tc::mma_bf16(tmem + 256 * h, tc::smem_desc(a0 + kk * 2 * M * 16 + h * 128 * 16, M * 16, 128),
+                                     tc::smem_desc(b0 + kk * 2 * N * 16, N * 16, 128), idesc,
+                                     (k > done || kk > 0) ? 1u : 0u);
+                tc::mma_commit(&empty[slot]);
             }
-    } else if (threadIdx.x == 0) {
-        atomicExch(p.err, 1);
+            tc::mma_commit(acc); // every MMA issued so far
+            ok = tc::mbar_wait(acc, uint32_t(turn & 1)) && ok;
+        }
+        ok = __syncthreads_and(ok);
+        tc::tc_fence_after();
+        if (ok) {
+            const int h = warp / 4, m = warp * 32 + lane;
+            float *g = mem.gW[l] + size_t(m) * N;
+            if (h * 128 < M)
+                for (int c0 = 0; c0 < N; c0 += 32) {
+                    float v[32];
+                    tc::tmem_ld32(tmem + 256 * h + (uint32_t((warp % 4) * 32) << 16) + c0, v);
+                    if (m < M)
+#pragma unroll
+                        for (int j = 0; j < 8; ++j)
+                            if (c0 + j * 4 < N)
+                                asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(g + c0 + j * 4),
+                                             "f"(v[j * 4]), "f"(v[j * 4 + 1]), "f"(v[j * 4 + 2]), "f"(v[j * 4 + 3])
+                                             : "memory");
+                }
+        } else if (threadIdx.x == 0) {
+            atomicExch(p.err, 1);
+        }
+        // the accumulators are read before the next piece's MMAs overwrite them
+        tc::tc_fence_before();
+        __syncthreads();
+        tc::tc_fence_after();
+        done = end;
     }
-    tc::tc_fence_before();
-    __syncthreads();
     if (warp == 0)
         tc::tmem_dealloc(tmem, 512);
 }

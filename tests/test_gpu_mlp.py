@@ -96,16 +96,19 @@ def test_training_fits_a_smooth_map(gpu):
 
 
 @pytest.mark.parametrize("shape,n", [((5, 64, 2, 3, 2), 16), ((20, 96, 1, 40, 1), 144), ((N_IN, WIDTH, HIDDEN, N_OUT, 1), 1008),
-                                     ((3, 16, 1, 1, 2), 128), ((200, 128, 2, 130, 1), 272)])
+                                     ((3, 16, 1, 1, 2), 128), ((200, 128, 2, 130, 1), 272),
+                                     ((N_IN, WIDTH, HIDDEN, N_OUT, MEMBERS), 528), ((N_IN, WIDTH, HIDDEN, N_OUT, MEMBERS), 2064),
+                                     ((4, 48, 8, 3, 8), 2064), ((4, 48, 2, 3, 1), 2176)])
 def test_gradients_of_other_shapes(gpu, shape, n):
     """The training kernels at widths and batches off their tiles (16 to 256
     wide, one to several 128-row tiles with a partial last one, inputs and
-    outputs wider than a slab), against the CPU checker with the bounds of
+    outputs wider than a slab; one, four and sixteen pieces of a batch, a CTA with
+    several, more CTAs than pieces), against the CPU checker with the bounds of
     test_gradients_match_cpu_oracle."""
     import torch
     n_in, width, hidden, n_out, members = shape
     m = gpu.Mlp()
-    m.init(n_in, width, hidden, n_out, members, max_batch=1024, seed=6)
+    m.init(n_in, width, hidden, n_out, members, max_batch=4096, seed=6)
     rng = np.random.default_rng(n)
     scal = [np.asarray(v, np.float32) for v in (rng.normal(size=n_in), rng.uniform(0.5, 2, n_in), rng.normal(size=n_out),
                                                 rng.uniform(0.5, 2, n_out))]
